@@ -88,7 +88,7 @@ def build_oracle(with_reference: bool | None = None) -> None:
     # the reference's sources: EMP_REFERENCE_DIR, else a `reference` directory beside the repository
     ref = os.environ.get("EMP_REFERENCE_DIR") or os.path.join(os.path.dirname(ROOT), "reference")
     if with_reference is None:
-        with_reference = os.path.isdir(ref)
+        with_reference = os.path.isfile(os.path.join(ref, "main.cu"))
     if with_reference and shutil.which("g++"):
         _run(["make", "-s", "-C", os.path.join(ROOT, "oracle"), "ref-cpu", f"REF={ref}"])
         if os.path.exists(NVCC):
