@@ -5,8 +5,9 @@
 //                             when a read is dropped) (k_map.cu)
 //   reduce  overlap.cu:206-293 -> duplicate removal by key buckets
 //                             (k_dedup.cu; the sort when 2n > M) +
-//                             init_list, then every round in the bucket
-//                             kernel (k_bucket.cu), or host-synchronised
+//                             init_list, then every round in the sweep
+//                             kernel (k_sweep.cu) or, for long lists, the
+//                             bucket kernel (k_bucket.cu); host-synchronised
 //                             rounds while a round's tables reach M/2
 //                             (k_round.cu, k_sort.cu, k_chunked.cu)
 // All tables stay in HBM; the host traffic is the FASTQ in and output.bin
@@ -154,7 +155,7 @@ struct emp_ctx {
     HostSlab slab;
     // emp_batch_run: the BktJob array and control block of one launch, their
     // host copies, and the launch's events
-    DevBuf batch_jobs, batch_ctl;
+    DevBuf batch_jobs, batch_ctl, batch_swp;
     PinnedBuf h_batch;
     cudaEvent_t batch_ev[2] = {};
     // the map phase of a batch of jobs: jobs on kMapStreams streams, so that
@@ -172,6 +173,7 @@ struct JobPrep {
     uint64_t n = 0, n_rec = 0, U = 0, M = 0, wpc = 0, ecap = 0, launches0 = 0;
     int L = 0, wpr = 0, rounds = 0;
     bool done = false;  // nothing more to run (empty input, no reads)
+    bool no_sweep = false;  // the rounds run in the bucket kernel (kCrowded)
 };
 
 struct emp_job {
@@ -196,6 +198,7 @@ struct emp_job {
     DevBuf dout;                 // output.bin records written on the device (after those in `out`)
     uint64_t dout_bytes = 0;
     PinnedBuf h_out;
+    DevBuf swp, swp_out;         // the sweep kernel's work memory and output bins (k_sweep.cu)
     DevBuf bk_lst0, bk_lst1, bk_cnt, bk_spill, bk_spans, bk_sfrom, bk_sto, bk_scratch, bk_job, bk_meta;  // bucket kernel
     PinnedBuf h_coop;
     cudaEvent_t sort_ev[2 * kSortPasses] = {};
@@ -234,6 +237,8 @@ enum MiscSlot { kMiscErr = 0, kMiscTotal = 1, kMiscLen = 2, kMiscN = 3, kMiscU =
 
 // internal: the pipeline's edge buffer was too small (never returned by the ABI)
 constexpr emp_status kNeedEdgeRoom = -1000;
+// internal: the sweep kernel met a group of too many equal keys (the bucket kernel takes the job)
+constexpr emp_status kCrowded = -1001;
 
 emp_status cuda_status(cudaError_t e) { return e == cudaSuccess ? EMP_OK : (e == cudaErrorMemoryAllocation ? EMP_E_NOMEM : EMP_E_CUDA); }
 
@@ -717,7 +722,8 @@ emp_status bucket_fetch(emp_job *j, const RoundEnv &env, cudaStream_t s) {
 // After the launch and a synchronisation: the job's counts and output size
 // from its launch description (copied back) and records.  kNeedEdgeRoom with
 // *needed set when its edge buffer was too small.
-emp_status bucket_collect(emp_job *j, int r0, uint64_t n_in, const BktJob &hj, uint64_t *needed) {
+template <class Launched>  // BktJob or SweepJob
+emp_status bucket_collect(emp_job *j, int r0, uint64_t n_in, const Launched &hj, uint64_t *needed) {
     emp_stats &st = j->st;
     if (hj.overflow) {
         *needed = hj.e_total;
@@ -796,6 +802,110 @@ emp_status run_rounds_bucket(emp_job *j, cudaStream_t s, const RoundEnv &env, in
     return bucket_collect(j, r0, n_in, *hj, needed);
 }
 
+// Profiling aid: the phases of a sweep launch (k_sweep.cu's mark), one line
+// each with the time since the one before (us).
+constexpr uint32_t kSweepTraceCap = 4096;
+void write_sweep_trace(emp_job *j, const char *path, cudaStream_t s) {
+    std::vector<uint64_t> t((size_t)kSweepTraceCap * kCoopTracePhases);
+    if (cudaMemcpyAsync(t.data(), j->coop_trace.p, t.size() * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return;
+    FILE *f = std::fopen(path, "w");
+    if (!f) return;
+    std::fprintf(f, "step,phase,us,r,R,prefixes,suffixes,ls,lp\n");
+    for (uint32_t i = 0; i < kSweepTraceCap; ++i) {
+        const uint64_t *p = &t[(size_t)i * kCoopTracePhases];
+        if (!p[3]) break;
+        std::fprintf(f, "%u,%u,%.2f,%u,%u,%u,%u,%u,%u\n", (unsigned)(p[0] >> 8), (unsigned)(p[0] & 255),
+                     i ? (p[3] - t[(size_t)(i - 1) * kCoopTracePhases + 3]) / 1e3 : 0.0, (unsigned)p[1], (unsigned)(p[1] >> 32),
+                     (unsigned)p[2], (unsigned)(p[2] >> 32), (unsigned)p[4], (unsigned)(p[4] >> 32));
+    }
+    std::fclose(f);
+}
+
+// Whether rounds over a list of n entries run in the sweep kernel
+// (k_sweep.cu): not when the caller shapes the bucket kernel's buckets or
+// regions.
+bool sweep_rounds_usable(const emp_job *j, uint64_t n) {
+    const emp_tuning &t = j->ctx->tune;
+    return !j->prep.no_sweep && t.round_driver == 0 && (!t.bucket_mean || t.bucket_mean == kBktMean) &&
+           (!t.region_cap || t.region_cap == kBktRegionCap) && n <= kSweepMaxEntries && sweep_grid_size() > 0;
+}
+
+// Buffers and launch description (host copy *hj) of rounds r0 .. of one job
+// in the sweep kernel: the list lk[cur] holds ns suffixes, then np prefixes.
+// The launch overwrites the list.
+emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t ns, uint64_t np,
+                         uint64_t ecap, uint32_t seg, SweepJob *hj) {
+    std::memset(hj, 0, sizeof(SweepJob));
+    hj->key[0] = j->lk0.as<uint64_t>();
+    hj->key[1] = j->lk1.as<uint64_t>();
+    hj->val = cur ? j->lv1.as<uint32_t>() : j->lv0.as<uint32_t>();
+    hj->cur0 = (uint8_t)cur;
+    hj->used_s = j->used_s.as<uint8_t>();
+    hj->used_p = j->used_p.as<uint8_t>();
+    hj->n_s = (uint32_t)ns;
+    hj->n_p = (uint32_t)np;
+    hj->seg = seg;
+    hj->L = env.L;
+    hj->rounds = env.rounds;
+    hj->r0 = r0;
+    hj->wpr = env.wpr;
+    hj->seq2 = env.seq2;
+    hj->tables = env.tables;
+    hj->ecap = ecap;
+    size_t zeroed = 0;
+    EMP_TRY(ensure(j, j->swp, sweep_layout(nullptr, hj, &zeroed)));
+    sweep_layout(j->swp.as<uint8_t>(), hj, &zeroed);
+    EMP_CUDA(cudaMemsetAsync(j->swp.p, 0, zeroed, s));
+    EMP_TRY(ensure(j, j->dout, (size_t)env.rounds * 12 + ecap * 8));
+    EMP_TRY(ensure(j, j->records, (size_t)env.rounds * sizeof(RoundRecord)));
+    if (!j->h_records.ensure((size_t)env.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
+    hj->out = j->dout.as<uint8_t>();
+    hj->records = j->records.as<RoundRecord>();
+    return EMP_OK;
+}
+
+// Rounds r0 .. of one job alone in the sweep kernel.
+emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t ns, uint64_t np,
+                            uint64_t ecap, uint64_t *needed) {
+    EMP_TRY(ensure(j, j->bk_job, sizeof(SweepJob)));
+    EMP_TRY(ensure(j, j->coop_ctl, sizeof(CoopCtl)));
+    if (!j->h_coop.ensure(sizeof(SweepJob) + sizeof(CoopCtl))) return EMP_E_NOMEM;
+    SweepJob *hj = j->h_coop.as<SweepJob>();
+    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + 1);
+    EMP_TRY(sweep_prepare(j, s, env, r0, cur, ns, np, ecap, sweep_segment_size(std::max(ns, np)), hj));
+    SweepOut go{};
+    size_t zeroed = 0;
+    const uint32_t bins = sweep_bins_max(ns + np, env.rounds - r0);
+    EMP_TRY(ensure(j, j->swp_out, sweep_out_layout(nullptr, bins, &go, &zeroed)));
+    sweep_out_layout(j->swp_out.as<uint8_t>(), bins, &go, &zeroed);
+    EMP_CUDA(cudaMemsetAsync(j->swp_out.p, 0, zeroed, s));
+    coop_ctl_init(j->ctx, hc, 1);
+    const bool trace = !j->ctx->trace_path.empty();
+    if (trace) {
+        EMP_TRY(ensure(j, j->coop_trace, (size_t)kSweepTraceCap * kCoopTracePhases * 8));
+        EMP_CUDA(cudaMemsetAsync(j->coop_trace.p, 0, j->coop_trace.bytes, s));
+        hc->trace = j->coop_trace.as<uint64_t>();
+        hc->trace_cap = kSweepTraceCap;
+    }
+    EMP_CUDA(cudaMemcpyAsync(j->bk_job.p, hj, sizeof(SweepJob), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaMemcpyAsync(j->coop_ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    cudaEvent_t e0 = j->upd_ev[0], e1 = j->upd_ev[1];
+    EMP_CUDA(cudaEventRecord(e0, s));
+    EMP_CUDA(launch_sweep(j->bk_job.as<SweepJob>(), j->coop_ctl.as<CoopCtl>(), go, s));
+    EMP_CUDA(cudaEventRecord(e1, s));
+    EMP_CUDA(cudaMemcpyAsync(hj, j->bk_job.p, sizeof(SweepJob), cudaMemcpyDeviceToHost, s));
+    EMP_CUDA(cudaMemcpyAsync(hc, j->coop_ctl.p, sizeof(CoopCtl), cudaMemcpyDeviceToHost, s));
+    EMP_TRY(bucket_fetch(j, env, s));
+    EMP_TRY(sync_and_check(j, s));
+    if (hc->err & kErrSpin) return EMP_E_TIMEOUT;
+    j->st.ms_round_kernel += ms_between(e0, e1);
+    if (trace) write_sweep_trace(j, j->ctx->trace_path.c_str(), s);
+    if (hj->crowded) return kCrowded;
+    return bucket_collect(j, r0, ns + np, *hj, needed);
+}
+
 // Round counters, output and used marks of a job, before its rounds.
 emp_status rounds_prelude(emp_job *j, cudaStream_t s) {
     emp_stats &st = j->st;
@@ -835,6 +945,7 @@ emp_status run_rounds(emp_job *j, cudaStream_t s, const RoundEnv &env, uint64_t 
         ++r;
     }
     if (r >= env.rounds) return EMP_OK;
+    if (sweep_rounds_usable(j, n_in)) return run_rounds_sweep(j, s, env, r, cur, S, P, ecap, needed);
     return run_rounds_bucket(j, s, env, r, cur, n_in, ecap, needed);
 }
 
@@ -1085,6 +1196,18 @@ RoundEnv job_env(emp_job *j) {
     return RoundEnv{q.L, q.rounds, q.M, q.wpc, j->ctx->tables.as<HashTables>(), j->seq2.as<uint32_t>(), q.wpr};
 }
 
+// The round drivers overwrite the list: build the initial one again from the
+// fingerprints and survivor marks, which the rounds leave intact.
+emp_status rebuild_list(emp_job *j, cudaStream_t s) {
+    const JobPrep &q = j->prep;
+    EMP_TRY(reset_chain(j, upd_tiles(2 * q.n), s));
+    launch_init_list(j->keys0.as<uint64_t>(), j->alive.as<uint8_t>(), q.n, j->lk0.as<uint64_t>(),
+                     j->lv0.as<uint32_t>(), j->status.as<uint64_t>(), chain_ctr(j),
+                     j->misc.as<uint64_t>() + kMiscU, err_word(j), s);
+    launch_dup_prefix_half(j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(), q.U, s);
+    return EMP_OK;
+}
+
 // All rounds of one job, restarting with a larger edge buffer when needed.
 emp_status job_rounds(emp_job *j, cudaStream_t s) {
     JobPrep &q = j->prep;
@@ -1094,16 +1217,14 @@ emp_status job_rounds(emp_job *j, cudaStream_t s) {
         uint64_t needed = 0;
         emp_status rc = run_rounds(j, s, env, q.U, q.ecap, &needed);
         if (rc == EMP_OK) return EMP_OK;
-        if (rc != kNeedEdgeRoom || attempt >= 2) return rc == kNeedEdgeRoom ? EMP_E_NOMEM : rc;
-        q.ecap = needed + needed / 4 + 1024;
-        j->ecap_hint = q.ecap;
-        // the round drivers overwrite the list buffers: build the initial list again
-        // from the fingerprints and survivor marks, which the rounds leave intact
-        EMP_TRY(reset_chain(j, upd_tiles(2 * q.n), s));
-        launch_init_list(j->keys0.as<uint64_t>(), j->alive.as<uint8_t>(), q.n, j->lk0.as<uint64_t>(),
-                         j->lv0.as<uint32_t>(), j->status.as<uint64_t>(), chain_ctr(j),
-                         j->misc.as<uint64_t>() + kMiscU, err_word(j), s);
-        launch_dup_prefix_half(j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(), q.U, s);
+        if (rc == kCrowded) {
+            q.no_sweep = true;
+        } else {
+            if (rc != kNeedEdgeRoom || attempt >= 3) return rc == kNeedEdgeRoom ? EMP_E_NOMEM : rc;
+            q.ecap = needed + needed / 4 + 1024;
+            j->ecap_hint = q.ecap;
+        }
+        EMP_TRY(rebuild_list(j, s));
     }
 }
 
@@ -1196,6 +1317,64 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
             q.ecap = needed + needed / 4 + 1024;
             j->ecap_hint = q.ecap;
             r = job_rounds(j, s);
+        }
+        rc[idx[k]] = r;
+    }
+    return EMP_OK;
+}
+
+// The same in one launch of the sweep kernel.
+emp_status batch_rounds_sweep(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &idx, std::vector<emp_status> &rc,
+                              cudaStream_t s) {
+    const size_t nb = idx.size();
+    EMP_TRY(ctx_ensure(ctx, ctx->batch_jobs, nb * sizeof(SweepJob), s));
+    EMP_TRY(ctx_ensure(ctx, ctx->batch_ctl, sizeof(CoopCtl), s));
+    if (!ctx->h_batch.ensure(nb * sizeof(SweepJob) + sizeof(CoopCtl))) return EMP_E_NOMEM;
+    if (!ctx->batch_ev[0]) {
+        for (auto &e : ctx->batch_ev) EMP_CUDA(cudaEventCreate(&e));
+    }
+    SweepJob *hj = ctx->h_batch.as<SweepJob>();
+    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + nb);
+    uint64_t side = 0, bins = 0;
+    for (int i : idx) {
+        side += jobs[i]->prep.U;
+        bins += sweep_bins_max(2 * jobs[i]->prep.U, jobs[i]->prep.rounds);
+    }
+    const uint32_t seg = sweep_segment_size(side);
+    for (size_t k = 0; k < nb; ++k) {
+        emp_job *j = jobs[idx[k]];
+        const JobPrep &q = j->prep;
+        EMP_TRY(rounds_prelude(j, s));
+        EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, seg, &hj[k]));
+    }
+    SweepOut go{};
+    size_t zeroed = 0;
+    EMP_TRY(ctx_ensure(ctx, ctx->batch_swp, sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed), s));
+    sweep_out_layout(ctx->batch_swp.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
+    EMP_CUDA(cudaMemsetAsync(ctx->batch_swp.p, 0, zeroed, s));
+    coop_ctl_init(ctx, hc, (uint32_t)nb);
+    EMP_CUDA(cudaMemcpyAsync(ctx->batch_jobs.p, hj, nb * sizeof(SweepJob), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaMemcpyAsync(ctx->batch_ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaEventRecord(ctx->batch_ev[0], s));
+    EMP_CUDA(launch_sweep(ctx->batch_jobs.as<SweepJob>(), ctx->batch_ctl.as<CoopCtl>(), go, s));
+    EMP_CUDA(cudaEventRecord(ctx->batch_ev[1], s));
+    EMP_CUDA(cudaMemcpyAsync(hj, ctx->batch_jobs.p, nb * sizeof(SweepJob), cudaMemcpyDeviceToHost, s));
+    EMP_CUDA(cudaMemcpyAsync(hc, ctx->batch_ctl.p, sizeof(CoopCtl), cudaMemcpyDeviceToHost, s));
+    for (size_t k = 0; k < nb; ++k) EMP_TRY(bucket_fetch(jobs[idx[k]], job_env(jobs[idx[k]]), s));
+    EMP_CUDA(cudaStreamSynchronize(s));
+    if (hc->err & kErrSpin) return EMP_E_TIMEOUT;
+    const float ms = ms_between(ctx->batch_ev[0], ctx->batch_ev[1]);
+    for (size_t k = 0; k < nb; ++k) {
+        emp_job *j = jobs[idx[k]];
+        JobPrep &q = j->prep;
+        j->st.ms_round_kernel += ms;  // the whole batch's launch
+        uint64_t needed = 0;
+        emp_status r = hj[k].crowded ? kCrowded : bucket_collect(j, 0, 2 * q.U, hj[k], &needed);
+        if (r == kNeedEdgeRoom || r == kCrowded) {  // alone again, with room for every edge or in the other kernel
+            if (r == kCrowded) q.no_sweep = true;
+            else j->ecap_hint = q.ecap = needed + needed / 4 + 1024;
+            r = rebuild_list(j, s);
+            if (r == EMP_OK) r = job_rounds(j, s);
         }
         rc[idx[k]] = r;
     }
@@ -1308,16 +1487,19 @@ emp_status close_jobs(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaSt
 emp_status run_batch(emp_ctx *ctx, emp_job **jobs, int n, cudaStream_t s) {
     std::vector<emp_status> rc((size_t)n, EMP_OK);
     EMP_TRY(map_batch(jobs, n, rc, s));
-    std::vector<int> batch, alone;
+    std::vector<int> sweep, bucket, alone;
     for (int i = 0; i < n; ++i) {
         if (rc[i] != EMP_OK || jobs[i]->prep.done) continue;
-        if (batch_eligible(jobs[i])) batch.push_back(i);
-        else alone.push_back(i);
+        if (!batch_eligible(jobs[i])) alone.push_back(i);
+        else if (sweep_rounds_usable(jobs[i], 2 * jobs[i]->prep.U)) sweep.push_back(i);
+        else bucket.push_back(i);
     }
-    if (!batch.empty()) {
-        const emp_status e = batch_rounds(ctx, jobs, batch, rc, s);
+    for (const std::vector<int> *batch : {&sweep, &bucket}) {
+        if (batch->empty()) continue;
+        const emp_status e = batch == &sweep ? batch_rounds_sweep(ctx, jobs, *batch, rc, s)
+                                             : batch_rounds(ctx, jobs, *batch, rc, s);
         if (e != EMP_OK)
-            for (int i : batch)
+            for (int i : *batch)
                 if (rc[i] == EMP_OK) rc[i] = e;
     }
     for (int i : alone) rc[i] = job_rounds(jobs[i], s);
@@ -1680,8 +1862,9 @@ emp_status emp_ctx_destroy(emp_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     for (auto &e : ctx->batch_ev)
         if (e) cudaEventDestroy(e);
-    ctx->in_use -= ctx->batch_jobs.bytes + ctx->batch_ctl.bytes;
+    ctx->in_use -= ctx->batch_jobs.bytes + ctx->batch_ctl.bytes + ctx->batch_swp.bytes;
     ctx->batch_jobs.release();
+    ctx->batch_swp.release();
     ctx->batch_ctl.release();
     for (int k = 0; k < kMapStreams; ++k) {
         if (ctx->map_streams[k]) {
@@ -1722,7 +1905,7 @@ emp_status emp_job_create(emp_ctx *ctx, const emp_params *p, emp_job **out) {
     }
     static_assert(kSlotHist >= kMiscSlots * sizeof(uint64_t) && kSlotCoop - kSlotHist >= kSortPasses * kSortRadix * 4,
                   "slab layout");
-    static_assert(kSlotCtl - kSlotCoop >= sizeof(BktJob) + sizeof(CoopCtl),
+    static_assert(kSlotCtl - kSlotCoop >= std::max(sizeof(BktJob), sizeof(SweepJob)) + sizeof(CoopCtl),
                   "slab layout");
     static_assert(kSlotBytes - kSlotRecords >= EMP_MAX_ROUNDS * sizeof(RoundRecord),
                   "slab layout");
@@ -1796,7 +1979,7 @@ static void release_buffers(emp_job *job) {
                       &job->coop_probe, &job->bk_lst0, &job->bk_lst1, &job->bk_cnt, &job->bk_spill, &job->bk_spans,
                       &job->bk_sfrom, &job->bk_sto, &job->bk_scratch, &job->bk_job, &job->dout,
                       &job->bk_meta, &job->xk0, &job->xv0, &job->xk1, &job->xv1, &job->ring_k, &job->ring_v,
-                      &job->cparts};
+                      &job->cparts, &job->swp, &job->swp_out};
     for (DevBuf *b : bufs) free_buf(job, *b);
     job->sorts_since_clear = 0;
 }

@@ -311,6 +311,85 @@ bool bucket_prologue_apart(const BktJob &host_job);
 cudaError_t measure_l2_read(uint64_t bytes, double *gbs);
 cudaError_t launch_bucket_prologue(BktJob *job, cudaStream_t s);
 
+// ---- many rounds per step (k_sweep.cu) -------------------------------------
+constexpr int kSweepThreads = 1024;  // threads of a sweep CTA (one CTA per SM)
+constexpr int kSweepMaxR = 32;       // rounds of a step at most
+// Longer lists run in the bucket kernel: beyond this one round of every entry
+// no longer fits filters and groups within L2 (112.7M entries: 24.4 ms there).
+constexpr uint64_t kSweepMaxEntries = 16ull << 20;
+constexpr int kSweepFirstR = 4;      // rounds of a job's first step
+constexpr int kSweepIters = 40;      // resolving iterations of a step at most (kSweepMaxR + 1 suffice)
+struct SweepCtr {  // one step of one job (zero at its start)
+    uint32_t ls, lp;  // live suffixes / prefixes (a launch that starts after host-driven rounds)
+    uint32_t pc;      // prefix candidates
+    uint32_t pairs;   // pairs of a suffix and a prefix
+    uint32_t ovf;     // they did not fit: the step runs again with fewer rounds
+    uint32_t fired_s, fired_p;  // entries matched
+};
+struct SweepGroup {  // all ones = empty
+    uint64_t key;    // key and round of the step
+    uint32_t head;   // its last prefix candidate
+    uint32_t pad;
+};
+struct SweepJob {
+    // the list at launch, [n_s suffixes | n_p prefixes]: key[cur0] holds the
+    // keys of round r0 - 1, val = rid | table << 31; both are overwritten
+    uint64_t *key[2];
+    uint32_t *val;
+    const uint8_t *used_s, *used_p;  // marks of rounds run before the launch (read when r0 > 0)
+    uint32_t n_s, n_p;
+    uint32_t seg;            // entries of a segment (a warp's unit of work), a multiple of 32
+    int32_t L, rounds, r0, wpr;
+    const uint32_t *seq2;    // read-major 2-bit bases, wpr words per read
+    const HashTables *tables;
+    uint64_t ecap;           // edges that fit `out`
+    uint8_t *out;            // output.bin records (12 * rounds + 8 * ecap bytes)
+    RoundRecord *records;    // [rounds]
+    // work memory (sweep_layout)
+    uint32_t w1_max;         // log2 words of filter 1
+    uint32_t gm_max;         // log2 group slots
+    uint32_t segs_s, segs_p;
+    uint32_t *filter1, *filter2;  // zero between steps
+    SweepCtr *ctr;           // [3]: step b uses ctr[b % 3]
+    uint32_t *fs, *fp;       // [round]: suffixes / prefixes matched
+    SweepGroup *groups;      // those of the step, empty between steps
+    uint32_t *T[2];          // [iteration % 2][entry]: round of the step that uses it
+    uint32_t *segcnt;        // live entries of each segment, suffixes then prefixes
+    uint4 *pcand;            // prefix candidates: value, entry, the group's next one, group
+    uint4 *pair;             // pairs: key and round, suffix, prefix (values)
+    uint2 *pair_e;           // their entries; bit 31 of the second: the pair matches
+    uint4 *rec, *rec2;       // matched entries: key, value, round
+    uint32_t *rank;          // their ranks within their output bins
+    uint32_t *binbase;       // [rounds - r0 + 1]: first output bin of each round
+    uint64_t *roff;          // [rounds]: offset of each round's record in `out`
+    // set by the launch
+    uint32_t nrec;           // matched entries (zero at launch)
+    uint32_t nbins;
+    uint32_t s0, p0;         // live suffixes / prefixes of round r0 (when r0 > 0)
+    uint32_t round;          // rounds run
+    uint32_t overflow;       // the edge buffer is too small (zero at launch)
+    uint32_t crowded;        // a group of too many entries: not a job for this kernel (zero at launch)
+    uint64_t e_total;        // edges
+    uint8_t cur0;
+};
+struct SweepOut {  // output bins of a launch's jobs (sweep_out_layout)
+    uint32_t *chg;    // [3][kSweepIters]: whether an iteration changed something
+    uint32_t *nbig;
+    uint32_t *cnt;    // records of each bin
+    uint64_t *off;    // their exclusive scan
+    uint64_t *ecnt;   // edges of each bin
+    uint64_t *eoff;   // their exclusive scan
+    uint32_t *round;  // its round
+    uint32_t *big;    // bins sorted by a whole CTA
+    uint64_t *part;
+};
+int sweep_grid_size();  // 0: no cooperative launch on this device
+uint32_t sweep_segment_size(uint64_t entries_per_side);
+uint32_t sweep_bins_max(uint64_t n_in, int rounds);
+size_t sweep_layout(uint8_t *base, SweepJob *job, size_t *zeroed);
+size_t sweep_out_layout(uint8_t *base, uint32_t bins, SweepOut *go, size_t *zeroed);
+cudaError_t launch_sweep(SweepJob *jobs, CoopCtl *ctl, const SweepOut &go, cudaStream_t s);
+
 void launch_join_count(const uint64_t *skeys, const uint32_t *svals, uint64_t n, uint32_t *cnt, cudaStream_t s);
 void launch_join_write(const uint64_t *skeys, const uint32_t *svals, uint64_t n, const uint32_t *cnt,
                        const uint64_t *offs, uint32_t *from, uint32_t *to, uint8_t *used_s, uint8_t *used_p,
