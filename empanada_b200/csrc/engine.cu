@@ -153,6 +153,7 @@ struct emp_ctx {
     uint64_t sort_cap = 0;
     uint64_t sort_calls = 0;
     HostSlab slab;
+    std::vector<emp_graph *> graphs;  // those whose arrays lie in the pool
     // emp_batch_run: the BktJob array and control block of one launch, their
     // host copies, and the launch's events
     DevBuf batch_jobs, batch_ctl, batch_swp;
@@ -1856,10 +1857,13 @@ emp_status emp_ctx_create(int device, uint64_t hbm_budget_bytes, emp_ctx **out) 
     return EMP_OK;
 }
 
+static void detach_graphs(emp_ctx *ctx);
+
 emp_status emp_ctx_destroy(emp_ctx *ctx) {
     if (!ctx) return EMP_E_INVAL;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    detach_graphs(ctx);
     for (auto &e : ctx->batch_ev)
         if (e) cudaEventDestroy(e);
     ctx->in_use -= ctx->batch_jobs.bytes + ctx->batch_ctl.bytes + ctx->batch_swp.bytes;
@@ -2471,8 +2475,16 @@ emp_status emp_run_file(const char *input_path, const char *output_path, const e
 }  // extern "C"
 
 // ---- unitigs of an output.bin ------------------------------------------------
+// A graph keeps its output.bin and its unitigs on the device; what is asked
+// for on the host is copied from there.  When its context goes first, the
+// context copies them to the host and the graph lives on without it.
 struct emp_graph {
-    emp_ctx *ctx = nullptr;
+    emp_ctx *ctx = nullptr;           // null: on the host
+    void *dev = nullptr;              // output.bin, order, starts (from the context's pool)
+    const uint8_t *d_bin = nullptr;
+    const uint32_t *d_order = nullptr;
+    const uint64_t *d_starts = nullptr;
+    uint64_t bytes = 0, unitigs = 0;
     std::vector<uint8_t> bin;         // the output.bin bytes (the L lines come from them)
     std::vector<uint64_t> rec_off;    // byte offset of every record
     uint64_t nodes = 0, edges = 0;
@@ -2480,6 +2492,47 @@ struct emp_graph {
     std::vector<uint64_t> starts;     // first position of every unitig, then `nodes`
     emp_graph_stats st{};
 };
+
+namespace {
+
+// the graph's arrays into its host vectors
+emp_status graph_to_host(emp_graph *g) {
+    if (g->order.size() == g->nodes) return EMP_OK;
+    if (!g->ctx) return EMP_E_NOMEM;  // the context went while there was no room for them
+    cudaSetDevice(g->ctx->device);
+    try {
+        g->bin.resize(g->bytes);
+        g->starts.resize(g->unitigs + 1);
+        g->order.resize(g->nodes);
+    } catch (...) {
+        g->order.clear();
+        return EMP_E_NOMEM;
+    }
+    if ((g->bytes && cudaMemcpy(g->bin.data(), g->d_bin, g->bytes, cudaMemcpyDeviceToHost) != cudaSuccess) ||
+        cudaMemcpy(g->starts.data(), g->d_starts, (g->unitigs + 1) * 8, cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(g->order.data(), g->d_order, g->nodes * 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
+        cudaGetLastError();
+        g->order.clear();
+        return EMP_E_CUDA;
+    }
+    return EMP_OK;
+}
+
+// the graph leaves its context
+void graph_detach(emp_graph *g) {
+    emp_ctx *c = g->ctx;
+    if (!c) return;
+    auto &v = c->graphs;
+    v.erase(std::remove(v.begin(), v.end(), g), v.end());
+    if (g->dev) {
+        cudaSetDevice(c->device);
+        cudaFreeAsync(g->dev, c->stream);
+    }
+    g->dev = nullptr;
+    g->ctx = nullptr;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -2504,91 +2557,111 @@ emp_status emp_graph_build(emp_ctx *ctx, const void *output_bin, uint64_t bytes,
         o += 12 + 8 * n;
     }
     g->edges = e0.back();
-    g->bin.assign(b, b + bytes);
+    g->bytes = bytes;
     cudaSetDevice(ctx->device);
     const uint32_t V = (uint32_t)g->nodes;
     const uint64_t E = g->edges, nrec = g->rec_off.size();
-    // one device allocation for everything, in the context's pool
-    const uint64_t scan_t = scan_tiles(V);
+    // two device allocations in the context's pool: what the graph keeps, and
+    // the build's work memory
     size_t off = 0;
     auto take = [&](size_t bytes_) { const size_t o = off; off = (off + bytes_ + 255) / 256 * 256; return o; };
-    const size_t o_bin = take(bytes + 16), o_roff = take(nrec * 8 + 8), o_e0 = take((nrec + 1) * 8);
-    const size_t o_from = take(E * 4 + 4), o_to = take(E * 4 + 4);
-    size_t o_node[15];
-    for (auto &x : o_node) x = take((size_t)V * 4);
-    const size_t o_start = take((size_t)V * 8), o_status = take(scan_t * 8 + 64), o_small = take(64);
+    const size_t o_bin = take(bytes + 16), o_order = take((size_t)V * 4), o_starts = take(((size_t)V + 1) * 8);
+    const size_t keep = off;
+    off = 0;
+    const uint64_t scan_t = scan_tiles(V);
+    const size_t o_roff = take(nrec * 8 + 8), o_e0 = take((nrec + 1) * 8);
+    size_t o_word[8], o_long[3];
+    for (auto &x : o_word) x = take((size_t)V * 4);
+    for (auto &x : o_long) x = take((size_t)V * 8);
+    const size_t o_tail = take(V), o_status = take(2 * scan_t * 8), o_small = take(512);
     cudaStream_t s = ctx->stream;
-    void *dev = nullptr;
-    if (cudaMallocFromPoolAsync(&dev, off, ctx->pool, s) != cudaSuccess) {
+    void *work = nullptr;
+    if (cudaMallocFromPoolAsync(&g->dev, keep, ctx->pool, s) != cudaSuccess) {
         cudaGetLastError();
         delete g;
         return EMP_E_NOMEM;
     }
-    uint8_t *d = static_cast<uint8_t *>(dev);
+    if (cudaMallocFromPoolAsync(&work, off, ctx->pool, s) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFreeAsync(g->dev, s);
+        delete g;
+        return EMP_E_NOMEM;
+    }
+    uint8_t *k = static_cast<uint8_t *>(g->dev), *d = static_cast<uint8_t *>(work);
     GraphBufs gb{};
-    gb.from = reinterpret_cast<uint32_t *>(d + o_from);
-    gb.to = reinterpret_cast<uint32_t *>(d + o_to);
-    uint32_t **node_arrays[15] = {&gb.dout, &gb.din, &gb.succ, &gb.pred, &gb.hop[0], &gb.hop[1], &gb.dist[0],
-                                  &gb.dist[1], &gb.mn[0], &gb.mn[1], &gb.nx[0], &gb.nx[1], &gb.size, &gb.order,
-                                  nullptr};
-    for (int k = 0; k < 14; ++k) *node_arrays[k] = reinterpret_cast<uint32_t *>(d + o_node[k]);
-    gb.start = reinterpret_cast<uint64_t *>(d + o_start);
+    uint32_t **words[8] = {&gb.succ, &gb.pred, &gb.size, &gb.is_head, &gb.mn[0], &gb.mn[1], &gb.nx[0], &gb.nx[1]};
+    for (int q = 0; q < 8; ++q) *words[q] = reinterpret_cast<uint32_t *>(d + o_word[q]);
+    uint64_t **longs[3] = {&gb.state, &gb.start, &gb.index};
+    for (int q = 0; q < 3; ++q) *longs[q] = reinterpret_cast<uint64_t *>(d + o_long[q]);
+    gb.tail = d + o_tail;
     gb.status = reinterpret_cast<uint64_t *>(d + o_status);
-    uint64_t *small = reinterpret_cast<uint64_t *>(d + o_small);  // tile counter, total, error, cycles
-    gb.tile_ctr = reinterpret_cast<uint32_t *>(small);
-    gb.total = small + 1;
-    gb.err = reinterpret_cast<uint32_t *>(small + 2);
-    gb.cycles = reinterpret_cast<uint32_t *>(small + 3);
+    gb.order = reinterpret_cast<uint32_t *>(k + o_order);
+    gb.starts = reinterpret_cast<uint64_t *>(k + o_starts);
+    uint64_t *small = reinterpret_cast<uint64_t *>(d + o_small);  // unitigs, nodes, then u32 words
+    uint32_t *sw = reinterpret_cast<uint32_t *>(small + 2);
+    gb.total = small;
+    gb.err = sw;
+    gb.cycles = sw + 1;
+    gb.undone = sw + 2;
+    gb.longer = sw + 3;
+    gb.tile_ctr = sw + 4;
+    gb.more = sw + 6;
+    static_assert(16 + (6 + kGraphJumps + 1) * 4 <= 512, "the small words fit");
+    g->d_bin = k + o_bin;
+    g->d_order = gb.order;
+    g->d_starts = gb.starts;
     emp_status rc = EMP_OK;
     cudaEvent_t ev[2] = {nullptr, nullptr};
-    PinnedBuf hs;
-    if (!hs.ensure(64)) rc = EMP_E_NOMEM;
-    if (rc == EMP_OK && (cudaEventCreate(&ev[0]) != cudaSuccess || cudaEventCreate(&ev[1]) != cudaSuccess))
-        rc = EMP_E_CUDA;
+    uint64_t hw[4] = {};  // small[0 .. 3]
+    uint32_t *hsw = reinterpret_cast<uint32_t *>(hw + 2);
+    auto fetch = [&]() {
+        cudaMemcpyAsync(hw, small, sizeof hw, cudaMemcpyDeviceToHost, s);
+        if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = EMP_E_CUDA;
+        else if (hsw[0] & kErrSpin) rc = EMP_E_TIMEOUT;
+        else if (hsw[0] & kErrCapacity) rc = EMP_E_FORMAT;  // an edge beyond the read-ends given
+    };
+    if (cudaEventCreate(&ev[0]) != cudaSuccess || cudaEventCreate(&ev[1]) != cudaSuccess) rc = EMP_E_CUDA;
     if (rc == EMP_OK) {
         cudaEventRecord(ev[0], s);
-        if (bytes) cudaMemcpyAsync(d + o_bin, b, bytes, cudaMemcpyHostToDevice, s);
+        if (bytes) cudaMemcpyAsync(k + o_bin, b, bytes, cudaMemcpyHostToDevice, s);
         if (nrec) cudaMemcpyAsync(d + o_roff, g->rec_off.data(), nrec * 8, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(d + o_e0, e0.data(), (nrec + 1) * 8, cudaMemcpyHostToDevice, s);
-        cudaMemsetAsync(gb.status, 0, scan_t * 8 + 64, s);
-        cudaMemsetAsync(small, 0, 64, s);
-        graph_build(d + o_bin, reinterpret_cast<uint64_t *>(d + o_roff), reinterpret_cast<uint64_t *>(d + o_e0),
+        cudaMemsetAsync(gb.status, 0, 2 * scan_t * 8, s);
+        cudaMemsetAsync(small, 0, 512, s);
+        graph_paths(k + o_bin, reinterpret_cast<uint64_t *>(d + o_roff), reinterpret_cast<uint64_t *>(d + o_e0),
                     (uint32_t)nrec, E, V, gb, s);
-        cudaEventRecord(ev[1], s);
-        g->order.resize(V);
-        std::vector<uint32_t> size(V);
-        cudaMemcpyAsync(g->order.data(), gb.order, (size_t)V * 4, cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(size.data(), gb.size, (size_t)V * 4, cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(hs.p, small, 32, cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = EMP_E_CUDA;
-        const uint64_t *hw = hs.as<uint64_t>();
-        if (rc == EMP_OK && (hw[2] & kErrSpin)) rc = EMP_E_TIMEOUT;
-        if (rc == EMP_OK && (hw[2] & kErrCapacity)) rc = EMP_E_FORMAT;  // an edge beyond the read-ends given
+        fetch();
+        if (rc == EMP_OK && hsw[2]) graph_cycles(V, gb, s);
         if (rc == EMP_OK) {
-            uint64_t pos = 0;
-            for (uint32_t u = 0; u < V; ++u)
-                if (size[u]) {
-                    g->starts.push_back(pos);
-                    pos += size[u];
-                    g->st.long_unitigs += size[u] >= 2;
-                }
-            g->starts.push_back(pos);
+            graph_place(V, gb, s);
+            cudaEventRecord(ev[1], s);
+            fetch();
+        }
+        if (rc == EMP_OK) {
+            g->unitigs = hw[0];
+            const uint64_t end = V;
+            cudaMemcpyAsync(gb.starts + g->unitigs, &end, 8, cudaMemcpyHostToDevice, s);
+            if (cudaStreamSynchronize(s) != cudaSuccess) rc = EMP_E_CUDA;
             g->st.nodes = V;
             g->st.edges = E;
-            g->st.unitigs = g->starts.size() - 1;
-            g->st.cycles = (uint32_t)hw[3];
+            g->st.unitigs = g->unitigs;
+            g->st.long_unitigs = hsw[3];
+            g->st.cycles = hsw[1];
             g->st.ms_build = ms_between(ev[0], ev[1]);
-            if (pos != V) rc = EMP_E_CUDA;
+            if (hw[1] != V) rc = EMP_E_CUDA;
         }
     }
     for (cudaEvent_t e : ev)
         if (e) cudaEventDestroy(e);
-    cudaFreeAsync(dev, s);
+    cudaFreeAsync(work, s);
     if (rc != EMP_OK) {
+        cudaFreeAsync(g->dev, s);
         cudaStreamSynchronize(s);
+        cudaGetLastError();
         delete g;
         return rc;
     }
+    ctx->graphs.push_back(g);
     *out = g;
     return EMP_OK;
 }
@@ -2601,13 +2674,18 @@ emp_status emp_graph_get_stats(emp_graph *g, emp_graph_stats *st) {
 
 emp_status emp_graph_unitigs(emp_graph *g, uint32_t *order, uint64_t order_cap, uint64_t *starts, uint64_t starts_cap) {
     if (!g) return EMP_E_INVAL;
-    if (order) {
-        if (order_cap < g->order.size()) return EMP_E_INVAL;
-        std::memcpy(order, g->order.data(), g->order.size() * 4);
+    if ((order && order_cap < g->nodes) || (starts && starts_cap < g->unitigs + 1)) return EMP_E_INVAL;
+    if (!g->ctx) {
+        EMP_TRY(graph_to_host(g));
+        if (order) std::memcpy(order, g->order.data(), g->nodes * 4);
+        if (starts) std::memcpy(starts, g->starts.data(), (g->unitigs + 1) * 8);
+        return EMP_OK;
     }
-    if (starts) {
-        if (starts_cap < g->starts.size()) return EMP_E_INVAL;
-        std::memcpy(starts, g->starts.data(), g->starts.size() * 8);
+    cudaSetDevice(g->ctx->device);
+    if ((order && cudaMemcpy(order, g->d_order, g->nodes * 4, cudaMemcpyDeviceToHost) != cudaSuccess) ||
+        (starts && cudaMemcpy(starts, g->d_starts, (g->unitigs + 1) * 8, cudaMemcpyDeviceToHost) != cudaSuccess)) {
+        cudaGetLastError();
+        return EMP_E_CUDA;
     }
     return EMP_OK;
 }
@@ -2628,6 +2706,8 @@ char *put_u64(char *p, uint64_t v) {
 
 emp_status emp_graph_write_gfa(emp_graph *g, const char *path, int32_t read_len) {
     if (!g || !path || read_len < 0) return EMP_E_INVAL;
+    const emp_status on_host = graph_to_host(g);
+    if (on_host != EMP_OK) return on_host;
     FILE *f = std::fopen(path, "wb");
     if (!f) return EMP_E_IO;
     std::vector<char> buf(1 << 22);
@@ -2714,8 +2794,18 @@ emp_status emp_graph_write_gfa(emp_graph *g, const char *path, int32_t read_len)
     return ok ? EMP_OK : EMP_E_IO;
 }
 
+// the graphs of a context that goes: their arrays to the host
+static void detach_graphs(emp_ctx *ctx) {
+    while (!ctx->graphs.empty()) {
+        emp_graph *g = ctx->graphs.back();
+        graph_to_host(g);
+        graph_detach(g);
+    }
+}
+
 emp_status emp_graph_destroy(emp_graph *g) {
     if (!g) return EMP_E_INVAL;
+    graph_detach(g);
     delete g;
     return EMP_OK;
 }

@@ -64,24 +64,30 @@ bool launch_dedup_hash(const uint64_t *keys, uint64_t n, uint32_t nb, void *scra
                        cudaStream_t s);
 
 // ---- unitigs of the overlap graph (k_graph.cu) ----------------------------
-// Device arrays of graph_build: per edge from/to (E), per node (nodes = 2n)
-// the degrees, succ/pred, two hop/dist and mn/nx buffers, unitig sizes (at
-// the heads), their starts (u64) and the nodes in unitig order; scan status
-// words (scan_tiles(nodes), zeroed), a tile counter and a total (zeroed),
-// the error word and a cycle counter (zeroed).
+// Device arrays of a graph's build, per node (nodes = 2n): succ/pred, jump
+// states (8-byte words), tail marks, unitig sizes (at the heads), head marks,
+// their scans; mn/nx only where there are cycles; scan status words (2 x
+// scan_tiles(nodes), zeroed); small words (zeroed).  order and starts are
+// the result.
+constexpr int kGraphJumps = 32;  // jumping passes at most (nodes < 2^31)
 struct GraphBufs {
-    uint32_t *from, *to;
-    uint32_t *dout, *din, *succ, *pred, *hop[2], *dist[2], *mn[2], *nx[2], *size, *order;
-    uint64_t *start;
+    uint32_t *succ, *pred, *size, *is_head, *mn[2], *nx[2];
+    uint64_t *state, *start, *index;
+    uint8_t *tail;
     uint64_t *status;
-    uint32_t *tile_ctr;
-    uint64_t *total;
-    uint32_t *err, *cycles;
+    uint32_t *tile_ctr;  // [2]
+    uint32_t *more;      // [kGraphJumps + 1]
+    uint64_t *total;     // [2]: unitigs, nodes
+    uint32_t *err, *cycles, *undone, *longer;
+    uint32_t *order;
+    uint64_t *starts;
 };
-// out: output.bin on the device; rec_off[k] its record k's byte offset,
-// rec_e0[k] the record's first edge (rec_e0[nrec] = E).
-void graph_build(const uint8_t *out, const uint64_t *rec_off, const uint64_t *rec_e0, uint32_t nrec, uint64_t E,
+// out: output.bin on the device (4-byte aligned); rec_off[k] its record k's
+// byte offset, rec_e0[k] the record's first edge (rec_e0[nrec] = E).
+void graph_paths(const uint8_t *out, const uint64_t *rec_off, const uint64_t *rec_e0, uint32_t nrec, uint64_t E,
                  uint32_t nodes, const GraphBufs &b, cudaStream_t s);
+void graph_cycles(uint32_t nodes, const GraphBufs &b, cudaStream_t s);
+void graph_place(uint32_t nodes, const GraphBufs &b, cudaStream_t s);
 
 // ---- radix sort (k_sort.cu) ---------------------------------------------
 constexpr int kSortBits = 8;
