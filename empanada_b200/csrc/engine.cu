@@ -135,6 +135,23 @@ struct HostSlab {
 
 }  // namespace
 
+// One sweep launch's descriptors (device and host), output bins and events.
+struct SweepBatch {
+    DevBuf jobs, ctl, out;
+    PinnedBuf host;
+    cudaEvent_t ev[2] = {};
+    uint64_t bytes() const { return jobs.bytes + ctl.bytes + out.bytes; }
+    void release() {
+        jobs.release();
+        ctl.release();
+        out.release();
+        for (auto &e : ev) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+    }
+};
+
 constexpr int kMapStreams = 32;     // streams of a batch's map phase at most
 constexpr int kMapStreamsDefault = 8;
 
@@ -156,7 +173,8 @@ struct emp_ctx {
     std::vector<emp_graph *> graphs;  // those whose arrays lie in the pool
     // emp_batch_run: the BktJob array and control block of one launch, their
     // host copies, and the launch's events
-    DevBuf batch_jobs, batch_ctl, batch_swp;
+    DevBuf batch_jobs, batch_ctl;
+    SweepBatch batch_swp;
     PinnedBuf h_batch;
     cudaEvent_t batch_ev[2] = {};
     // the map phase of a batch of jobs: jobs on kMapStreams streams, so that
@@ -1324,60 +1342,68 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
     return EMP_OK;
 }
 
-// The same in one launch of the sweep kernel.
-emp_status batch_rounds_sweep(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &idx, std::vector<emp_status> &rc,
-                              cudaStream_t s) {
-    const size_t nb = idx.size();
-    EMP_TRY(ctx_ensure(ctx, ctx->batch_jobs, nb * sizeof(SweepJob), s));
-    EMP_TRY(ctx_ensure(ctx, ctx->batch_ctl, sizeof(CoopCtl), s));
-    if (!ctx->h_batch.ensure(nb * sizeof(SweepJob) + sizeof(CoopCtl))) return EMP_E_NOMEM;
-    if (!ctx->batch_ev[0]) {
-        for (auto &e : ctx->batch_ev) EMP_CUDA(cudaEventCreate(&e));
+// One launch of the sweep kernel over all rounds of several jobs (lists
+// ready): queued by launch, read by collect once the stream has been waited for.
+emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<emp_job *> &jobs, cudaStream_t s) {
+    const size_t nb = jobs.size();
+    EMP_TRY(ctx_ensure(ctx, sb.jobs, nb * sizeof(SweepJob), s));
+    EMP_TRY(ctx_ensure(ctx, sb.ctl, sizeof(CoopCtl), s));
+    if (!sb.host.ensure(nb * sizeof(SweepJob) + sizeof(CoopCtl))) return EMP_E_NOMEM;
+    if (!sb.ev[0]) {
+        for (auto &e : sb.ev) EMP_CUDA(cudaEventCreate(&e));
     }
-    SweepJob *hj = ctx->h_batch.as<SweepJob>();
+    SweepJob *hj = sb.host.as<SweepJob>();
     CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + nb);
     uint64_t side = 0, bins = 0;
-    for (int i : idx) {
-        side += jobs[i]->prep.U;
-        bins += sweep_bins_max(2 * jobs[i]->prep.U, jobs[i]->prep.rounds);
+    for (emp_job *j : jobs) {
+        side += j->prep.U;
+        bins += sweep_bins_max(2 * j->prep.U, j->prep.rounds);
     }
     const uint32_t seg = sweep_segment_size(side);
     for (size_t k = 0; k < nb; ++k) {
-        emp_job *j = jobs[idx[k]];
+        emp_job *j = jobs[k];
         const JobPrep &q = j->prep;
         EMP_TRY(rounds_prelude(j, s));
         EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, seg, &hj[k]));
     }
     SweepOut go{};
     size_t zeroed = 0;
-    EMP_TRY(ctx_ensure(ctx, ctx->batch_swp, sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed), s));
-    sweep_out_layout(ctx->batch_swp.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
-    EMP_CUDA(cudaMemsetAsync(ctx->batch_swp.p, 0, zeroed, s));
+    EMP_TRY(ctx_ensure(ctx, sb.out, sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed), s));
+    sweep_out_layout(sb.out.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
+    EMP_CUDA(cudaMemsetAsync(sb.out.p, 0, zeroed, s));
     coop_ctl_init(ctx, hc, (uint32_t)nb);
-    EMP_CUDA(cudaMemcpyAsync(ctx->batch_jobs.p, hj, nb * sizeof(SweepJob), cudaMemcpyHostToDevice, s));
-    EMP_CUDA(cudaMemcpyAsync(ctx->batch_ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
-    EMP_CUDA(cudaEventRecord(ctx->batch_ev[0], s));
-    EMP_CUDA(launch_sweep(ctx->batch_jobs.as<SweepJob>(), ctx->batch_ctl.as<CoopCtl>(), go, s));
-    EMP_CUDA(cudaEventRecord(ctx->batch_ev[1], s));
-    EMP_CUDA(cudaMemcpyAsync(hj, ctx->batch_jobs.p, nb * sizeof(SweepJob), cudaMemcpyDeviceToHost, s));
-    EMP_CUDA(cudaMemcpyAsync(hc, ctx->batch_ctl.p, sizeof(CoopCtl), cudaMemcpyDeviceToHost, s));
-    for (size_t k = 0; k < nb; ++k) EMP_TRY(bucket_fetch(jobs[idx[k]], job_env(jobs[idx[k]]), s));
-    EMP_CUDA(cudaStreamSynchronize(s));
-    if (hc->err & kErrSpin) return EMP_E_TIMEOUT;
-    const float ms = ms_between(ctx->batch_ev[0], ctx->batch_ev[1]);
+    EMP_CUDA(cudaMemcpyAsync(sb.jobs.p, hj, nb * sizeof(SweepJob), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaMemcpyAsync(sb.ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaEventRecord(sb.ev[0], s));
+    EMP_CUDA(launch_sweep(sb.jobs.as<SweepJob>(), sb.ctl.as<CoopCtl>(), go, s));
+    EMP_CUDA(cudaEventRecord(sb.ev[1], s));
+    EMP_CUDA(cudaMemcpyAsync(hj, sb.jobs.p, nb * sizeof(SweepJob), cudaMemcpyDeviceToHost, s));
+    EMP_CUDA(cudaMemcpyAsync(hc, sb.ctl.p, sizeof(CoopCtl), cudaMemcpyDeviceToHost, s));
+    for (emp_job *j : jobs) EMP_TRY(bucket_fetch(j, job_env(j), s));
+    return EMP_OK;
+}
+
+// Per-job status of the launch in rc; a job whose edges did not fit, or that
+// is not one for the sweep kernel, runs again alone.
+emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &jobs, std::vector<emp_status> &rc,
+                               cudaStream_t s) {
+    const size_t nb = jobs.size();
+    const SweepJob *hj = sb.host.as<SweepJob>();
+    if (reinterpret_cast<const CoopCtl *>(hj + nb)->err & kErrSpin) return EMP_E_TIMEOUT;
+    const float ms = ms_between(sb.ev[0], sb.ev[1]);
     for (size_t k = 0; k < nb; ++k) {
-        emp_job *j = jobs[idx[k]];
+        emp_job *j = jobs[k];
         JobPrep &q = j->prep;
         j->st.ms_round_kernel += ms;  // the whole batch's launch
         uint64_t needed = 0;
         emp_status r = hj[k].crowded ? kCrowded : bucket_collect(j, 0, 2 * q.U, hj[k], &needed);
-        if (r == kNeedEdgeRoom || r == kCrowded) {  // alone again, with room for every edge or in the other kernel
+        if (r == kNeedEdgeRoom || r == kCrowded) {
             if (r == kCrowded) q.no_sweep = true;
             else j->ecap_hint = q.ecap = needed + needed / 4 + 1024;
             r = rebuild_list(j, s);
             if (r == EMP_OK) r = job_rounds(j, s);
         }
-        rc[idx[k]] = r;
+        rc[k] = r;
     }
     return EMP_OK;
 }
@@ -1495,12 +1521,19 @@ emp_status run_batch(emp_ctx *ctx, emp_job **jobs, int n, cudaStream_t s) {
         else if (sweep_rounds_usable(jobs[i], 2 * jobs[i]->prep.U)) sweep.push_back(i);
         else bucket.push_back(i);
     }
-    for (const std::vector<int> *batch : {&sweep, &bucket}) {
-        if (batch->empty()) continue;
-        const emp_status e = batch == &sweep ? batch_rounds_sweep(ctx, jobs, *batch, rc, s)
-                                             : batch_rounds(ctx, jobs, *batch, rc, s);
+    if (!sweep.empty()) {
+        std::vector<emp_job *> js;
+        for (int i : sweep) js.push_back(jobs[i]);
+        std::vector<emp_status> src(js.size(), EMP_OK);
+        emp_status e = sweep_batch_launch(ctx, ctx->batch_swp, js, s);
+        if (e == EMP_OK) e = cuda_status(cudaStreamSynchronize(s));
+        if (e == EMP_OK) e = sweep_batch_collect(ctx->batch_swp, js, src, s);
+        for (size_t k = 0; k < sweep.size(); ++k) rc[sweep[k]] = e != EMP_OK ? e : src[k];
+    }
+    if (!bucket.empty()) {
+        const emp_status e = batch_rounds(ctx, jobs, bucket, rc, s);
         if (e != EMP_OK)
-            for (int i : *batch)
+            for (int i : bucket)
                 if (rc[i] == EMP_OK) rc[i] = e;
     }
     for (int i : alone) rc[i] = job_rounds(jobs[i], s);
@@ -1522,6 +1555,8 @@ struct emp_server {
     emp_server_params p{};
     std::deque<emp_job *> queue;     // submitted, not yet admitted
     std::vector<emp_job *> live;     // in the bucket-kernel batch
+    std::vector<emp_job *> sweep;    // those that run all rounds in the next sweep launch
+    SweepBatch sb;
     std::vector<emp_job *> finished; // completed, not yet handed out
     uint64_t admitted = 0;           // footprint estimates of the admitted jobs
     DevBuf d_jobs, d_ctl;
@@ -1539,6 +1574,11 @@ void server_complete(emp_server *srv, emp_job *j) {
     srv->finished.push_back(j);
 }
 
+// whether the job runs only a share of its rounds in a launch
+bool shares(const emp_server *srv, const emp_job *j) {
+    return !srv->p.share_min_entries || 2 * j->prep.U >= srv->p.share_min_entries;
+}
+
 // One step: the launch of at most rounds_per_launch rounds of every job in
 // the batch goes first, so that the FASTQ copies of newly admitted jobs run
 // beside it; then the admitted jobs' map phase (queued behind the launch),
@@ -1551,16 +1591,35 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     const auto ts = std::chrono::steady_clock::now();
     const uint64_t budget = srv->p.hbm_budget_bytes ? srv->p.hbm_budget_bytes : ctx->budget;
     std::vector<emp_job *> adm;
-    while (!srv->queue.empty() && (int)(srv->live.size() + adm.size()) < srv->p.max_jobs) {
+    while (!srv->queue.empty() && (int)(srv->live.size() + srv->sweep.size() + adm.size()) < srv->p.max_jobs) {
         emp_job *j = srv->queue.front();
         const uint64_t est = served_footprint(j->F);
-        if (budget && srv->admitted + est > budget && !(srv->live.empty() && adm.empty())) break;
+        const bool idle = srv->live.empty() && srv->sweep.empty() && adm.empty();
+        if (budget && srv->admitted + est > budget && !idle) break;
         srv->queue.pop_front();
         srv->admitted += est;
         j->admit_est = est;
         adm.push_back(j);
     }
-    // ---- the launch (not waited for yet)
+    // ---- the launches (not waited for yet): all rounds of the short jobs in
+    // one sweep launch, the long jobs' share of theirs in the bucket kernel
+    std::vector<emp_job *> swept;
+    swept.swap(srv->sweep);
+    emp_status sweep_rc = EMP_OK;
+    struct SweptGuard {  // a step that ends early: the launch has overwritten their lists, so they fail
+        emp_server *srv;
+        std::vector<emp_job *> &jobs;
+        cudaStream_t s;
+        bool closed = false;
+        ~SweptGuard() {
+            if (closed || jobs.empty()) return;
+            cudaStreamSynchronize(s);
+            std::vector<emp_status> rc(jobs.size(), EMP_E_CUDA);
+            close_jobs(jobs.data(), (int)jobs.size(), rc, s);
+            for (emp_job *j : jobs) server_complete(srv, j);
+        }
+    } swept_guard{srv, swept, s};
+    if (!swept.empty()) sweep_rc = sweep_batch_launch(ctx, srv->sb, swept, s);
     const size_t nb = srv->live.size();
     BktJob *hj = nullptr;
     CoopCtl *hc = nullptr;
@@ -1582,7 +1641,7 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
         bool any_unlimited = false;
         for (size_t k = 0; k < nb; ++k) {
             hj[k] = srv->live[k]->bk;
-            const bool large = !srv->p.share_min_entries || 2 * srv->live[k]->prep.U >= srv->p.share_min_entries;
+            const bool large = shares(srv, srv->live[k]);
             hj[k].iter_share = large ? share : 0u;
             any_unlimited |= !large;
         }
@@ -1610,11 +1669,16 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
         std::vector<emp_status> crc;
         // a lone job in an idle server (nothing in flight, nothing queued)
         // runs alone, as emp_job_run runs it: one launch for all its rounds
-        const bool solo = nb == 0 && n == 1 && srv->queue.empty();
+        const bool solo = nb == 0 && swept.empty() && n == 1 && srv->queue.empty();
         for (int i = 0; i < n; ++i) {
             emp_job *j = adm[i];
             JobPrep &q = j->prep;
             const bool fits = !srv->p.batch_max_entries || 2 * q.U <= srv->p.batch_max_entries;
+            if (rc[i] == EMP_OK && !q.done && batch_eligible(j) && fits && !solo && !shares(srv, j) &&
+                sweep_rounds_usable(j, 2 * q.U)) {
+                srv->sweep.push_back(j);
+                continue;
+            }
             if (rc[i] == EMP_OK && !q.done && batch_eligible(j) && fits && !solo) {
                 rc[i] = rounds_prelude(j, s);
                 if (rc[i] == EMP_OK) rc[i] = bucket_prepare(j, s, job_env(j), 0, 0, 2 * q.U, q.ecap, 1u, &j->bk);
@@ -1638,11 +1702,9 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
         ss.admitted += (uint64_t)n;
         ss.ms_admit += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }
-    if (!nb) {
-        srv->live.swap(joining);
-        return EMP_OK;
-    }
-    // ---- the launch's results
+    if (!nb) srv->live.swap(joining);
+    if (!nb && swept.empty()) return EMP_OK;
+    // ---- the launches' results
     const auto tw = std::chrono::steady_clock::now();
     EMP_CUDA(cudaStreamSynchronize(s));
     const auto tr = std::chrono::steady_clock::now();
@@ -1652,6 +1714,18 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
         std::chrono::steady_clock::time_point t;
         ~ResultClock() { acc += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t).count(); }
     } result_clock{ss.ms_results, tr};
+    if (!swept.empty()) {
+        swept_guard.closed = true;
+        std::vector<emp_status> rc(swept.size(), EMP_OK);
+        if (sweep_rc == EMP_OK) sweep_rc = sweep_batch_collect(srv->sb, swept, rc, s);
+        if (sweep_rc != EMP_OK) rc.assign(swept.size(), sweep_rc);
+        ss.launches += 1;
+        ss.batch_jobs += swept.size();
+        ss.ms_kernel += ms_between(srv->sb.ev[0], srv->sb.ev[1]);
+        close_jobs(swept.data(), (int)swept.size(), rc, s);
+        for (emp_job *j : swept) server_complete(srv, j);
+    }
+    if (!nb) return sweep_rc == EMP_E_TIMEOUT ? EMP_E_TIMEOUT : EMP_OK;
     const bool timed_out = (hc->err & kErrSpin) != 0;
     const float ms = ms_between(srv->ev[0], srv->ev[1]);
     ss.launches += 1;
@@ -1674,7 +1748,7 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     }
     still.insert(still.end(), joining.begin(), joining.end());
     srv->live.swap(still);
-    if (done.empty()) return EMP_OK;
+    if (done.empty()) return sweep_rc == EMP_E_TIMEOUT ? EMP_E_TIMEOUT : EMP_OK;
     EMP_CUDA(cudaStreamSynchronize(s));
     std::vector<emp_status> rc(done.size(), timed_out ? EMP_E_TIMEOUT : EMP_OK);
     for (size_t k = 0; k < done.size() && !timed_out; ++k) {
@@ -1690,7 +1764,7 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     }
     close_jobs(done.data(), (int)done.size(), rc, s);
     for (emp_job *j : done) server_complete(srv, j);
-    return timed_out ? EMP_E_TIMEOUT : EMP_OK;
+    return timed_out || sweep_rc == EMP_E_TIMEOUT ? EMP_E_TIMEOUT : EMP_OK;
 }
 
 }  // namespace
@@ -1866,7 +1940,7 @@ emp_status emp_ctx_destroy(emp_ctx *ctx) {
     detach_graphs(ctx);
     for (auto &e : ctx->batch_ev)
         if (e) cudaEventDestroy(e);
-    ctx->in_use -= ctx->batch_jobs.bytes + ctx->batch_ctl.bytes + ctx->batch_swp.bytes;
+    ctx->in_use -= ctx->batch_jobs.bytes + ctx->batch_ctl.bytes + ctx->batch_swp.bytes();
     ctx->batch_jobs.release();
     ctx->batch_swp.release();
     ctx->batch_ctl.release();
@@ -2205,10 +2279,12 @@ emp_status emp_server_destroy(emp_server *srv) {
     };
     for (emp_job *j : srv->queue) drop(j);
     for (emp_job *j : srv->live) drop(j);
+    for (emp_job *j : srv->sweep) drop(j);
     for (emp_job *j : srv->finished) j->server = nullptr;
     for (auto &e : srv->ev)
         if (e) cudaEventDestroy(e);
-    srv->ctx->in_use -= srv->d_jobs.bytes + srv->d_ctl.bytes;
+    srv->ctx->in_use -= srv->d_jobs.bytes + srv->d_ctl.bytes + srv->sb.bytes();
+    srv->sb.release();
     delete srv;
     return EMP_OK;
 }
@@ -2253,7 +2329,7 @@ emp_status emp_server_get_stats(emp_server *srv, emp_server_stats *st) {
 emp_status emp_server_counts(emp_server *srv, int *queued, int *in_flight, int *finished) {
     if (!srv) return EMP_E_INVAL;
     if (queued) *queued = (int)srv->queue.size();
-    if (in_flight) *in_flight = (int)srv->live.size();
+    if (in_flight) *in_flight = (int)(srv->live.size() + srv->sweep.size());
     if (finished) *finished = (int)srv->finished.size();
     return EMP_OK;
 }
