@@ -166,7 +166,7 @@ struct emp_ctx {
     cudaMemPool_t pool = nullptr;
     DevBuf tables;  // HashTables, then ChunkWeights
     // emp_sort_pairs working set, kept for the next call
-    DevBuf sort_k1, sort_v1, sort_scr, sort_err;
+    DevBuf sort_k1, sort_v1, sort_scr;
     uint64_t sort_cap = 0;
     uint64_t sort_calls = 0;
     HostSlab slab;
@@ -396,7 +396,7 @@ uint32_t *err_word(emp_job *j) { return reinterpret_cast<uint32_t *>(j->misc.as<
 // the sort scratch must start zeroed and be re-zeroed before its epoch wraps
 emp_status ensure_sort_scratch(emp_job *j, uint64_t n_max, cudaStream_t s) {
     const size_t need = sort_scratch_bytes(n_max);
-    if (need > j->sort_scratch.bytes || j->sorts_since_clear > 100000) {
+    if (need > j->sort_scratch.bytes || j->sorts_since_clear > kSortsPerClear) {
         EMP_TRY(ensure(j, j->sort_scratch, need));
         EMP_CUDA(cudaMemsetAsync(j->sort_scratch.p, 0, j->sort_scratch.bytes, s));
         j->sorts_since_clear = 0;
@@ -411,13 +411,13 @@ void timed_sort(emp_job *j, uint64_t n, cudaStream_t s) {
     j->sort_timed = true;
     ++j->sorts_since_clear;
     sort_pairs(j->sk0.as<uint64_t>(), j->sv0.as<uint32_t>(), j->sk1.as<uint64_t>(), j->sv1.as<uint32_t>(), n,
-               j->sort_scratch.p, j->misc.as<uint64_t>() + kMiscSortN, err_word(j), s, j->sort_ev);
+               j->sort_scratch.p, err_word(j), s, j->sort_ev);
 }
 
 // stable sort of (k, v)[0..n) in place through (k1, v1), on the job's sort scratch
 void seg_sort(emp_job *j, uint64_t *k, uint32_t *v, uint64_t *k1, uint32_t *v1, uint64_t n, cudaStream_t s) {
     ++j->sorts_since_clear;
-    sort_pairs(k, v, k1, v1, n, j->sort_scratch.p, j->misc.as<uint64_t>() + kMiscSortN, err_word(j), s);
+    sort_pairs(k, v, k1, v1, n, j->sort_scratch.p, err_word(j), s);
 }
 
 // The reference's fingerprint sort of a table of n > M entries
@@ -2904,23 +2904,26 @@ emp_status emp_sort_pairs(emp_ctx *ctx, uint64_t *d_keys, uint32_t *d_vals, uint
         return true;
     };
     // the working set is kept in the context for the next call
-    if (n > ctx->sort_cap || ctx->sort_calls > 100000) {
-        if (!grow(ctx->sort_k1, n * 8) || !grow(ctx->sort_v1, n * 4) || !grow(ctx->sort_scr, sort_scratch_bytes(n)) ||
-            !grow(ctx->sort_err, 16))
+    if (n > ctx->sort_cap || ctx->sort_calls > kSortsPerClear) {
+        if (!grow(ctx->sort_k1, n * 8) || !grow(ctx->sort_v1, n * 4) || !grow(ctx->sort_scr, sort_scratch_bytes(n)))
             return EMP_E_NOMEM;
         if (cudaMemsetAsync(ctx->sort_scr.p, 0, ctx->sort_scr.bytes, s) != cudaSuccess) return EMP_E_CUDA;
         ctx->sort_cap = n;
         ctx->sort_calls = 0;
     }
     ++ctx->sort_calls;
-    // sort_err: the error word, then (8 bytes in) the device copy of n
-    uint64_t *err = ctx->sort_err.as<uint64_t>();
-    cudaMemsetAsync(err, 0, 8, s);
-    sort_pairs(d_keys, d_vals, ctx->sort_k1.as<uint64_t>(), ctx->sort_v1.as<uint32_t>(), n, ctx->sort_scr.p, err + 1,
-               reinterpret_cast<uint32_t *>(err), s);
-    uint32_t herr = 0;
-    cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, s);
-    if (cudaStreamSynchronize(s) != cudaSuccess) return EMP_E_CUDA;
+    uint32_t *flags = sort_flags(ctx->sort_scr.p);  // radix sort needed, error
+    uint64_t *k1 = ctx->sort_k1.as<uint64_t>();
+    uint32_t *v1 = ctx->sort_v1.as<uint32_t>();
+    uint32_t h[2] = {0, 0};
+    sort_groups(d_keys, d_vals, k1, v1, n, ctx->sort_scr.p, flags + 1, s);
+    for (int radix = 0;; radix = 1) {
+        cudaMemcpyAsync(h, flags, sizeof h, cudaMemcpyDeviceToHost, s);
+        if (cudaStreamSynchronize(s) != cudaSuccess) return EMP_E_CUDA;
+        if (!h[0] || radix) break;
+        sort_radix(d_keys, d_vals, k1, v1, n, ctx->sort_scr.p, flags + 1, s);  // uneven keys
+    }
+    const uint32_t herr = h[1];
     if (herr & kErrSpin) return EMP_E_TIMEOUT;
     return EMP_OK;
 }

@@ -4,9 +4,10 @@
 // library routine).
 //
 // The array holds, for at most kStaticMaxPairs pairs:
-//   [alternate keys 8 B/pair][alternate values 4 B/pair][error word, n]
-//   [SortScratch header][look-back words, one per (4096-pair tile, digit)]
-// Each call clears the error word, the header and the look-back words of its
+//   [alternate keys 8 B/pair][alternate values 4 B/pair]
+//   [SortScratch header with the error word][look-back words, one per (4096-pair tile, digit)]
+//   [group bounds]
+// Each call clears the header and the look-back words of its
 // own tiles before the sort reads them.  Every call on a device uses the
 // same array: calls whose GPU work overlaps (other streams, other host
 // threads) race on it and give wrong results.
@@ -23,10 +24,10 @@ constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 constexpr size_t kOffK1 = 0;
 constexpr size_t kOffV1 = align_up(kOffK1 + kStaticMaxPairs * sizeof(uint64_t));
-constexpr size_t kOffWord = align_up(kOffV1 + kStaticMaxPairs * sizeof(uint32_t));  // u32 error, u64 n at +8
-constexpr size_t kOffScr = align_up(kOffWord + 16);
+constexpr size_t kOffScr = align_up(kOffV1 + kStaticMaxPairs * sizeof(uint32_t));
 constexpr size_t kMaxTiles = (kStaticMaxPairs + kSortTile - 1) / kSortTile;
-constexpr size_t kScrBytes = sizeof(SortScratch) + kMaxTiles * kSortRadix * sizeof(uint64_t);
+constexpr size_t kScrBytes = sizeof(SortScratch) + kMaxTiles * kSortRadix * sizeof(uint64_t) +
+                             (kStaticMaxPairs / (kGroupMean / 2) + 4) * sizeof(uint64_t);
 constexpr size_t kStaticBytes = align_up(kOffScr + kScrBytes);  // 12.6 MB at 2^20 pairs
 
 static __device__ __align__(256) uint8_t g_sort_static[kStaticBytes];
@@ -68,23 +69,28 @@ extern "C" emp_status emp_sort_pairs_static(uint64_t *d_keys, uint32_t *d_vals, 
     const emp_status rc = static_scratch(&base);
     if (rc != EMP_OK) return rc;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    uint32_t *err = reinterpret_cast<uint32_t *>(base + kOffWord);
-    uint64_t *n_dev = reinterpret_cast<uint64_t *>(base + kOffWord + 8);
-    const size_t scr_bytes = sort_scratch_bytes(n);  // header + look-back words of n's tiles
-    if (cudaMemsetAsync(err, 0, sizeof(uint32_t), s) != cudaSuccess ||
-        cudaMemsetAsync(base + kOffScr, 0, scr_bytes, s) != cudaSuccess) {
+    uint8_t *scr = base + kOffScr;
+    uint32_t *flags = sort_flags(scr);  // radix sort needed, error
+    // header + look-back words of n's tiles
+    if (cudaMemsetAsync(scr, 0, sort_scratch_bytes(n), s) != cudaSuccess) {
         cudaGetLastError();
         return EMP_E_CUDA;
     }
-    sort_pairs(d_keys, d_vals, reinterpret_cast<uint64_t *>(base + kOffK1), reinterpret_cast<uint32_t *>(base + kOffV1),
-               n, base + kOffScr, n_dev, err, s, nullptr);
-    if (cudaGetLastError() != cudaSuccess) return EMP_E_CUDA;
-    uint32_t herr = 0;
-    if (cudaMemcpyAsync(&herr, err, sizeof herr, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess) {
-        cudaGetLastError();
-        return EMP_E_CUDA;
+    uint64_t *k1 = reinterpret_cast<uint64_t *>(base + kOffK1);
+    uint32_t *v1 = reinterpret_cast<uint32_t *>(base + kOffV1);
+    uint32_t h[2] = {0, 0};
+    sort_groups(d_keys, d_vals, k1, v1, n, scr, flags + 1, s);
+    for (int radix = 0;; radix = 1) {
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(h, flags, sizeof h, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
+            cudaGetLastError();
+            return EMP_E_CUDA;
+        }
+        if (!h[0] || radix) break;
+        sort_radix(d_keys, d_vals, k1, v1, n, scr, flags + 1, s);  // uneven keys
     }
+    const uint32_t herr = h[1];
     if (herr & kErrSpin) return EMP_E_TIMEOUT;
     return EMP_OK;
 }

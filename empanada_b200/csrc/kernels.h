@@ -89,40 +89,42 @@ void graph_paths(const uint8_t *out, const uint64_t *rec_off, const uint64_t *re
 void graph_cycles(uint32_t nodes, const GraphBufs &b, cudaStream_t s);
 void graph_place(uint32_t nodes, const GraphBufs &b, cudaStream_t s);
 
-// ---- radix sort (k_sort.cu) ---------------------------------------------
+// ---- sort of (fingerprint, value) pairs (k_sort.cu) ------------------------
 constexpr int kSortBits = 8;
 constexpr int kSortRadix = 1 << kSortBits;
-constexpr int kSortPasses = 8;           // 59-bit sort keys
+constexpr int kSortPasses = 8;           // digits of a full radix sort
 constexpr uint32_t kSortTile = 4096;
 __host__ __device__ inline uint64_t sort_tiles(uint64_t n) { return (n + kSortTile - 1) / kSortTile; }
 constexpr uint32_t kSmallSort = 4096;    // up to this many pairs: one CTA sorts in shared memory
+constexpr uint32_t kGroupMean = 2900;    // pairs of a key-range group at most, on average
 struct SortScratch {
     uint32_t hist[kSortPasses][kSortRadix];  // digit counts of the pairs being sorted
     uint32_t tile_ctr[kSortPasses];          // per-pass tile tickets
     uint32_t epoch;                          // look-back epoch of the current sort
-    uint32_t pad[7];
-    // followed by sort_tiles(n_max) * kSortRadix epoch-tagged look-back words
+    uint32_t radix;                          // the pairs need the full radix sort
+    uint32_t err;                            // error word for callers without one of their own
+    uint32_t pad[5];
+    // followed by sort_tiles(n_max) * kSortRadix epoch-tagged look-back words,
+    // then the group bounds
 };
-// Start a new sort on this scratch: advance the epoch, reset the tickets and
-// (zero_hist) the histogram.  One CTA.
-void launch_sort_prepare(SortScratch *sc, bool zero_hist, cudaStream_t s);
-// Bytes of scratch a sort of up to n pairs needs (histograms, tile tickets,
-// epoch, look-back words).  Zero it once after allocation; it resets itself
-// between sorts (re-zero after 100000 sorts, before the epoch can wrap).
+// Bytes of scratch a sort of up to n pairs needs.  Zero it once after
+// allocation; it resets itself between sorts (re-zero after 50000 sorts,
+// before the epoch can wrap).
 size_t sort_scratch_bytes(uint64_t n);
-// Stable sort of (keys, vals) by sort_key(key, val), count *n_dev (device)
-// with n_max >= *n_dev sizing the grid.  Ping-pongs between (k0,v0) and
-// (k1,v1); kSortPasses is even, so the result ends in (k0,v0) (returns 0).
-// pass_events (optional, 2*kSortPasses events) bracket each digit pass.
-int sort_pairs_dev(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, const uint64_t *n_dev, uint64_t n_max,
-                   void *scratch, uint32_t *err, cudaStream_t s, cudaEvent_t *pass_events = nullptr);
-// The same without the prepare step: the caller has already prepared the
-// scratch (pipeline rounds prepare the next sort in their round_end kernel).
-void sort_pairs_prepared(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, const uint64_t *n_dev,
-                         uint64_t n_max, SortScratch *sc, uint32_t *err, cudaStream_t s);
-// Same with a host count (copied into the device word n_dev first).
-int sort_pairs(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch, uint64_t *n_dev,
-               uint32_t *err, cudaStream_t s, cudaEvent_t *pass_events = nullptr);
+constexpr uint64_t kSortsPerClear = 50000;
+// Stable sort of (keys, vals) by sort_key(key, val), ping-ponging between
+// (k0,v0) and (k1,v1); the result is in (k0,v0).  Queued whole: sort_pairs.
+// In two halves, for a caller that waits for the stream anyway: sort_groups,
+// and sort_radix if sort_flags(scratch)[0] (device) is then nonzero;
+// sort_flags(scratch)[1], zero when sort_groups starts, can serve as err.
+// events (optional, 2*kSortPasses events) bracket the passes.
+void sort_pairs(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch, uint32_t *err,
+                cudaStream_t s, cudaEvent_t *events = nullptr);
+void sort_groups(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch, uint32_t *err,
+                 cudaStream_t s);
+void sort_radix(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch, uint32_t *err,
+                cudaStream_t s, cudaEvent_t *events = nullptr);
+uint32_t *sort_flags(void *scratch);
 
 // ---- sort of a table larger than M (k_chunked.cu) --------------------------
 struct ChunkPart {  // one merge partition: A entries [a0, a0+pa), B entries [b0, b0+pb)
