@@ -90,21 +90,30 @@ EMP_DEV bool is_n_class(uint8_t c) { return (c & 0xC0u) == 0x40u && (c & 8u); }
 EMP_DEV uint64_t next_sfx(uint64_t key, uint32_t v, uint32_t pw1, uint32_t pw2) {
     uint32_t f1 = (uint32_t)(key >> 32), f2 = (uint32_t)key;
     uint32_t e = v + 1u;
-    uint32_t t1 = mod1((uint64_t)(e * pw1));  // 32-bit product < 2^31, as in the reference
-    uint32_t t2 = mod2((uint64_t)(e * pw2));
+    uint32_t t1 = mod_fold32<3u, kP1>(e * pw1);  // 32-bit product < 2^31, as in the reference
+    uint32_t t2 = mod_fold32<33u, kP2>(e * pw2);
     f1 = f1 >= t1 ? f1 - t1 : f1 + kP1 - t1;
     f2 = f2 >= t2 ? f2 - t2 : f2 + kP2 - t2;
     return ((uint64_t)f1 << 32) | f2;
 }
 
-// PrevPfx: drop the last base (code v).  Subtraction and product wrap mod 2^64
-// exactly like the reference's uint64_t expression.
+// PrevPfx: drop the last base (code v), (f - enc) * R^-1 mod P.  P1 = -1 mod 5
+// and P2 = -1 mod 7, so for f - enc = R k + m the quotient is k + m (P + 1) / R:
+// a sixth of the instructions of the product with the inverse and its folds.
+// Where f < enc, subtraction and product wrap mod 2^64 exactly like the
+// reference's uint64_t expression.
+static_assert((kP1 + 1u) % kR1 == 0 && (kP2 + 1u) % kR2 == 0, "P = -1 mod R");
 EMP_DEV uint64_t prev_pfx(uint64_t key, uint32_t v, uint32_t inv1, uint32_t inv2) {
-    uint64_t f1 = key >> 32, f2 = key & 0xffffffffull;
-    uint64_t e = v + 1u;
-    uint64_t x1 = (uint64_t)inv1 * (f1 - e);
-    uint64_t x2 = (uint64_t)inv2 * (f2 - e);
-    return ((uint64_t)mod1(x1) << 32) | mod2(x2);
+    const uint32_t f1 = (uint32_t)(key >> 32), f2 = (uint32_t)key, e = v + 1u;
+    if (f1 < e || f2 < e) {
+        const uint64_t x1 = (uint64_t)inv1 * ((uint64_t)f1 - e);
+        const uint64_t x2 = (uint64_t)inv2 * ((uint64_t)f2 - e);
+        return ((uint64_t)mod1(x1) << 32) | mod2(x2);
+    }
+    const uint32_t y1 = f1 - e, k1 = y1 / kR1, y2 = f2 - e, k2 = y2 / kR2;
+    const uint32_t g1 = k1 + (y1 - k1 * kR1) * ((kP1 + 1u) / kR1);
+    const uint32_t g2 = k2 + (y2 - k2 * kR2) * ((kP2 + 1u) / kR2);
+    return ((uint64_t)g1 << 32) | g2;
 }
 
 // 59-bit sort key: (fp1, fp2) order-preserving in 58 bits, table bit below.

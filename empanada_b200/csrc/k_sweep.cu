@@ -164,23 +164,11 @@ EMP_DEV void step_sfx(uint32_t &f1, uint32_t &f2, uint2 t) {
     f1 = f1 >= t.x ? f1 - t.x : f1 + kP1 - t.x;
     f2 = f2 >= t.y ? f2 - t.y : f2 + kP2 - t.y;
 }
-// PrevPfx: (f - enc) / R mod P.  P1 = -1 mod 5 and P2 = -1 mod 7, so for y =
-// R k + m the quotient is k + m (P + 1) / R (a sixth of the instructions of
-// the product with the inverse and its two folds).  Where f < enc the
-// reference's difference wraps in 64 bits (overlap.cu:77-91): prev_pfx.
 EMP_DEV void step_pfx(uint32_t &f1, uint32_t &f2, uint32_t v, uint32_t inv1, uint32_t inv2) {
-    const uint32_t e = v + 1u;
-    if (f1 < e || f2 < e) {
-        const uint64_t k = prev_pfx(((uint64_t)f1 << 32) | f2, v, inv1, inv2);
-        f1 = (uint32_t)(k >> 32);
-        f2 = (uint32_t)k;
-        return;
-    }
-    const uint32_t y1 = f1 - e, k1 = y1 / kR1, y2 = f2 - e, k2 = y2 / kR2;
-    f1 = k1 + (y1 - k1 * kR1) * ((kP1 + 1u) / kR1);
-    f2 = k2 + (y2 - k2 * kR2) * ((kP2 + 1u) / kR2);
+    const uint64_t k = prev_pfx(((uint64_t)f1 << 32) | f2, v, inv1, inv2);
+    f1 = (uint32_t)(k >> 32);
+    f2 = (uint32_t)k;
 }
-static_assert((kP1 + 1u) % kR1 == 0 && (kP2 + 1u) % kR2 == 0, "P = -1 mod R");
 
 // ---------------------------------------------------------------- groups
 // slot of a group: (key, round), the last prefix candidate that entered it
