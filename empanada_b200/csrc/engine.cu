@@ -137,13 +137,13 @@ struct HostSlab {
 
 // One sweep launch's descriptors (device and host), output bins and events.
 struct SweepBatch {
-    DevBuf jobs, ctl, out;
-    PinnedBuf host;
+    DevBuf jobs, out;  // descriptors, control block and round records; output bins
+    PinnedBuf host;    // the same as `jobs`
+    size_t records = 0;  // offset of the round records
     cudaEvent_t ev[2] = {};
-    uint64_t bytes() const { return jobs.bytes + ctl.bytes + out.bytes; }
+    uint64_t bytes() const { return jobs.bytes + out.bytes; }
     void release() {
         jobs.release();
-        ctl.release();
         out.release();
         for (auto &e : ev) {
             if (e) cudaEventDestroy(e);
@@ -193,6 +193,7 @@ struct JobPrep {
     int L = 0, wpr = 0, rounds = 0;
     bool done = false;  // nothing more to run (empty input, no reads)
     bool no_sweep = false;  // the rounds run in the bucket kernel (kCrowded)
+    bool one_half = false;  // the list's prefix half, a copy of the suffixes', is not written (the sweep kernel needs none)
 };
 
 struct emp_job {
@@ -251,7 +252,7 @@ namespace {
 
 // misc device words (u64 slots)
 enum MiscSlot { kMiscErr = 0, kMiscTotal = 1, kMiscLen = 2, kMiscN = 3, kMiscU = 4, kMiscNout = 5, kMiscSout = 6,
-                kMiscE = 7, kMiscCtr = 8, kMiscParts = 9, kMiscSortN = 10, kMiscLen0 = 11, kMiscKept = 12,
+                kMiscE = 7, kMiscParts = 9, kMiscSortN = 10, kMiscLen0 = 11, kMiscKept = 12,
                 kMiscSlots = 16 };
 
 // internal: the pipeline's edge buffer was too small (never returned by the ABI)
@@ -383,14 +384,15 @@ void append_bytes(std::vector<uint8_t> &o, const void *p, size_t n) {
     o.insert(o.end(), b, b + n);
 }
 
-// reset look-back status words + tile counter for a chained scan over `tiles`
+// Tile counter (64 bytes) and look-back status words of a chained scan over
+// `tiles`, zeroed (a scan of one tile reads neither).
 emp_status reset_chain(emp_job *j, uint64_t tiles, cudaStream_t s) {
     EMP_TRY(ensure(j, j->status, tiles * sizeof(uint64_t) + 64));
-    EMP_CUDA(cudaMemsetAsync(j->status.p, 0, tiles * sizeof(uint64_t), s));
-    EMP_CUDA(cudaMemsetAsync(j->misc.as<uint64_t>() + kMiscCtr, 0, sizeof(uint64_t), s));
+    if (tiles > 1) EMP_CUDA(cudaMemsetAsync(j->status.p, 0, tiles * sizeof(uint64_t) + 64, s));
     return EMP_OK;
 }
-uint32_t *chain_ctr(emp_job *j) { return reinterpret_cast<uint32_t *>(j->misc.as<uint64_t>() + kMiscCtr); }
+uint32_t *chain_ctr(emp_job *j) { return j->status.as<uint32_t>(); }
+uint64_t *chain_words(emp_job *j) { return j->status.as<uint64_t>() + 8; }
 uint32_t *err_word(emp_job *j) { return reinterpret_cast<uint32_t *>(j->misc.as<uint64_t>() + kMiscErr); }
 
 // the sort scratch must start zeroed and be re-zeroed before its epoch wraps
@@ -511,7 +513,7 @@ emp_status sync_round(emp_job *j, cudaStream_t s, const RoundEnv &env, int r, in
     a.tables = env.tables;
     a.L = env.L;
     a.round = r;
-    a.status = j->status.as<uint64_t>();
+    a.status = chain_words(j);
     a.tile_ctr = chain_ctr(j);
     a.n_out = dm + kMiscNout;
     a.s_out = dm + kMiscSout;
@@ -552,7 +554,7 @@ emp_status sync_round(emp_job *j, cudaStream_t s, const RoundEnv &env, int r, in
     EMP_TRY(ensure(j, j->offs, N * 8));
     launch_join_count(sk, sv, N, j->cnt.as<uint32_t>(), s);
     EMP_TRY(reset_chain(j, scan_tiles(N), s));
-    launch_scan_u32_u64(j->cnt.as<uint32_t>(), j->offs.as<uint64_t>(), N, j->status.as<uint64_t>(), chain_ctr(j),
+    launch_scan_u32_u64(j->cnt.as<uint32_t>(), j->offs.as<uint64_t>(), N, chain_words(j), chain_ctr(j),
                         dm + kMiscE, err_word(j), s);
     EMP_TRY(sync_and_check(j, s));
     account_sort(j);
@@ -579,7 +581,7 @@ emp_status sync_round(emp_job *j, cudaStream_t s, const RoundEnv &env, int r, in
         EMP_TRY(ensure(j, j->parts, pcap * sizeof(SearchPart)));
         EMP_TRY(reset_chain(j, upd_tiles(N), s));
         launch_split_tables(sk, sv, N, j->akeys.as<uint64_t>(), j->apos.as<uint32_t>(), j->bkeys.as<uint64_t>(),
-                            j->status.as<uint64_t>(), chain_ctr(j), err_word(j), s);
+                            chain_words(j), chain_ctr(j), err_word(j), s);
         launch_search_partitions(j->akeys.as<uint64_t>(), S, j->bkeys.as<uint64_t>(), P, M / 2,
                                  j->apos.as<uint32_t>(), j->offs.as<uint64_t>(), E, j->parts.as<SearchPart>(), pcap,
                                  dm + kMiscParts, err_word(j), s);
@@ -873,27 +875,30 @@ emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0
     hj->seq2 = env.seq2;
     hj->tables = env.tables;
     hj->ecap = ecap;
+    hj->one_half = j->prep.one_half ? 1 : 0;
     size_t zeroed = 0;
     EMP_TRY(ensure(j, j->swp, sweep_layout(nullptr, hj, &zeroed)));
     sweep_layout(j->swp.as<uint8_t>(), hj, &zeroed);
-    EMP_CUDA(cudaMemsetAsync(j->swp.p, 0, zeroed, s));
     EMP_TRY(ensure(j, j->dout, (size_t)env.rounds * 12 + ecap * 8));
-    EMP_TRY(ensure(j, j->records, (size_t)env.rounds * sizeof(RoundRecord)));
-    if (!j->h_records.ensure((size_t)env.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
     hj->out = j->dout.as<uint8_t>();
-    hj->records = j->records.as<RoundRecord>();
     return EMP_OK;
 }
 
 // Rounds r0 .. of one job alone in the sweep kernel.
 emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t ns, uint64_t np,
                             uint64_t ecap, uint64_t *needed) {
-    EMP_TRY(ensure(j, j->bk_job, sizeof(SweepJob)));
-    EMP_TRY(ensure(j, j->coop_ctl, sizeof(CoopCtl)));
-    if (!j->h_coop.ensure(sizeof(SweepJob) + sizeof(CoopCtl))) return EMP_E_NOMEM;
-    SweepJob *hj = j->h_coop.as<SweepJob>();
-    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + 1);
+    // descriptor, control block and round records in one device buffer, laid
+    // out as the job's host slot has them: one copy each way
+    constexpr size_t kRec = kSlotRecords - kSlotCoop;
+    const size_t rec_bytes = (size_t)env.rounds * sizeof(RoundRecord);
+    EMP_TRY(ensure(j, j->coop_ctl, kRec + rec_bytes));
+    if (!j->h_coop.ensure(sizeof(SweepJob) + sizeof(CoopCtl)) || !j->h_records.ensure(rec_bytes)) return EMP_E_NOMEM;
+    uint8_t *dev = j->coop_ctl.as<uint8_t>();
+    SweepJob *hj = j->h_coop.as<SweepJob>(), *dj = reinterpret_cast<SweepJob *>(dev);
+    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + 1), *dc = reinterpret_cast<CoopCtl *>(dj + 1);
     EMP_TRY(sweep_prepare(j, s, env, r0, cur, ns, np, ecap, sweep_segment_size(std::max(ns, np)), hj));
+    hj->records = reinterpret_cast<RoundRecord *>(dev + kRec);
+    EMP_CUDA(cudaMemsetAsync(j->swp.p, 0, (size_t)hj->zeroed * 16, s));
     SweepOut go{};
     size_t zeroed = 0;
     const uint32_t bins = sweep_bins_max(ns + np, env.rounds - r0);
@@ -908,16 +913,14 @@ emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int
         hc->trace = j->coop_trace.as<uint64_t>();
         hc->trace_cap = kSweepTraceCap;
     }
-    EMP_CUDA(cudaMemcpyAsync(j->bk_job.p, hj, sizeof(SweepJob), cudaMemcpyHostToDevice, s));
-    EMP_CUDA(cudaMemcpyAsync(j->coop_ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaMemcpyAsync(dev, hj, sizeof(SweepJob) + sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
     cudaEvent_t e0 = j->upd_ev[0], e1 = j->upd_ev[1];
     EMP_CUDA(cudaEventRecord(e0, s));
-    EMP_CUDA(launch_sweep(j->bk_job.as<SweepJob>(), j->coop_ctl.as<CoopCtl>(), go, s));
+    EMP_CUDA(launch_sweep(dj, dc, go, false, s));
     EMP_CUDA(cudaEventRecord(e1, s));
-    EMP_CUDA(cudaMemcpyAsync(hj, j->bk_job.p, sizeof(SweepJob), cudaMemcpyDeviceToHost, s));
-    EMP_CUDA(cudaMemcpyAsync(hc, j->coop_ctl.p, sizeof(CoopCtl), cudaMemcpyDeviceToHost, s));
-    EMP_TRY(bucket_fetch(j, env, s));
-    EMP_TRY(sync_and_check(j, s));
+    static_assert(kSlotBytes >= kSlotRecords + EMP_MAX_ROUNDS * sizeof(RoundRecord), "the records stay in the slot");
+    EMP_CUDA(cudaMemcpyAsync(hj, dev, kRec + rec_bytes, cudaMemcpyDeviceToHost, s));
+    EMP_CUDA(cudaStreamSynchronize(s));
     if (hc->err & kErrSpin) return EMP_E_TIMEOUT;
     j->st.ms_round_kernel += ms_between(e0, e1);
     if (trace) write_sweep_trace(j, j->ctx->trace_path.c_str(), s);
@@ -925,8 +928,8 @@ emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int
     return bucket_collect(j, r0, ns + np, *hj, needed);
 }
 
-// Round counters, output and used marks of a job, before its rounds.
-emp_status rounds_prelude(emp_job *j, cudaStream_t s) {
+// Round counters and output of a job, before its rounds.
+void rounds_prelude(emp_job *j) {
     emp_stats &st = j->st;
     st.n_rounds = 0;
     st.n_edges = 0;
@@ -936,9 +939,13 @@ emp_status rounds_prelude(emp_job *j, cudaStream_t s) {
     std::memset(st.edges, 0, sizeof st.edges);
     j->out.clear();
     j->dout_bytes = 0;
-    EMP_CUDA(cudaMemsetAsync(j->used_s.p, 0, j->used_s.bytes, s));
-    EMP_CUDA(cudaMemsetAsync(j->used_p.p, 0, j->used_p.bytes, s));
-    return EMP_OK;
+}
+
+// The list whole: [suffixes | prefixes].
+void whole_list(emp_job *j, cudaStream_t s) {
+    if (j->prep.one_half)
+        launch_dup_prefix_half(j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(), j->prep.U, s);
+    j->prep.one_half = false;
 }
 
 // All rounds: synchronous ones while a round could split into several search
@@ -949,7 +956,7 @@ emp_status run_rounds(emp_job *j, cudaStream_t s, const RoundEnv &env, uint64_t 
     if (!j->upd_ev[0]) {  // per-round events, made when a job first runs rounds on its own
         for (auto &e : j->upd_ev) EMP_CUDA(cudaEventCreate(&e));
     }
-    EMP_TRY(rounds_prelude(j, s));
+    rounds_prelude(j);
     int cur = 0, r = 0;
     uint64_t n_in = 2 * U, S = U, P = U;
     const uint64_t M = env.M;
@@ -957,7 +964,13 @@ emp_status run_rounds(emp_job *j, cudaStream_t s, const RoundEnv &env, uint64_t 
     // host-synchronised rounds (one full sort each) while a round may split
     // into several search partitions, and while the list is too large for the
     // bucket kernel
-    while (r < env.rounds && (!bucket || S >= M / 2 || P >= M / 2 || n_in > kBktMaxEntries)) {
+    auto host_round = [&]() { return r < env.rounds && (!bucket || S >= M / 2 || P >= M / 2 || n_in > kBktMaxEntries); };
+    if (host_round()) {  // the only rounds that mark what they use by read-end
+        whole_list(j, s);
+        EMP_CUDA(cudaMemsetAsync(j->used_s.p, 0, j->used_s.bytes, s));
+        EMP_CUDA(cudaMemsetAsync(j->used_p.p, 0, j->used_p.bytes, s));
+    }
+    while (host_round()) {
         bool stop = false;
         EMP_TRY(sync_round(j, s, env, r, cur, n_in, S, P, stop));
         if (stop) return EMP_OK;
@@ -965,6 +978,7 @@ emp_status run_rounds(emp_job *j, cudaStream_t s, const RoundEnv &env, uint64_t 
     }
     if (r >= env.rounds) return EMP_OK;
     if (sweep_rounds_usable(j, n_in)) return run_rounds_sweep(j, s, env, r, cur, S, P, ecap, needed);
+    whole_list(j, s);
     return run_rounds_bucket(j, s, env, r, cur, n_in, ecap, needed);
 }
 
@@ -1004,7 +1018,7 @@ emp_status map_begin(emp_job *j, cudaStream_t s) {
     EMP_TRY(ensure(j, j->tile_excl, T * 8));
     launch_nl_count(j->fq.as<uint8_t>(), F, j->tile_counts.as<uint32_t>(), j->misc.as<uint64_t>() + kMiscLen0, s);
     EMP_TRY(reset_chain(j, scan_tiles(T), s));
-    launch_scan_u32_u64(j->tile_counts.as<uint32_t>(), j->tile_excl.as<uint64_t>(), T, j->status.as<uint64_t>(),
+    launch_scan_u32_u64(j->tile_counts.as<uint32_t>(), j->tile_excl.as<uint64_t>(), T, chain_words(j),
                         chain_ctr(j), j->misc.as<uint64_t>() + kMiscTotal, err_word(j), s);
     return EMP_OK;
 }
@@ -1053,16 +1067,12 @@ emp_status map_records(emp_job *j, cudaStream_t s) {
 
 // The read pass (K2) with `wpr` read-major words per read.
 emp_status launch_reads(emp_job *j, cudaStream_t s, int wpr) {
-    uint64_t *hm = j->h_misc.as<uint64_t>();
     uint64_t *dm = j->misc.as<uint64_t>();
     const uint64_t n_rec = j->prep.n_rec;
     j->prep.wpr = wpr;
     EMP_TRY(ensure(j, j->keys0, n_rec * 16));
     EMP_TRY(ensure(j, j->seq2, n_rec * (uint64_t)wpr * 4));
     EMP_TRY(ensure(j, j->keep, n_rec * 4));
-    const uint32_t mm[4] = {0xffffffffu, 0u, 0u, 0u};  // length extremes, then the kept count
-    std::memcpy(hm + kMiscLen, mm, 16);
-    EMP_CUDA(cudaMemcpyAsync(dm + kMiscLen, hm + kMiscLen, 16, cudaMemcpyHostToDevice, s));
     launch_read_pass(j->fq.as<uint8_t>(), j->F, j->tile_excl.as<uint64_t>(), j->ctx->tables.as<HashTables>(),
                      reinterpret_cast<const ChunkWeights *>(j->ctx->tables.as<uint8_t>() + sizeof(HashTables)),
                      j->keys0.as<uint64_t>(), j->seq2.as<uint32_t>(), wpr, j->keep.as<uint32_t>(), dm + kMiscN,
@@ -1091,6 +1101,7 @@ emp_status map_keys(emp_job *j, cudaStream_t s) {
     const uint64_t n = hm[kMiscN];
     uint32_t mm2[2];
     std::memcpy(mm2, hm + kMiscLen, 8);
+    mm2[0] = ~mm2[0];
     int L = 0;
     if (n) {
         if (mm2[0] != mm2[1]) return EMP_E_FORMAT;
@@ -1109,6 +1120,7 @@ emp_status map_keys(emp_job *j, cudaStream_t s) {
     const uint64_t n2 = 2 * n;
     if (n2 >= (1ull << 31)) return EMP_E_UNSUPPORTED;
     if (q.wpr != (L + 15) / 16) {  // the kept reads are not as long as the first record: lay the words out again
+        EMP_CUDA(cudaMemsetAsync(dm + kMiscLen, 0, 16, s));  // length extremes, kept count
         EMP_TRY(launch_reads(j, s, (L + 15) / 16));
         EMP_TRY(sync_and_check(j, s));
         if (hm[kMiscErr] & kErrBadBase) return EMP_E_FORMAT;
@@ -1117,7 +1129,7 @@ emp_status map_keys(emp_job *j, cudaStream_t s) {
         EMP_TRY(ensure(j, j->keys_tmp, n * 16));
         EMP_TRY(ensure(j, j->seq2_tmp, n * (uint64_t)q.wpr * 4));
         EMP_TRY(reset_chain(j, scan_tiles(q.n_rec), s));
-        launch_scan_u32_u32(j->keep.as<uint32_t>(), j->keep.as<uint32_t>(), q.n_rec, j->status.as<uint64_t>(),
+        launch_scan_u32_u32(j->keep.as<uint32_t>(), j->keep.as<uint32_t>(), q.n_rec, chain_words(j),
                             chain_ctr(j), dm + kMiscKept, err_word(j), s);
         launch_compact_reads(j->keep.as<uint32_t>(), q.n_rec, n, j->keys0.as<uint64_t>(), j->seq2.as<uint32_t>(),
                              q.wpr, j->keys_tmp.as<uint64_t>(), j->seq2_tmp.as<uint32_t>(), s);
@@ -1148,16 +1160,17 @@ emp_status map_keys(emp_job *j, cudaStream_t s) {
     const uint32_t nbd = n2 <= q.M && j->ctx->tune.dedup_driver == 0 ? dedup_buckets(n2) : 0u;
     bool hashed = false;
     if (nbd) {  // in core: the smallest rid of every fingerprint survives, no sort needed
-        EMP_TRY(ensure(j, j->dedup_scr, dedup_scratch_bytes(nbd)));
-        EMP_TRY(reset_chain(j, scan_tiles(nbd), s));
+        if (!j->dedup_scr.p) {
+            EMP_TRY(ensure(j, j->dedup_scr, kDedupScratch));
+            EMP_CUDA(cudaMemsetAsync(j->dedup_scr.p, 0, kDedupScratch, s));
+        }
         hashed = launch_dedup_hash(j->keys0.as<uint64_t>(), n2, nbd, j->dedup_scr.p, j->sk0.as<uint64_t>(),
-                                   j->sv0.as<uint32_t>(), j->alive.as<uint8_t>(), j->status.as<uint64_t>(),
-                                   chain_ctr(j), dm + kMiscSortN, err_word(j), s);
+                                   j->sv0.as<uint32_t>(), j->alive.as<uint8_t>(), err_word(j), s);
     }
     if (!hashed) EMP_TRY(dedup_by_sort(j, s));
     EMP_TRY(reset_chain(j, upd_tiles(n2), s));
     launch_init_list(j->keys0.as<uint64_t>(), j->alive.as<uint8_t>(), n, j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(),
-                     j->status.as<uint64_t>(), chain_ctr(j), dm + kMiscU, err_word(j), s);
+                     chain_words(j), chain_ctr(j), dm + kMiscU, err_word(j), s);
     return EMP_OK;
 }
 
@@ -1192,7 +1205,7 @@ emp_status map_list(emp_job *j, cudaStream_t s) {
         EMP_TRY(dedup_by_sort(j, s));
         EMP_TRY(reset_chain(j, upd_tiles(2 * q.n), s));
         launch_init_list(j->keys0.as<uint64_t>(), j->alive.as<uint8_t>(), q.n, j->lk0.as<uint64_t>(),
-                         j->lv0.as<uint32_t>(), j->status.as<uint64_t>(), chain_ctr(j), dm + kMiscU, err_word(j), s);
+                         j->lv0.as<uint32_t>(), chain_words(j), chain_ctr(j), dm + kMiscU, err_word(j), s);
         EMP_TRY(sync_and_check(j, s));
     }
     if (j->h_misc.as<uint64_t>()[kMiscErr] & kErrHang) return EMP_E_HANG;
@@ -1201,9 +1214,10 @@ emp_status map_list(emp_job *j, cudaStream_t s) {
     const uint64_t U = j->h_misc.as<uint64_t>()[kMiscU];
     q.U = U;
     j->st.n_unique = U;
-    launch_dup_prefix_half(j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(), U, s);
-    cudaEventRecord(j->map_ev[2], s);
     q.rounds = q.L - j->p.min_ovlp;
+    q.one_half = true;
+    if (!(q.U < q.M / 2 && sweep_rounds_usable(j, 2 * U))) whole_list(j, s);
+    cudaEventRecord(j->map_ev[2], s);
     if (q.rounds <= 0) return EMP_OK;
     const uint64_t ecap0 = j->ctx->tune.edge_cap ? j->ctx->tune.edge_cap : (4 * U > (1u << 20) ? 4 * U : (1u << 20));
     q.ecap = j->ecap_hint ? j->ecap_hint : ecap0;
@@ -1218,12 +1232,13 @@ RoundEnv job_env(emp_job *j) {
 // The round drivers overwrite the list: build the initial one again from the
 // fingerprints and survivor marks, which the rounds leave intact.
 emp_status rebuild_list(emp_job *j, cudaStream_t s) {
-    const JobPrep &q = j->prep;
+    JobPrep &q = j->prep;
     EMP_TRY(reset_chain(j, upd_tiles(2 * q.n), s));
     launch_init_list(j->keys0.as<uint64_t>(), j->alive.as<uint8_t>(), q.n, j->lk0.as<uint64_t>(),
-                     j->lv0.as<uint32_t>(), j->status.as<uint64_t>(), chain_ctr(j),
+                     j->lv0.as<uint32_t>(), chain_words(j), chain_ctr(j),
                      j->misc.as<uint64_t>() + kMiscU, err_word(j), s);
-    launch_dup_prefix_half(j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(), q.U, s);
+    q.one_half = true;
+    whole_list(j, s);
     return EMP_OK;
 }
 
@@ -1277,7 +1292,7 @@ emp_status run_job(emp_job *j, cudaStream_t s) {
         cudaEventRecord(j->map_ev[3], s);
         cudaEventRecord(j->map_ev[4], s);
     }
-    EMP_TRY(sync_and_check(j, s));
+    EMP_CUDA(cudaStreamSynchronize(s));
     EMP_CUDA(cudaGetLastError());
     job_finish(j);
     return EMP_OK;
@@ -1310,7 +1325,8 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
     for (size_t k = 0; k < nb; ++k) {
         emp_job *j = jobs[idx[k]];
         const JobPrep &q = j->prep;
-        EMP_TRY(rounds_prelude(j, s));
+        rounds_prelude(j);
+        whole_list(j, s);
         EMP_TRY(bucket_prepare(j, s, job_env(j), 0, 0, 2 * q.U, q.ecap, 1u, &hj[k]));
     }
     coop_ctl_init(ctx, hc, (uint32_t)nb);
@@ -1346,25 +1362,30 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
 // ready): queued by launch, read by collect once the stream has been waited for.
 emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<emp_job *> &jobs, cudaStream_t s) {
     const size_t nb = jobs.size();
-    EMP_TRY(ctx_ensure(ctx, sb.jobs, nb * sizeof(SweepJob), s));
-    EMP_TRY(ctx_ensure(ctx, sb.ctl, sizeof(CoopCtl), s));
-    if (!sb.host.ensure(nb * sizeof(SweepJob) + sizeof(CoopCtl))) return EMP_E_NOMEM;
-    if (!sb.ev[0]) {
-        for (auto &e : sb.ev) EMP_CUDA(cudaEventCreate(&e));
-    }
-    SweepJob *hj = sb.host.as<SweepJob>();
-    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + nb);
-    uint64_t side = 0, bins = 0;
+    uint64_t side = 0, bins = 0, recs = 0;
     for (emp_job *j : jobs) {
         side += j->prep.U;
         bins += sweep_bins_max(2 * j->prep.U, j->prep.rounds);
+        recs += (uint64_t)j->prep.rounds;
     }
+    sb.records = (nb * sizeof(SweepJob) + sizeof(CoopCtl) + 255) / 256 * 256;
+    const size_t total = sb.records + recs * sizeof(RoundRecord);
+    EMP_TRY(ctx_ensure(ctx, sb.jobs, total, s));
+    if (!sb.host.ensure(total)) return EMP_E_NOMEM;
+    if (!sb.ev[0]) {
+        for (auto &e : sb.ev) EMP_CUDA(cudaEventCreate(&e));
+    }
+    SweepJob *hj = sb.host.as<SweepJob>(), *dj = sb.jobs.as<SweepJob>();
+    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + nb), *dc = reinterpret_cast<CoopCtl *>(dj + nb);
+    RoundRecord *rec = reinterpret_cast<RoundRecord *>(sb.jobs.as<uint8_t>() + sb.records);
     const uint32_t seg = sweep_segment_size(side);
     for (size_t k = 0; k < nb; ++k) {
         emp_job *j = jobs[k];
         const JobPrep &q = j->prep;
-        EMP_TRY(rounds_prelude(j, s));
+        rounds_prelude(j);
         EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, seg, &hj[k]));
+        hj[k].records = rec;
+        rec += q.rounds;
     }
     SweepOut go{};
     size_t zeroed = 0;
@@ -1372,14 +1393,11 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     sweep_out_layout(sb.out.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
     EMP_CUDA(cudaMemsetAsync(sb.out.p, 0, zeroed, s));
     coop_ctl_init(ctx, hc, (uint32_t)nb);
-    EMP_CUDA(cudaMemcpyAsync(sb.jobs.p, hj, nb * sizeof(SweepJob), cudaMemcpyHostToDevice, s));
-    EMP_CUDA(cudaMemcpyAsync(sb.ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaMemcpyAsync(dj, hj, nb * sizeof(SweepJob) + sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
     EMP_CUDA(cudaEventRecord(sb.ev[0], s));
-    EMP_CUDA(launch_sweep(sb.jobs.as<SweepJob>(), sb.ctl.as<CoopCtl>(), go, s));
+    EMP_CUDA(launch_sweep(dj, dc, go, true, s));
     EMP_CUDA(cudaEventRecord(sb.ev[1], s));
-    EMP_CUDA(cudaMemcpyAsync(hj, sb.jobs.p, nb * sizeof(SweepJob), cudaMemcpyDeviceToHost, s));
-    EMP_CUDA(cudaMemcpyAsync(hc, sb.ctl.p, sizeof(CoopCtl), cudaMemcpyDeviceToHost, s));
-    for (emp_job *j : jobs) EMP_TRY(bucket_fetch(j, job_env(j), s));
+    EMP_CUDA(cudaMemcpyAsync(hj, dj, total, cudaMemcpyDeviceToHost, s));
     return EMP_OK;
 }
 
@@ -1391,10 +1409,14 @@ emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &job
     const SweepJob *hj = sb.host.as<SweepJob>();
     if (reinterpret_cast<const CoopCtl *>(hj + nb)->err & kErrSpin) return EMP_E_TIMEOUT;
     const float ms = ms_between(sb.ev[0], sb.ev[1]);
+    const RoundRecord *rec = reinterpret_cast<const RoundRecord *>(sb.host.as<uint8_t>() + sb.records);
     for (size_t k = 0; k < nb; ++k) {
         emp_job *j = jobs[k];
         JobPrep &q = j->prep;
         j->st.ms_round_kernel += ms;  // the whole batch's launch
+        if (!j->h_records.ensure((size_t)q.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
+        std::memcpy(j->h_records.p, rec, (size_t)q.rounds * sizeof(RoundRecord));
+        rec += q.rounds;
         uint64_t needed = 0;
         emp_status r = hj[k].crowded ? kCrowded : bucket_collect(j, 0, 2 * q.U, hj[k], &needed);
         if (r == kNeedEdgeRoom || r == kCrowded) {
@@ -1491,13 +1513,11 @@ emp_status close_jobs(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaSt
             cudaEventRecord(jobs[i]->map_ev[3], s);
             cudaEventRecord(jobs[i]->map_ev[4], s);
         }
-        rc[i] = map_fetch(jobs[i], s);
     }
     EMP_CUDA(cudaStreamSynchronize(s));
     EMP_CUDA(cudaGetLastError());
     emp_status first = EMP_OK;
     for (int i = 0; i < n; ++i) {
-        if (rc[i] == EMP_OK) rc[i] = map_check(jobs[i]);
         if (rc[i] == EMP_OK) {
             job_finish(jobs[i]);
         } else {
@@ -1680,8 +1700,9 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
                 continue;
             }
             if (rc[i] == EMP_OK && !q.done && batch_eligible(j) && fits && !solo) {
-                rc[i] = rounds_prelude(j, s);
-                if (rc[i] == EMP_OK) rc[i] = bucket_prepare(j, s, job_env(j), 0, 0, 2 * q.U, q.ecap, 1u, &j->bk);
+                rounds_prelude(j);
+                whole_list(j, s);
+                rc[i] = bucket_prepare(j, s, job_env(j), 0, 0, 2 * q.U, q.ecap, 1u, &j->bk);
                 if (rc[i] == EMP_OK) {
                     joining.push_back(j);
                     continue;

@@ -10,7 +10,8 @@
 //
 //   hist     per-CTA shared-memory histogram of the key buckets (the top
 //            bits of fp1 scaled to nb buckets), added into global counts
-//   (scan)   bucket starts, copied to the bucket cursors
+//   scan     bucket starts and cursors (one CTA); the counts zeroed for the
+//            next call
 //   scatter  each (key, rid) to its bucket: a CTA ranks a tile of keys per
 //            bucket in shared memory and reserves each bucket's run with one
 //            atomic (up to 2048 buckets), or one atomic per run of equal
@@ -50,10 +51,33 @@ __global__ void __launch_bounds__(kDT) dedup_hist_kernel(const uint64_t *__restr
         if (s_hist[i]) atomicAdd(counts + i, s_hist[i]);
 }
 
-// cursor[b] = start[b] (the exclusive scan of the counts)
-__global__ void __launch_bounds__(kDT) dedup_cursor_kernel(const uint64_t *__restrict__ start, uint32_t nb,
-                                                           uint32_t *__restrict__ cursor) {
-    for (uint32_t b = blockIdx.x * kDT + threadIdx.x; b < nb; b += gridDim.x * kDT) cursor[b] = (uint32_t)start[b];
+// start[b] = cursor[b] = the exclusive scan of the counts (one CTA), which
+// are zeroed for the next call.
+constexpr int kScanT = 1024;
+__global__ void __launch_bounds__(kScanT) dedup_scan_kernel(uint32_t *__restrict__ counts, uint32_t nb,
+                                                            uint32_t *__restrict__ start,
+                                                            uint32_t *__restrict__ cursor) {
+    __shared__ uint32_t s_warp[32];
+    uint32_t run = 0;
+    for (uint32_t b0 = 0; b0 < nb; b0 += 4 * kScanT) {
+        uint32_t c[4], sum = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t b = b0 + 4 * threadIdx.x + q;
+            c[q] = b < nb ? counts[b] : 0u;
+            if (b < nb) counts[b] = 0;
+            sum += c[q];
+        }
+        uint32_t tot;
+        uint32_t x = run + block_exclusive_scan<kScanT, uint32_t>(sum, s_warp, &tot);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t b = b0 + 4 * threadIdx.x + q;
+            if (b < nb) start[b] = cursor[b] = x;
+            x += c[q];
+        }
+        run += tot;
+    }
 }
 
 __global__ void __launch_bounds__(kDT) dedup_scatter_kernel(const uint64_t *__restrict__ keys, uint64_t n,
@@ -127,7 +151,7 @@ constexpr size_t kMarkSmem = kDedupSlots * (8 + 4);
 
 __global__ void __launch_bounds__(kDT) dedup_mark_hash_kernel(const uint64_t *__restrict__ pk,
                                                               const uint32_t *__restrict__ pr,
-                                                              const uint64_t *__restrict__ start, uint32_t nb,
+                                                              const uint32_t *__restrict__ start, uint32_t nb,
                                                               uint64_t n, uint8_t *__restrict__ alive,
                                                               uint32_t *err) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -181,8 +205,6 @@ uint32_t dedup_buckets(uint64_t n) {
     return (uint32_t)(nb > kDedupMaxBuckets ? kDedupMaxBuckets : nb);
 }
 
-size_t dedup_scratch_bytes(uint32_t nb) { return (size_t)nb * (4 + 8 + 4) + 64; }
-
 // Shared-memory attributes of the kernels, set once per device.
 static bool dedup_setup(int &sms) {
     constexpr int kDevs = 64;
@@ -209,20 +231,16 @@ static bool dedup_setup(int &sms) {
 }
 
 bool launch_dedup_hash(const uint64_t *keys, uint64_t n, uint32_t nb, void *scratch, uint64_t *pk, uint32_t *pr,
-                       uint8_t *alive, uint64_t *status, uint32_t *tile_ctr, uint64_t *total, uint32_t *err,
-                       cudaStream_t s) {
+                       uint8_t *alive, uint32_t *err, cudaStream_t s) {
     int sms = 0;
     if (!n || !nb || !dedup_setup(sms)) return false;
     uint32_t *counts = reinterpret_cast<uint32_t *>(scratch);
-    uint64_t *start = reinterpret_cast<uint64_t *>(counts + ((nb + 1) & ~1u));
-    uint32_t *cursor = reinterpret_cast<uint32_t *>(start + nb);
-    cudaMemsetAsync(counts, 0, (size_t)nb * 4, s);
+    uint32_t *start = counts + kDedupMaxBuckets, *cursor = start + kDedupMaxBuckets;
     const uint64_t per = (n + kDT - 1) / kDT;
     const unsigned g_hist = (unsigned)(per < (uint64_t)sms * 4 ? per : (uint64_t)sms * 4);
     count_launch(4);
     dedup_hist_kernel<<<g_hist, kDT, nb * 4, s>>>(keys, n, nb, counts);
-    launch_scan_u32_u64(counts, start, nb, status, tile_ctr, total, err, s);
-    dedup_cursor_kernel<<<(nb + kDT - 1) / kDT, kDT, 0, s>>>(start, nb, cursor);
+    dedup_scan_kernel<<<1, kScanT, 0, s>>>(counts, nb, start, cursor);
     if (nb <= kTiledBuckets) {
         const uint64_t tiles = (n + kScatterTile - 1) / kScatterTile;
         const unsigned g_t = (unsigned)(tiles < (uint64_t)sms * 8 ? tiles : (uint64_t)sms * 8);

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kRT, 4) read_pass_kernel(const uint8_t *__rest
                                                         uint32_t *len_minmax, uint32_t *err) {
     extern __shared__ __align__(16) uint8_t read_smem[];
     ReadSmem &sm = *reinterpret_cast<ReadSmem *>(read_smem);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31;
     for (int i = tid; i < kChunks * 8; i += kRT) sm.chunk[i >> 3][i & 7] = weights->w[i >> 3][i & 7];
     for (int i = tid; i < (int)kRecCap; i += kRT) sm.end[i] = kNoEnd;  // each use resets its slots
     if (tid < 16) sm.win[tid >> 3][kWinWords + (tid & 7)] = 0;
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kRT, 4) read_pass_kernel(const uint8_t *__rest
     if (lane == 0) {
         if (kept) atomicAdd(reinterpret_cast<unsigned long long *>(n_kept), (unsigned long long)kept);
         if (lmax) {
-            atomicMin(len_minmax, lmin);
+            atomicMax(len_minmax, ~lmin);
             atomicMax(len_minmax + 1, lmax);
         }
         if (anybad) atomicOr(err, kErrBadBase);

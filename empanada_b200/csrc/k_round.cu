@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) init_list_kernel(const uint64_t *__restri
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[8];
     __shared__ uint64_t s_base;
-    if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
+    if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(tile_ctr, 1u) : 0u;
     __syncthreads();
     const uint32_t tile = s_tile;
     const uint64_t base = (uint64_t)tile * kUpdTile, n2 = 2 * n;
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256) update_compact_kernel(RoundArgs a) {
     __shared__ uint64_t s_base;
     __shared__ uint32_t s_sfx;
     if (threadIdx.x == 0) {
-        s_tile = atomicAdd(a.tile_ctr, 1u);
+        s_tile = gridDim.x > 1 ? atomicAdd(a.tile_ctr, 1u) : 0u;
         s_sfx = 0;
     }
     __syncthreads();
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) split_tables_kernel(const uint64_t *__res
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[8];
     __shared__ uint64_t s_base;
-    if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
+    if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(tile_ctr, 1u) : 0u;
     __syncthreads();
     const uint32_t tile = s_tile;
     const uint64_t base = (uint64_t)tile * kUpdTile;

@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(256) scan_kernel(const uint32_t *__restrict__ 
     __shared__ uint32_t s_tile;
     __shared__ uint64_t s_warp[8];
     __shared__ uint64_t s_base;
-    if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
+    if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(tile_ctr, 1u) : 0u;
     __syncthreads();
     const uint32_t tile = s_tile;
     const uint64_t base = (uint64_t)tile * kScanTile;

@@ -299,6 +299,8 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
     const uint32_t cnt = kPass != 2 && b == 0 ? lim : __ldcg(segcnt);
     const uint64_t e0 = (uint64_t)side0 + o;
     uint64_t *kin = J.key[l.cur], *kadv = J.key[l.cur ^ 1];
+    // the first step's prefixes may be the suffixes' entries, read from there
+    const bool half = kPfx && b == 0 && J.one_half;
     uint32_t *const T0 = J.T[0], *const T1 = J.T[1];
     const uint32_t *told = tg & 1u ? T1 : T0;
     uint32_t *const lval = J.val;
@@ -315,8 +317,8 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
         uint64_t key = 0;
         uint32_t val = 0;
         if (live) {
-            key = __ldcg(kin + e);
-            val = __ldcg(lval + e);
+            key = __ldcg(kin + (half ? e - side0 : e));
+            val = __ldcg(lval + (half ? e - side0 : e)) | (half ? 0x80000000u : 0u);
             if (kPass != 2) {
                 if (b) live = l.retry || t_round(__ldcg(told + e), tg) == kNever;
                 else if (host_used) live = used[val & 0x7fffffffu] == 0;
@@ -328,7 +330,7 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
             en = e0 + live_n + __popc(m & lanemask_lt_u32());
             live_n += __popc(m);
             __syncwarp();
-            if (live && en != e) {
+            if (live && (en != e || half)) {
                 lval[en] = val;
                 kin[en] = key;
             }
@@ -884,7 +886,7 @@ EMP_DEV void mark(SweepTrace &t, uint32_t phase, uint32_t b, const SweepJob *job
     ++t.n;
 }
 
-__global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *ctl, SweepOut go) {
+__global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *ctl, SweepOut go, int zero) {
     extern __shared__ __align__(16) uint8_t smem_all[];
     SShared &sh = *reinterpret_cast<SShared *>(smem_all);
     uint8_t *smem = smem_all + kSweepShared;
@@ -912,6 +914,16 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
     __syncthreads();
     SweepTrace tr{ctl, 0u};
     mark(tr, 0, 0, jobs, sh);
+    if (zero) {
+        const uint32_t total = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t { return (jobs[j].zeroed + 4 * kST - 1) / (4 * kST); });
+        for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
+            const int j = job_of(sh.pref, J, t);
+            uint4 *p = reinterpret_cast<uint4 *>(jobs[j].filter1);
+            const uint32_t lo = (t - sh.pref[j]) * 4 * kST, hi = min(lo + 4 * kST, jobs[j].zeroed);
+            for (uint32_t i = lo + tid; i < hi; i += kST) p[i] = make_uint4(0, 0, 0, 0);
+        }
+        if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
+    }
     uint32_t tg = 0;  // resolving iterations of the launch
     for (uint32_t b = 0;; ++b) {
         if (b && tid < J) next_step(jobs[tid], sh.loc[tid], b);
@@ -1085,6 +1097,7 @@ size_t sweep_layout(uint8_t *base, SweepJob *J, size_t *zeroed) {
     J->fs = reinterpret_cast<uint32_t *>(take((size_t)rounds * 4));
     J->fp = reinterpret_cast<uint32_t *>(take((size_t)rounds * 4));
     *zeroed = o;
+    J->zeroed = (uint32_t)(o / 16);
     J->groups = reinterpret_cast<SweepGroup *>(take(sizeof(SweepGroup) << gm));
     for (int k = 0; k < 2; ++k) J->T[k] = reinterpret_cast<uint32_t *>(take(n * 4));
     J->segcnt = reinterpret_cast<uint32_t *>(take((size_t)(J->segs_s + J->segs_p) * 4));
@@ -1151,11 +1164,12 @@ int sweep_grid_size() {
     return g - 1;
 }
 
-cudaError_t launch_sweep(SweepJob *jobs, CoopCtl *ctl, const SweepOut &go, cudaStream_t s) {
+cudaError_t launch_sweep(SweepJob *jobs, CoopCtl *ctl, const SweepOut &go, bool zero, cudaStream_t s) {
     const int grid = sweep_grid_size();
     if (grid <= 0) return cudaErrorNotSupported;
     SweepOut g = go;
-    void *args[] = {&jobs, &ctl, &g};
+    int z = zero ? 1 : 0;
+    void *args[] = {&jobs, &ctl, &g, &z};
     count_launch();
     return cudaLaunchCooperativeKernel((const void *)sweep_kernel, dim3(grid), dim3(kST), args, kSweepSmem, s);
 }

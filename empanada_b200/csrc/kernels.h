@@ -18,7 +18,7 @@ inline void count_launch(uint64_t k = 1) { g_launches.fetch_add(k, std::memory_o
 constexpr uint32_t kScanTile = 4096;  // u32 inputs per tile
 __host__ __device__ inline uint64_t scan_tiles(uint64_t n) { return (n + kScanTile - 1) / kScanTile; }
 // out[i] = sum(in[0..i)); *total = sum(in).  status: scan_tiles(n) u64,
-// tile_ctr: one u32; both must be zero.  out may alias in.
+// tile_ctr: one u32; both must be zero (more than one tile).  out may alias in.
 void launch_scan_u32_u64(const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *status, uint32_t *tile_ctr,
                          uint64_t *total, uint32_t *err, cudaStream_t s);
 void launch_scan_u32_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint64_t *status, uint32_t *tile_ctr,
@@ -34,8 +34,9 @@ void launch_nl_count(const uint8_t *fq, uint64_t F, uint32_t *tile_counts, uint6
 // keep[k] = 1 iff the record's sequence line holds no N-class byte and is not
 // empty; keys[2k] / keys[2k+1] = fingerprint of its read / of the reverse
 // complement, seq2[k * wpr + w] = its bases 16w .. 16w+15 (2 bits each, zero
-// past the read); *n_kept += the kept count (start it at 0), the kept reads'
-// length extremes in len_minmax, kErrBadBase in *err.  Reads longer than
+// past the read); *n_kept += the kept count (start it at 0), the complement of
+// the kept reads' shortest length and the longest in len_minmax (maxima; start
+// them at 0), kErrBadBase in *err.  Reads longer than
 // kMaxReadLen are classified but not hashed.
 void launch_read_pass(const uint8_t *fq, uint64_t F, const uint64_t *tile_excl, const HashTables *tables,
                       const ChunkWeights *weights, uint64_t *keys, uint32_t *seq2, int wpr, uint32_t *keep,
@@ -50,18 +51,17 @@ void launch_columns(const uint32_t *seq2, uint64_t n, int L, int wpr, uint32_t *
 // ---- duplicate removal without a sort (k_dedup.cu) -------------------------
 // alive[e] = 1 iff read-end e has the smallest rid of its fingerprint (the
 // survivor of the reference's in-core sort + unique).  nb key buckets from
-// dedup_buckets(n) (0: use the sort); scratch: dedup_scratch_bytes(nb);
-// pk/pr: n pairs of room; status: scan_tiles(nb) zeroed look-back words,
-// *tile_ctr zeroed.  kErrDedupFull in *err: a bucket overflowed, use the sort.
-// Returns false when the kernels cannot run on this device.
+// dedup_buckets(n) (0: use the sort); scratch: kDedupScratch bytes, zeroed
+// once (each call leaves it ready for the next); pk/pr: n pairs of room.
+// kErrDedupFull in *err: a bucket overflowed, use the sort.  Returns false
+// when the kernels cannot run on this device.
 constexpr uint32_t kDedupMean = 4096;
 constexpr uint32_t kDedupMaxBuckets = 16384;
 constexpr uint64_t kDedupMaxEnds = (uint64_t)kDedupMaxBuckets * 6000;
+constexpr size_t kDedupScratch = (size_t)kDedupMaxBuckets * (4 + 4 + 4);  // counts, starts, cursors
 uint32_t dedup_buckets(uint64_t n);
-size_t dedup_scratch_bytes(uint32_t nb);
 bool launch_dedup_hash(const uint64_t *keys, uint64_t n, uint32_t nb, void *scratch, uint64_t *pk, uint32_t *pr,
-                       uint8_t *alive, uint64_t *status, uint32_t *tile_ctr, uint64_t *total, uint32_t *err,
-                       cudaStream_t s);
+                       uint8_t *alive, uint32_t *err, cudaStream_t s);
 
 // ---- unitigs of the overlap graph (k_graph.cu) ----------------------------
 // Device arrays of a graph's build, per node (nodes = 2n): succ/pred, jump
@@ -355,6 +355,7 @@ struct SweepJob {
     RoundRecord *records;    // [rounds]
     // work memory (sweep_layout)
     uint32_t w1_max;         // log2 words of filter 1
+    uint32_t zeroed;         // bytes to be zero at the start, in units of 16
     uint32_t gm_max;         // log2 group slots
     uint32_t segs_s, segs_p;
     uint32_t *filter1, *filter2;  // zero between steps
@@ -379,6 +380,7 @@ struct SweepJob {
     uint32_t crowded;        // a group of too many entries: not a job for this kernel (zero at launch)
     uint64_t e_total;        // edges
     uint8_t cur0;
+    uint8_t one_half;        // the list at launch holds the suffixes only: the prefixes are the same entries
 };
 struct SweepOut {  // output bins of a launch's jobs (sweep_out_layout)
     uint32_t *chg;    // [3][kSweepIters]: whether an iteration changed something
@@ -396,7 +398,9 @@ uint32_t sweep_segment_size(uint64_t entries_per_side);
 uint32_t sweep_bins_max(uint64_t n_in, int rounds);
 size_t sweep_layout(uint8_t *base, SweepJob *job, size_t *zeroed);
 size_t sweep_out_layout(uint8_t *base, uint32_t bins, SweepOut *go, size_t *zeroed);
-cudaError_t launch_sweep(SweepJob *jobs, CoopCtl *ctl, const SweepOut &go, cudaStream_t s);
+// zero: the launch itself zeroes the jobs' memory (their first `zeroed` bytes
+// from filter1), else the caller has.
+cudaError_t launch_sweep(SweepJob *jobs, CoopCtl *ctl, const SweepOut &go, bool zero, cudaStream_t s);
 
 void launch_join_count(const uint64_t *skeys, const uint32_t *svals, uint64_t n, uint32_t *cnt, cudaStream_t s);
 void launch_join_write(const uint64_t *skeys, const uint32_t *svals, uint64_t n, const uint32_t *cnt,
