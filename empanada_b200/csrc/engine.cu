@@ -1393,6 +1393,13 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     sweep_out_layout(sb.out.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
     EMP_CUDA(cudaMemsetAsync(sb.out.p, 0, zeroed, s));
     coop_ctl_init(ctx, hc, (uint32_t)nb);
+    if (!ctx->trace_path.empty()) {
+        emp_job *j = jobs[0];
+        EMP_TRY(ensure(j, j->coop_trace, (size_t)kSweepTraceCap * kCoopTracePhases * 8));
+        EMP_CUDA(cudaMemsetAsync(j->coop_trace.p, 0, j->coop_trace.bytes, s));
+        hc->trace = j->coop_trace.as<uint64_t>();
+        hc->trace_cap = kSweepTraceCap;
+    }
     EMP_CUDA(cudaMemcpyAsync(dj, hj, nb * sizeof(SweepJob) + sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
     EMP_CUDA(cudaEventRecord(sb.ev[0], s));
     EMP_CUDA(launch_sweep(dj, dc, go, true, s));
@@ -1409,6 +1416,7 @@ emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &job
     const SweepJob *hj = sb.host.as<SweepJob>();
     if (reinterpret_cast<const CoopCtl *>(hj + nb)->err & kErrSpin) return EMP_E_TIMEOUT;
     const float ms = ms_between(sb.ev[0], sb.ev[1]);
+    if (nb && !jobs[0]->ctx->trace_path.empty()) write_sweep_trace(jobs[0], jobs[0]->ctx->trace_path.c_str(), s);
     const RoundRecord *rec = reinterpret_cast<const RoundRecord *>(sb.host.as<uint8_t>() + sb.records);
     for (size_t k = 0; k < nb; ++k) {
         emp_job *j = jobs[k];

@@ -362,6 +362,7 @@ struct SweepJob {
     SweepCtr *ctr;           // [3]: step b uses ctr[b % 3]
     uint32_t *fs, *fp;       // [round]: suffixes / prefixes matched
     SweepGroup *groups;      // those of the step, empty between steps
+    uint64_t *bases;         // each suffix's bases of the step, 2 bits a round
     uint32_t *T[2];          // [iteration % 2][entry]: round of the step that uses it
     uint32_t *segcnt;        // live entries of each segment, suffixes then prefixes
     uint4 *pcand;            // prefix candidates: value, entry, the group's next one, group
