@@ -63,9 +63,9 @@ struct SweepLoc {  // a job's step, the same in every CTA
     uint32_t r;          // first round of this step
     uint32_t R;          // rounds of this step
     uint32_t ls, lp;     // live suffixes and prefixes at its start
+    uint32_t w1, w2;     // words of the two filters
     uint8_t act;         // the job runs this step
     uint8_t cur;         // key array that holds the keys of round r - 1
-    uint8_t w1, w2;      // log2 of the two filters' words
     uint8_t gm, gclean;  // log2 of the group slots in use, and of those emptied so far
     uint8_t retry;       // the step before did not fit: its rounds again
 };
@@ -136,12 +136,12 @@ EMP_DEV uint32_t kq_f1(uint64_t k) { return (uint32_t)(k >> 35); }
 EMP_DEV uint32_t kq_f2(uint64_t k) { return (uint32_t)(k >> 6) & kMask29; }
 EMP_DEV uint32_t kq_q(uint64_t k) { return (uint32_t)k & 63u; }
 
-// word and bits of (key, round) in a filter of 2^log words
+// word and bits of (key, round) in a filter of `words` words
 EMP_DEV uint32_t filter_mix(uint32_t f1, uint32_t f2, uint32_t q) {
     uint32_t h = f1 * 0x9E3779B1u + f2 * 0x85EBCA77u + q * 0xC2B2AE3Du;
     return h ^ (h >> 15);
 }
-EMP_DEV uint32_t filter_word(uint32_t h, uint32_t log) { return (h * 0x2C1B3C6Du) >> (32 - log); }
+EMP_DEV uint32_t filter_word(uint32_t h, uint32_t words) { return __umulhi(h * 0x2C1B3C6Du, words); }
 EMP_DEV uint32_t filter_bits3(uint32_t h) {
     const uint32_t g = h * 0x297A2D39u;
     return (1u << (g >> 27)) | (1u << ((g >> 22) & 31u)) | (1u << ((g >> 17) & 31u));
@@ -315,7 +315,7 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
     uint32_t *const lval = J.val;
     const uint8_t *used = kPfx ? J.used_p : J.used_s;
     uint32_t *const filter = kPass == 2 ? J.filter2 : J.filter1;
-    const uint32_t log = kPass == 2 ? l.w2 : l.w1, R = l.R, len0 = (uint32_t)J.L - l.r - 1u;
+    const uint32_t words = kPass == 2 ? l.w2 : l.w1, R = l.R, len0 = (uint32_t)J.L - l.r - 1u;
     const uint32_t inv1 = J.tables->inv1, inv2 = J.tables->inv2;
     const bool host_used = J.r0 > 0;
     uint64_t *const win = J.bases + o;  // the suffixes' bases of the step, from pass A to pass C
@@ -377,8 +377,8 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
                     g2[u] = f2;
                     if (live) {
                         const uint32_t h = filter_mix(f1, f2, q);
-                        if (kPass == 0) red_or(filter + filter_word(h, log), filter_bits3(h));
-                        else fw[u] = __ldcg(filter + filter_word(h, log));
+                        if (kPass == 0) red_or(filter + filter_word(h, words), filter_bits3(h));
+                        else fw[u] = __ldcg(filter + filter_word(h, words));
                     }
                 }
             }
@@ -560,15 +560,15 @@ EMP_DEV void clear_filters(SweepJob *jobs, int J, SShared &sh) {
     constexpr uint32_t kWords = kST * 16;  // per tile: four 16-byte stores a thread
     const uint32_t total = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t {
         const SweepLoc &l = sh.loc[j];
-        return l.act ? ((1u << l.w1) + kWords - 1) / kWords + ((1u << l.w2) + kWords - 1) / kWords : 0u;
+        return l.act ? (l.w1 + kWords - 1) / kWords + (l.w2 + kWords - 1) / kWords : 0u;
     });
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const int j = job_of(sh.pref, J, t);
         const SweepLoc &l = sh.loc[j];
         uint32_t k = t - sh.pref[j];
-        const uint32_t t1 = ((1u << l.w1) + kWords - 1) / kWords;
+        const uint32_t t1 = (l.w1 + kWords - 1) / kWords;
         uint32_t *f = k < t1 ? jobs[j].filter1 : jobs[j].filter2;
-        const uint32_t words = k < t1 ? 1u << l.w1 : 1u << l.w2;
+        const uint32_t words = k < t1 ? l.w1 : l.w2;
         if (k >= t1) k -= t1;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -878,12 +878,10 @@ EMP_DEV void next_step(SweepJob &J, SweepLoc &l, uint32_t b) {
 EMP_DEV void size_filters(const SweepJob &J, SweepLoc &l, uint64_t all) {
     const uint64_t cap = all ? kFilterKeys / all : 1;
     if (l.R > cap) l.R = cap < 1 ? 1u : (uint32_t)cap;
-    const uint64_t most = (uint64_t)1 << (J.w1_max + 2);  // 8 bits per key where the filter's memory ends
-    while (l.R > 1 && (uint64_t)l.ls * l.R > most) l.R = (l.R + 1) / 2;
-    uint32_t w = pow2_log(((uint64_t)l.ls * l.R + 1) / 2);  // 16 bits per (entry, round)
-    w = w < 10 ? 10u : w;
-    l.w1 = (uint8_t)(w < J.w1_max ? w : J.w1_max);
-    l.w2 = (uint8_t)(l.w1 > 12 ? l.w1 - 2 : 10);
+    while (l.R > 1 && (uint64_t)l.ls * l.R > 4ull * J.w1_max) l.R = (l.R + 1) / 2;  // 8 bits per key where memory ends
+    const uint64_t w = ((uint64_t)l.ls * l.R + 1) / 2;  // 16 bits per (entry, round)
+    l.w1 = (uint32_t)(w < 1024 ? 1024 : w < J.w1_max ? (w + 3) / 4 * 4 : J.w1_max);
+    l.w2 = l.w1 > 4096 ? (l.w1 / 4 + 3) / 4 * 4 : 1024;
 }
 
 // Profiling aid: at the end of a phase, (phase | step << 8, job 0's first
@@ -1100,17 +1098,16 @@ size_t sweep_layout(uint8_t *base, SweepJob *J, size_t *zeroed) {
     };
     const uint64_t ns = J->n_s, np = J->n_p, n = ns + np;
     const int rounds = J->rounds;
-    // filter 1 holds four rounds of every suffix at 16 bits each
-    uint32_t w1 = 10;
-    while (w1 < 24 && (1ull << w1) < 2 * ns) ++w1;
-    J->w1_max = w1;
+    // filter 1 holds eight rounds of every suffix at 16 bits each
+    const uint64_t w1 = ns < 256 ? 1024 : 4 * ns < (1u << 24) ? 4 * ns : 1u << 24;
+    J->w1_max = (uint32_t)w1;
     uint32_t gm = 10;
     while ((1ull << gm) < np + np / 4) ++gm;
     J->gm_max = gm;
     J->segs_s = (uint32_t)((ns + J->seg - 1) / J->seg);
     J->segs_p = (uint32_t)((np + J->seg - 1) / J->seg);
-    J->filter1 = reinterpret_cast<uint32_t *>(take((size_t)4 << w1));
-    J->filter2 = reinterpret_cast<uint32_t *>(take((size_t)4 << (w1 > 12 ? w1 - 2 : 10)));
+    J->filter1 = reinterpret_cast<uint32_t *>(take((size_t)4 * w1));
+    J->filter2 = reinterpret_cast<uint32_t *>(take((size_t)4 * (w1 > 4096 ? w1 / 4 + 4 : 1024)));
     J->ctr = reinterpret_cast<SweepCtr *>(take(3 * sizeof(SweepCtr)));
     J->fs = reinterpret_cast<uint32_t *>(take((size_t)rounds * 4));
     J->fp = reinterpret_cast<uint32_t *>(take((size_t)rounds * 4));

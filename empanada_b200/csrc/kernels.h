@@ -354,7 +354,7 @@ struct SweepJob {
     uint8_t *out;            // output.bin records (12 * rounds + 8 * ecap bytes)
     RoundRecord *records;    // [rounds]
     // work memory (sweep_layout)
-    uint32_t w1_max;         // log2 words of filter 1
+    uint32_t w1_max;         // words of filter 1
     uint32_t zeroed;         // bytes to be zero at the start, in units of 16
     uint32_t gm_max;         // log2 group slots
     uint32_t segs_s, segs_p;
