@@ -28,6 +28,7 @@
 #include <sys/stat.h>
 
 #include "../../include/empanada.h"
+#include "hostcopy.h"
 #include "ingest.h"
 #include "kernels.h"
 
@@ -170,6 +171,7 @@ struct emp_ctx {
     uint64_t sort_cap = 0;
     uint64_t sort_calls = 0;
     HostSlab slab;
+    HostStage stage;                  // pageable copies
     std::vector<emp_graph *> graphs;  // those whose arrays lie in the pool
     // emp_batch_run: the BktJob array and control block of one launch, their
     // host copies, and the launch's events
@@ -2159,7 +2161,10 @@ static emp_status feed(emp_job *job, const void *src, uint64_t n, int last, cuda
         cudaEventCreate(&a);
         cudaEventCreate(&b);
         cudaEventRecord(a, job->ctx->stream);
-        cudaError_t e = cudaMemcpyAsync(job->fq.as<uint8_t>() + job->F, src, n, kind, job->ctx->stream);
+        cudaError_t e = kind == cudaMemcpyHostToDevice
+                            ? job->ctx->stage.to_device(job->ctx->device, job->fq.as<uint8_t>() + job->F, src, n,
+                                                        job->ctx->stream)
+                            : cudaMemcpyAsync(job->fq.as<uint8_t>() + job->F, src, n, kind, job->ctx->stream);
         cudaEventRecord(b, job->ctx->stream);
         cudaError_t e2 = cudaStreamSynchronize(job->ctx->stream);
         if (kind == cudaMemcpyHostToDevice) job->ms_h2d += ms_between(a, b);
@@ -2379,8 +2384,8 @@ emp_status emp_job_output_copy(emp_job *job, void *dst, uint64_t cap) {
     if (host) std::memcpy(dst, job->out.data(), host);
     if (job->dout_bytes) {  // records of the device-resident rounds follow those of the host-driven ones
         cudaSetDevice(job->ctx->device);
-        if (cudaMemcpy(static_cast<uint8_t *>(dst) + host, job->dout.p, job->dout_bytes, cudaMemcpyDeviceToHost) !=
-            cudaSuccess) {
+        if (job->ctx->stage.to_host(job->ctx->device, static_cast<uint8_t *>(dst) + host, job->dout.p,
+                                    job->dout_bytes) != cudaSuccess) {
             cudaGetLastError();
             return EMP_E_CUDA;
         }
@@ -2441,7 +2446,7 @@ emp_status emp_job_fingerprints(emp_job *job, uint64_t *keys, uint64_t cap, uint
     if (!job->n_ends || (!keys && cap == 0)) return EMP_OK;  // size query
     if (!keys || cap < job->n_ends) return EMP_E_INVAL;
     cudaSetDevice(job->ctx->device);
-    if (cudaMemcpy(keys, job->keys0.p, job->n_ends * 8, cudaMemcpyDeviceToHost) != cudaSuccess) return EMP_E_CUDA;
+    if (job->ctx->stage.to_host(job->ctx->device, keys, job->keys0.p, job->n_ends * 8) != cudaSuccess) return EMP_E_CUDA;
     return EMP_OK;
 }
 
@@ -2613,9 +2618,11 @@ emp_status graph_to_host(emp_graph *g) {
         g->order.clear();
         return EMP_E_NOMEM;
     }
-    if ((g->bytes && cudaMemcpy(g->bin.data(), g->d_bin, g->bytes, cudaMemcpyDeviceToHost) != cudaSuccess) ||
-        cudaMemcpy(g->starts.data(), g->d_starts, (g->unitigs + 1) * 8, cudaMemcpyDeviceToHost) != cudaSuccess ||
-        cudaMemcpy(g->order.data(), g->d_order, g->nodes * 4, cudaMemcpyDeviceToHost) != cudaSuccess) {
+    HostStage &st = g->ctx->stage;
+    const int dev = g->ctx->device;
+    if ((g->bytes && st.to_host(dev, g->bin.data(), g->d_bin, g->bytes) != cudaSuccess) ||
+        st.to_host(dev, g->starts.data(), g->d_starts, (g->unitigs + 1) * 8) != cudaSuccess ||
+        st.to_host(dev, g->order.data(), g->d_order, g->nodes * 4) != cudaSuccess) {
         cudaGetLastError();
         g->order.clear();
         return EMP_E_CUDA;
@@ -2728,7 +2735,7 @@ emp_status emp_graph_build(emp_ctx *ctx, const void *output_bin, uint64_t bytes,
     if (cudaEventCreate(&ev[0]) != cudaSuccess || cudaEventCreate(&ev[1]) != cudaSuccess) rc = EMP_E_CUDA;
     if (rc == EMP_OK) {
         cudaEventRecord(ev[0], s);
-        if (bytes) cudaMemcpyAsync(k + o_bin, b, bytes, cudaMemcpyHostToDevice, s);
+        if (bytes) ctx->stage.to_device(ctx->device, k + o_bin, b, bytes, s);
         if (nrec) cudaMemcpyAsync(d + o_roff, g->rec_off.data(), nrec * 8, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(d + o_e0, e0.data(), (nrec + 1) * 8, cudaMemcpyHostToDevice, s);
         cudaMemsetAsync(gb.status, 0, 2 * scan_t * 8, s);
@@ -2787,8 +2794,9 @@ emp_status emp_graph_unitigs(emp_graph *g, uint32_t *order, uint64_t order_cap, 
         return EMP_OK;
     }
     cudaSetDevice(g->ctx->device);
-    if ((order && cudaMemcpy(order, g->d_order, g->nodes * 4, cudaMemcpyDeviceToHost) != cudaSuccess) ||
-        (starts && cudaMemcpy(starts, g->d_starts, (g->unitigs + 1) * 8, cudaMemcpyDeviceToHost) != cudaSuccess)) {
+    emp_ctx *c = g->ctx;
+    if ((order && c->stage.to_host(c->device, order, g->d_order, g->nodes * 4) != cudaSuccess) ||
+        (starts && c->stage.to_host(c->device, starts, g->d_starts, (g->unitigs + 1) * 8) != cudaSuccess)) {
         cudaGetLastError();
         return EMP_E_CUDA;
     }
