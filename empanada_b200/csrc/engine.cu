@@ -856,10 +856,11 @@ bool sweep_rounds_usable(const emp_job *j, uint64_t n) {
 }
 
 // Buffers and launch description (host copy *hj) of rounds r0 .. of one job
-// in the sweep kernel: the list lk[cur] holds ns suffixes, then np prefixes.
+// in the sweep kernel: the list lk[cur] holds ns suffixes, then np prefixes;
+// side: the suffixes (or prefixes, if more) of all jobs of the launch.
 // The launch overwrites the list.
 emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t ns, uint64_t np,
-                         uint64_t ecap, uint32_t seg, SweepJob *hj) {
+                         uint64_t ecap, uint64_t side, SweepJob *hj) {
     std::memset(hj, 0, sizeof(SweepJob));
     hj->key[0] = j->lk0.as<uint64_t>();
     hj->key[1] = j->lk1.as<uint64_t>();
@@ -869,7 +870,8 @@ emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0
     hj->used_p = j->used_p.as<uint8_t>();
     hj->n_s = (uint32_t)ns;
     hj->n_p = (uint32_t)np;
-    hj->seg = seg;
+    hj->seg = sweep_segment_size(side);
+    hj->shard_log = sweep_shard_log(np, side);
     hj->L = env.L;
     hj->rounds = env.rounds;
     hj->r0 = r0;
@@ -898,7 +900,7 @@ emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int
     uint8_t *dev = j->coop_ctl.as<uint8_t>();
     SweepJob *hj = j->h_coop.as<SweepJob>(), *dj = reinterpret_cast<SweepJob *>(dev);
     CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + 1), *dc = reinterpret_cast<CoopCtl *>(dj + 1);
-    EMP_TRY(sweep_prepare(j, s, env, r0, cur, ns, np, ecap, sweep_segment_size(std::max(ns, np)), hj));
+    EMP_TRY(sweep_prepare(j, s, env, r0, cur, ns, np, ecap, std::max(ns, np), hj));
     hj->records = reinterpret_cast<RoundRecord *>(dev + kRec);
     EMP_CUDA(cudaMemsetAsync(j->swp.p, 0, (size_t)hj->zeroed * 16, s));
     SweepOut go{};
@@ -1380,12 +1382,11 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     SweepJob *hj = sb.host.as<SweepJob>(), *dj = sb.jobs.as<SweepJob>();
     CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + nb), *dc = reinterpret_cast<CoopCtl *>(dj + nb);
     RoundRecord *rec = reinterpret_cast<RoundRecord *>(sb.jobs.as<uint8_t>() + sb.records);
-    const uint32_t seg = sweep_segment_size(side);
     for (size_t k = 0; k < nb; ++k) {
         emp_job *j = jobs[k];
         const JobPrep &q = j->prep;
         rounds_prelude(j);
-        EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, seg, &hj[k]));
+        EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, side, &hj[k]));
         hj[k].records = rec;
         rec += q.rounds;
     }

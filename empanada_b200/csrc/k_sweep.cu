@@ -8,11 +8,11 @@
 //   A  every live suffix: its keys of the R rounds (NextSfx, overlap.cu:57-75)
 //      into a Bloom filter (one 32-bit word, three bits per (round, key))
 //   B  every live prefix: its R keys (PrevPfx, overlap.cu:77-91) against that
-//      filter; a hit is a candidate: it enters a hash table of (key, round)
-//      groups and a second, small filter
+//      filter; a hit is a candidate: it enters a chain of its (key, round)'s
+//      hash and a second, small filter
 //   C  every live suffix again: its keys against the second filter, then the
-//      hash table; a suffix whose key is there makes a pair (suffix, prefix,
-//      round) with each prefix of the group from another read (get_edges,
+//      the chain; a suffix whose key is there makes a pair (suffix, prefix,
+//      round) with each prefix of that key from another read (get_edges,
 //      overlap.cu:557-603)
 //   resolve  no entry was removed inside the step, so a pair may hold entries
 //      that an earlier round of the step uses (remove_used, overlap.cu:694-710).
@@ -39,7 +39,7 @@
 // per round, and a grid barrier is paid per phase of a step of up to 32
 // rounds.  Bound: random L2 accesses (measured on this chip 188 G/s for a
 // reduction, 276 G/s for a load, 121 G/s for a compare-and-swap, a sixth of
-// that beyond 64 MB), which is why the filters and groups of a step are kept
+// that beyond 64 MB), which is why the filters and chains of a step are kept
 // within L2 (kFilterKeys).  All rounds, bucket kernel -> here: 2,000 x 100
 // reads 1.16 -> 0.29 ms, 100k x 150 1.90 -> 0.53, 1.2M x 250 8.03 -> 4.0,
 // 256 sets (13.2M reads) 71 -> 37 ms.
@@ -52,7 +52,6 @@ namespace {
 constexpr int kST = kSweepThreads;      // 1024: one CTA per SM
 constexpr int kSW = kST / 32;
 constexpr uint32_t kNever = 0xffffffffu;
-constexpr uint64_t kNoGroup = ~0ull;    // empty slot of the group table
 constexpr uint64_t kFilterKeys = 25u << 20;  // (entry, round) keys of a step's first filters: 48 MB, within L2
 constexpr uint32_t kU = 4;              // filter accesses of a lane in flight
 constexpr uint32_t kQCap = 32 * (kU + 1);  // queued candidates per warp
@@ -64,9 +63,11 @@ struct SweepLoc {  // a job's step, the same in every CTA
     uint32_t R;          // rounds of this step
     uint32_t ls, lp;     // live suffixes and prefixes at its start
     uint32_t w1, w2;     // words of the two filters
+    uint32_t cands;      // prefix candidates that the step found
+    uint32_t pc, pairs;  // places up to the last one given to a candidate and a pair
     uint8_t act;         // the job runs this step
     uint8_t cur;         // key array that holds the keys of round r - 1
-    uint8_t gm, gclean;  // log2 of the group slots in use, and of those emptied so far
+    uint8_t gm, gclean;  // log2 of the chain heads in use, and of those emptied so far
     uint8_t retry;       // the step before did not fit: its rounds again
 };
 
@@ -168,6 +169,14 @@ EMP_DEV uint64_t step_bases(const SweepJob &J, uint32_t val, uint32_t r, uint32_
     return s ? x ^ 0xAAAAAAAAAAAAAAAAull : x;  // the complement's codes
 }
 
+// the line of the first of them on its way
+EMP_DEV void prefetch_bases(const SweepJob &J, uint32_t val, uint32_t r, uint32_t R) {
+    const bool inc = val >> 31 == (val & 1u);
+    const uint32_t start = inc ? r : (uint32_t)J.L - r - R;
+    const uint32_t *row = J.seq2 + (uint64_t)((val & 0x7fffffffu) >> 1) * J.wpr + (start >> 4);
+    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(__cvta_generic_to_global(row)));
+}
+
 // NextSfx on the two fingerprints: t = (enc * R^(len - 1)) mod P of both
 EMP_DEV void step_sfx(uint32_t &f1, uint32_t &f2, uint2 t) {
     f1 = f1 >= t.x ? f1 - t.x : f1 + kP1 - t.x;
@@ -179,31 +188,23 @@ EMP_DEV void step_pfx(uint32_t &f1, uint32_t &f2, uint32_t v, uint32_t inv1, uin
     f2 = (uint32_t)k;
 }
 
-// ---------------------------------------------------------------- groups
-// slot of a group: (key, round), the last prefix candidate that entered it
-EMP_DEV uint32_t group_hash(uint64_t k, uint32_t mask) { return (uint32_t)((k * 0x9E3779B97F4A7C15ull) >> 32) & mask; }
-EMP_DEV uint32_t group_insert(SweepGroup *gr, uint32_t mask, uint64_t k) {
-    uint32_t s = group_hash(k, mask);
-    for (uint32_t probes = 0; probes <= mask; ++probes) {
-        const uint64_t old = atomicCAS(reinterpret_cast<unsigned long long *>(&gr[s].key), (unsigned long long)kNoGroup,
-                                       (unsigned long long)k);
-        if (old == kNoGroup || old == k) return s;
-        s = (s + 1) & mask;
-    }
-    return kNever;
+// ---------------------------------------------------------------- candidates
+// chain of (key, round): the last candidate that entered it is the head
+EMP_DEV uint32_t chain_hash(uint64_t k, uint32_t mask) { return (uint32_t)((k * 0x9E3779B97F4A7C15ull) >> 32) & mask; }
+
+// Places of a step's candidates and pairs are handed out by 2^shard_log
+// counters (all warps of the grid reach their flushes about together, and one
+// counter takes 0.71 ns for each).  Runs of 32 places go round the counters,
+// so that what a warp writes at once stays together.
+EMP_DEV uint32_t shard_of(const SweepJob &J) { return blockIdx.x & ((1u << J.shard_log) - 1u); }
+EMP_DEV uint32_t place(const SweepJob &J, uint32_t k, uint32_t p) {  // place p of counter k
+    return (((p >> 5) << J.shard_log | k) << 5) | (p & 31u);
 }
-// the group's last prefix candidate; kNever: no such group
-EMP_DEV uint32_t group_find(const SweepGroup *gr, uint32_t mask, uint64_t k) {
-    uint32_t s = group_hash(k, mask);
-    for (uint32_t probes = 0; probes <= mask; ++probes) {
-        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(gr + s));
-        const uint64_t h = (uint64_t)v.x | ((uint64_t)v.y << 32);
-        if (h == k) return v.z;
-        if (h == kNoGroup) return kNever;
-        s = (s + 1) & mask;
-    }
-    return kNever;
+// whether place x has been given out; n: the counter that gives it
+EMP_DEV const SweepShard &shard_at(const SweepJob &J, const SweepCtr &c, uint32_t x) {
+    return c.shard[(x >> 5) & ((1u << J.shard_log) - 1u)];
 }
+EMP_DEV bool given(const SweepJob &J, uint32_t x, uint32_t n) { return (((x >> 5) >> J.shard_log) << 5 | (x & 31u)) < n; }
 
 // T of iteration tg (numbered through the launch): word = (number
 // complemented, 26 bits | round, 6 bits), so that atomicMin prefers the newer
@@ -224,36 +225,32 @@ EMP_DEV void queue_push(Queue &w, bool f, uint64_t kq, uint32_t e, uint32_t val)
     w.n += __popc(m);
 }
 
-// up to 32 queued prefixes -> candidates, groups, second filter
+// up to 32 queued prefixes -> candidates, chains, second filter
 EMP_DEV void flush_prefixes(SweepJob &J, SweepCtr &c, Queue &w, const SweepLoc &l) {
     const uint32_t lane = threadIdx.x & 31, n = w.n < 32u ? w.n : 32u;
     __syncwarp();
     const uint32_t at = w.n - n;
     uint32_t pos = 0;
-    if (lane == 0) pos = atomicAdd(&c.pc, n);
-    pos = __shfl_sync(0xffffffffu, pos, 0) + lane;
+    if (lane == 0) pos = atomicAdd(&c.shard[shard_of(J)].pc, n);
+    pos = place(J, shard_of(J), __shfl_sync(0xffffffffu, pos, 0) + lane);
     if (lane < n) {
         const uint4 x = w.q[at + lane];
-        const uint64_t kq = (uint64_t)x.x | ((uint64_t)x.y << 32);
-        const uint32_t slots = 1u << l.gm;
-        uint32_t g = kNever, prev = kNever;
-        if (pos < J.n_p && (pos < slots - slots / 4 || l.gm == J.gm_max)) {
-            g = group_insert(J.groups, slots - 1, kq);
-            if (g != kNever) {
-                prev = atomicExch(&J.groups[g].head, pos);
-                const uint32_t h = filter_mix(kq_f1(kq), kq_f2(kq), kq_q(kq));
-                red_or(J.filter2 + filter_word(h, l.w2), filter_bits3(h));
-            }
+        if (pos < J.p_cap) {
+            const uint64_t kq = (uint64_t)x.x | ((uint64_t)x.y << 32);
+            const uint32_t next = atomicExch(J.heads + chain_hash(kq, (1u << l.gm) - 1u), pos);
+            const uint32_t h = filter_mix(kq_f1(kq), kq_f2(kq), kq_q(kq));
+            red_or(J.filter2 + filter_word(h, l.w2), filter_bits3(h));
+            J.pcand[pos] = make_uint4(x.x, x.y, x.z, next);
+        } else {
+            c.ovf = 1;
         }
-        if (pos < J.n_p) J.pcand[pos] = make_uint4(x.w, x.z, prev, g);
-        if (g == kNever) c.ovf = 1;
     }
     w.n = at;
     __syncwarp();
 }
 
-// up to 32 queued suffixes -> a pair with every prefix of another read in the
-// group of their key; the step's first T (nothing removed yet) from the pairs
+// up to 32 queued suffixes -> a pair with every prefix of another read with
+// their key; the step's first T (nothing removed yet) from the pairs
 EMP_DEV void flush_suffixes(SweepJob &J, SweepCtr &c, Queue &w, const SweepLoc &l, uint32_t tg) {
     const uint32_t lane = threadIdx.x & 31, n = w.n < 32u ? w.n : 32u;
     __syncwarp();
@@ -262,29 +259,34 @@ EMP_DEV void flush_suffixes(SweepJob &J, SweepCtr &c, Queue &w, const SweepLoc &
     uint32_t p = kNever;
     if (lane < n) {
         x = w.q[at + lane];
-        p = group_find(J.groups, (1u << l.gm) - 1, (uint64_t)x.x | ((uint64_t)x.y << 32));
+        p = __ldcg(J.heads + chain_hash((uint64_t)x.x | ((uint64_t)x.y << 32), (1u << l.gm) - 1u));
     }
     uint32_t *const T = J.T[tg & 1u];
-    const uint32_t walk = l.R > 1 ? 64u : 4096u, cap = J.n_s + J.n_p, t = t_word(tg, x.x & 63u);
+    const uint32_t walk = l.R > 1 ? 64u : 4096u, t = t_word(tg, x.x & 63u);
     for (uint32_t k = 0; __any_sync(0xffffffffu, p != kNever); ++k) {
-        uint4 y = make_uint4(0, 0, kNever, 0);
+        uint4 y = make_uint4(0, 0, 0, kNever);
         if (p != kNever) y = __ldcg(J.pcand + p);
-        const bool pair = p != kNever && ((y.x ^ x.w) & 0x7ffffffeu) != 0;
+        bool pair = p != kNever && y.x == x.x && y.y == x.y;
+        uint32_t vp = 0;
+        if (pair) {
+            vp = __ldcg(J.val + y.z);
+            pair = ((vp ^ x.w) & 0x7ffffffeu) != 0;
+        }
         const uint32_t m = __ballot_sync(0xffffffffu, pair);
         if (m) {
             uint32_t pos = 0;
-            if (lane == 0) pos = atomicAdd(&c.pairs, (uint32_t)__popc(m));
-            pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(m & lanemask_lt_u32());
-            if (pair && pos < cap) {
-                J.pair[pos] = make_uint4(x.x, x.y, x.w, y.x);
-                J.pair_e[pos] = make_uint2(x.z, y.y | 0x80000000u);
+            if (lane == 0) pos = atomicAdd(&c.shard[shard_of(J)].pairs, (uint32_t)__popc(m));
+            pos = place(J, shard_of(J), __shfl_sync(0xffffffffu, pos, 0) + __popc(m & lanemask_lt_u32()));
+            if (pair && pos < J.pair_cap) {
+                J.pair[pos] = make_uint4(x.x, x.y, x.w, vp);
+                J.pair_e[pos] = make_uint2(x.z, y.z | 0x80000000u);
                 red_min(T + x.z, t);
-                red_min(T + y.y, t);
+                red_min(T + y.z, t);
             }
-            if (pair && pos >= cap) c.ovf = 1;
+            if (pair && pos >= J.pair_cap) c.ovf = 1;
         }
-        p = y.z;
-        if (k >= walk) {  // a crowded group: fewer rounds at once, or another kernel
+        p = y.w;
+        if (k >= walk) {  // a crowded chain: fewer rounds at once, or another kernel
             c.ovf = 1;
             break;
         }
@@ -320,20 +322,30 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
     const bool host_used = J.r0 > 0;
     uint64_t *const win = J.bases + o;  // the suffixes' bases of the step, from pass A to pass C
     uint32_t live_n = 0;
+    const uint64_t from = half ? e0 - side0 : e0;  // where the entries are read
+    // the entries of the chunk after this one are on their way while it is worked on
+    uint64_t nkey = 0, nbases = 0;
+    uint32_t nval = 0, nold = kNever;
+    auto fetch = [&](uint32_t x) {
+        if (x >= cnt) return;
+        nkey = __ldcg(kin + from + x);
+        nval = __ldcg(lval + from + x);
+        if (kPass != 2 && b && !l.retry) nold = __ldcg(told + e0 + x);
+        if (kPass == 2) nbases = __ldcg(win + x);
+    };
+    fetch(lane);
     for (uint32_t x0 = 0; x0 < cnt; x0 += 32) {
         const uint32_t x = x0 + lane;
         const uint64_t e = e0 + x;
         bool live = x < cnt;
-        uint64_t key = 0;
-        uint32_t val = 0;
-        if (live) {
-            key = __ldcg(kin + (half ? e - side0 : e));
-            val = __ldcg(lval + (half ? e - side0 : e)) | (half ? 0x80000000u : 0u);
-            if (kPass != 2) {
-                if (b) live = l.retry || t_round(__ldcg(told + e), tg) == kNever;
-                else if (host_used) live = used[val & 0x7fffffffu] == 0;
-            }
+        const uint64_t key = nkey;
+        const uint32_t val = nval | (half ? 0x80000000u : 0u);
+        uint64_t bases = nbases;
+        if (kPass != 2 && live) {
+            if (b) live = t_round(nold, tg) == kNever;
+            else if (host_used) live = used[val & 0x7fffffffu] == 0;
         }
+        fetch(x + 32);
         uint64_t en = e;
         if (kPass != 2) {
             const uint32_t m = __ballot_sync(0xffffffffu, live);  // every lane has read its entry
@@ -350,14 +362,9 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
             }
         }
         uint32_t f1 = (uint32_t)(key >> 32), f2 = (uint32_t)key;
-        uint64_t bases = 0;
-        if (live) {
-            if (kPass == 2) {
-                bases = __ldcg(win + x);
-            } else {
-                bases = step_bases(J, val, l.r, R);
-                if (kPass == 0) win[en - e0] = bases;
-            }
+        if (kPass != 2 && live) {
+            bases = step_bases(J, val, l.r, R);
+            if (kPass == 0) win[en - e0] = bases;
         }
         for (uint32_t q0 = 0; q0 < R; q0 += kU) {
             uint32_t g1[kU], g2[kU], fw[kU];
@@ -396,6 +403,8 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
                     else flush_suffixes(J, c, w, l, tg + 1);
                 }
             }
+            if (kPass != 2 && q0 == 0 && x + 32 < cnt && t_round(nold, tg) == kNever)
+                prefetch_bases(J, nval | (half ? 0x80000000u : 0u), l.r, R);
         }
         if (kPass != 0 && live) kadv[en] = ((uint64_t)f1 << 32) | f2;
     }
@@ -439,21 +448,20 @@ EMP_DEV void sweep_pass(SweepJob *jobs, int J, uint32_t b, uint32_t tg, SShared 
 // as true; iteration tg takes it from T[tg - 1] and T[tg] is the smallest
 // round of each entry's matching pairs.  When no status changes T[tg] = T[tg
 // - 1] is the solution.
-EMP_DEV uint32_t live_pairs(const SweepLoc &l, const SweepCtr &c) {
-    return l.act && !__ldcg(&c.ovf) ? __ldcg(&c.pairs) : 0u;
-}
 EMP_DEV void resolve_pairs(SweepJob *jobs, int J, uint32_t b, uint32_t tg, uint32_t *chg, SShared &sh) {
     const uint32_t total = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t {
-        return (live_pairs(sh.loc[j], jobs[j].ctr[b % 3]) + kST - 1) / kST;
+        return sh.loc[j].act ? (sh.loc[j].pairs + kST - 1) / kST : 0u;
     });
     bool changed = false;
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const int j = job_of(sh.pref, J, t);
         SweepJob &jb = jobs[j];
         const uint32_t x = (t - sh.pref[j]) * kST + threadIdx.x;
-        if (x >= __ldcg(&jb.ctr[b % 3].pairs)) continue;
+        if (x >= sh.loc[j].pairs) continue;
+        const uint32_t given_n = __ldcg(&shard_at(jb, jb.ctr[b % 3], x).pairs);
         const uint32_t q = __ldcg(reinterpret_cast<const uint32_t *>(jb.pair + x)) & 63u;
         const uint2 e = __ldcg(jb.pair_e + x);
+        if (!given(jb, x, given_n)) continue;
         const uint32_t ep = e.y & 0x7fffffffu;
         const uint32_t *T0 = jb.T[(tg - 1) & 1u];
         uint32_t *T1 = jb.T[tg & 1u];
@@ -484,11 +492,11 @@ EMP_DEV uint32_t block_append(uint32_t f, uint32_t *ctr, SShared &sh) {
 }
 
 // The step's matching pairs: a record for each of their entries (the first
-// pair of an entry claims it), the counts per round; groups emptied, filters
+// pair of an entry claims it), the counts per round; chains emptied, filters
 // zeroed.
 EMP_DEV void commit_step(SweepJob *jobs, int J, uint32_t b, uint32_t tg, SShared &sh) {
     uint32_t total = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t {
-        return (live_pairs(sh.loc[j], jobs[j].ctr[b % 3]) + kST - 1) / kST;
+        return sh.loc[j].act ? (sh.loc[j].pairs + kST - 1) / kST : 0u;
     });
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const int j = job_of(sh.pref, J, t);
@@ -499,9 +507,10 @@ EMP_DEV void commit_step(SweepJob *jobs, int J, uint32_t b, uint32_t tg, SShared
         const uint32_t x = (t - sh.pref[j]) * kST + threadIdx.x;
         uint4 v = make_uint4(0, 0, 0, 0);
         bool fs = false, fp = false;
-        if (x < __ldcg(&c.pairs)) {
+        if (x < sh.loc[j].pairs) {
+            const uint32_t given_n = __ldcg(&shard_at(jb, c, x).pairs);
             const uint2 e = __ldcg(jb.pair_e + x);
-            if (e.y >> 31) {
+            if (given(jb, x, given_n) && e.y >> 31) {
                 v = __ldcg(jb.pair + x);
                 uint32_t *T = jb.T[tg & 1u];
                 fs = (atomicExch(T + e.x, t_word(tg, kClaimed)) & 63u) != kClaimed;
@@ -524,34 +533,37 @@ EMP_DEV void commit_step(SweepJob *jobs, int J, uint32_t b, uint32_t tg, SShared
         __syncthreads();
     }
     total = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t {
-        return sh.loc[j].act ? (min(__ldcg(&jobs[j].ctr[b % 3].pc), jobs[j].n_p) + kST - 1) / kST : 0u;
+        if (!sh.loc[j].act) return 0u;
+        return (sh.loc[j].pc + kST - 1) / kST;
     });
-    for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {  // every group has a prefix
+    for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {  // every chain has a candidate
         const int j = job_of(sh.pref, J, t);
         SweepJob &jb = jobs[j];
         const uint32_t x = (t - sh.pref[j]) * kST + threadIdx.x;
-        if (x < min(__ldcg(&jb.ctr[b % 3].pc), jb.n_p)) {
-            const uint32_t g = __ldcg(&jb.pcand[x].w);
-            if (g != kNever) *reinterpret_cast<uint4 *>(jb.groups + g) = make_uint4(kNever, kNever, kNever, kNever);
+        if (x < sh.loc[j].pc) {
+            const uint32_t given_n = __ldcg(&shard_at(jb, jb.ctr[b % 3], x).pc);
+            const uint2 k = __ldcg(reinterpret_cast<const uint2 *>(jb.pcand + x));
+            if (!given(jb, x, given_n)) continue;
+            jb.heads[chain_hash((uint64_t)k.x | ((uint64_t)k.y << 32), (1u << sh.loc[j].gm) - 1u)] = kNever;
         }
     }
 }
 
-// group slots that no step of the job has used yet: emptied
-EMP_DEV void clean_groups(SweepJob *jobs, int J, SShared &sh) {
-    constexpr uint32_t kSlots = kST * 4;
+// chain heads that no step of the job has used yet: emptied
+EMP_DEV void clean_heads(SweepJob *jobs, int J, SShared &sh) {
+    constexpr uint32_t kTile = kST * 16;  // heads per tile: four 16-byte stores a thread
     const uint32_t total = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t {
         const SweepLoc &l = sh.loc[j];
         if (!l.act || l.gm <= l.gclean) return 0u;
         const uint32_t lo = l.gclean ? 1u << l.gclean : 0u;
-        return ((1u << l.gm) - lo + kSlots - 1) / kSlots;
+        return ((1u << l.gm) - lo + kTile - 1) / kTile;
     });
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
         const int j = job_of(sh.pref, J, t);
         const SweepLoc &l = sh.loc[j];
-        const uint32_t lo = (l.gclean ? 1u << l.gclean : 0u) + (t - sh.pref[j]) * kSlots, hi = min(lo + kSlots, 1u << l.gm);
-        uint4 *g = reinterpret_cast<uint4 *>(jobs[j].groups);
-        for (uint32_t i = lo + threadIdx.x; i < hi; i += kST) g[i] = make_uint4(kNever, kNever, kNever, kNever);
+        const uint32_t lo = (l.gclean ? 1u << l.gclean : 0u) + (t - sh.pref[j]) * kTile, hi = min(lo + kTile, 1u << l.gm);
+        for (uint32_t i = lo + 4 * threadIdx.x; i < hi; i += 4 * kST)  // all multiples of four
+            *reinterpret_cast<uint4 *>(jobs[j].heads + i) = make_uint4(kNever, kNever, kNever, kNever);
     }
 }
 
@@ -837,7 +849,29 @@ EMP_DEV void write_bin_cta(const uint4 *sorted, uint32_t c, uint32_t *from, uint
     }
 }
 
-// the job's step after step b - 1: its first round, its length, its groups
+// What pass B and C of a job's step found, in one read of its counters.
+EMP_DEV void step_counts(const SweepJob &J, const SweepCtr &c, SweepLoc &l) {
+    const uint32_t last = (1u << J.shard_log) - 1u, ovf = __ldcg(&c.ovf);
+    uint2 n = __ldcg(reinterpret_cast<const uint2 *>(&c.shard[0]));
+    uint32_t all = n.x, mc = n.x, mp = n.y;
+    if (last) {
+        uint2 v[kSweepShards];
+#pragma unroll
+        for (uint32_t k = 1; k < kSweepShards; ++k)  // in flight together
+            v[k] = __ldcg(reinterpret_cast<const uint2 *>(&c.shard[min(k, last)]));
+#pragma unroll
+        for (uint32_t k = 1; k < kSweepShards; ++k) {
+            all += k <= last ? v[k].x : 0u;
+            mc = max(mc, v[k].x);
+            mp = max(mp, v[k].y);
+        }
+    }
+    l.cands = all;
+    l.pc = min(((mc + 31) & ~31u) << J.shard_log, J.p_cap);
+    l.pairs = ovf ? 0u : min(((mp + 31) & ~31u) << J.shard_log, J.pair_cap);
+}
+
+// the job's step after step b - 1: its first round, its length, its chains
 EMP_DEV void next_step(SweepJob &J, SweepLoc &l, uint32_t b) {
     if (!l.act) return;
     const SweepCtr &c = J.ctr[(b - 1) % 3];
@@ -848,18 +882,17 @@ EMP_DEV void next_step(SweepJob &J, SweepLoc &l, uint32_t b) {
     }
     l.retry = __ldcg(&c.ovf) != 0;
     if (l.retry) {  // too many candidates: the same rounds again, fewer at once
-        if (l.R == 1 && l.gm == J.gm_max) {
+        if (l.R == 1) {
             l.act = 0;
             if (blockIdx.x == 0) J.crowded = 1;
         }
         l.R = l.R > 4 ? l.R / 4 : 1u;
-        l.gm = (uint8_t)J.gm_max;
         return;
     }
     const uint32_t us = __ldcg(&c.fired_s), up = __ldcg(&c.fired_p);
     // about one candidate per live entry and step, were none removed
     const uint64_t want = us ? (uint64_t)l.ls * l.R / us : (uint64_t)kSweepMaxR;
-    const uint64_t tried = (uint64_t)l.lp * l.R, cands = __ldcg(&c.pc);
+    const uint64_t tried = (uint64_t)l.lp * l.R, cands = l.cands;
     l.ls -= us;
     l.lp -= up;
     l.r += l.R;
@@ -869,8 +902,8 @@ EMP_DEV void next_step(SweepJob &J, SweepLoc &l, uint32_t b) {
     const uint32_t left = (uint32_t)J.rounds > l.r ? (uint32_t)J.rounds - l.r : 0u;
     l.R = R < left ? R : left;
     l.act = left > 0 && l.ls > 0 && l.lp > 0;
-    // twice the groups that the last step's rate of candidates gives
-    const uint32_t gm = pow2_log(2 * (cands * ((uint64_t)l.lp * l.R) / (tried ? tried : 1)) + 1024);
+    // a chain per candidate that the last step's rate gives
+    const uint32_t gm = pow2_log(cands * ((uint64_t)l.lp * l.R) / (tried ? tried : 1) + 1024);
     l.gm = (uint8_t)min(gm, (uint32_t)J.gm_max);
 }
 // filter sizes of a step, its rounds cut so that all jobs' first filters stay
@@ -890,13 +923,12 @@ struct SweepTrace {
     CoopCtl *ctl;
     uint32_t n;
 };
-EMP_DEV void mark(SweepTrace &t, uint32_t phase, uint32_t b, const SweepJob *jobs, const SShared &sh) {
+EMP_DEV void mark(SweepTrace &t, uint32_t phase, uint32_t b, const SShared &sh) {
     if (!t.ctl->trace || blockIdx.x != 0 || threadIdx.x != 0 || t.n >= t.ctl->trace_cap) return;
-    const SweepCtr &c = jobs[0].ctr[b % 3];
     uint64_t *p = t.ctl->trace + (uint64_t)t.n * kCoopTracePhases;
     p[0] = phase | (uint64_t)b << 8;
     p[1] = sh.loc[0].r | (uint64_t)sh.loc[0].R << 32;
-    p[2] = __ldcg(&c.pc) | (uint64_t)__ldcg(&c.pairs) << 32;
+    p[2] = sh.loc[0].cands | (uint64_t)sh.loc[0].pairs << 32;
     p[3] = globaltimer();
     p[4] = sh.loc[0].ls | (uint64_t)sh.loc[0].lp << 32;
     ++t.n;
@@ -925,11 +957,11 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         l.retry = 0;
         l.cur = x.cur0;
         l.gclean = 0;
-        l.gm = (uint8_t)min(pow2_log((uint64_t)x.n_p + 1024), (uint32_t)x.gm_max);
+        l.gm = (uint8_t)min(pow2_log((uint64_t)x.n_p / 2 + 1024), (uint32_t)x.gm_max);
     }
     __syncthreads();
     SweepTrace tr{ctl, 0u};
-    mark(tr, 0, 0, jobs, sh);
+    mark(tr, 0, 0, sh);
     if (zero) {
         const uint32_t total = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t { return (jobs[j].zeroed + 4 * kST - 1) / (4 * kST); });
         for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
@@ -947,19 +979,23 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         block_exclusive_scan<kST, uint64_t>(tid < J && sh.loc[tid].act ? (uint64_t)sh.loc[tid].ls : 0ull, sh.scan64, &all);
         if (tid < J) size_filters(jobs[tid], sh.loc[tid], all);
         if (!__syncthreads_or(tid < J && sh.loc[tid].act)) break;
-        mark(tr, 1, b, jobs, sh);
+        mark(tr, 1, b, sh);
         uint32_t *chg = go.chg + (b % 3) * kSweepIters;
-        clean_groups(jobs, J, sh);
+        clean_heads(jobs, J, sh);
         sweep_pass<0>(jobs, J, b, tg, sh, smem);
         if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-        mark(tr, 2, b, jobs, sh);
+        mark(tr, 2, b, sh);
         sweep_pass<1>(jobs, J, b, tg, sh, smem);
         if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-        mark(tr, 3, b, jobs, sh);
+        mark(tr, 3, b, sh);
         if (blockIdx.x == gridDim.x - 1) {  // the next step's counters (last read two steps ago)
+            for (uint32_t k = tid; k < (uint32_t)J * kSweepShards; k += kST) {
+                SweepShard &x = jobs[k / kSweepShards].ctr[(b + 1) % 3].shard[k % kSweepShards];
+                x.pc = x.pairs = 0;
+            }
             if (tid < J) {
-                uint32_t *c = reinterpret_cast<uint32_t *>(&jobs[tid].ctr[(b + 1) % 3]);
-                for (uint32_t k = 0; k < sizeof(SweepCtr) / 4; ++k) c[k] = 0;
+                SweepCtr &c = jobs[tid].ctr[(b + 1) % 3];
+                c.ls = c.lp = c.ovf = c.fired_s = c.fired_p = 0;
                 if (b == 0 && jobs[tid].r0 > 0) {
                     jobs[tid].s0 = __ldcg(&jobs[tid].ctr[0].ls);
                     jobs[tid].p0 = __ldcg(&jobs[tid].ctr[0].lp);
@@ -969,25 +1005,26 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         }
         sweep_pass<2>(jobs, J, b, tg, sh, smem);
         if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-        mark(tr, 4, b, jobs, sh);
+        mark(tr, 4, b, sh);
         ++tg;  // the T of the pairs as pass C found them: final where every step is one round
-        if (__syncthreads_or(tid < J && sh.loc[tid].R > 1 && live_pairs(sh.loc[tid], jobs[tid].ctr[b % 3]))) {
+        if (tid < J && sh.loc[tid].act) step_counts(jobs[tid], jobs[tid].ctr[b % 3], sh.loc[tid]);
+        if (__syncthreads_or(tid < J && sh.loc[tid].act && sh.loc[tid].R > 1 && sh.loc[tid].pairs)) {
             for (uint32_t it = 0; it < (uint32_t)kSweepIters; ++it) {  // kSweepMaxR + 1 suffice
                 resolve_pairs(jobs, J, b, ++tg, chg + it, sh);
                 if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-                mark(tr, 5, b, jobs, sh);
+                mark(tr, 5, b, sh);
                 if (!__ldcg(chg + it)) break;
             }
         }
         clear_filters(jobs, J, sh);
         commit_step(jobs, J, b, tg, sh);
         if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-        mark(tr, 6, b, jobs, sh);
+        mark(tr, 6, b, sh);
     }
     // ---- output: the rounds' sizes, the records by (round, key range)
     for (int j = blockIdx.x; j < J; j += gridDim.x) round_sizes(jobs[j], sh);
     if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-    mark(tr, 11, 0, jobs, sh);
+    mark(tr, 11, 0, sh);
     const uint32_t nb = sweep_prefix(sh, sh.bin0, J, [&](int j) -> uint32_t { return vld(jobs[j].nbins); });
     uint32_t tiles = sweep_prefix(sh, sh.pref, J, [&](int j) -> uint32_t { return (vld(jobs[j].nrec) + kST - 1) / kST; });
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -997,9 +1034,9 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
             jobs[j].rank[x] = atomicAdd(go.cnt + sh.bin0[j] + rec_bin(jobs[j], __ldcg(jobs[j].rec + x)), 1u);
     }
     if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-    mark(tr, 12, 0, jobs, sh);
+    mark(tr, 12, 0, sh);
     if (!grid_scan(go.cnt, go.off, nb, go.part, ctl, sh)) return;
-    mark(tr, 20, 0, jobs, sh);
+    mark(tr, 20, 0, sh);
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const int j = job_of(sh.pref, J, t);
         const uint32_t x = (t - sh.pref[j]) * kST + tid;
@@ -1010,7 +1047,7 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         }
     }
     if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-    mark(tr, 13, 0, jobs, sh);
+    mark(tr, 13, 0, sh);
     WarpBin &wb = reinterpret_cast<WarpBin *>(smem)[warp];
     for (uint32_t t = warp * gridDim.x + blockIdx.x; t < nb; t += gridDim.x * kSW) {
         const int j = job_of(sh.bin0, J, t);
@@ -1025,7 +1062,7 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         if (lane == 0 && c <= kBinCap) go.ecnt[t] = e;
     }
     if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-    mark(tr, 14, 0, jobs, sh);
+    mark(tr, 14, 0, sh);
     const uint32_t nbig = vld(*go.nbig);
     if (nbig) {
         for (uint32_t k = blockIdx.x; k < nbig; k += gridDim.x) {
@@ -1037,14 +1074,14 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
             __syncthreads();
         }
         if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-    mark(tr, 15, 0, jobs, sh);
+    mark(tr, 15, 0, sh);
     }
     if (!grid_scan(go.ecnt, go.eoff, nb, go.part, ctl, sh)) return;
-    mark(tr, 21, 0, jobs, sh);
+    mark(tr, 21, 0, sh);
     for (int j = blockIdx.x; j < J; j += gridDim.x) round_places(jobs[j], sh.bin0[j], go.eoff, sh);
     if (!grid_barrier_raw(ctl, &sh.flag, &sh.gen)) return;
-    mark(tr, 16, 0, jobs, sh);
-    auto place = [&](uint32_t t, int &j, uint32_t *&from, uint32_t *&to, uint64_t &o, uint64_t &at) -> bool {
+    mark(tr, 16, 0, sh);
+    auto place_bin = [&](uint32_t t, int &j, uint32_t *&from, uint32_t *&to, uint64_t &o, uint64_t &at) -> bool {
         j = job_of(sh.bin0, J, t);
         const SweepJob &jb = jobs[j];
         if (vld(jb.overflow)) return false;
@@ -1062,7 +1099,7 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         int j;
         uint32_t *from, *to;
         uint64_t o, at;
-        if (place(t, j, from, to, o, at)) write_bin_warp(jobs[j].rec + at, c, from, to, o, wb);
+        if (place_bin(t, j, from, to, o, at)) write_bin_warp(jobs[j].rec + at, c, from, to, o, wb);
     }
     __syncthreads();
     for (uint32_t k = blockIdx.x; k < nbig; k += gridDim.x) {
@@ -1070,7 +1107,7 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         int j;
         uint32_t *from, *to;
         uint64_t o, at;
-        if (place(t, j, from, to, o, at)) write_bin_cta(jobs[j].rec + at, __ldcg(go.cnt + t), from, to, o, sh);
+        if (place_bin(t, j, from, to, o, at)) write_bin_cta(jobs[j].rec + at, __ldcg(go.cnt + t), from, to, o, sh);
     }
 }
 
@@ -1083,6 +1120,16 @@ uint32_t sweep_segment_size(uint64_t entries_per_side) {
     const uint64_t warps = 148ull * kSW;
     uint64_t s = (entries_per_side / warps + 31) / 32 * 32;
     return (uint32_t)(s < 32 ? 32 : s > 1024 ? 1024 : s);
+}
+
+// a job of `entries` of a launch's entries per side: its share of the warps
+// that draw places, and none for a few thousand entries
+uint32_t sweep_shard_log(uint64_t entries, uint64_t entries_per_side) {
+    uint32_t k = 0;
+    while ((2u << k) <= kSweepShards && (2ull << k) * entries_per_side <= kSweepShards * entries &&
+           (8192ull << k) <= entries)
+        ++k;
+    return k;
 }
 
 uint32_t sweep_bins_max(uint64_t n_in, int rounds) { return (uint32_t)(n_in / kBinMean) + (uint32_t)rounds + 1; }
@@ -1102,8 +1149,11 @@ size_t sweep_layout(uint8_t *base, SweepJob *J, size_t *zeroed) {
     const uint64_t w1 = ns < 256 ? 1024 : 4 * ns < (1u << 24) ? 4 * ns : 1u << 24;
     J->w1_max = (uint32_t)w1;
     uint32_t gm = 10;
-    while ((1ull << gm) < np + np / 4) ++gm;
+    while ((1ull << gm) < np) ++gm;
     J->gm_max = gm;
+    // a quarter more than every shard's share
+    J->p_cap = (uint32_t)(((np + np / 4) >> J->shard_log) / 32 + 2) << (J->shard_log + 5);
+    J->pair_cap = (uint32_t)(((n + n / 4) >> J->shard_log) / 32 + 2) << (J->shard_log + 5);
     J->segs_s = (uint32_t)((ns + J->seg - 1) / J->seg);
     J->segs_p = (uint32_t)((np + J->seg - 1) / J->seg);
     J->filter1 = reinterpret_cast<uint32_t *>(take((size_t)4 * w1));
@@ -1113,13 +1163,13 @@ size_t sweep_layout(uint8_t *base, SweepJob *J, size_t *zeroed) {
     J->fp = reinterpret_cast<uint32_t *>(take((size_t)rounds * 4));
     *zeroed = o;
     J->zeroed = (uint32_t)(o / 16);
-    J->groups = reinterpret_cast<SweepGroup *>(take(sizeof(SweepGroup) << gm));
+    J->heads = reinterpret_cast<uint32_t *>(take((size_t)4 << gm));
     J->bases = reinterpret_cast<uint64_t *>(take(ns * 8));
     for (int k = 0; k < 2; ++k) J->T[k] = reinterpret_cast<uint32_t *>(take(n * 4));
     J->segcnt = reinterpret_cast<uint32_t *>(take((size_t)(J->segs_s + J->segs_p) * 4));
-    J->pcand = reinterpret_cast<uint4 *>(take(np * 16));
-    J->pair = reinterpret_cast<uint4 *>(take(n * 16));
-    J->pair_e = reinterpret_cast<uint2 *>(take(n * 8));
+    J->pcand = reinterpret_cast<uint4 *>(take((size_t)J->p_cap * 16));
+    J->pair = reinterpret_cast<uint4 *>(take((size_t)J->pair_cap * 16));
+    J->pair_e = reinterpret_cast<uint2 *>(take((size_t)J->pair_cap * 8));
     J->rec = reinterpret_cast<uint4 *>(take(n * 16));
     J->rec2 = reinterpret_cast<uint4 *>(take(n * 16));
     J->rank = reinterpret_cast<uint32_t *>(take(n * 4));

@@ -327,17 +327,18 @@ constexpr int kSweepMaxR = 32;       // rounds of a step at most
 constexpr uint64_t kSweepMaxEntries = 16ull << 20;
 constexpr int kSweepFirstR = 4;      // rounds of a job's first step
 constexpr int kSweepIters = 40;      // resolving iterations of a step at most (kSweepMaxR + 1 suffice)
-struct SweepCtr {  // one step of one job (zero at its start)
-    uint32_t ls, lp;  // live suffixes / prefixes (a launch that starts after host-driven rounds)
+constexpr uint32_t kSweepShards = 16;  // counters of a job's candidates and pairs at most
+struct SweepShard {   // in a cache line of its own
     uint32_t pc;      // prefix candidates
     uint32_t pairs;   // pairs of a suffix and a prefix
+    uint32_t pad[30];
+};
+struct SweepCtr {  // one step of one job (zero at its start)
+    SweepShard shard[kSweepShards];
+    uint32_t ls, lp;  // live suffixes / prefixes (a launch that starts after host-driven rounds)
     uint32_t ovf;     // they did not fit: the step runs again with fewer rounds
     uint32_t fired_s, fired_p;  // entries matched
-};
-struct SweepGroup {  // all ones = empty
-    uint64_t key;    // key and round of the step
-    uint32_t head;   // its last prefix candidate
-    uint32_t pad;
+    uint32_t pad[27];
 };
 struct SweepJob {
     // the list at launch, [n_s suffixes | n_p prefixes]: key[cur0] holds the
@@ -346,6 +347,7 @@ struct SweepJob {
     uint32_t *val;
     const uint8_t *used_s, *used_p;  // marks of rounds run before the launch (read when r0 > 0)
     uint32_t n_s, n_p;
+    uint32_t shard_log;      // log2 of the counters of its candidates and pairs
     uint32_t seg;            // entries of a segment (a warp's unit of work), a multiple of 32
     int32_t L, rounds, r0, wpr;
     const uint32_t *seq2;    // read-major 2-bit bases, wpr words per read
@@ -356,16 +358,17 @@ struct SweepJob {
     // work memory (sweep_layout)
     uint32_t w1_max;         // words of filter 1
     uint32_t zeroed;         // bytes to be zero at the start, in units of 16
-    uint32_t gm_max;         // log2 group slots
+    uint32_t gm_max;         // log2 chain heads
+    uint32_t p_cap, pair_cap;  // places of candidates and pairs
     uint32_t segs_s, segs_p;
     uint32_t *filter1, *filter2;  // zero between steps
     SweepCtr *ctr;           // [3]: step b uses ctr[b % 3]
     uint32_t *fs, *fp;       // [round]: suffixes / prefixes matched
-    SweepGroup *groups;      // those of the step, empty between steps
+    uint32_t *heads;         // chains of the step's candidates by (key, round): the last one; empty between steps
     uint64_t *bases;         // each suffix's bases of the step, 2 bits a round
     uint32_t *T[2];          // [iteration % 2][entry]: round of the step that uses it
     uint32_t *segcnt;        // live entries of each segment, suffixes then prefixes
-    uint4 *pcand;            // prefix candidates: value, entry, the group's next one, group
+    uint4 *pcand;            // prefix candidates: key and round, entry, the chain's next one
     uint4 *pair;             // pairs: key and round, suffix, prefix (values)
     uint2 *pair_e;           // their entries; bit 31 of the second: the pair matches
     uint4 *rec, *rec2;       // matched entries: key, value, round
@@ -378,7 +381,7 @@ struct SweepJob {
     uint32_t s0, p0;         // live suffixes / prefixes of round r0 (when r0 > 0)
     uint32_t round;          // rounds run
     uint32_t overflow;       // the edge buffer is too small (zero at launch)
-    uint32_t crowded;        // a group of too many entries: not a job for this kernel (zero at launch)
+    uint32_t crowded;        // a chain of too many entries: not a job for this kernel (zero at launch)
     uint64_t e_total;        // edges
     uint8_t cur0;
     uint8_t one_half;        // the list at launch holds the suffixes only: the prefixes are the same entries
@@ -396,6 +399,7 @@ struct SweepOut {  // output bins of a launch's jobs (sweep_out_layout)
 };
 int sweep_grid_size();  // 0: no cooperative launch on this device
 uint32_t sweep_segment_size(uint64_t entries_per_side);
+uint32_t sweep_shard_log(uint64_t entries, uint64_t entries_per_side);
 uint32_t sweep_bins_max(uint64_t n_in, int rounds);
 size_t sweep_layout(uint8_t *base, SweepJob *job, size_t *zeroed);
 size_t sweep_out_layout(uint8_t *base, uint32_t bins, SweepOut *go, size_t *zeroed);
