@@ -871,6 +871,7 @@ emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0
     hj->n_s = (uint32_t)ns;
     hj->n_p = (uint32_t)np;
     hj->seg = sweep_segment_size(side);
+    hj->first_r = sweep_first_rounds(j->prep.U, 2 * j->prep.n);
     hj->shard_log = sweep_shard_log(np, side);
     hj->L = env.L;
     hj->rounds = env.rounds;

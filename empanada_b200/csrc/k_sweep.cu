@@ -55,7 +55,7 @@ constexpr uint32_t kNever = 0xffffffffu;
 constexpr uint64_t kFilterKeys = 25u << 20;  // (entry, round) keys of a step's first filters: 48 MB, within L2
 constexpr uint32_t kU = 4;              // filter accesses of a lane in flight
 constexpr uint32_t kQCap = 32 * (kU + 1);  // queued candidates per warp
-constexpr uint32_t kBinMean = 48;       // matched entries per output bin aimed at
+constexpr uint32_t kBinMean = 32;       // matched entries per output bin aimed at
 constexpr uint32_t kBinCap = 192;       // up to this many: one warp, in shared memory
 
 struct SweepLoc {  // a job's step, the same in every CTA
@@ -317,7 +317,7 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
     uint32_t *const lval = J.val;
     const uint8_t *used = kPfx ? J.used_p : J.used_s;
     uint32_t *const filter = kPass == 2 ? J.filter2 : J.filter1;
-    const uint32_t words = kPass == 2 ? l.w2 : l.w1, R = l.R, len0 = (uint32_t)J.L - l.r - 1u;
+    const uint32_t words = kPass == 2 ? l.w2 : l.w1, len0 = (uint32_t)J.L - l.r - 1u;
     const uint32_t inv1 = J.tables->inv1, inv2 = J.tables->inv2;
     const bool host_used = J.r0 > 0;
     uint64_t *const win = J.bases + o;  // the suffixes' bases of the step, from pass A to pass C
@@ -325,8 +325,9 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
     const uint64_t from = half ? e0 - side0 : e0;  // where the entries are read
     // the entries of the chunk after this one are on their way while it is worked on
     uint64_t nkey = 0, nbases = 0;
-    uint32_t nval = 0, nold = kNever;
+    uint32_t nval = 0, nold = kNever, nfull = 0;
     auto fetch = [&](uint32_t x) {
+        if (kPass != 0) nfull = __ldcg(&c.ovf);
         if (x >= cnt) return;
         nkey = __ldcg(kin + from + x);
         nval = __ldcg(lval + from + x);
@@ -338,6 +339,9 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
         const uint32_t x = x0 + lane;
         const uint64_t e = e0 + x;
         bool live = x < cnt;
+        // the step does not fit and runs again: nothing more to find
+        const uint32_t R = kPass != 0 && __any_sync(0xffffffffu, nfull) ? 0u : l.R;
+        if (kPass == 2 && R == 0) break;
         const uint64_t key = nkey;
         const uint32_t val = nval | (half ? 0x80000000u : 0u);
         uint64_t bases = nbases;
@@ -363,7 +367,7 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
         }
         uint32_t f1 = (uint32_t)(key >> 32), f2 = (uint32_t)key;
         if (kPass != 2 && live) {
-            bases = step_bases(J, val, l.r, R);
+            bases = step_bases(J, val, l.r, l.R);
             if (kPass == 0) win[en - e0] = bases;
         }
         for (uint32_t q0 = 0; q0 < R; q0 += kU) {
@@ -404,7 +408,7 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
                 }
             }
             if (kPass != 2 && q0 == 0 && x + 32 < cnt && t_round(nold, tg) == kNever)
-                prefetch_bases(J, nval | (half ? 0x80000000u : 0u), l.r, R);
+                prefetch_bases(J, nval | (half ? 0x80000000u : 0u), l.r, l.R);
         }
         if (kPass != 0 && live) kadv[en] = ((uint64_t)f1 << 32) | f2;
     }
@@ -952,7 +956,7 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
         l.ls = x.n_s;
         l.lp = x.n_p;
         const uint32_t left = x.rounds > x.r0 ? (uint32_t)(x.rounds - x.r0) : 0u;
-        l.R = left < (uint32_t)kSweepFirstR ? left : (uint32_t)kSweepFirstR;
+        l.R = min(left, x.first_r);
         l.act = left > 0 && x.n_s > 0;
         l.retry = 0;
         l.cur = x.cur0;
@@ -1130,6 +1134,18 @@ uint32_t sweep_shard_log(uint64_t entries, uint64_t entries_per_side) {
            (8192ull << k) <= entries)
         ++k;
     return k;
+}
+
+// Rounds of a job's first step, for about one candidate per entry: U unique
+// keys among n2 read-ends give the reads that start at a base and strand
+// (lambda; U / n2 = (1 - e^-lambda) / lambda of them differ), and an entry
+// finds a partner in a round with nearly that probability.  A dense set's
+// step that does not fit runs again with fewer rounds.
+uint32_t sweep_first_rounds(uint64_t U, uint64_t n2) {
+    const double d = n2 > U ? 1.0 - (double)U / (double)n2 : 0.0;
+    const double lambda = 2.0 * d * (1.0 + d * (2.0 / 3.0));
+    const double r = lambda > 0 ? 0.8 / lambda : 4.0;
+    return r < 1.0 ? 1u : r > 4.0 ? 4u : (uint32_t)r;
 }
 
 uint32_t sweep_bins_max(uint64_t n_in, int rounds) { return (uint32_t)(n_in / kBinMean) + (uint32_t)rounds + 1; }

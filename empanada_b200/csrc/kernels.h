@@ -325,7 +325,6 @@ constexpr int kSweepMaxR = 32;       // rounds of a step at most
 // Longer lists run in the bucket kernel: beyond this one round of every entry
 // no longer fits filters and groups within L2 (112.7M entries: 24.4 ms there).
 constexpr uint64_t kSweepMaxEntries = 16ull << 20;
-constexpr int kSweepFirstR = 4;      // rounds of a job's first step
 constexpr int kSweepIters = 40;      // resolving iterations of a step at most (kSweepMaxR + 1 suffice)
 constexpr uint32_t kSweepShards = 16;  // counters of a job's candidates and pairs at most
 struct SweepShard {   // in a cache line of its own
@@ -347,6 +346,7 @@ struct SweepJob {
     uint32_t *val;
     const uint8_t *used_s, *used_p;  // marks of rounds run before the launch (read when r0 > 0)
     uint32_t n_s, n_p;
+    uint32_t first_r;        // rounds of its first step
     uint32_t shard_log;      // log2 of the counters of its candidates and pairs
     uint32_t seg;            // entries of a segment (a warp's unit of work), a multiple of 32
     int32_t L, rounds, r0, wpr;
@@ -399,6 +399,7 @@ struct SweepOut {  // output bins of a launch's jobs (sweep_out_layout)
 };
 int sweep_grid_size();  // 0: no cooperative launch on this device
 uint32_t sweep_segment_size(uint64_t entries_per_side);
+uint32_t sweep_first_rounds(uint64_t U, uint64_t n2);
 uint32_t sweep_shard_log(uint64_t entries, uint64_t entries_per_side);
 uint32_t sweep_bins_max(uint64_t n_in, int rounds);
 size_t sweep_layout(uint8_t *base, SweepJob *job, size_t *zeroed);
