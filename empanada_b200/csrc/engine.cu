@@ -776,6 +776,21 @@ emp_status bucket_collect(emp_job *j, int r0, uint64_t n_in, const Launched &hj,
     return EMP_OK;
 }
 
+// Whether rounds over a list of n entries run in the sweep kernel
+// (k_sweep.cu): not when the caller shapes the bucket kernel's buckets or
+// regions.
+bool sweep_rounds_usable(const emp_job *j, uint64_t n) {
+    const emp_tuning &t = j->ctx->tune;
+    return !j->prep.no_sweep && t.round_driver == 0 && (!t.bucket_mean || t.bucket_mean == kBktMean) &&
+           (!t.region_cap || t.region_cap == kBktRegionCap) &&
+           (n <= kSweepMaxEntries ||
+            (n <= kSweepMaxSparse && sweep_first_rounds(j->prep.U, 2 * j->prep.n) >= kSweepSparseR)) &&
+           sweep_grid_size() > 0;
+}
+
+emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t ns, uint64_t np,
+                            uint64_t ecap, uint64_t *needed, bool handed = false);
+
 // Rounds r0 .. of one job alone in the bucket kernel: one cooperative launch,
 // one grid barrier per round.
 emp_status run_rounds_bucket(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t n_in,
@@ -807,6 +822,7 @@ emp_status run_rounds_bucket(emp_job *j, cudaStream_t s, const RoundEnv &env, in
         hc->probe = j->coop_probe.as<uint64_t>();
     }
     hj->pre_done = bucket_prologue_apart(*hj) ? 1u : 0u;
+    hj->hand = sweep_rounds_usable(j, 0) ? 1u : 0u;
     EMP_CUDA(cudaMemcpyAsync(j->bk_job.p, hj, sizeof(BktJob), cudaMemcpyHostToDevice, s));
     EMP_CUDA(cudaMemcpyAsync(j->coop_ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
     cudaEvent_t e0 = j->upd_ev[0], e1 = j->upd_ev[1];
@@ -822,7 +838,15 @@ emp_status run_rounds_bucket(emp_job *j, cudaStream_t s, const RoundEnv &env, in
     st.ms_round_kernel += ms_between(e0, e1);
     if (trace_path) write_coop_trace(j, trace_path, env.rounds, r0, j->h_records.as<RoundRecord>(), s, 1, "round_us");
     if (probe_env) write_coop_probe(j, probe_path.c_str(), grid, s);
-    return bucket_collect(j, r0, n_in, *hj, needed);
+    EMP_TRY(bucket_collect(j, r0, n_in, *hj, needed));
+    if (!hj->hand_iter) return EMP_OK;
+    // the rounds from r1 on in the sweep kernel, their edges behind those of the rounds before
+    const int r1 = r0 + (int)hj->hand_iter;
+    const uint64_t ns = hj->hand_s, np = hj->hand_n - ns, E = st.n_edges;
+    EMP_CUDA(launch_bucket_list(j->bk_job.as<BktJob>(), j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(), s));
+    const emp_status rc = run_rounds_sweep(j, s, env, r1, 0, ns, np, ecap - E, needed, true);
+    if (rc == kNeedEdgeRoom) *needed += E;
+    return rc == EMP_E_NOMEM ? kCrowded : rc;  // all of them here, then
 }
 
 // Profiling aid: the phases of a sweep launch (k_sweep.cu's mark), one line
@@ -846,21 +870,12 @@ void write_sweep_trace(emp_job *j, const char *path, cudaStream_t s) {
     std::fclose(f);
 }
 
-// Whether rounds over a list of n entries run in the sweep kernel
-// (k_sweep.cu): not when the caller shapes the bucket kernel's buckets or
-// regions.
-bool sweep_rounds_usable(const emp_job *j, uint64_t n) {
-    const emp_tuning &t = j->ctx->tune;
-    return !j->prep.no_sweep && t.round_driver == 0 && (!t.bucket_mean || t.bucket_mean == kBktMean) &&
-           (!t.region_cap || t.region_cap == kBktRegionCap) && n <= kSweepMaxEntries && sweep_grid_size() > 0;
-}
-
 // Buffers and launch description (host copy *hj) of rounds r0 .. of one job
 // in the sweep kernel: the list lk[cur] holds ns suffixes, then np prefixes;
 // side: the suffixes (or prefixes, if more) of all jobs of the launch.
 // The launch overwrites the list.
 emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t ns, uint64_t np,
-                         uint64_t ecap, uint64_t side, SweepJob *hj) {
+                         uint64_t ecap, uint64_t side, bool handed, SweepJob *hj) {
     std::memset(hj, 0, sizeof(SweepJob));
     hj->key[0] = j->lk0.as<uint64_t>();
     hj->key[1] = j->lk1.as<uint64_t>();
@@ -871,7 +886,9 @@ emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0
     hj->n_s = (uint32_t)ns;
     hj->n_p = (uint32_t)np;
     hj->seg = sweep_segment_size(side);
-    hj->first_r = sweep_first_rounds(j->prep.U, 2 * j->prep.n);
+    hj->first_r = handed ? kHandRate : sweep_first_rounds(j->prep.U, 2 * j->prep.n);
+    hj->marked = r0 > 0 && !handed;
+    hj->stepped = handed;
     hj->shard_log = sweep_shard_log(np, side);
     hj->L = env.L;
     hj->rounds = env.rounds;
@@ -884,14 +901,16 @@ emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0
     size_t zeroed = 0;
     EMP_TRY(ensure(j, j->swp, sweep_layout(nullptr, hj, &zeroed)));
     sweep_layout(j->swp.as<uint8_t>(), hj, &zeroed);
-    EMP_TRY(ensure(j, j->dout, (size_t)env.rounds * 12 + ecap * 8));
-    hj->out = j->dout.as<uint8_t>();
+    // behind the records of the rounds that ran before, whose buffer held all
+    EMP_TRY(ensure(j, j->dout, (size_t)j->dout_bytes + (size_t)(env.rounds - r0) * 12 + ecap * 8));
+    hj->out = j->dout.as<uint8_t>() + j->dout_bytes;
     return EMP_OK;
 }
 
-// Rounds r0 .. of one job alone in the sweep kernel.
+// Rounds r0 .. of one job alone in the sweep kernel; handed: the bucket
+// kernel's launch left them.
 emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0, int cur, uint64_t ns, uint64_t np,
-                            uint64_t ecap, uint64_t *needed) {
+                            uint64_t ecap, uint64_t *needed, bool handed) {
     // descriptor, control block and round records in one device buffer, laid
     // out as the job's host slot has them: one copy each way
     constexpr size_t kRec = kSlotRecords - kSlotCoop;
@@ -901,7 +920,7 @@ emp_status run_rounds_sweep(emp_job *j, cudaStream_t s, const RoundEnv &env, int
     uint8_t *dev = j->coop_ctl.as<uint8_t>();
     SweepJob *hj = j->h_coop.as<SweepJob>(), *dj = reinterpret_cast<SweepJob *>(dev);
     CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + 1), *dc = reinterpret_cast<CoopCtl *>(dj + 1);
-    EMP_TRY(sweep_prepare(j, s, env, r0, cur, ns, np, ecap, std::max(ns, np), hj));
+    EMP_TRY(sweep_prepare(j, s, env, r0, cur, ns, np, ecap, std::max(ns, np), handed, hj));
     hj->records = reinterpret_cast<RoundRecord *>(dev + kRec);
     EMP_CUDA(cudaMemsetAsync(j->swp.p, 0, (size_t)hj->zeroed * 16, s));
     SweepOut go{};
@@ -1387,7 +1406,7 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
         emp_job *j = jobs[k];
         const JobPrep &q = j->prep;
         rounds_prelude(j);
-        EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, side, &hj[k]));
+        EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, side, false, &hj[k]));
         hj[k].records = rec;
         rec += q.rounds;
     }

@@ -1474,6 +1474,18 @@ EMP_DEV RoundShape round_shape(const BktJob &J, uint32_t iter) {
     return z;
 }
 
+// Whether the launch leaves round z.r and those after it to the sweep kernel,
+// which takes many rounds per step: at 20.7M entries a round of two per step
+// costs 57 us per million entries there, of six 29, against 33 here; below a
+// few million a round costs the 15 us of its phases here whatever it holds.
+// The hand-over itself costs about 0.15 ms.
+EMP_DEV bool hand_over(const BktJob &J, uint32_t iter, const RoundShape &z) {
+    if (!J.hand || !z.active || iter < 2 || J.rounds - z.r < kHandRounds) return false;
+    const uint64_t n = __ldcg(&J.meta[z.r].n), n1 = __ldcg(&J.meta[z.r - 1].n), s = __ldcg(&J.meta[z.r].s);
+    return n > s && ((n <= kHandMost && (n1 - n) * kHandRate < n1) ||
+                     (n <= kHandFew && J.rounds - z.r >= kHandFewRounds));
+}
+
 // The next tile this CTA runs (job, bucket, iteration), whose two regions
 // are pulled into L2 while this one is worked on; job = nullptr: none.
 struct NextTile {
@@ -1598,8 +1610,17 @@ EMP_COLD void place_edges(BktJob *jobs, int J, uint32_t its, BShared &sh, uint8_
     for (int j = 0; j < J; ++j) {
         BktJob &x = jobs[j];
         const uint32_t ran = x.iter_share && x.iter_share < its ? x.iter_share : its;
-        if (round_shape(x, x.iter0 + ran).active) continue;  // resumes in the next launch
-        if (blockIdx.x == 0 && threadIdx.x == 0) x.done = 1;
+        const RoundShape left = round_shape(x, x.iter0 + ran);
+        const bool handed = hand_over(x, x.iter0 + ran, left);
+        if (left.active && !handed) continue;  // resumes in the next launch
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            x.done = 1;
+            if (handed) {
+                x.hand_iter = x.iter0 + ran;
+                x.hand_n = __ldcg(&x.meta[left.r].n);
+                x.hand_s = __ldcg(&x.meta[left.r].s);
+            }
+        }
         const uint32_t r0 = (uint32_t)x.r0;
         // the rounds that ran: round r ran iff r < rounds and it had a suffix
         // (build_graph's loop condition, overlap.cu:258); they form a prefix
@@ -1611,7 +1632,7 @@ EMP_COLD void place_edges(BktJob *jobs, int J, uint32_t its, BShared &sh, uint8_
         }
         uint32_t ran_all;
         block_exclusive_scan<kT, uint32_t>(nran, sh.scan32, &ran_all);
-        const uint32_t r1 = r0 + ran_all;
+        const uint32_t r1 = handed ? (uint32_t)left.r : r0 + ran_all;
         uint64_t P[kRPT], E[kRPT], e_my = 0, b_my = 0;
 #pragma unroll
         for (int q = 0; q < kRPT; ++q) {
@@ -1741,9 +1762,9 @@ __global__ void __launch_bounds__(kT, 2) bucket_rounds_kernel(BktJob *jobs, Coop
             const RoundShape z = round_shape(jobs[j], jobs[j].iter0 + it);
             sh.shp_nb[j] = z.nb;
             sh.shp_nbn[j] = z.nb_next;
-            return z.active ? z.nb : 0u;
+            return z.active && !hand_over(jobs[j], jobs[j].iter0 + it, z) ? z.nb : 0u;
         });
-        if (total == 0) break;  // no job has a round left
+        if (total == 0) break;  // no job has a round left to run here
         probe(ctl, it, 1);
         tile_loop_ahead(sh, ticket, J, total, [&](int j, uint32_t b, uint32_t next) {
             const uint32_t g = jobs[j].iter0 + it;
@@ -1834,7 +1855,44 @@ __global__ void __launch_bounds__(kPreT) bucket_prologue_kernel(const BktJob *jo
     }
 }
 
+// The list left to the sweep kernel: one warp per bin copies its region, the
+// spilled entries follow one by one.
+__global__ void __launch_bounds__(256) bucket_list_kernel(BktJob *job, uint64_t *__restrict__ keys,
+                                                          uint32_t *__restrict__ vals) {
+    const BktJob &J = *job;
+    const uint32_t lane = threadIdx.x & 31, warps = gridDim.x * 8, w0 = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const RoundShape z = round_shape(J, J.hand_iter);
+    const ListIn li = list_in(J, J.hand_iter);
+    auto draw = [&](uint32_t table, uint32_t n) -> uint64_t {  // places for n entries of a table (lane 0)
+        return atomicAdd(&job->hand_ctr[table], n) + (table ? J.hand_s : 0ull);
+    };
+    for (uint32_t b = w0; b < 2 * z.nb; b += warps) {
+        const uint32_t n = min(li.cnt[b], li.cap);
+        if (!n) continue;
+        uint64_t at = lane == 0 ? draw(b & 1u, n) : 0;
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (uint32_t i = lane; i < n; i += 32) {
+            const uint4 e = li.lst[(uint64_t)b * li.cap + i];
+            keys[at + i] = e.x | (uint64_t)e.y << 32;
+            vals[at + i] = e.z;
+        }
+    }
+    const uint32_t ns = *li.spill_n;
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < ns; i += gridDim.x * 256) {
+        const uint4 e = li.spill[i];
+        const uint64_t at = draw(li.stag[i] & 1u, 1u);
+        keys[at] = e.x | (uint64_t)e.y << 32;
+        vals[at] = e.z;
+    }
+}
+
 }  // namespace
+
+cudaError_t launch_bucket_list(BktJob *job, uint64_t *keys, uint32_t *vals, cudaStream_t s) {
+    count_launch();
+    bucket_list_kernel<<<148 * 8, 256, 0, s>>>(job, keys, vals);
+    return cudaGetLastError();
+}
 
 bool bucket_prologue_apart(const BktJob &hj) {
     return hj.iter0 == 0 && hj.n_in > 0 && bkt_count(hj.n_in, hj.wave, hj.mean) > kBktMaxBuckets;

@@ -319,7 +319,7 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
     uint32_t *const filter = kPass == 2 ? J.filter2 : J.filter1;
     const uint32_t words = kPass == 2 ? l.w2 : l.w1, len0 = (uint32_t)J.L - l.r - 1u;
     const uint32_t inv1 = J.tables->inv1, inv2 = J.tables->inv2;
-    const bool host_used = J.r0 > 0;
+    const bool host_used = J.marked, stepped = b == 0 && J.stepped;
     uint64_t *const win = J.bases + o;  // the suffixes' bases of the step, from pass A to pass C
     uint32_t live_n = 0;
     const uint64_t from = half ? e0 - side0 : e0;  // where the entries are read
@@ -379,7 +379,8 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
                 if (q < R) {  // the same in every lane
                     const uint32_t v = (uint32_t)bases & 3u;
                     bases >>= 2;
-                    if (kPfx) {
+                    if (u == 0 && q0 == 0 && stepped) {
+                    } else if (kPfx) {
                         step_pfx(f1, f2, v, inv1, inv2);
                     } else {
                         step_sfx(f1, f2, mult[(len0 - q) * 4 + v]);
@@ -651,7 +652,7 @@ EMP_DEV void round_sizes(SweepJob &J, SShared &sh) {
     uint32_t ts, tp, tb, tr;
     const uint32_t es = block_exclusive_scan<kST, uint32_t>(fs, sh.scan32, &ts);
     const uint32_t ep = block_exclusive_scan<kST, uint32_t>(fp, sh.scan32, &tp);
-    const uint32_t s0 = J.r0 > 0 ? vld(J.s0) : J.n_s, p0 = J.r0 > 0 ? vld(J.p0) : J.n_p;
+    const uint32_t s0 = J.marked ? vld(J.s0) : J.n_s, p0 = J.marked ? vld(J.p0) : J.n_p;
     const uint32_t S = s0 - es, P = p0 - ep;
     block_exclusive_scan<kST, uint32_t>(t < nr && S > 0 ? 1u : 0u, sh.scan32, &tr);
     const uint32_t c = fs + fp;
@@ -885,7 +886,7 @@ EMP_DEV void next_step(SweepJob &J, SweepLoc &l, uint32_t b) {
     if (!l.act) return;
     const SweepCtr &c = J.ctr[(b - 1) % 3];
     l.gclean = max(l.gclean, l.gm);
-    if (b == 1 && J.r0 > 0) {  // counted by the first step
+    if (b == 1 && J.marked) {  // counted by the first step
         l.ls = __ldcg(&c.ls);
         l.lp = __ldcg(&c.lp);
     }
@@ -1005,7 +1006,7 @@ __global__ void __launch_bounds__(kST, 1) sweep_kernel(SweepJob *jobs, CoopCtl *
             if (tid < J) {
                 SweepCtr &c = jobs[tid].ctr[(b + 1) % 3];
                 c.ls = c.lp = c.ovf = c.fired_s = c.fired_p = 0;
-                if (b == 0 && jobs[tid].r0 > 0) {
+                if (b == 0 && jobs[tid].marked) {
                     jobs[tid].s0 = __ldcg(&jobs[tid].ctr[0].ls);
                     jobs[tid].p0 = __ldcg(&jobs[tid].ctr[0].lp);
                 }

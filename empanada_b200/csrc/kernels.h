@@ -305,7 +305,20 @@ struct BktJob {
     uint64_t e_total;        // edges of the finished rounds of this launch
     uint64_t e_stage;        // staging buffer fill
     BktRound *meta;          // [rounds + 1], zeroed; round r at meta[r]
+    uint32_t hand;           // the launch may leave its last rounds to the sweep kernel (a job alone)
+    uint32_t hand_iter;      // it did, after this many iterations
+    uint64_t hand_n, hand_s; // entries and suffixes of the list it left
+    uint32_t hand_ctr[2];    // entries that launch_bucket_list has placed (zero at launch)
 };
+// When the rounds go over to the sweep kernel: at most kHandMost entries left
+// and fewer than 1 / kHandRate of them used in the last round, with
+// kHandRounds to come, or kHandFew left with kHandFewRounds to come.
+constexpr uint64_t kHandMost = 12ull << 20, kHandFew = 3ull << 20;
+constexpr uint32_t kHandRate = 6;
+constexpr int kHandRounds = 16, kHandFewRounds = 64;
+// The list of round r0 + hand_iter as [suffixes | prefixes], each in any
+// order, with that round's keys.
+cudaError_t launch_bucket_list(BktJob *job, uint64_t *keys, uint32_t *vals, cudaStream_t s);
 size_t bkt_scratch_bytes(uint64_t n_max);
 constexpr uint32_t kBktRegionCap = 2048;  // entries per (bucket, table) region: 15 sigma above the mean of 1450
 int bucket_grid_size();                             // 0: no cooperative launch on this device
@@ -322,9 +335,15 @@ cudaError_t launch_bucket_prologue(BktJob *job, cudaStream_t s);
 // ---- many rounds per step (k_sweep.cu) -------------------------------------
 constexpr int kSweepThreads = 1024;  // threads of a sweep CTA (one CTA per SM)
 constexpr int kSweepMaxR = 32;       // rounds of a step at most
-// Longer lists run in the bucket kernel: beyond this one round of every entry
-// no longer fits filters and groups within L2 (112.7M entries: 24.4 ms there).
-constexpr uint64_t kSweepMaxEntries = 16ull << 20;
+// Which lists start in the sweep kernel: up to kSweepMaxEntries entries, and
+// sparse ones (a first step of kSweepSparseR rounds) up to kSweepMaxSparse.
+// The others' first rounds run in the bucket kernel, which uses many entries
+// per round as cheaply as few.  All rounds, bucket kernel / sweep kernel /
+// handed over: 7.2M entries of a dense set 2.87 / 2.49 ms / -, 14.7M 3.94 /
+// 4.45 / 3.74, 21.4M with errors 16.9 / 11.5 / 10.9; sparse 15.5M 22.8 / 11.9
+// / 13.2, 22.8M 10.9 / 10.0 / 11.2, 41.8M 18.9 / 20.5 / -.
+constexpr uint64_t kSweepMaxEntries = 9ull << 20, kSweepMaxSparse = 24ull << 20;
+constexpr uint32_t kSweepSparseR = 4;
 constexpr int kSweepIters = 40;      // resolving iterations of a step at most (kSweepMaxR + 1 suffice)
 constexpr uint32_t kSweepShards = 16;  // counters of a job's candidates and pairs at most
 struct SweepShard {   // in a cache line of its own
@@ -344,7 +363,7 @@ struct SweepJob {
     // keys of round r0 - 1, val = rid | table << 31; both are overwritten
     uint64_t *key[2];
     uint32_t *val;
-    const uint8_t *used_s, *used_p;  // marks of rounds run before the launch (read when r0 > 0)
+    const uint8_t *used_s, *used_p;  // marks of rounds run before the launch (read when `marked`)
     uint32_t n_s, n_p;
     uint32_t first_r;        // rounds of its first step
     uint32_t shard_log;      // log2 of the counters of its candidates and pairs
@@ -378,12 +397,14 @@ struct SweepJob {
     // set by the launch
     uint32_t nrec;           // matched entries (zero at launch)
     uint32_t nbins;
-    uint32_t s0, p0;         // live suffixes / prefixes of round r0 (when r0 > 0)
+    uint32_t s0, p0;         // live suffixes / prefixes of round r0 (when `marked`)
     uint32_t round;          // rounds run
     uint32_t overflow;       // the edge buffer is too small (zero at launch)
     uint32_t crowded;        // a chain of too many entries: not a job for this kernel (zero at launch)
     uint64_t e_total;        // edges
     uint8_t cur0;
+    uint8_t marked;          // entries used before the launch are in the list, marked
+    uint8_t stepped;         // key[cur0] holds the keys of round r0 itself
     uint8_t one_half;        // the list at launch holds the suffixes only: the prefixes are the same entries
 };
 struct SweepOut {  // output bins of a launch's jobs (sweep_out_layout)
