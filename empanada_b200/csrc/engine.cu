@@ -194,6 +194,8 @@ struct JobPrep {
     uint64_t n = 0, n_rec = 0, U = 0, M = 0, wpc = 0, ecap = 0, launches0 = 0;
     int L = 0, wpr = 0, rounds = 0;
     bool done = false;  // nothing more to run (empty input, no reads)
+    bool dev_out = false;   // host-driven rounds left their records on the device
+    bool host_out = false;  // they go to host memory instead (no device memory to hold them)
     bool no_sweep = false;  // the rounds run in the bucket kernel (kCrowded)
     bool one_half = false;  // the list's prefix half, a copy of the suffixes', is not written (the sweep kernel needs none)
 };
@@ -254,7 +256,7 @@ namespace {
 
 // misc device words (u64 slots)
 enum MiscSlot { kMiscErr = 0, kMiscTotal = 1, kMiscLen = 2, kMiscN = 3, kMiscU = 4, kMiscNout = 5, kMiscSout = 6,
-                kMiscE = 7, kMiscParts = 9, kMiscSortN = 10, kMiscLen0 = 11, kMiscKept = 12,
+                kMiscE = 7, kMiscParts = 9, kMiscSortN = 10, kMiscLen0 = 11, kMiscKept = 12, kMiscRecs = 13,
                 kMiscSlots = 16 };
 
 // internal: the pipeline's edge buffer was too small (never returned by the ABI)
@@ -442,11 +444,20 @@ emp_status chunked_sort(emp_job *j, uint64_t *k, uint32_t *v, uint64_t *k1, uint
     EMP_TRY(ensure(j, j->cparts, pcap * sizeof(ChunkPart)));
     // sorted by key, then (stably) by chunk: each chunk sorted on its own
     seg_sort(j, k, v, k1, v1, n, s);
-    launch_chunk_keys(v, n, lst, M, j->xk0.as<uint64_t>(), j->xv0.as<uint32_t>(), s);
-    seg_sort(j, j->xk0.as<uint64_t>(), j->xv0.as<uint32_t>(), j->xk1.as<uint64_t>(), j->xv1.as<uint32_t>(), n, s);
+    // up to 256 chunks: one digit pass (6.7M entries in two chunks, 0.65 ms as
+    // a sort of any keys, whose groups do not fit, 0.08 so)
+    const bool digit = (n - 1) / M < (1u << kSortBits);
+    launch_chunk_keys(v, n, lst, M, digit ? kTopDigitShift : 32, j->xk0.as<uint64_t>(), j->xv0.as<uint32_t>(), s);
+    if (digit) {
+        ++j->sorts_since_clear;
+        sort_top_digit(j->xk0.as<uint64_t>(), j->xv0.as<uint32_t>(), j->xk1.as<uint64_t>(), j->xv1.as<uint32_t>(), n,
+                       j->sort_scratch.p, err_word(j), s);
+    } else {
+        seg_sort(j, j->xk0.as<uint64_t>(), j->xv0.as<uint32_t>(), j->xk1.as<uint64_t>(), j->xv1.as<uint32_t>(), n, s);
+    }
     uint64_t *rk = j->ring_k.as<uint64_t>();
     uint32_t *rv = j->ring_v.as<uint32_t>();
-    launch_ring_gather(k, v, j->xv0.as<uint32_t>(), n, rk, rv, s);
+    launch_ring_gather(k, v, digit ? j->xv1.as<uint32_t>() : j->xv0.as<uint32_t>(), n, rk, rv, s);
     // the FIFO of sorted tables (ring start, entries), oldest first
     std::deque<std::pair<uint64_t, uint64_t>> q;
     for (uint64_t off = 0; off < n; off += M) q.emplace_back(off, n - off < M ? n - off : M);
@@ -477,6 +488,25 @@ void emit_record(emp_job *j, int32_t ovlp, uint64_t e0, uint64_t e1) {
         append_bytes(j->out, j->h_to.as<uint32_t>() + e0, ne * 4);
     }
     j->st.n_records += 1;
+}
+
+// Room for `bytes` of output on the device, `ahead` more when it grows; the
+// records that are there stay.
+emp_status dout_room(emp_job *j, size_t bytes, size_t ahead, cudaStream_t s) {
+    if (!j->dout_bytes) {
+        if (bytes <= j->dout.bytes) return EMP_OK;
+        const emp_status rc = ahead ? ensure(j, j->dout, bytes + ahead) : EMP_E_NOMEM;
+        return rc == EMP_OK ? rc : ensure(j, j->dout, bytes);
+    }
+    if (bytes <= j->dout.bytes) return EMP_OK;
+    DevBuf nb;
+    if (!ahead || ctx_ensure(j->ctx, nb, bytes + ahead, s) != EMP_OK) EMP_TRY(ctx_ensure(j->ctx, nb, bytes, s));
+    const cudaError_t e = cudaMemcpyAsync(nb.p, j->dout.p, j->dout_bytes, cudaMemcpyDeviceToDevice, s);
+    swap_buf(nb, j->dout);
+    j->ctx->in_use -= nb.bytes;
+    cudaFreeAsync(nb.p, s);
+    nb.p = nullptr;
+    return cuda_status(e);
 }
 
 struct RoundEnv {
@@ -564,16 +594,32 @@ emp_status sync_round(emp_job *j, cudaStream_t s, const RoundEnv &env, int r, in
     if (E) {
         EMP_TRY(ensure(j, j->efrom, E * 4));
         EMP_TRY(ensure(j, j->eto, E * 4));
-        if (!j->h_from.ensure(E * 4) || !j->h_to.ensure(E * 4)) return EMP_E_NOMEM;
         launch_join_write(sk, sv, N, j->cnt.as<uint32_t>(), j->offs.as<uint64_t>(), j->efrom.as<uint32_t>(),
                           j->eto.as<uint32_t>(), j->used_s.as<uint8_t>(), j->used_p.as<uint8_t>(), s);
-        EMP_CUDA(cudaMemcpyAsync(j->h_from.p, j->efrom.p, E * 4, cudaMemcpyDeviceToHost, s));
-        EMP_CUDA(cudaMemcpyAsync(j->h_to.p, j->eto.p, E * 4, cudaMemcpyDeviceToHost, s));
-        EMP_CUDA(cudaStreamSynchronize(s));
+        if (j->prep.host_out) {
+            if (!j->h_from.ensure(E * 4) || !j->h_to.ensure(E * 4)) return EMP_E_NOMEM;
+            EMP_CUDA(cudaMemcpyAsync(j->h_from.p, j->efrom.p, E * 4, cudaMemcpyDeviceToHost, s));
+            EMP_CUDA(cudaMemcpyAsync(j->h_to.p, j->eto.p, E * 4, cudaMemcpyDeviceToHost, s));
+            EMP_CUDA(cudaStreamSynchronize(s));
+        }
     }
     const int32_t ovlp = env.L - 1 - r;
+    // the round's records, behind those before it: on the device, for the
+    // output's one copy out (through host arrays and a host vector 33 MB of
+    // them took 7 ms of 15)
+    auto records = [&](const SearchPart *parts, uint64_t np, uint64_t nrec, uint64_t nedge) -> emp_status {
+        const size_t bytes = 12 * nrec + 8 * nedge;
+        j->prep.dev_out = true;
+        EMP_TRY(dout_room(j, j->dout_bytes + bytes, (size_t)env.rounds * 12 + j->prep.ecap * 8, s));
+        launch_write_records(parts, np, E, ovlp, j->efrom.as<uint32_t>(), j->eto.as<uint32_t>(),
+                             j->dout.as<uint8_t>() + j->dout_bytes, s);
+        j->dout_bytes += bytes;
+        st.n_records += nrec;
+        return EMP_OK;
+    };
     if (!split) {
-        emit_record(j, ovlp, 0, E);
+        if (j->prep.host_out) emit_record(j, ovlp, 0, E);
+        else EMP_TRY(records(nullptr, 0, 1, E));
     } else {
         // search partitions of windows M/2; each two-sided one is a record
         EMP_TRY(ensure(j, j->akeys, S * 8));
@@ -586,17 +632,21 @@ emp_status sync_round(emp_job *j, cudaStream_t s, const RoundEnv &env, int r, in
                             chain_words(j), chain_ctr(j), err_word(j), s);
         launch_search_partitions(j->akeys.as<uint64_t>(), S, j->bkeys.as<uint64_t>(), P, M / 2,
                                  j->apos.as<uint32_t>(), j->offs.as<uint64_t>(), E, j->parts.as<SearchPart>(), pcap,
-                                 dm + kMiscParts, err_word(j), s);
+                                 dm + kMiscParts, dm + kMiscRecs, err_word(j), s);
         EMP_TRY(sync_and_check(j, s));
         if (hm[kMiscErr] & kErrHang) return EMP_E_HANG;
         if (hm[kMiscErr] & kErrCapacity) return EMP_E_UNSUPPORTED;
         const uint64_t np = hm[kMiscParts];
-        if (!j->h_parts.ensure(np * sizeof(SearchPart) + 16)) return EMP_E_NOMEM;
-        EMP_CUDA(cudaMemcpyAsync(j->h_parts.p, j->parts.p, np * sizeof(SearchPart), cudaMemcpyDeviceToHost, s));
-        EMP_CUDA(cudaStreamSynchronize(s));
-        const SearchPart *ps = j->h_parts.as<SearchPart>();
-        for (uint64_t q = 0; q < np; ++q)
-            if (ps[q].pa && ps[q].pb) emit_record(j, ovlp, ps[q].e0, ps[q].e1);
+        if (!j->prep.host_out) {
+            EMP_TRY(records(j->parts.as<SearchPart>(), np, hm[kMiscRecs], hm[kMiscRecs + 1]));
+        } else {
+            if (!j->h_parts.ensure(np * sizeof(SearchPart) + 16)) return EMP_E_NOMEM;
+            EMP_CUDA(cudaMemcpyAsync(j->h_parts.p, j->parts.p, np * sizeof(SearchPart), cudaMemcpyDeviceToHost, s));
+            EMP_CUDA(cudaStreamSynchronize(s));
+            const SearchPart *ps = j->h_parts.as<SearchPart>();
+            for (uint64_t q = 0; q < np; ++q)
+                if (ps[q].pa && ps[q].pb) emit_record(j, ovlp, ps[q].e0, ps[q].e1);
+        }
     }
     st.n_edges += E;
     if (r < EMP_MAX_ROUNDS) st.edges[r] = E;
@@ -696,7 +746,8 @@ emp_status bucket_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r
     EMP_TRY(ensure(j, j->bk_scratch, bkt_scratch_bytes(nmax)));
     EMP_TRY(ensure(j, j->bk_meta, ((size_t)env.rounds + 1) * sizeof(BktRound)));
     EMP_CUDA(cudaMemsetAsync(j->bk_meta.p, 0, ((size_t)env.rounds + 1) * sizeof(BktRound), s));
-    EMP_TRY(ensure(j, j->dout, (size_t)env.rounds * 12 + ecap * 8));
+    // behind the records of host-driven rounds
+    EMP_TRY(dout_room(j, (size_t)j->dout_bytes + (size_t)env.rounds * 12 + ecap * 8, 0, s));
     EMP_TRY(ensure(j, j->records, (size_t)env.rounds * sizeof(RoundRecord)));
     if (!j->h_records.ensure((size_t)env.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
     std::memset(hj, 0, sizeof(BktJob));
@@ -722,7 +773,7 @@ emp_status bucket_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r
     hj->spans = j->bk_spans.as<BktSpan>();
     hj->sfrom = j->bk_sfrom.as<uint32_t>();
     hj->sto = j->bk_sto.as<uint32_t>();
-    hj->out = j->dout.as<uint8_t>();
+    hj->out = j->dout.as<uint8_t>() + j->dout_bytes;
     hj->ecap = ecap;
     hj->records = j->records.as<RoundRecord>();
     hj->scratch = j->bk_scratch.as<uint8_t>();
@@ -902,7 +953,7 @@ emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0
     EMP_TRY(ensure(j, j->swp, sweep_layout(nullptr, hj, &zeroed)));
     sweep_layout(j->swp.as<uint8_t>(), hj, &zeroed);
     // behind the records of the rounds that ran before, whose buffer held all
-    EMP_TRY(ensure(j, j->dout, (size_t)j->dout_bytes + (size_t)(env.rounds - r0) * 12 + ecap * 8));
+    EMP_TRY(dout_room(j, (size_t)j->dout_bytes + (size_t)(env.rounds - r0) * 12 + ecap * 8, 0, s));
     hj->out = j->dout.as<uint8_t>() + j->dout_bytes;
     return EMP_OK;
 }
@@ -1277,6 +1328,9 @@ emp_status job_rounds(emp_job *j, cudaStream_t s) {
         if (rc == EMP_OK) return EMP_OK;
         if (rc == kCrowded) {
             q.no_sweep = true;
+        } else if (rc == EMP_E_NOMEM && q.dev_out && !q.host_out) {
+            q.host_out = true;
+            free_buf(j, j->dout);
         } else {
             if (rc != kNeedEdgeRoom || attempt >= 3) return rc == kNeedEdgeRoom ? EMP_E_NOMEM : rc;
             q.ecap = needed + needed / 4 + 1024;

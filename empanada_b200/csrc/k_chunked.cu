@@ -61,7 +61,7 @@ EMP_DEV uint64_t rid_lower(const uint32_t *lst, uint64_t lo, uint64_t hi, uint32
 // below the entry's -- the position in the id-sorted table that the
 // reference cuts into chunks (regenerate_fingerprints, overlap.cu:605-667).
 __global__ void chunk_keys_kernel(const uint32_t *__restrict__ v, uint64_t n, const uint32_t *__restrict__ lst,
-                                  uint64_t M, uint64_t *__restrict__ ck, uint32_t *__restrict__ ci) {
+                                  uint64_t M, int shift, uint64_t *__restrict__ ck, uint32_t *__restrict__ ci) {
     uint64_t n_even = 0;
     if (lst) {  // the parity boundary of the list
         uint64_t lo = 0, hi = n;
@@ -75,7 +75,7 @@ __global__ void chunk_keys_kernel(const uint32_t *__restrict__ v, uint64_t n, co
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t rid = rid_of(v[i]);
         const uint64_t rank = lst ? rid_lower(lst, 0, n_even, rid) + (rid_lower(lst, n_even, n, rid) - n_even) : rid;
-        ck[i] = (rank / M) << 32;  // sort_key keeps the chunk order (chunk < 2^34)
+        ck[i] = (rank / M) << shift;
         ci[i] = (uint32_t)i;
     }
 }
@@ -195,10 +195,10 @@ int grid_for(uint64_t n) {
 
 }  // namespace
 
-void launch_chunk_keys(const uint32_t *v, uint64_t n, const uint32_t *lst, uint64_t M, uint64_t *ck, uint32_t *ci,
-                       cudaStream_t s) {
+void launch_chunk_keys(const uint32_t *v, uint64_t n, const uint32_t *lst, uint64_t M, int shift, uint64_t *ck,
+                       uint32_t *ci, cudaStream_t s) {
     count_launch();
-    chunk_keys_kernel<<<grid_for(n), 256, 0, s>>>(v, n, lst, M, ck, ci);
+    chunk_keys_kernel<<<grid_for(n), 256, 0, s>>>(v, n, lst, M, shift, ck, ci);
 }
 
 void launch_ring_gather(const uint64_t *k, const uint32_t *v, const uint32_t *idx, uint64_t n, uint64_t *rk,

@@ -247,9 +247,9 @@ EMP_DEV uint64_t lower_bound_dev(const uint64_t *a, uint64_t lo, uint64_t hi, ui
 __global__ void search_partitions_kernel(const uint64_t *__restrict__ A, uint64_t S, const uint64_t *__restrict__ B,
                                          uint64_t P, uint64_t h, const uint32_t *__restrict__ apos,
                                          const uint64_t *__restrict__ offs, uint64_t E, SearchPart *parts,
-                                         uint64_t cap, uint64_t *count, uint32_t *err) {
+                                         uint64_t cap, uint64_t *count, uint64_t *recs, uint32_t *err) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    uint64_t offA = 0, offB = 0, np = 0;
+    uint64_t offA = 0, offB = 0, np = 0, nrec = 0, nedge = 0;
     bool failed = false;
     auto eoff = [&](uint64_t rank) -> uint64_t { return rank < S ? offs[apos[rank]] : E; };
     auto push = [&](uint64_t pa, uint64_t pb) -> bool {
@@ -262,6 +262,11 @@ __global__ void search_partitions_kernel(const uint64_t *__restrict__ A, uint64_
         parts[np].pb = pb;
         parts[np].e0 = eoff(offA);
         parts[np].e1 = eoff(offA + pa);
+        parts[np].off = 12 * nrec + 8 * nedge;
+        if (pa && pb) {  // a record
+            ++nrec;
+            nedge += parts[np].e1 - parts[np].e0;
+        }
         ++np;
         return true;
     };
@@ -291,6 +296,36 @@ __global__ void search_partitions_kernel(const uint64_t *__restrict__ A, uint64_
         else if (offB == P && offA < S) push(S - offA, 0);
     }
     *count = np;
+    recs[0] = nrec;
+    recs[1] = nedge;
+}
+
+// u64 n, i32 ovlp_len, from[n], to[n] (write_edges_binary, overlap.cu:148-161)
+__global__ void write_records_kernel(const SearchPart *__restrict__ parts, uint64_t np, uint64_t E, int32_t ovlp,
+                                     const uint32_t *__restrict__ from, const uint32_t *__restrict__ to, uint8_t *out) {
+    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const SearchPart whole{1, 1, 0, E, 0};
+    for (uint64_t q = t; q < (parts ? np : 1); q += step) {
+        const SearchPart p = parts ? parts[q] : whole;
+        if (!p.pa || !p.pb) continue;
+        uint32_t *h = reinterpret_cast<uint32_t *>(out + p.off);
+        h[0] = (uint32_t)(p.e1 - p.e0);
+        h[1] = (uint32_t)((p.e1 - p.e0) >> 32);
+        h[2] = (uint32_t)ovlp;
+    }
+    for (uint64_t e = t; e < E; e += step) {
+        uint64_t lo = 0, hi = parts ? np : 1;  // the last partition that starts at or before e
+        while (hi - lo > 1) {
+            const uint64_t m = (lo + hi) >> 1;
+            if (parts[m].e0 <= e) lo = m;
+            else hi = m;
+        }
+        const SearchPart p = parts ? parts[lo] : whole;
+        if (!p.pa || !p.pb || e >= p.e1) continue;
+        uint32_t *f = reinterpret_cast<uint32_t *>(out + p.off + 12);
+        f[e - p.e0] = from[e];
+        f[(p.e1 - p.e0) + (e - p.e0)] = to[e];
+    }
 }
 
 static unsigned grid_for(uint64_t work, unsigned per_block, unsigned cap) {
@@ -348,9 +383,15 @@ void launch_split_tables(const uint64_t *skeys, const uint32_t *svals, uint64_t 
 
 void launch_search_partitions(const uint64_t *akeys, uint64_t S, const uint64_t *bkeys, uint64_t P, uint64_t h,
                               const uint32_t *apos, const uint64_t *offs, uint64_t E, SearchPart *parts,
-                              uint64_t cap, uint64_t *count, uint32_t *err, cudaStream_t s) {
+                              uint64_t cap, uint64_t *count, uint64_t *recs, uint32_t *err, cudaStream_t s) {
     count_launch();
-    search_partitions_kernel<<<1, 32, 0, s>>>(akeys, S, bkeys, P, h, apos, offs, E, parts, cap, count, err);
+    search_partitions_kernel<<<1, 32, 0, s>>>(akeys, S, bkeys, P, h, apos, offs, E, parts, cap, count, recs, err);
+}
+
+void launch_write_records(const SearchPart *parts, uint64_t np, uint64_t E, int32_t ovlp, const uint32_t *from,
+                          const uint32_t *to, uint8_t *out, cudaStream_t s) {
+    count_launch();
+    write_records_kernel<<<grid_for(E > np ? E : np, 256, 148 * 16), 256, 0, s>>>(parts, np, E, ovlp, from, to, out);
 }
 
 void launch_join_count(const uint64_t *skeys, const uint32_t *svals, uint64_t n, uint32_t *cnt, cudaStream_t s) {

@@ -425,6 +425,20 @@ void sort_radix(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t
     }
 }
 
+void sort_top_digit(const uint64_t *k0, const uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch,
+                    uint32_t *err, cudaStream_t s) {
+    static_assert(kTopDigitShift == kKeyBits - kSortBits + 2, "bit b >= 32 of a key is bit b - 2 of its sort key");
+    if (!n) return;
+    const SortGrid sg = sort_setup();
+    SortScratch *sc = reinterpret_cast<SortScratch *>(scratch);
+    const uint64_t hb = (n + 2047) / 2048;
+    count_launch(3);
+    sort_prepare_kernel<<<1, 256, 0, s>>>(sc, false);
+    group_hist_kernel<1><<<(unsigned)(hb < 148 * 4 ? hb : 148 * 4), 512, 0, s>>>(k0, n, sc);
+    onesweep_kernel<<<sweep_grid(n, sg), kBlkThreads, kOnesweepSmem, s>>>(k0, v0, k1, v1, n, 0, kKeyBits - kSortBits, 0u,
+                                                                          sc, err);
+}
+
 void sort_pairs(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch, uint32_t *err,
                 cudaStream_t s, cudaEvent_t *events) {
     if (events) cudaEventRecord(events[0], s);  // the first pass's events take in the groups

@@ -125,17 +125,22 @@ void sort_groups(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_
 void sort_radix(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch, uint32_t *err,
                 cudaStream_t s, cudaEvent_t *events = nullptr);
 uint32_t *sort_flags(void *scratch);
+// Stable sort by the key's top digit alone (its bits kTopDigitShift ..), into
+// (k1, v1); the other bits of the sort key are zero above it.
+constexpr int kTopDigitShift = 53;
+void sort_top_digit(const uint64_t *k0, const uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch,
+                    uint32_t *err, cudaStream_t s);
 
 // ---- sort of a table larger than M (k_chunked.cu) --------------------------
 struct ChunkPart {  // one merge partition: A entries [a0, a0+pa), B entries [b0, b0+pb)
     uint64_t a0, pa, b0, pb;
 };
-// Chunk of each entry of (v)[0..n) as a sort key ((rank / M) << 32) with its
+// Chunk of each entry of (v)[0..n) as a sort key ((rank / M) << shift) with its
 // index: rank = read-end id when lst is null (the table holds ids 0..n-1 in
 // order), else the entry's rank among the ids of lst (the table in list
 // order: even ids ascending, then odd ids ascending).
-void launch_chunk_keys(const uint32_t *v, uint64_t n, const uint32_t *lst, uint64_t M, uint64_t *ck, uint32_t *ci,
-                       cudaStream_t s);
+void launch_chunk_keys(const uint32_t *v, uint64_t n, const uint32_t *lst, uint64_t M, int shift, uint64_t *ck,
+                       uint32_t *ci, cudaStream_t s);
 // (rk, rv)[i] = (k, v)[idx[i]], i < n
 void launch_ring_gather(const uint64_t *k, const uint32_t *v, const uint32_t *idx, uint64_t n, uint64_t *rk,
                         uint32_t *rv, cudaStream_t s);
@@ -188,11 +193,17 @@ void launch_split_tables(const uint64_t *skeys, const uint32_t *svals, uint64_t 
 struct SearchPart {
     uint64_t pa, pb;  // suffixes / prefixes in the partition
     uint64_t e0, e1;  // its edges in the round's edge list
+    uint64_t off;     // its record's offset among the round's (12 bytes and 8 an edge each); one-sided: none
 };
 // One thread walks the reference's partition loop with windows of h = M/2.
+// count[0]: the partitions; recs[0], recs[1]: the two-sided ones, their edges.
 void launch_search_partitions(const uint64_t *akeys, uint64_t S, const uint64_t *bkeys, uint64_t P, uint64_t h,
                               const uint32_t *apos, const uint64_t *offs, uint64_t E, SearchPart *parts,
-                              uint64_t cap, uint64_t *count, uint32_t *err, cudaStream_t s);
+                              uint64_t cap, uint64_t *count, uint64_t *recs, uint32_t *err, cudaStream_t s);
+// The records of a round's partitions (parts null: one record of all E edges)
+// at `out`, from its edges in list order.
+void launch_write_records(const SearchPart *parts, uint64_t np, uint64_t E, int32_t ovlp, const uint32_t *from,
+                          const uint32_t *to, uint8_t *out, cudaStream_t s);
 // ---- per-round counts of the all-rounds kernel --------------------------
 struct RoundRecord {
     uint64_t S, P, E, e0;  // table sizes, edges, first edge of the round
