@@ -52,7 +52,12 @@ namespace {
 constexpr int kST = kSweepThreads;      // 1024: one CTA per SM
 constexpr int kSW = kST / 32;
 constexpr uint32_t kNever = 0xffffffffu;
-constexpr uint64_t kFilterKeys = 25u << 20;  // (entry, round) keys of a step's first filters: 48 MB, within L2
+// (entry, round) keys of a step's first filters at most, and those up to which
+// a key has 12 bits instead of 10.  Fewer keys a step would stay within L2 (a
+// batch of 13.2M reads: 25M keys of 16 bits 29.8 ms, 56M of 12 26.2, 80M of 10
+// 26.0, 112M of 12 27.4), but then every live entry is read and compacted for
+// fewer rounds; fewer bits cost false candidates.
+constexpr uint64_t kFilterKeys = 80u << 20, kFilterRoomy = 32u << 20;
 constexpr uint32_t kU = 4;              // filter accesses of a lane in flight
 constexpr uint32_t kQCap = 32 * (kU + 1);  // queued candidates per warp
 constexpr uint32_t kBinMean = 32;       // matched entries per output bin aimed at
@@ -319,7 +324,7 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
     uint32_t *const filter = kPass == 2 ? J.filter2 : J.filter1;
     const uint32_t words = kPass == 2 ? l.w2 : l.w1, len0 = (uint32_t)J.L - l.r - 1u;
     const uint32_t inv1 = J.tables->inv1, inv2 = J.tables->inv2;
-    const bool host_used = J.marked, stepped = b == 0 && J.stepped;
+    const bool host_used = J.marked, stepped = J.stepped && l.r == (uint32_t)J.r0;  // in every try of the first step
     uint64_t *const win = J.bases + o;  // the suffixes' bases of the step, from pass A to pass C
     uint32_t live_n = 0;
     const uint64_t from = half ? e0 - side0 : e0;  // where the entries are read
@@ -922,7 +927,8 @@ EMP_DEV void size_filters(const SweepJob &J, SweepLoc &l, uint64_t all) {
     const uint64_t cap = all ? kFilterKeys / all : 1;
     if (l.R > cap) l.R = cap < 1 ? 1u : (uint32_t)cap;
     while (l.R > 1 && (uint64_t)l.ls * l.R > 4ull * J.w1_max) l.R = (l.R + 1) / 2;  // 8 bits per key where memory ends
-    const uint64_t w = ((uint64_t)l.ls * l.R + 1) / 2;  // 16 bits per (entry, round)
+    const uint64_t keys = (uint64_t)l.ls * l.R;
+    const uint64_t w = all * l.R <= kFilterRoomy ? (keys * 3 + 7) / 8 : (keys * 5 + 15) / 16;
     l.w1 = (uint32_t)(w < 1024 ? 1024 : w < J.w1_max ? (w + 3) / 4 * 4 : J.w1_max);
     l.w2 = l.w1 > 4096 ? (l.w1 / 4 + 3) / 4 * 4 : 1024;
 }
@@ -1170,7 +1176,7 @@ size_t sweep_layout(uint8_t *base, SweepJob *J, size_t *zeroed) {
     };
     const uint64_t ns = J->n_s, np = J->n_p, n = ns + np;
     const int rounds = J->rounds;
-    // filter 1 holds eight rounds of every suffix at 16 bits each
+    // filter 1 holds twelve rounds of every suffix at 10 bits each
     const uint64_t w1 = ns < 256 ? 1024 : 4 * ns < (1u << 24) ? 4 * ns : 1u << 24;
     J->w1_max = (uint32_t)w1;
     uint32_t gm = 10;
