@@ -153,7 +153,9 @@ struct SweepBatch {
     }
 };
 
-constexpr int kMapStreams = 32;     // streams of a batch's map phase at most
+// emp_tuning::map_streams: accepted and reported, without effect since a
+// batch's map phase is one launch per kernel
+constexpr int kMapStreams = 32;
 constexpr int kMapStreamsDefault = 8;
 
 struct emp_ctx {
@@ -179,10 +181,11 @@ struct emp_ctx {
     SweepBatch batch_swp;
     PinnedBuf h_batch;
     cudaEvent_t batch_ev[2] = {};
-    // the map phase of a batch of jobs: jobs on kMapStreams streams, so that
-    // the small kernels of small read sets run side by side
-    cudaStream_t map_streams[kMapStreams] = {};
-    cudaEvent_t map_ev[kMapStreams + 1] = {};
+    // the map phase of a batch of jobs: arguments, block lists and fetched
+    // words of a stage's launches; the phase's start, its reads, its lists
+    DevBuf many;
+    PinnedBuf h_many;
+    cudaEvent_t many_ev[3] = {};
     emp_tuning tune{};  // engine choices (zero fields: defaults)
     // profiling aids, read from the environment when the context is made:
     // EMP_COOP_TRACE=<file> (per-round durations of the bucket kernel),
@@ -194,6 +197,8 @@ struct JobPrep {
     uint64_t n = 0, n_rec = 0, U = 0, M = 0, wpc = 0, ecap = 0, launches0 = 0;
     int L = 0, wpr = 0, rounds = 0;
     bool done = false;  // nothing more to run (empty input, no reads)
+    bool shared = false;    // the map phase ran in launches for a whole batch, which took
+    float ms_map = 0, ms_dedup = 0;
     bool dev_out = false;   // host-driven rounds left their records on the device
     bool host_out = false;  // they go to host memory instead (no device memory to hold them)
     bool no_sweep = false;  // the rounds run in the bucket kernel (kCrowded)
@@ -1061,7 +1066,103 @@ emp_status run_rounds(emp_job *j, cudaStream_t s, const RoundEnv &env, uint64_t 
 // a count before sizing the next step (one stream synchronisation between
 // stages; a batch of jobs shares it).  A stage returns EMP_OK with j->prep.done
 // set once the job has nothing more to run.
-emp_status map_begin(emp_job *j, cudaStream_t s) {
+// The launches of a stage for all jobs of a batch, collected and then queued
+// as one per kernel, their arguments and block lists in one copy: ten launches
+// and five copies a job on eight streams took 10.3 ms for 256 jobs, this 7.1
+// (6.5 of it kernels), and the calls themselves 3 ms more.
+struct MapMany {
+    std::vector<NlArgs> nl;
+    std::vector<ScanArgs> scan;
+    std::vector<ReadArgs> read;
+    std::vector<DedupArgs> dedup;
+    std::vector<InitArgs> init;
+    std::vector<emp_job *> fetch;
+    uint32_t nb_max = 0;
+};
+// Queue what was collected, then the fetched jobs' words into their host
+// slots; waits for the stream.
+emp_status many_flush(emp_ctx *c, MapMany &m, cudaStream_t s) {
+    if (!m.read.empty()) {  // two turns of the resident CTAs, by the jobs' tiles
+        uint64_t tiles = 0;
+        for (const ReadArgs &a : m.read) tiles += parse_tiles(a.F);
+        const uint64_t want = 2ull * read_pass_grid();
+        for (ReadArgs &a : m.read) {
+            const uint64_t t = parse_tiles(a.F), b = (t * want + tiles - 1) / tiles;
+            a.blocks = (uint32_t)(b < t ? b : t);
+        }
+    }
+    // blocks of entry k of list q: nl, scan, read, hist, scatter, mark, init
+    auto blocks_of = [&](int q, size_t k) -> uint32_t {
+        switch (q) {
+            case 0: return (uint32_t)parse_tiles(m.nl[k].F);
+            case 1: return (uint32_t)scan_tiles(m.scan[k].n);
+            case 2: return m.read[k].blocks;
+            case 3: return m.dedup[k].hist_blocks;
+            case 4: return m.dedup[k].scatter_blocks;
+            case 5: return m.dedup[k].mark_blocks;
+            default: return (uint32_t)upd_tiles(2 * m.init[k].n);
+        }
+    };
+    const size_t entries[7] = {m.nl.size(),    m.scan.size(),  m.read.size(), m.dedup.size(),
+                               m.dedup.size(), m.dedup.size(), m.init.size()};
+    size_t nblk[7] = {};
+    for (int q = 0; q < 7; ++q)
+        for (size_t k = 0; k < entries[q]; ++k) nblk[q] += blocks_of(q, k);
+    size_t total = 0, at[13];
+    int part = 0;
+    auto add = [&](size_t bytes) {
+        at[part++] = total;
+        total += (bytes + 255) / 256 * 256;
+    };
+    add(m.nl.size() * sizeof(NlArgs));
+    add(m.scan.size() * sizeof(ScanArgs));
+    add(m.read.size() * sizeof(ReadArgs));
+    add(m.dedup.size() * sizeof(DedupArgs));
+    add(m.init.size() * sizeof(InitArgs));
+    for (size_t b : nblk) add(b * sizeof(uint2));
+    add(m.fetch.size() * sizeof(uint64_t *));
+    static_assert(kMiscSlots == 16, "a job's words as launch_gather_words takes them");
+    const size_t words = m.fetch.size() * kMiscSlots * 8;
+    EMP_TRY(ctx_ensure(c, c->many, total + words + 256, s));
+    if (!c->h_many.ensure(total + words + 256)) return EMP_E_NOMEM;
+    uint8_t *h = c->h_many.as<uint8_t>(), *d = c->many.as<uint8_t>();
+    auto put = [&](int k, const auto &v) {
+        if (!v.empty()) std::memcpy(h + at[k], v.data(), v.size() * sizeof(v[0]));
+    };
+    put(0, m.nl);
+    put(1, m.scan);
+    put(2, m.read);
+    put(3, m.dedup);
+    put(4, m.init);
+    for (int q = 0; q < 7; ++q) {
+        uint2 *o = reinterpret_cast<uint2 *>(h + at[5 + q]);
+        for (size_t k = 0; k < entries[q]; ++k) {
+            const uint32_t c = blocks_of(q, k);
+            for (uint32_t b = 0; b < c; ++b) *o++ = make_uint2((uint32_t)k, b);
+        }
+    }
+    uint64_t **src = reinterpret_cast<uint64_t **>(h + at[12]);
+    for (size_t k = 0; k < m.fetch.size(); ++k) src[k] = m.fetch[k]->misc.as<uint64_t>();
+    if (total) EMP_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, s));
+    auto blocks = [&](int k) { return ManyBlocks{reinterpret_cast<const uint2 *>(d + at[5 + k]), (uint32_t)nblk[k]}; };
+    launch_nl_count_many(reinterpret_cast<const NlArgs *>(d + at[0]), blocks(0), s);
+    launch_scan_many(reinterpret_cast<const ScanArgs *>(d + at[1]), blocks(1), s);
+    launch_read_pass_many(reinterpret_cast<const ReadArgs *>(d + at[2]), blocks(2), s);
+    launch_dedup_many(reinterpret_cast<const DedupArgs *>(d + at[3]), (uint32_t)m.dedup.size(), m.nb_max, blocks(3),
+                      blocks(4), blocks(5), s);
+    launch_init_list_many(reinterpret_cast<const InitArgs *>(d + at[4]), blocks(6), s);
+    launch_gather_words(reinterpret_cast<const uint64_t *const *>(d + at[12]), (uint32_t)m.fetch.size(),
+                        reinterpret_cast<uint64_t *>(d + total), s);
+    if (words) EMP_CUDA(cudaMemcpyAsync(h + total, d + total, words, cudaMemcpyDeviceToHost, s));
+    EMP_CUDA(cudaStreamSynchronize(s));
+    EMP_CUDA(cudaGetLastError());
+    for (size_t k = 0; k < m.fetch.size(); ++k)
+        std::memcpy(m.fetch[k]->h_misc.p, h + total + k * kMiscSlots * 8, kMiscSlots * 8);
+    m = MapMany{};
+    return EMP_OK;
+}
+
+emp_status map_begin(emp_job *j, cudaStream_t s, MapMany *mm = nullptr) {
     emp_stats &st = j->st;
     j->stream = s;
     if (j->feed_pending) {  // the FASTQ is still being copied in
@@ -1080,26 +1181,38 @@ emp_status map_begin(emp_job *j, cudaStream_t s) {
     j->prep.launches0 = g_launches.load();
     j->prep.M = j->p.reduce_mem / 16;
     if (j->prep.M < 2) return EMP_E_INVAL;
-    cudaEventRecord(j->map_ev[0], s);
+    j->prep.shared = mm != nullptr;
+    if (!mm) cudaEventRecord(j->map_ev[0], s);
     EMP_TRY(ensure(j, j->misc, kMiscSlots * sizeof(uint64_t)));
     if (!j->h_misc.ensure(kMiscSlots * sizeof(uint64_t)) || !j->h_hist.ensure(kSortPasses * kSortRadix * 4))
         return EMP_E_NOMEM;
-    EMP_CUDA(cudaMemsetAsync(j->misc.p, 0, kMiscSlots * sizeof(uint64_t), s));
     const uint64_t F = j->F;
+    if (!mm || !F) EMP_CUDA(cudaMemsetAsync(j->misc.p, 0, kMiscSlots * sizeof(uint64_t), s));
     if (!F) return EMP_OK;
     // ---- K1: newline index
     const uint64_t T = parse_tiles(F);
     EMP_TRY(ensure(j, j->tile_counts, T * 4));
     EMP_TRY(ensure(j, j->tile_excl, T * 8));
-    launch_nl_count(j->fq.as<uint8_t>(), F, j->tile_counts.as<uint32_t>(), j->misc.as<uint64_t>() + kMiscLen0, s);
+    uint64_t *dm = j->misc.as<uint64_t>();
     EMP_TRY(reset_chain(j, scan_tiles(T), s));
+    if (mm) {
+        mm->nl.push_back(NlArgs{j->fq.as<uint8_t>(), F, j->tile_counts.as<uint32_t>(), dm + kMiscLen0, dm});
+        mm->scan.push_back(ScanArgs{j->tile_counts.as<uint32_t>(), j->tile_excl.as<uint64_t>(), T, chain_words(j),
+                                    chain_ctr(j), dm + kMiscTotal, err_word(j)});
+        return EMP_OK;
+    }
+    launch_nl_count(j->fq.as<uint8_t>(), F, j->tile_counts.as<uint32_t>(), dm + kMiscLen0, s);
     launch_scan_u32_u64(j->tile_counts.as<uint32_t>(), j->tile_excl.as<uint64_t>(), T, chain_words(j),
                         chain_ctr(j), j->misc.as<uint64_t>() + kMiscTotal, err_word(j), s);
     return EMP_OK;
 }
 
 // queue the copy of the job's device words that the next stage reads
-emp_status map_fetch(emp_job *j, cudaStream_t s) {
+emp_status map_fetch(emp_job *j, cudaStream_t s, MapMany *mm = nullptr) {
+    if (mm) {
+        mm->fetch.push_back(j);
+        return EMP_OK;
+    }
     EMP_CUDA(cudaMemcpyAsync(j->h_misc.p, j->misc.p, kMiscSlots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     return EMP_OK;
 }
@@ -1113,10 +1226,10 @@ void map_finish_empty(emp_job *j, cudaStream_t s) {
     j->prep.done = true;
 }
 
-emp_status launch_reads(emp_job *j, cudaStream_t s, int wpr);
+emp_status launch_reads(emp_job *j, cudaStream_t s, int wpr, MapMany *mm);
 emp_status dedup_by_sort(emp_job *j, cudaStream_t s);
 
-emp_status map_records(emp_job *j, cudaStream_t s) {
+emp_status map_records(emp_job *j, cudaStream_t s, MapMany *mm = nullptr) {
     EMP_TRY(map_check(j));
     uint64_t *hm = j->h_misc.as<uint64_t>();
     uint64_t *dm = j->misc.as<uint64_t>();
@@ -1137,22 +1250,30 @@ emp_status map_records(emp_job *j, cudaStream_t s) {
     // length needs another layout.
     const uint64_t len0 = hm[kMiscLen0];
     const int wpr = len0 >= 1 && len0 <= (uint64_t)kMaxReadLen ? (int)((len0 + 15) / 16) : kMaxReadLen / 16;
-    return launch_reads(j, s, wpr);
+    return launch_reads(j, s, wpr, mm);
 }
 
 // The read pass (K2) with `wpr` read-major words per read.
-emp_status launch_reads(emp_job *j, cudaStream_t s, int wpr) {
+emp_status launch_reads(emp_job *j, cudaStream_t s, int wpr, MapMany *mm) {
     uint64_t *dm = j->misc.as<uint64_t>();
     const uint64_t n_rec = j->prep.n_rec;
     j->prep.wpr = wpr;
     EMP_TRY(ensure(j, j->keys0, n_rec * 16));
     EMP_TRY(ensure(j, j->seq2, n_rec * (uint64_t)wpr * 4));
     EMP_TRY(ensure(j, j->keep, n_rec * 4));
+    if (mm) {
+        mm->read.push_back(ReadArgs{
+            j->fq.as<uint8_t>(), j->F, j->tile_excl.as<uint64_t>(), j->ctx->tables.as<HashTables>(),
+            reinterpret_cast<const ChunkWeights *>(j->ctx->tables.as<uint8_t>() + sizeof(HashTables)),
+            j->keys0.as<uint64_t>(), j->seq2.as<uint32_t>(), wpr, 0u, j->keep.as<uint32_t>(), dm + kMiscN,
+            reinterpret_cast<uint32_t *>(dm + kMiscLen), err_word(j)});
+        return EMP_OK;
+    }
     launch_read_pass(j->fq.as<uint8_t>(), j->F, j->tile_excl.as<uint64_t>(), j->ctx->tables.as<HashTables>(),
                      reinterpret_cast<const ChunkWeights *>(j->ctx->tables.as<uint8_t>() + sizeof(HashTables)),
                      j->keys0.as<uint64_t>(), j->seq2.as<uint32_t>(), wpr, j->keep.as<uint32_t>(), dm + kMiscN,
                      reinterpret_cast<uint32_t *>(dm + kMiscLen), err_word(j), s);
-    cudaEventRecord(j->map_ev[1], s);
+    if (!j->prep.shared) cudaEventRecord(j->map_ev[1], s);
     return EMP_OK;
 }
 
@@ -1166,7 +1287,7 @@ bool columns_needed(const emp_ctx *c, uint64_t n, uint64_t M) {
     return !bucket_rounds_usable(c) || 2 * n >= M / 2 || 4 * n > kBktMaxEntries;
 }
 
-emp_status map_keys(emp_job *j, cudaStream_t s) {
+emp_status map_keys(emp_job *j, cudaStream_t s, MapMany *mm = nullptr) {
     EMP_TRY(map_check(j));
     JobPrep &q = j->prep;
     uint64_t *hm = j->h_misc.as<uint64_t>();
@@ -1196,7 +1317,7 @@ emp_status map_keys(emp_job *j, cudaStream_t s) {
     if (n2 >= (1ull << 31)) return EMP_E_UNSUPPORTED;
     if (q.wpr != (L + 15) / 16) {  // the kept reads are not as long as the first record: lay the words out again
         EMP_CUDA(cudaMemsetAsync(dm + kMiscLen, 0, 16, s));  // length extremes, kept count
-        EMP_TRY(launch_reads(j, s, (L + 15) / 16));
+        EMP_TRY(launch_reads(j, s, (L + 15) / 16, nullptr));
         EMP_TRY(sync_and_check(j, s));
         if (hm[kMiscErr] & kErrBadBase) return EMP_E_FORMAT;
     }
@@ -1238,6 +1359,21 @@ emp_status map_keys(emp_job *j, cudaStream_t s) {
         if (!j->dedup_scr.p) {
             EMP_TRY(ensure(j, j->dedup_scr, kDedupScratch));
             EMP_CUDA(cudaMemsetAsync(j->dedup_scr.p, 0, kDedupScratch, s));
+        }
+        DedupArgs a;
+        if (mm && nbd <= kDedupTiled &&
+            dedup_args(&a, j->keys0.as<uint64_t>(), n2, nbd, j->dedup_scr.p, j->sk0.as<uint64_t>(),
+                       j->sv0.as<uint32_t>(), j->alive.as<uint8_t>(), err_word(j))) {
+            const uint64_t tiles = upd_tiles(n2);
+            EMP_TRY(ensure(j, j->status, tiles * sizeof(uint64_t) + 64));
+            a.hist_blocks = (uint32_t)((n2 + 2047) / 2048);  // the other jobs fill the chip
+            a.zero = j->status.as<uint64_t>();               // as reset_chain does
+            a.zero_n = (uint32_t)tiles + 8;
+            mm->dedup.push_back(a);
+            mm->nb_max = std::max(mm->nb_max, nbd);
+            mm->init.push_back(InitArgs{j->keys0.as<uint64_t>(), j->alive.as<uint8_t>(), n, j->lk0.as<uint64_t>(),
+                                        j->lv0.as<uint32_t>(), chain_words(j), chain_ctr(j), dm + kMiscU, err_word(j)});
+            return EMP_OK;
         }
         hashed = launch_dedup_hash(j->keys0.as<uint64_t>(), n2, nbd, j->dedup_scr.p, j->sk0.as<uint64_t>(),
                                    j->sv0.as<uint32_t>(), j->alive.as<uint8_t>(), err_word(j), s);
@@ -1343,12 +1479,14 @@ emp_status job_rounds(emp_job *j, cudaStream_t s) {
 // Timings and counts of a finished job (after its stream is synchronised).
 void job_finish(emp_job *j) {
     emp_stats &st = j->st;
-    if (!j->prep.done) {
-        st.ms_map = ms_between(j->map_ev[0], j->map_ev[1]);
-        st.ms_dedup = ms_between(j->map_ev[1], j->map_ev[2]);
+    const JobPrep &q = j->prep;
+    if (!q.done) {
+        st.ms_map = q.shared ? q.ms_map : ms_between(j->map_ev[0], j->map_ev[1]);
+        st.ms_dedup = q.shared ? q.ms_dedup : ms_between(j->map_ev[1], j->map_ev[2]);
         st.ms_rounds = ms_between(j->map_ev[2], j->map_ev[3]);
     }
-    st.ms_total = ms_between(j->map_ev[0], j->map_ev[4]);
+    st.ms_total = !q.shared ? ms_between(j->map_ev[0], j->map_ev[4])
+                            : q.ms_map + q.ms_dedup + (q.done ? 0.f : ms_between(j->map_ev[2], j->map_ev[4]));
     st.output_bytes = j->out.size() + j->dout_bytes;
     st.gpu_launches = g_launches.load() - j->prep.launches0;
     j->have_result = true;
@@ -1523,69 +1661,46 @@ emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStr
     auto fail = [&](int i, emp_status e) {
         if (rc[i] == EMP_OK) rc[i] = e;
     };
-    // job i on stream i mod K (K = 1: s itself), every stream after s's work so far
-    emp_ctx *ctx = n ? jobs[0]->ctx : nullptr;
-    const int want = ctx && ctx->tune.map_streams ? (int)ctx->tune.map_streams : kMapStreamsDefault;
-    const int K = n > 1 ? std::min(n, want) : 1;
-    std::vector<cudaStream_t> st((size_t)K, s);
-    if (K > 1) {
-        for (int k = 0; k <= kMapStreams; ++k)
-            if (!ctx->map_ev[k]) EMP_CUDA(cudaEventCreateWithFlags(&ctx->map_ev[k], cudaEventDisableTiming));
-        EMP_CUDA(cudaEventRecord(ctx->map_ev[kMapStreams], s));  // the last event: the start of the phase
-        for (int k = 0; k < K; ++k) {
-            if (!ctx->map_streams[k]) EMP_CUDA(cudaStreamCreateWithFlags(&ctx->map_streams[k], cudaStreamNonBlocking));
-            st[k] = ctx->map_streams[k];
-            EMP_CUDA(cudaStreamWaitEvent(st[k], ctx->map_ev[kMapStreams], 0));
-        }
-    }
-    auto sync_all = [&]() -> emp_status {
-        for (cudaStream_t q : st) EMP_CUDA(cudaStreamSynchronize(q));
+    if (n == 1) {
+        auto one = [&](emp_status e) {
+            fail(0, e);
+            if (live(0)) fail(0, map_fetch(jobs[0], s));
+            return cuda_status(cudaStreamSynchronize(s));
+        };
+        EMP_TRY(one(map_begin(jobs[0], s)));
+        if (live(0)) EMP_TRY(one(map_records(jobs[0], s)));
+        if (live(0)) EMP_TRY(one(map_keys(jobs[0], s)));
+        if (live(0)) fail(0, map_list(jobs[0], s));
         return EMP_OK;
-    };
-    // largest jobs first, each to the stream with the fewest FASTQ bytes so
-    // far (so that no stream ends a stage long after the others)
-    std::vector<int> order((size_t)n), sid((size_t)n, 0);
-    for (int i = 0; i < n; ++i) order[(size_t)i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return jobs[a]->F > jobs[b]->F; });
-    {
-        std::vector<uint64_t> load((size_t)K, 0);
-        for (int i : order) {
-            const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-            sid[(size_t)i] = k;
-            load[(size_t)k] += jobs[i]->F + 4096;
-        }
     }
-    auto stages = [&]() -> emp_status {
-        for (int i : order) {
-            fail(i, map_begin(jobs[i], st[sid[i]]));
-            if (rc[i] == EMP_OK) fail(i, map_fetch(jobs[i], st[sid[i]]));
-        }
-        EMP_TRY(sync_all());
-        for (int i : order) {
+    if (n < 1) return EMP_OK;
+    emp_ctx *ctx = jobs[0]->ctx;
+    for (auto &e : ctx->many_ev)
+        if (!e) EMP_CUDA(cudaEventCreate(&e));
+    MapMany mm;
+    auto stage = [&](auto step) {
+        for (int i = 0; i < n; ++i) {
             if (!live(i)) continue;
-            fail(i, map_records(jobs[i], st[sid[i]]));
-            if (live(i)) fail(i, map_fetch(jobs[i], st[sid[i]]));
+            fail(i, step(jobs[i]));
+            if (live(i)) fail(i, map_fetch(jobs[i], s, &mm));
         }
-        EMP_TRY(sync_all());
-        for (int i : order) {
-            if (!live(i)) continue;
-            fail(i, map_keys(jobs[i], st[sid[i]]));
-            if (live(i)) fail(i, map_fetch(jobs[i], st[sid[i]]));
-        }
-        EMP_TRY(sync_all());
-        for (int i : order)
-            if (live(i)) fail(i, map_list(jobs[i], st[sid[i]]));
-        return EMP_OK;
+        return many_flush(ctx, mm, s);
     };
-    const emp_status e = stages();
-    if (K > 1) {  // the rest of the jobs' work (and any error path) is on s, after all of this
-        for (int k = 0; k < K; ++k) {
-            cudaEventRecord(ctx->map_ev[k], st[k]);
-            cudaStreamWaitEvent(s, ctx->map_ev[k], 0);
-        }
-        for (int i = 0; i < n; ++i) jobs[i]->stream = s;
+    EMP_CUDA(cudaEventRecord(ctx->many_ev[0], s));
+    EMP_TRY(stage([&](emp_job *j) { return map_begin(j, s, &mm); }));
+    EMP_TRY(stage([&](emp_job *j) { return map_records(j, s, &mm); }));
+    EMP_CUDA(cudaEventRecord(ctx->many_ev[1], s));
+    EMP_TRY(stage([&](emp_job *j) { return map_keys(j, s, &mm); }));
+    EMP_CUDA(cudaEventRecord(ctx->many_ev[2], s));
+    EMP_CUDA(cudaEventSynchronize(ctx->many_ev[2]));
+    const float ms_map = ms_between(ctx->many_ev[0], ctx->many_ev[1]);
+    const float ms_dedup = ms_between(ctx->many_ev[1], ctx->many_ev[2]);
+    for (int i = 0; i < n; ++i) {
+        jobs[i]->prep.ms_map = ms_map;
+        jobs[i]->prep.ms_dedup = ms_dedup;
+        if (live(i)) fail(i, map_list(jobs[i], s));
     }
-    return e;
+    return EMP_OK;
 }
 
 // Close jobs[0..n) whose work is all queued: their last events, one
@@ -2046,17 +2161,12 @@ emp_status emp_ctx_destroy(emp_ctx *ctx) {
     detach_graphs(ctx);
     for (auto &e : ctx->batch_ev)
         if (e) cudaEventDestroy(e);
-    ctx->in_use -= ctx->batch_jobs.bytes + ctx->batch_ctl.bytes + ctx->batch_swp.bytes();
+    ctx->in_use -= ctx->batch_jobs.bytes + ctx->batch_ctl.bytes + ctx->batch_swp.bytes() + ctx->many.bytes;
+    ctx->many.release();
     ctx->batch_jobs.release();
     ctx->batch_swp.release();
     ctx->batch_ctl.release();
-    for (int k = 0; k < kMapStreams; ++k) {
-        if (ctx->map_streams[k]) {
-            cudaStreamSynchronize(ctx->map_streams[k]);
-            cudaStreamDestroy(ctx->map_streams[k]);
-        }
-    }
-    for (auto &e : ctx->map_ev)
+    for (auto &e : ctx->many_ev)
         if (e) cudaEventDestroy(e);
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);

@@ -39,24 +39,35 @@ __device__ __forceinline__ uint32_t dedup_bucket(uint64_t key, uint32_t nb) {
     return (uint32_t)(((key >> 32) * (uint64_t)nb) >> 29);  // fp1 < 2^29
 }
 
-__global__ void __launch_bounds__(kDT) dedup_hist_kernel(const uint64_t *__restrict__ keys, uint64_t n,
-                                                         uint32_t nb, uint32_t *__restrict__ counts) {
+EMP_DEV void dedup_hist_block(const DedupArgs &a, uint32_t bid) {
+    const uint64_t *const __restrict__ keys = a.keys;
+    const uint64_t n = a.n;
+    const uint32_t nb = a.nb;
+    uint32_t *const __restrict__ counts = a.counts;
+    if (bid == 0 && a.zero)
+        for (uint32_t i = threadIdx.x; i < a.zero_n; i += kDT) a.zero[i] = 0;
     extern __shared__ uint32_t s_hist[];  // nb
     for (uint32_t i = threadIdx.x; i < nb; i += kDT) s_hist[i] = 0;
     __syncthreads();
-    for (uint64_t e = (uint64_t)blockIdx.x * kDT + threadIdx.x; e < n; e += (uint64_t)gridDim.x * kDT)
+    for (uint64_t e = (uint64_t)bid * kDT + threadIdx.x; e < n; e += (uint64_t)a.hist_blocks * kDT)
         atomicAdd(&s_hist[dedup_bucket(__ldg(keys + e), nb)], 1u);
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < nb; i += kDT)
         if (s_hist[i]) atomicAdd(counts + i, s_hist[i]);
 }
+__global__ void __launch_bounds__(kDT) dedup_hist_kernel(const DedupArgs a) { dedup_hist_block(a, blockIdx.x); }
+__global__ void __launch_bounds__(kDT) dedup_hist_many_kernel(const DedupArgs *a, const uint2 *blk) {
+    const uint2 b = blk[blockIdx.x];
+    dedup_hist_block(a[b.x], b.y);
+}
 
 // start[b] = cursor[b] = the exclusive scan of the counts (one CTA), which
 // are zeroed for the next call.
 constexpr int kScanT = 1024;
-__global__ void __launch_bounds__(kScanT) dedup_scan_kernel(uint32_t *__restrict__ counts, uint32_t nb,
-                                                            uint32_t *__restrict__ start,
-                                                            uint32_t *__restrict__ cursor) {
+EMP_DEV void dedup_scan_block(const DedupArgs &a) {
+    uint32_t *const __restrict__ counts = a.counts, *const __restrict__ start = a.start;
+    uint32_t *const __restrict__ cursor = a.cursor;
+    const uint32_t nb = a.nb;
     __shared__ uint32_t s_warp[32];
     uint32_t run = 0;
     for (uint32_t b0 = 0; b0 < nb; b0 += 4 * kScanT) {
@@ -79,6 +90,8 @@ __global__ void __launch_bounds__(kScanT) dedup_scan_kernel(uint32_t *__restrict
         run += tot;
     }
 }
+__global__ void __launch_bounds__(kScanT) dedup_scan_kernel(const DedupArgs a) { dedup_scan_block(a); }
+__global__ void __launch_bounds__(kScanT) dedup_scan_many_kernel(const DedupArgs *a) { dedup_scan_block(a[blockIdx.x]); }
 
 __global__ void __launch_bounds__(kDT) dedup_scatter_kernel(const uint64_t *__restrict__ keys, uint64_t n,
                                                             uint32_t nb, uint32_t *__restrict__ cursor,
@@ -104,16 +117,18 @@ __global__ void __launch_bounds__(kDT) dedup_scatter_kernel(const uint64_t *__re
 // The same for few buckets (nb <= kTiledBuckets), where the bucket cursors
 // would be hot: a CTA ranks a tile of kScatterTile keys per bucket in shared
 // memory and reserves each bucket's run with one atomic.
-constexpr uint32_t kTiledBuckets = 2048;
+constexpr uint32_t kTiledBuckets = kDedupTiled;
 constexpr int kScatterPer = 16;
 constexpr uint32_t kScatterTile = kDT * kScatterPer;
 
-__global__ void __launch_bounds__(kDT) dedup_scatter_tiled_kernel(const uint64_t *__restrict__ keys, uint64_t n,
-                                                                  uint32_t nb, uint32_t *__restrict__ cursor,
-                                                                  uint64_t *__restrict__ pk,
-                                                                  uint32_t *__restrict__ pr) {
+EMP_DEV void dedup_scatter_tiled_block(const DedupArgs &a, uint32_t bid) {
+    const uint64_t *const __restrict__ keys = a.keys;
+    const uint64_t n = a.n;
+    const uint32_t nb = a.nb;
+    uint32_t *const __restrict__ cursor = a.cursor, *const __restrict__ pr = a.pr;
+    uint64_t *const __restrict__ pk = a.pk;
     __shared__ uint32_t s_cnt[kTiledBuckets];
-    for (uint64_t t0 = (uint64_t)blockIdx.x * kScatterTile; t0 < n; t0 += (uint64_t)gridDim.x * kScatterTile) {
+    for (uint64_t t0 = (uint64_t)bid * kScatterTile; t0 < n; t0 += (uint64_t)a.scatter_blocks * kScatterTile) {
         for (uint32_t b = threadIdx.x; b < nb; b += kDT) s_cnt[b] = 0;
         __syncthreads();
         uint64_t k[kScatterPer];
@@ -142,6 +157,13 @@ __global__ void __launch_bounds__(kDT) dedup_scatter_tiled_kernel(const uint64_t
         __syncthreads();
     }
 }
+__global__ void __launch_bounds__(kDT) dedup_scatter_tiled_kernel(const DedupArgs a) {
+    dedup_scatter_tiled_block(a, blockIdx.x);
+}
+__global__ void __launch_bounds__(kDT) dedup_scatter_many_kernel(const DedupArgs *a, const uint2 *blk) {
+    const uint2 b = blk[blockIdx.x];
+    dedup_scatter_tiled_block(a[b.x], b.y);
+}
 
 __device__ __forceinline__ uint32_t dedup_slot(uint64_t key) {
     return (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> 40) & (kDedupSlots - 1);
@@ -149,16 +171,18 @@ __device__ __forceinline__ uint32_t dedup_slot(uint64_t key) {
 
 constexpr size_t kMarkSmem = kDedupSlots * (8 + 4);
 
-__global__ void __launch_bounds__(kDT) dedup_mark_hash_kernel(const uint64_t *__restrict__ pk,
-                                                              const uint32_t *__restrict__ pr,
-                                                              const uint32_t *__restrict__ start, uint32_t nb,
-                                                              uint64_t n, uint8_t *__restrict__ alive,
-                                                              uint32_t *err) {
+EMP_DEV void dedup_mark_block(const DedupArgs &a, uint32_t bid) {
+    const uint64_t *const __restrict__ pk = a.pk;
+    const uint32_t *const __restrict__ pr = a.pr, *const __restrict__ start = a.start;
+    const uint32_t nb = a.nb;
+    const uint64_t n = a.n;
+    uint8_t *const __restrict__ alive = a.alive;
+    uint32_t *const err = a.err;
     extern __shared__ __align__(16) uint8_t smem[];
     uint64_t *s_key = reinterpret_cast<uint64_t *>(smem);
     uint32_t *s_min = reinterpret_cast<uint32_t *>(s_key + kDedupSlots);
     __shared__ uint32_t s_used;
-    for (uint32_t b = blockIdx.x; b < nb; b += gridDim.x) {
+    for (uint32_t b = bid; b < nb; b += a.mark_blocks) {
         for (uint32_t i = threadIdx.x; i < kDedupSlots; i += kDT) {
             s_key[i] = kDedupEmpty;
             s_min[i] = 0xffffffffu;
@@ -196,6 +220,11 @@ __global__ void __launch_bounds__(kDT) dedup_mark_hash_kernel(const uint64_t *__
         __syncthreads();
     }
 }
+__global__ void __launch_bounds__(kDT) dedup_mark_hash_kernel(const DedupArgs a) { dedup_mark_block(a, blockIdx.x); }
+__global__ void __launch_bounds__(kDT) dedup_mark_many_kernel(const DedupArgs *a, const uint2 *blk) {
+    const uint2 b = blk[blockIdx.x];
+    dedup_mark_block(a[b.x], b.y);
+}
 
 }  // namespace
 
@@ -220,6 +249,8 @@ static bool dedup_setup(int &sms) {
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     if (cudaFuncSetAttribute(dedup_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(kDedupMaxBuckets * 4)) != cudaSuccess ||
+        cudaFuncSetAttribute(dedup_mark_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarkSmem) !=
+            cudaSuccess ||
         cudaFuncSetAttribute(dedup_mark_hash_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarkSmem) !=
             cudaSuccess) {
         cudaGetLastError();
@@ -230,28 +261,42 @@ static bool dedup_setup(int &sms) {
     return true;
 }
 
-bool launch_dedup_hash(const uint64_t *keys, uint64_t n, uint32_t nb, void *scratch, uint64_t *pk, uint32_t *pr,
-                       uint8_t *alive, uint32_t *err, cudaStream_t s) {
+bool dedup_args(DedupArgs *a, const uint64_t *keys, uint64_t n, uint32_t nb, void *scratch, uint64_t *pk, uint32_t *pr,
+                uint8_t *alive, uint32_t *err) {
     int sms = 0;
     if (!n || !nb || !dedup_setup(sms)) return false;
     uint32_t *counts = reinterpret_cast<uint32_t *>(scratch);
     uint32_t *start = counts + kDedupMaxBuckets, *cursor = start + kDedupMaxBuckets;
-    const uint64_t per = (n + kDT - 1) / kDT;
-    const unsigned g_hist = (unsigned)(per < (uint64_t)sms * 4 ? per : (uint64_t)sms * 4);
-    count_launch(4);
-    dedup_hist_kernel<<<g_hist, kDT, nb * 4, s>>>(keys, n, nb, counts);
-    dedup_scan_kernel<<<1, kScanT, 0, s>>>(counts, nb, start, cursor);
-    if (nb <= kTiledBuckets) {
-        const uint64_t tiles = (n + kScatterTile - 1) / kScatterTile;
-        const unsigned g_t = (unsigned)(tiles < (uint64_t)sms * 8 ? tiles : (uint64_t)sms * 8);
-        dedup_scatter_tiled_kernel<<<g_t, kDT, 0, s>>>(keys, n, nb, cursor, pk, pr);
-    } else {
-        const unsigned g_sc = (unsigned)(per < (uint64_t)sms * 8 ? per : (uint64_t)sms * 8);
-        dedup_scatter_kernel<<<g_sc, kDT, 0, s>>>(keys, n, nb, cursor, pk, pr);
-    }
-    const unsigned g_mark = nb < (uint32_t)sms * 2 ? nb : (uint32_t)sms * 2;
-    dedup_mark_hash_kernel<<<g_mark, kDT, kMarkSmem, s>>>(pk, pr, start, nb, n, alive, err);
+    const uint64_t per = (n + kDT - 1) / kDT, tiles = (n + kScatterTile - 1) / kScatterTile, most = (uint64_t)sms;
+    *a = DedupArgs{keys, n, nb, 0u, 0u, 0u, counts, start, cursor, pk, pr, alive, err, nullptr, 0u};
+    a->hist_blocks = (uint32_t)(per < most * 4 ? per : most * 4);
+    a->scatter_blocks = (uint32_t)(nb <= kTiledBuckets ? (tiles < most * 8 ? tiles : most * 8)
+                                                       : (per < most * 8 ? per : most * 8));
+    a->mark_blocks = nb < most * 2 ? nb : (uint32_t)most * 2;
     return true;
+}
+
+bool launch_dedup_hash(const uint64_t *keys, uint64_t n, uint32_t nb, void *scratch, uint64_t *pk, uint32_t *pr,
+                       uint8_t *alive, uint32_t *err, cudaStream_t s) {
+    DedupArgs a;
+    if (!dedup_args(&a, keys, n, nb, scratch, pk, pr, alive, err)) return false;
+    count_launch(4);
+    dedup_hist_kernel<<<a.hist_blocks, kDT, nb * 4, s>>>(a);
+    dedup_scan_kernel<<<1, kScanT, 0, s>>>(a);
+    if (nb <= kTiledBuckets) dedup_scatter_tiled_kernel<<<a.scatter_blocks, kDT, 0, s>>>(a);
+    else dedup_scatter_kernel<<<a.scatter_blocks, kDT, 0, s>>>(keys, n, nb, a.cursor, pk, pr);
+    dedup_mark_hash_kernel<<<a.mark_blocks, kDT, kMarkSmem, s>>>(a);
+    return true;
+}
+
+void launch_dedup_many(const DedupArgs *a, uint32_t jobs, uint32_t nb_max, ManyBlocks hist, ManyBlocks scatter,
+                       ManyBlocks mark, cudaStream_t s) {
+    if (!jobs) return;
+    count_launch(4);
+    dedup_hist_many_kernel<<<hist.n, kDT, nb_max * 4, s>>>(a, hist.blk);
+    dedup_scan_many_kernel<<<jobs, kScanT, 0, s>>>(a);
+    dedup_scatter_many_kernel<<<scatter.n, kDT, 0, s>>>(a, scatter.blk);
+    dedup_mark_many_kernel<<<mark.n, kDT, kMarkSmem, s>>>(a, mark.blk);
 }
 
 }  // namespace emp

@@ -45,11 +45,15 @@ EMP_DEV uint32_t first_nl_after(const uint4 &v, uint32_t off, uint32_t after) {
     return best;
 }
 
-__global__ void __launch_bounds__(256) nl_count_kernel(const uint8_t *__restrict__ fq, uint64_t F,
-                                                       uint32_t *__restrict__ tile_counts, uint64_t *len0) {
+EMP_DEV void nl_count_block(const NlArgs &A, const uint32_t bid) {
+    const uint8_t *const __restrict__ fq = A.fq;
+    const uint64_t F = A.F;
+    uint32_t *const tile_counts = A.tile_counts;
+    uint64_t *const len0 = A.len0;
+    if (bid == 0 && A.zero && threadIdx.x < 16) A.zero[threadIdx.x] = 0;
     __shared__ uint32_t s_warp[8];
     __shared__ uint32_t s_nl[2];
-    const uint64_t base = (uint64_t)blockIdx.x * kParseTile;
+    const uint64_t base = (uint64_t)bid * kParseTile;
     uint32_t c = 0;
     uint4 blk[4];
 #pragma unroll
@@ -68,14 +72,14 @@ __global__ void __launch_bounds__(256) nl_count_kernel(const uint8_t *__restrict
 #pragma unroll
     for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = c;
-    if (blockIdx.x == 0 && threadIdx.x == 0) s_nl[0] = s_nl[1] = 0xffffffffu;
+    if (bid == 0 && threadIdx.x == 0) s_nl[0] = s_nl[1] = 0xffffffffu;
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t t = 0;
         for (int w = 0; w < 8; ++w) t += s_warp[w];
-        tile_counts[blockIdx.x] = t;
+        tile_counts[bid] = t;
     }
-    if (blockIdx.x != 0) return;
+    if (bid != 0) return;
     // tile 0: the first record's sequence line lies between newlines 0 and 1
     // (a hint for sizing the read-major word store; 0 when not found here)
     uint32_t a = 0xffffffffu;
@@ -92,6 +96,11 @@ __global__ void __launch_bounds__(256) nl_count_kernel(const uint8_t *__restrict
     }
     __syncthreads();
     if (threadIdx.x == 0) *len0 = (s_nl[0] != 0xffffffffu && s_nl[1] != 0xffffffffu) ? s_nl[1] - s_nl[0] - 1 : 0;
+}
+__global__ void __launch_bounds__(256) nl_count_kernel(const NlArgs a) { nl_count_block(a, blockIdx.x); }
+__global__ void __launch_bounds__(256) nl_count_many_kernel(const NlArgs *a, const uint2 *blk) {
+    const uint2 b = blk[blockIdx.x];
+    nl_count_block(a[b.x], b.y);
 }
 
 // 0x80 in every byte of t that is zero, 0 elsewhere (no carries between bytes)
@@ -249,13 +258,18 @@ EMP_DEV void stage_window(const uint8_t *fq, uint64_t F, uint64_t tile, uint32_t
     }
 }
 
-__global__ void __launch_bounds__(kRT, 4) read_pass_kernel(const uint8_t *__restrict__ fq, uint64_t F,
-                                                        const uint64_t *__restrict__ tile_excl,
-                                                        const HashTables *__restrict__ tables,
-                                                        const ChunkWeights *__restrict__ weights,
-                                                        uint64_t *__restrict__ keys, uint32_t *__restrict__ seq2,
-                                                        int wpr, uint32_t *__restrict__ keep_out, uint64_t *n_kept,
-                                                        uint32_t *len_minmax, uint32_t *err) {
+EMP_DEV void read_pass_block(const ReadArgs &A, const uint32_t bid) {
+    const uint8_t *const __restrict__ fq = A.fq;
+    const uint64_t F = A.F;
+    const uint64_t *const __restrict__ tile_excl = A.tile_excl;
+    const HashTables *const __restrict__ tables = A.tables;
+    const ChunkWeights *const __restrict__ weights = A.weights;
+    uint64_t *const __restrict__ keys = A.keys;
+    uint32_t *const __restrict__ seq2 = A.seq2, *const __restrict__ keep_out = A.keep;
+    uint64_t *const n_kept = A.n_kept;
+    uint32_t *const len_minmax = A.len_minmax, *const err = A.err;
+    const int wpr = A.wpr;
+    const uint32_t nblk = A.blocks;
     extern __shared__ __align__(16) uint8_t read_smem[];
     ReadSmem &sm = *reinterpret_cast<ReadSmem *>(read_smem);
     const int tid = threadIdx.x, lane = tid & 31;
@@ -270,10 +284,10 @@ __global__ void __launch_bounds__(kRT, 4) read_pass_kernel(const uint8_t *__rest
     __syncthreads();
     const uint64_t ntiles = parse_tiles(F);
     uint32_t lmin = 0xffffffffu, lmax = 0u, bad_kept = 0u, kept = 0u;
-    if (blockIdx.x < ntiles) stage_window(fq, F, blockIdx.x, sm.win[0], &sm.bar[0]);
+    if (bid < ntiles) stage_window(fq, F, bid, sm.win[0], &sm.bar[0]);
     int buf = 0;
     uint32_t parity = 0;  // bit b: the phase buffer b's barrier completes next
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
+    for (uint64_t tile = bid; tile < ntiles; tile += nblk, buf ^= 1) {
         const uint64_t T0 = tile * kParseTile;
         const bool win_eof = T0 + kWin >= F;  // the window holds the rest of the input
         const uint64_t E = tile_excl[tile];   // newlines before the tile
@@ -286,7 +300,7 @@ __global__ void __launch_bounds__(kRT, 4) read_pass_kernel(const uint8_t *__rest
             }
             return;
         }
-        if (tile + gridDim.x < ntiles) stage_window(fq, F, tile + gridDim.x, sm.win[buf ^ 1], &sm.bar[buf ^ 1]);
+        if (tile + nblk < ntiles) stage_window(fq, F, tile + nblk, sm.win[buf ^ 1], &sm.bar[buf ^ 1]);
         const uint32_t *win = sm.win[buf];
         // ---- locate.  Thread t holds tile bytes [64t, 64t + 64) (four 16-byte
         // chunks, read in an order rotated by t so that a quarter-warp's
@@ -459,6 +473,13 @@ __global__ void __launch_bounds__(kRT, 4) read_pass_kernel(const uint8_t *__rest
         if (anybad) atomicOr(err, kErrBadBase);
     }
 }
+__global__ void __launch_bounds__(kRT, 4) read_pass_kernel(const __grid_constant__ ReadArgs a) {
+    read_pass_block(a, blockIdx.x);
+}
+__global__ void __launch_bounds__(kRT, 4) read_pass_many_kernel(const ReadArgs *a, const uint2 *blk) {
+    const uint2 b = blk[blockIdx.x];
+    read_pass_block(a[b.x], b.y);
+}
 
 // Kept records to consecutive indices: pos = exclusive scan of keep (a
 // record is kept iff pos[k+1] > pos[k], the last one iff its pos < n_kept).
@@ -512,13 +533,15 @@ static unsigned grid_for(uint64_t work, unsigned per_block, unsigned cap) {
 void launch_nl_count(const uint8_t *fq, uint64_t F, uint32_t *tile_counts, uint64_t *len0, cudaStream_t s) {
     if (!F) return;
     count_launch();
-    nl_count_kernel<<<(unsigned)parse_tiles(F), 256, 0, s>>>(fq, F, tile_counts, len0);
+    nl_count_kernel<<<(unsigned)parse_tiles(F), 256, 0, s>>>(NlArgs{fq, F, tile_counts, len0, nullptr});
+}
+void launch_nl_count_many(const NlArgs *a, ManyBlocks b, cudaStream_t s) {
+    if (!b.n) return;
+    count_launch();
+    nl_count_many_kernel<<<b.n, 256, 0, s>>>(a, b.blk);
 }
 
-void launch_read_pass(const uint8_t *fq, uint64_t F, const uint64_t *tile_excl, const HashTables *tables,
-                      const ChunkWeights *weights, uint64_t *keys, uint32_t *seq2, int wpr, uint32_t *keep, uint64_t *n_kept, uint32_t *len_minmax,
-                      uint32_t *err, cudaStream_t s) {
-    if (!F) return;
+uint32_t read_pass_grid() {
     // persistent grid (SMs x resident CTAs) and the shared-memory attribute, once per device
     constexpr int kDevs = 64;
     static std::atomic<int> grid[kDevs] = {};
@@ -532,6 +555,8 @@ void launch_read_pass(const uint8_t *fq, uint64_t F, const uint64_t *tile_excl, 
         int sms = 148, occ = 1;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(read_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ReadSmem));
+        cudaFuncSetAttribute(read_pass_many_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(ReadSmem));
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, read_pass_kernel, kRT, sizeof(ReadSmem)) !=
                 cudaSuccess ||
             occ < 1)
@@ -540,9 +565,32 @@ void launch_read_pass(const uint8_t *fq, uint64_t F, const uint64_t *tile_excl, 
         g = sms * occ;
         grid[dev].store(g, std::memory_order_release);
     }
+    return (uint32_t)g;
+}
+
+void launch_read_pass(const uint8_t *fq, uint64_t F, const uint64_t *tile_excl, const HashTables *tables,
+                      const ChunkWeights *weights, uint64_t *keys, uint32_t *seq2, int wpr, uint32_t *keep, uint64_t *n_kept, uint32_t *len_minmax,
+                      uint32_t *err, cudaStream_t s) {
+    if (!F) return;
+    ReadArgs a{fq, F, tile_excl, tables, weights, keys, seq2, wpr, 0u, keep, n_kept, len_minmax, err};
+    a.blocks = grid_for(parse_tiles(F), 1, read_pass_grid());
     count_launch();
-    read_pass_kernel<<<grid_for(parse_tiles(F), 1, (unsigned)g), kRT, sizeof(ReadSmem), s>>>(
-        fq, F, tile_excl, tables, weights, keys, seq2, wpr, keep, n_kept, len_minmax, err);
+    read_pass_kernel<<<a.blocks, kRT, sizeof(ReadSmem), s>>>(a);
+}
+void launch_read_pass_many(const ReadArgs *a, ManyBlocks b, cudaStream_t s) {
+    if (!b.n) return;
+    read_pass_grid();  // the kernel's attributes
+    count_launch();
+    read_pass_many_kernel<<<b.n, kRT, sizeof(ReadSmem), s>>>(a, b.blk);
+}
+__global__ void __launch_bounds__(256) gather_words_kernel(const uint64_t *const *src, uint32_t jobs, uint64_t *out) {
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (i < jobs * 16) out[i] = src[i >> 4][i & 15];
+}
+void launch_gather_words(const uint64_t *const *src, uint32_t jobs, uint64_t *out, cudaStream_t s) {
+    if (!jobs) return;
+    count_launch();
+    gather_words_kernel<<<(jobs * 16 + 255) / 256, 256, 0, s>>>(src, jobs, out);
 }
 
 void launch_compact_reads(const uint32_t *pos, uint64_t n_rec, uint64_t n_kept, const uint64_t *keys,

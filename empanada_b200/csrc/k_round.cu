@@ -37,15 +37,18 @@ __global__ void dedup_mark_kernel(const uint64_t *__restrict__ k, const uint32_t
 
 constexpr int kChunks = kUpdTile / 256;  // 8
 
-__global__ void __launch_bounds__(256) init_list_kernel(const uint64_t *__restrict__ keys0,
-                                                        const uint8_t *__restrict__ alive, uint64_t n,
-                                                        uint64_t *__restrict__ lk, uint32_t *__restrict__ lv,
-                                                        uint64_t *status, uint32_t *tile_ctr, uint64_t *count,
-                                                        uint32_t *err) {
+EMP_DEV void init_list_block(const InitArgs &a) {
+    const uint64_t *const __restrict__ keys0 = a.keys0;
+    const uint8_t *const __restrict__ alive = a.alive;
+    const uint64_t n = a.n;
+    uint64_t *const __restrict__ lk = a.lk;
+    uint32_t *const __restrict__ lv = a.lv;
+    uint64_t *const status = a.status, *const count = a.count;
+    uint32_t *const err = a.err;
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[8];
     __shared__ uint64_t s_base;
-    if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(tile_ctr, 1u) : 0u;
+    if (threadIdx.x == 0) s_tile = 2 * n > kUpdTile ? atomicAdd(a.tile_ctr, 1u) : 0u;
     __syncthreads();
     const uint32_t tile = s_tile;
     const uint64_t base = (uint64_t)tile * kUpdTile, n2 = 2 * n;
@@ -76,6 +79,11 @@ __global__ void __launch_bounds__(256) init_list_kernel(const uint64_t *__restri
         }
     }
     if (threadIdx.x == 0 && (uint64_t)tile == upd_tiles(n2) - 1) *count = s_base + running;
+}
+__global__ void __launch_bounds__(256) init_list_kernel(const InitArgs a) { init_list_block(a); }
+// a job's tiles draw their numbers from its own counter
+__global__ void __launch_bounds__(256) init_list_many_kernel(const InitArgs *a, const uint2 *blk) {
+    init_list_block(a[blk[blockIdx.x].x]);
 }
 
 __global__ void iota_kernel(uint32_t *__restrict__ v, uint64_t n) {
@@ -348,8 +356,13 @@ void launch_init_list(const uint64_t *keys0, const uint8_t *alive, uint64_t n, u
         return;
     }
     count_launch();
-    init_list_kernel<<<(unsigned)upd_tiles(2 * n), 256, 0, s>>>(keys0, alive, n, lkeys, lvals, status, tile_ctr,
-                                                                 count, err);
+    init_list_kernel<<<(unsigned)upd_tiles(2 * n), 256, 0, s>>>(
+        InitArgs{keys0, alive, n, lkeys, lvals, status, tile_ctr, count, err});
+}
+void launch_init_list_many(const InitArgs *a, ManyBlocks b, cudaStream_t s) {
+    if (!b.n) return;
+    count_launch();
+    init_list_many_kernel<<<b.n, 256, 0, s>>>(a, b.blk);
 }
 
 void launch_iota(uint32_t *v, uint64_t n, cudaStream_t s) {

@@ -11,13 +11,12 @@
 namespace emp {
 
 template <typename OutT>
-__global__ void __launch_bounds__(256) scan_kernel(const uint32_t *__restrict__ in, OutT *out, uint64_t n,
-                                                   uint64_t *status, uint32_t *tile_ctr, uint64_t *total,
-                                                   uint32_t *err) {
+EMP_DEV void scan_block(const uint32_t *__restrict__ in, OutT *out, uint64_t n, uint64_t *status, uint32_t *tile_ctr,
+                        uint64_t *total, uint32_t *err) {
     __shared__ uint32_t s_tile;
     __shared__ uint64_t s_warp[8];
     __shared__ uint64_t s_base;
-    if (threadIdx.x == 0) s_tile = gridDim.x > 1 ? atomicAdd(tile_ctr, 1u) : 0u;
+    if (threadIdx.x == 0) s_tile = n > kScanTile ? atomicAdd(tile_ctr, 1u) : 0u;
     __syncthreads();
     const uint32_t tile = s_tile;
     const uint64_t base = (uint64_t)tile * kScanTile;
@@ -53,6 +52,23 @@ __global__ void __launch_bounds__(256) scan_kernel(const uint32_t *__restrict__ 
         }
     }
     if (threadIdx.x == 0 && (uint64_t)tile == scan_tiles(n) - 1) *total = tb + running;
+}
+
+template <typename OutT>
+__global__ void __launch_bounds__(256) scan_kernel(const uint32_t *__restrict__ in, OutT *out, uint64_t n,
+                                                   uint64_t *status, uint32_t *tile_ctr, uint64_t *total,
+                                                   uint32_t *err) {
+    scan_block<OutT>(in, out, n, status, tile_ctr, total, err);
+}
+// a job's tiles draw their numbers from its own counter
+__global__ void __launch_bounds__(256) scan_many_kernel(const ScanArgs *a, const uint2 *blk) {
+    const ScanArgs &x = a[blk[blockIdx.x].x];
+    scan_block<uint64_t>(x.in, x.out, x.n, x.status, x.tile_ctr, x.total, x.err);
+}
+void launch_scan_many(const ScanArgs *a, ManyBlocks b, cudaStream_t s) {
+    if (!b.n) return;
+    count_launch();
+    scan_many_kernel<<<b.n, 256, 0, s>>>(a, b.blk);
 }
 
 void launch_scan_u32_u64(const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *status, uint32_t *tile_ctr,

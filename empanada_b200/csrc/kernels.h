@@ -24,6 +24,86 @@ void launch_scan_u32_u64(const uint32_t *in, uint64_t *out, uint64_t n, uint64_t
 void launch_scan_u32_u32(const uint32_t *in, uint32_t *out, uint64_t n, uint64_t *status, uint32_t *tile_ctr,
                          uint64_t *total, uint32_t *err, cudaStream_t s);
 
+// ---- one launch for many jobs ----------------------------------------------
+// The map phase's kernels take their arguments as a struct: one by value, or
+// an array of them with a list of blocks, (job, block of the job) each.  A
+// job's map phase is about ten launches of a few microseconds; a batch of 256
+// spent 8 ms of host time on them.
+struct NlArgs {
+    const uint8_t *fq;
+    uint64_t F;
+    uint32_t *tile_counts;
+    uint64_t *len0;
+    uint64_t *zero;  // set: 16 words to zero before (len0 may be one of them)
+};
+struct ScanArgs {
+    const uint32_t *in;
+    uint64_t *out;
+    uint64_t n;
+    uint64_t *status;
+    uint32_t *tile_ctr;
+    uint64_t *total;
+    uint32_t *err;
+};
+struct HashTables;
+struct ChunkWeights;
+struct ReadArgs {
+    const uint8_t *fq;
+    uint64_t F;
+    const uint64_t *tile_excl;
+    const HashTables *tables;
+    const ChunkWeights *weights;
+    uint64_t *keys;
+    uint32_t *seq2;
+    int wpr;
+    uint32_t blocks;  // CTAs that share the job's tiles
+    uint32_t *keep;
+    uint64_t *n_kept;
+    uint32_t *len_minmax;
+    uint32_t *err;
+};
+struct DedupArgs {
+    const uint64_t *keys;
+    uint64_t n;
+    uint32_t nb;
+    uint32_t hist_blocks, scatter_blocks, mark_blocks;
+    uint32_t *counts, *start, *cursor;
+    uint64_t *pk;
+    uint32_t *pr;
+    uint8_t *alive;
+    uint32_t *err;
+    uint64_t *zero;   // set: words to zero for a later kernel
+    uint32_t zero_n;
+};
+struct InitArgs {
+    const uint64_t *keys0;
+    const uint8_t *alive;
+    uint64_t n;
+    uint64_t *lk;
+    uint32_t *lv;
+    uint64_t *status;
+    uint32_t *tile_ctr;
+    uint64_t *count;
+    uint32_t *err;
+};
+struct ManyBlocks {
+    const uint2 *blk;
+    uint32_t n;
+};
+void launch_nl_count_many(const NlArgs *a, ManyBlocks b, cudaStream_t s);
+void launch_scan_many(const ScanArgs *a, ManyBlocks b, cudaStream_t s);
+void launch_read_pass_many(const ReadArgs *a, ManyBlocks b, cudaStream_t s);
+uint32_t read_pass_grid();  // CTAs of it that are resident at once
+// the four steps' block lists; nb_max: most buckets of a job (at most kDedupTiled)
+constexpr uint32_t kDedupTiled = 2048;
+bool dedup_args(DedupArgs *a, const uint64_t *keys, uint64_t n, uint32_t nb, void *scratch, uint64_t *pk, uint32_t *pr,
+                uint8_t *alive, uint32_t *err);
+void launch_dedup_many(const DedupArgs *a, uint32_t jobs, uint32_t nb_max, ManyBlocks hist, ManyBlocks scatter,
+                       ManyBlocks mark, cudaStream_t s);
+void launch_init_list_many(const InitArgs *a, ManyBlocks b, cudaStream_t s);
+// out[16 j ..] = the 16 words at src[j]
+void launch_gather_words(const uint64_t *const *src, uint32_t jobs, uint64_t *out, cudaStream_t s);
+
 // ---- map phase (k_map.cu) -------------------------------------------------
 constexpr uint64_t kParseTile = 16384;  // FASTQ bytes per tile
 __host__ __device__ inline uint64_t parse_tiles(uint64_t F) { return (F + kParseTile - 1) / kParseTile; }

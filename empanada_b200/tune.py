@@ -7,9 +7,6 @@ the workload it times); they differ in speed:
                  Smaller buckets give more of them per round (better balance
                  across the SMs, more buckets in flight), larger ones fewer
                  per-bucket fixed costs.
-``map_streams``  streams a batch's map phase spreads its jobs over (batches
-                 only): more streams run more small jobs' kernels side by
-                 side, at more launch and synchronisation overhead.
 ``dedup_driver`` duplicate removal by key buckets and hash sets (0) or by
                  sorting every fingerprint (1).
 
@@ -34,7 +31,7 @@ from . import _native
 
 # the defaults first: they win ties
 JOB_CANDIDATES = {"bucket_mean": [2900, 2175, 1450], "dedup_driver": [0, 1]}
-BATCH_CANDIDATES = {"bucket_mean": [2900, 2175, 1450], "map_streams": [8, 16, 32, 4]}
+BATCH_CANDIDATES = {"bucket_mean": [2900, 2175, 1450]}
 
 
 def enabled() -> bool:
