@@ -787,9 +787,14 @@ def main():
             kname = "coop_rounds_kernel"
             what = ("all rounds, Bloom-filter driver: per round 13 B + 1/4 B per entry in, 24 B per kept entry, "
                     "72 B per candidate, 8 B per edge")
+        elif 2 * st["n_unique"] <= 9 << 20:  # lists that start in the sweep kernel whatever their density
+            kname = "sweep_kernel"
+            what = ("all rounds in one launch, many per step; counted as one pass per round over the live entries: "
+                    "16 B per entry, 16 B per entry kept for the next round, 8 B per edge")
         else:
             kname = "bucket_rounds_kernel"
-            what = ("all rounds in one launch (with the prologue launch of a directly binned job, timed together): "
+            what = ("all rounds in one launch (with the prologue launch of a directly binned job and the sweep launch that "
+                    "takes over the last rounds, timed together): "
                     "per round 16 B gathered per entry, 16 B written per entry kept for the next round, 8 B per edge")
     elif sort_ms >= upd_ms:  # the radix-sort digit pass dominates
         per_launch = 24.0 * sort_elems / max(sort_passes, 1)

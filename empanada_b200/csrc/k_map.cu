@@ -20,6 +20,8 @@
 //   compact_reads the kept records to consecutive indices (only when the
 //                 N filter or an empty line dropped one)
 //   columns       read-major words -> column-major words (only when needed)
+// nl_count and read_pass also run once for all jobs of a batch (the _many
+// kernels): a block's job and its number within the job come from a list.
 #include <atomic>
 
 #include "sort_block.cuh"

@@ -11,7 +11,7 @@
 //      filter; a hit is a candidate: it enters a chain of its (key, round)'s
 //      hash and a second, small filter
 //   C  every live suffix again: its keys against the second filter, then the
-//      the chain; a suffix whose key is there makes a pair (suffix, prefix,
+//      chain; a suffix whose key is there makes a pair (suffix, prefix,
 //      round) with each prefix of that key from another read (get_edges,
 //      overlap.cu:557-603)
 //   resolve  no entry was removed inside the step, so a pair may hold entries
@@ -37,12 +37,16 @@
 // round for a long time (an entry beyond a sequencing error or a coverage
 // gap): here such an entry costs a hash step and three random L2 accesses
 // per round, and a grid barrier is paid per phase of a step of up to 32
-// rounds.  Bound: random L2 accesses (measured on this chip 188 G/s for a
-// reduction, 276 G/s for a load, 121 G/s for a compare-and-swap, a sixth of
-// that beyond 64 MB), which is why the filters and chains of a step are kept
-// within L2 (kFilterKeys).  All rounds, bucket kernel -> here: 2,000 x 100
-// reads 1.16 -> 0.29 ms, 100k x 150 1.90 -> 0.53, 1.2M x 250 8.03 -> 4.0,
-// 256 sets (13.2M reads) 71 -> 37 ms.
+// rounds.  Bound: random accesses.  A lane's own line costs the load unit of
+// an SM one cycle for a load (276 G/s on the chip), 1.5 for a reduction (188),
+// 2.3 for an exchange (121), a sixth of that rate where they leave L2; a late
+// step of 1.2M x 250 reads (16M keys) runs its reductions at 160 G/s and its
+// loads at 160.  What is left around them: a chunk's entries and bases (on
+// their way a chunk ahead), the candidates' chain of an exchange and two
+// stores, warps that end early (they draw their segments), and for a few
+// thousand entries the latency of 8 barriers a step, 60 us.  All rounds,
+// bucket kernel -> here: 2,000 x 100 reads 1.16 -> 0.245 ms, 100k x 150 1.90
+// -> 0.505, 1.2M x 250 8.03 -> 3.17, 256 sets (13.2M reads) 71 -> 26 ms.
 #include "coop_common.cuh"
 
 namespace emp {

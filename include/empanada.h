@@ -110,9 +110,11 @@ emp_status emp_ctx_destroy(emp_ctx *ctx);
  * autotuner, empanada_b200.tune, picks them by timing) or serve tests.  A
  * zero field means its default.  Set them while no job of the context runs. */
 typedef struct emp_tuning {
-    int32_t round_driver;     /* 0: the bucket kernel for every round that cannot split into
-                                 several search partitions; 1: host-synchronised rounds only */
-    uint32_t bucket_mean;     /* bucket kernel: entries per key bucket aimed at, 512..3000 (default 2900) */
+    int32_t round_driver;     /* 0: the sweep kernel, and the bucket kernel for long lists, for every
+                                 round that cannot split into several search partitions;
+                                 1: host-synchronised rounds only */
+    uint32_t bucket_mean;     /* bucket kernel: entries per key bucket aimed at, 512..3000 (default 2900;
+                                 another value keeps every such round in the bucket kernel) */
     uint32_t region_cap;      /* bucket kernel: entries per (bucket, table) region, 1..2048 (default 2048);
                                  a region's overflow goes to a spill area */
     int32_t dedup_driver;     /* 0: duplicate removal by key buckets and hash sets where 2n <= M (the
@@ -177,7 +179,8 @@ emp_status emp_job_run(emp_job *job, void *stream);
 /* emp_job_run of njobs independent jobs of one context (at most 1024, each
  * once) as one batch: the map phase of every job with one stream
  * synchronisation per stage for the whole batch, and the rounds of all jobs
- * whose lists fit the bucket kernel in a single launch of it.  Replaces one
+ * whose rounds cannot split in one launch of the sweep kernel (and one of the
+ * bucket kernel for the long ones).  Replaces one
  * run of the reference's whole program (main.cu:42-71, then build_graph,
  * overlap.cu:206-293) per read set; each job's output is byte-identical to
  * emp_job_run's.  Returns the first failing job's status (jobs that failed
@@ -193,9 +196,9 @@ emp_status emp_job_status(emp_job *job);
  * submitted; each step admits queued jobs (first come, first served, while
  * the footprint estimates of the jobs in flight stay within the budget: 4 B
  * per FASTQ byte + 64 MiB per job), runs their map phase, adds them to the
- * batch, and runs one bucket-kernel launch of at most rounds_per_launch
- * rounds of every job in the batch; jobs join and leave the batch between
- * launches.  A job too large for the batch, or whose rounds split into
+ * batch, and runs all rounds of its short jobs in one launch and at most
+ * rounds_per_launch rounds of every long one (share_min_entries) in another;
+ * jobs join and leave the batch between launches.  A job too large for the batch, or whose rounds split into
  * several search partitions, runs alone within the step, and so does a job
  * admitted alone into an idle server (no job in flight or queued), as
  * emp_job_run runs it.  Every job's output
