@@ -22,6 +22,7 @@
 #include <cstring>
 #include <deque>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1656,7 +1657,7 @@ emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &job
 // The map phase of jobs[0..n) with one stream synchronisation per stage for
 // all of them; a job that fails gets its status in rc.  Jobs left with rc
 // EMP_OK and prep.done unset have their lists ready for the rounds.
-emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
+emp_status map_batch_stages(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
     auto live = [&](int i) { return rc[i] == EMP_OK && !jobs[i]->prep.done; };
     auto fail = [&](int i, emp_status e) {
         if (rc[i] == EMP_OK) rc[i] = e;
@@ -1701,6 +1702,15 @@ emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStr
         if (live(i)) fail(i, map_list(jobs[i], s));
     }
     return EMP_OK;
+}
+
+// The same with a failed host allocation (the stages' lists) as a status.
+emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
+    try {
+        return map_batch_stages(jobs, n, rc, s);
+    } catch (const std::bad_alloc &) {
+        return EMP_E_NOMEM;
+    }
 }
 
 // Close jobs[0..n) whose work is all queued: their last events, one
