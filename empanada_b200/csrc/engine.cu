@@ -300,6 +300,15 @@ emp_status ctx_ensure(emp_ctx *c, DevBuf &b, size_t bytes, cudaStream_t s) {
     return EMP_OK;
 }
 
+// Size for a buffer that grows with the batch: each larger batch than any
+// before would otherwise allocate, and page-locking a few MB takes a
+// millisecond (a burst through the server: 112 ms of 2 s).
+size_t roomy(size_t bytes) {
+    size_t r = 1u << 20;
+    while (r < bytes) r *= 2;
+    return r;
+}
+
 // a job's buffers grow in the order of the stream its current run uses
 emp_status ensure(emp_job *j, DevBuf &b, size_t bytes) {
     return ctx_ensure(j->ctx, b, bytes, j->stream ? j->stream : j->ctx->stream);
@@ -1124,8 +1133,9 @@ emp_status many_flush(emp_ctx *c, MapMany &m, cudaStream_t s) {
     add(m.fetch.size() * sizeof(uint64_t *));
     static_assert(kMiscSlots == 16, "a job's words as launch_gather_words takes them");
     const size_t words = m.fetch.size() * kMiscSlots * 8;
-    EMP_TRY(ctx_ensure(c, c->many, total + words + 256, s));
-    if (!c->h_many.ensure(total + words + 256)) return EMP_E_NOMEM;
+    const size_t room = roomy(total + words + 256);
+    EMP_TRY(ctx_ensure(c, c->many, room, s));
+    if (!c->h_many.ensure(room)) return EMP_E_NOMEM;
     uint8_t *h = c->h_many.as<uint8_t>(), *d = c->many.as<uint8_t>();
     auto put = [&](int k, const auto &v) {
         if (!v.empty()) std::memcpy(h + at[k], v.data(), v.size() * sizeof(v[0]));
@@ -1587,8 +1597,8 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     }
     sb.records = (nb * sizeof(SweepJob) + sizeof(CoopCtl) + 255) / 256 * 256;
     const size_t total = sb.records + recs * sizeof(RoundRecord);
-    EMP_TRY(ctx_ensure(ctx, sb.jobs, total, s));
-    if (!sb.host.ensure(total)) return EMP_E_NOMEM;
+    EMP_TRY(ctx_ensure(ctx, sb.jobs, roomy(total), s));
+    if (!sb.host.ensure(roomy(total))) return EMP_E_NOMEM;
     if (!sb.ev[0]) {
         for (auto &e : sb.ev) EMP_CUDA(cudaEventCreate(&e));
     }
@@ -1605,7 +1615,7 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     }
     SweepOut go{};
     size_t zeroed = 0;
-    EMP_TRY(ctx_ensure(ctx, sb.out, sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed), s));
+    EMP_TRY(ctx_ensure(ctx, sb.out, roomy(sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed)), s));
     sweep_out_layout(sb.out.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
     EMP_CUDA(cudaMemsetAsync(sb.out.p, 0, zeroed, s));
     coop_ctl_init(ctx, hc, (uint32_t)nb);
