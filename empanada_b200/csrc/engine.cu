@@ -524,6 +524,18 @@ emp_status dout_room(emp_job *j, size_t bytes, size_t ahead, cudaStream_t s) {
     return cuda_status(e);
 }
 
+// Edge buffers of more edges than this are refused: no device holds them, and
+// their sizes in bytes would wrap further on.
+constexpr uint64_t kMostEdges = 1ull << 40;
+
+// Room in dout, behind the records that are there, for those of a launch over
+// `rounds` rounds with up to ecap edges (the kernels check their edges against
+// ecap alone).
+emp_status records_room(emp_job *j, int rounds, uint64_t ecap, cudaStream_t s) {
+    if (ecap > kMostEdges) return EMP_E_NOMEM;
+    return dout_room(j, (size_t)j->dout_bytes + (size_t)rounds * 12 + ecap * 8, 0, s);
+}
+
 struct RoundEnv {
     int L;
     int rounds;
@@ -625,7 +637,7 @@ emp_status sync_round(emp_job *j, cudaStream_t s, const RoundEnv &env, int r, in
     auto records = [&](const SearchPart *parts, uint64_t np, uint64_t nrec, uint64_t nedge) -> emp_status {
         const size_t bytes = 12 * nrec + 8 * nedge;
         j->prep.dev_out = true;
-        EMP_TRY(dout_room(j, j->dout_bytes + bytes, (size_t)env.rounds * 12 + j->prep.ecap * 8, s));
+        EMP_TRY(dout_room(j, j->dout_bytes + bytes, (size_t)env.rounds * 12 + std::min(j->prep.ecap, kMostEdges) * 8, s));
         launch_write_records(parts, np, E, ovlp, j->efrom.as<uint32_t>(), j->eto.as<uint32_t>(),
                              j->dout.as<uint8_t>() + j->dout_bytes, s);
         j->dout_bytes += bytes;
@@ -750,6 +762,7 @@ emp_status bucket_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r
     const uint64_t list_entries = (uint64_t)nb_max * 2 * cap;
     const uint64_t iters = (uint64_t)(env.rounds - r0) + 1;  // lists of iterations 0 .. rounds - r0
     const size_t cnt_bytes = iters * 2 * nb_max * 4;
+    EMP_TRY(records_room(j, env.rounds, ecap, s));
     EMP_TRY(ensure(j, j->bk_lst0, list_entries * sizeof(BktEntry)));
     EMP_TRY(ensure(j, j->bk_lst1, list_entries * sizeof(BktEntry)));
     EMP_TRY(ensure(j, j->bk_cnt, cnt_bytes + iters * 4));
@@ -761,8 +774,6 @@ emp_status bucket_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r
     EMP_TRY(ensure(j, j->bk_scratch, bkt_scratch_bytes(nmax)));
     EMP_TRY(ensure(j, j->bk_meta, ((size_t)env.rounds + 1) * sizeof(BktRound)));
     EMP_CUDA(cudaMemsetAsync(j->bk_meta.p, 0, ((size_t)env.rounds + 1) * sizeof(BktRound), s));
-    // behind the records of host-driven rounds
-    EMP_TRY(dout_room(j, (size_t)j->dout_bytes + (size_t)env.rounds * 12 + ecap * 8, 0, s));
     EMP_TRY(ensure(j, j->records, (size_t)env.rounds * sizeof(RoundRecord)));
     if (!j->h_records.ensure((size_t)env.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
     std::memset(hj, 0, sizeof(BktJob));
@@ -904,11 +915,13 @@ emp_status run_rounds_bucket(emp_job *j, cudaStream_t s, const RoundEnv &env, in
     st.ms_round_kernel += ms_between(e0, e1);
     if (trace_path) write_coop_trace(j, trace_path, env.rounds, r0, j->h_records.as<RoundRecord>(), s, 1, "round_us");
     if (probe_env) write_coop_probe(j, probe_path.c_str(), grid, s);
+    const uint64_t host_edges = st.n_edges;  // of the host-driven rounds before, which are not in ecap
     EMP_TRY(bucket_collect(j, r0, n_in, *hj, needed));
     if (!hj->hand_iter) return EMP_OK;
-    // the rounds from r1 on in the sweep kernel, their edges behind those of the rounds before
+    // the rounds from r1 on in the sweep kernel, their edges behind those of the
+    // rounds before: what this launch left of its ecap edges
     const int r1 = r0 + (int)hj->hand_iter;
-    const uint64_t ns = hj->hand_s, np = hj->hand_n - ns, E = st.n_edges;
+    const uint64_t ns = hj->hand_s, np = hj->hand_n - ns, E = st.n_edges - host_edges;
     EMP_CUDA(launch_bucket_list(j->bk_job.as<BktJob>(), j->lk0.as<uint64_t>(), j->lv0.as<uint32_t>(), s));
     const emp_status rc = run_rounds_sweep(j, s, env, r1, 0, ns, np, ecap - E, needed, true);
     if (rc == kNeedEdgeRoom) *needed += E;
@@ -968,7 +981,7 @@ emp_status sweep_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r0
     EMP_TRY(ensure(j, j->swp, sweep_layout(nullptr, hj, &zeroed)));
     sweep_layout(j->swp.as<uint8_t>(), hj, &zeroed);
     // behind the records of the rounds that ran before, whose buffer held all
-    EMP_TRY(dout_room(j, (size_t)j->dout_bytes + (size_t)(env.rounds - r0) * 12 + ecap * 8, 0, s));
+    EMP_TRY(records_room(j, env.rounds - r0, ecap, s));
     hj->out = j->dout.as<uint8_t>() + j->dout_bytes;
     return EMP_OK;
 }
