@@ -1681,6 +1681,7 @@ emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &job
 // all of them; a job that fails gets its status in rc.  Jobs left with rc
 // EMP_OK and prep.done unset have their lists ready for the rounds.
 emp_status map_batch_stages(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
+    for (int i = 0; i < n; ++i) jobs[i]->prep = JobPrep{};  // a job's last set may have ended it early
     auto live = [&](int i) { return rc[i] == EMP_OK && !jobs[i]->prep.done; };
     auto fail = [&](int i, emp_status e) {
         if (rc[i] == EMP_OK) rc[i] = e;
