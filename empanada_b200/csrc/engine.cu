@@ -1729,17 +1729,32 @@ emp_status map_batch_stages(emp_job **jobs, int n, std::vector<emp_status> &rc, 
 }
 
 // The same with a failed host allocation (the stages' lists) as a status.
+// Where there is no room for what the jobs share, they go one after another,
+// each with a status of its own.
 emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
-    try {
-        return map_batch_stages(jobs, n, rc, s);
-    } catch (const std::bad_alloc &) {
-        return EMP_E_NOMEM;
+    auto stages = [&](emp_job **js, int k, std::vector<emp_status> &r) -> emp_status {
+        try {
+            return map_batch_stages(js, k, r, s);
+        } catch (const std::bad_alloc &) {
+            return EMP_E_NOMEM;
+        }
+    };
+    emp_status e = stages(jobs, n, rc);
+    if (e != EMP_E_NOMEM || n < 2) return e;
+    EMP_CUDA(cudaStreamSynchronize(s));
+    std::vector<emp_status> one(1);
+    for (int i = 0; i < n; ++i) {
+        one[0] = EMP_OK;
+        e = stages(jobs + i, 1, one);
+        if (e != EMP_OK && e != EMP_E_NOMEM) return e;
+        rc[i] = e != EMP_OK ? e : one[0];
     }
+    return EMP_OK;
 }
 
 // Close jobs[0..n) whose work is all queued: their last events, one
 // synchronisation, then results (rc[i] == EMP_OK) or none.  Sets each job's
-// last_rc; returns the first failure.
+// last_rc, whatever happens; returns the first failure.
 emp_status close_jobs(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
     for (int i = 0; i < n; ++i) {
         if (rc[i] != EMP_OK) continue;
@@ -1748,10 +1763,11 @@ emp_status close_jobs(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaSt
             cudaEventRecord(jobs[i]->map_ev[4], s);
         }
     }
-    EMP_CUDA(cudaStreamSynchronize(s));
-    EMP_CUDA(cudaGetLastError());
+    const cudaError_t synced = cudaStreamSynchronize(s), last = cudaGetLastError();
+    const emp_status all = cuda_status(synced != cudaSuccess ? synced : last);
     emp_status first = EMP_OK;
     for (int i = 0; i < n; ++i) {
+        if (rc[i] == EMP_OK) rc[i] = all;
         if (rc[i] == EMP_OK) {
             job_finish(jobs[i]);
         } else {
@@ -1767,7 +1783,8 @@ emp_status close_jobs(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaSt
 // ones in one bucket-kernel launch, the others' rounds one job after another.
 emp_status run_batch(emp_ctx *ctx, emp_job **jobs, int n, cudaStream_t s) {
     std::vector<emp_status> rc((size_t)n, EMP_OK);
-    EMP_TRY(map_batch(jobs, n, rc, s));
+    const emp_status mapped = map_batch(jobs, n, rc, s);
+    if (mapped != EMP_OK) rc.assign((size_t)n, mapped);
     std::vector<int> sweep, bucket, alone;
     for (int i = 0; i < n; ++i) {
         if (rc[i] != EMP_OK || jobs[i]->prep.done) continue;
@@ -1860,19 +1877,19 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     std::vector<emp_job *> swept;
     swept.swap(srv->sweep);
     emp_status sweep_rc = EMP_OK;
-    struct SweptGuard {  // a step that ends early: the launch has overwritten their lists, so they fail
+    struct HeldGuard {  // a step that ends early: the jobs that are in none of the server's lists fail
         emp_server *srv;
         std::vector<emp_job *> &jobs;
         cudaStream_t s;
         bool closed = false;
-        ~SweptGuard() {
+        ~HeldGuard() {
             if (closed || jobs.empty()) return;
             cudaStreamSynchronize(s);
             std::vector<emp_status> rc(jobs.size(), EMP_E_CUDA);
             close_jobs(jobs.data(), (int)jobs.size(), rc, s);
             for (emp_job *j : jobs) server_complete(srv, j);
         }
-    } swept_guard{srv, swept, s};
+    } adm_guard{srv, adm, s}, swept_guard{srv, swept, s};
     if (!swept.empty()) sweep_rc = sweep_batch_launch(ctx, srv->sb, swept, s);
     const size_t nb = srv->live.size();
     BktJob *hj = nullptr;
@@ -1911,12 +1928,18 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     }
     ss.ms_launch += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - ts).count();
     // ---- the admitted jobs' map phase
+    emp_status map_rc = EMP_OK;  // of the phase as a whole: every admitted job comes back with it
+    auto step_rc = [&](bool timed_out) {
+        return timed_out || sweep_rc == EMP_E_TIMEOUT ? EMP_E_TIMEOUT : map_rc == EMP_E_CUDA ? map_rc : EMP_OK;
+    };
     std::vector<emp_job *> joining;
     if (!adm.empty()) {
         const auto t0 = std::chrono::steady_clock::now();
         const int n = (int)adm.size();
         std::vector<emp_status> rc((size_t)n, EMP_OK);
-        EMP_TRY(map_batch(adm.data(), n, rc, s));
+        adm_guard.closed = true;
+        map_rc = map_batch(adm.data(), n, rc, s);
+        if (map_rc != EMP_OK) rc.assign((size_t)n, map_rc);
         const auto t1 = std::chrono::steady_clock::now();
         ss.ms_map += std::chrono::duration<double, std::milli>(t1 - t0).count();
         std::vector<emp_job *> close;
@@ -1958,7 +1981,7 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
         ss.ms_admit += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }
     if (!nb) srv->live.swap(joining);
-    if (!nb && swept.empty()) return EMP_OK;
+    if (!nb && swept.empty()) return step_rc(false);
     // ---- the launches' results
     const auto tw = std::chrono::steady_clock::now();
     EMP_CUDA(cudaStreamSynchronize(s));
@@ -1980,7 +2003,7 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
         close_jobs(swept.data(), (int)swept.size(), rc, s);
         for (emp_job *j : swept) server_complete(srv, j);
     }
-    if (!nb) return sweep_rc == EMP_E_TIMEOUT ? EMP_E_TIMEOUT : EMP_OK;
+    if (!nb) return step_rc(false);
     const bool timed_out = (hc->err & kErrSpin) != 0;
     const float ms = ms_between(srv->ev[0], srv->ev[1]);
     ss.launches += 1;
@@ -2003,7 +2026,7 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     }
     still.insert(still.end(), joining.begin(), joining.end());
     srv->live.swap(still);
-    if (done.empty()) return sweep_rc == EMP_E_TIMEOUT ? EMP_E_TIMEOUT : EMP_OK;
+    if (done.empty()) return step_rc(false);
     EMP_CUDA(cudaStreamSynchronize(s));
     std::vector<emp_status> rc(done.size(), timed_out ? EMP_E_TIMEOUT : EMP_OK);
     for (size_t k = 0; k < done.size() && !timed_out; ++k) {
@@ -2019,7 +2042,7 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     }
     close_jobs(done.data(), (int)done.size(), rc, s);
     for (emp_job *j : done) server_complete(srv, j);
-    return timed_out || sweep_rc == EMP_E_TIMEOUT ? EMP_E_TIMEOUT : EMP_OK;
+    return step_rc(timed_out);
 }
 
 }  // namespace
