@@ -142,6 +142,7 @@ struct SweepBatch {
     DevBuf jobs, out;  // descriptors, control block and round records; output bins
     PinnedBuf host;    // the same as `jobs`
     size_t records = 0;  // offset of the round records
+    std::vector<size_t> in, out_of_it;  // the jobs of the launch; those with no room for it, which run alone
     cudaEvent_t ev[2] = {};
     uint64_t bytes() const { return jobs.bytes + out.bytes; }
     void release() {
@@ -1599,47 +1600,69 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
 }
 
 // One launch of the sweep kernel over all rounds of several jobs (lists
-// ready): queued by launch, read by collect once the stream has been waited for.
+// ready): queued by launch, read by collect once the stream has been waited
+// for.  A job whose buffers are refused is left out of it, and all of them
+// where there is no room for what they share.
 emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<emp_job *> &jobs, cudaStream_t s) {
     const size_t nb = jobs.size();
     uint64_t side = 0, bins = 0, recs = 0;
     for (emp_job *j : jobs) {
         side += j->prep.U;
-        bins += sweep_bins_max(2 * j->prep.U, j->prep.rounds);
         recs += (uint64_t)j->prep.rounds;
     }
+    sb.in.clear();
+    sb.out_of_it.clear();
+    auto none = [&](emp_status e) -> emp_status {
+        if (e != EMP_E_NOMEM) return e;
+        sb.in.clear();
+        sb.out_of_it.resize(nb);
+        for (size_t k = 0; k < nb; ++k) sb.out_of_it[k] = k;
+        return EMP_OK;
+    };
     sb.records = (nb * sizeof(SweepJob) + sizeof(CoopCtl) + 255) / 256 * 256;
     const size_t total = sb.records + recs * sizeof(RoundRecord);
-    EMP_TRY(ctx_ensure(ctx, sb.jobs, roomy(total), s));
-    if (!sb.host.ensure(roomy(total))) return EMP_E_NOMEM;
+    const emp_status room = ctx_ensure(ctx, sb.jobs, roomy(total), s);
+    if (room != EMP_OK) return none(room);
+    if (!sb.host.ensure(roomy(total))) return none(EMP_E_NOMEM);
     if (!sb.ev[0]) {
         for (auto &e : sb.ev) EMP_CUDA(cudaEventCreate(&e));
     }
     SweepJob *hj = sb.host.as<SweepJob>(), *dj = sb.jobs.as<SweepJob>();
-    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + nb), *dc = reinterpret_cast<CoopCtl *>(dj + nb);
     RoundRecord *rec = reinterpret_cast<RoundRecord *>(sb.jobs.as<uint8_t>() + sb.records);
     for (size_t k = 0; k < nb; ++k) {
         emp_job *j = jobs[k];
         const JobPrep &q = j->prep;
+        SweepJob &d = hj[sb.in.size()];
         rounds_prelude(j);
-        EMP_TRY(sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, side, false, &hj[k]));
-        hj[k].records = rec;
+        const emp_status e = sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, side, false, &d);
+        if (e == EMP_E_NOMEM) {
+            sb.out_of_it.push_back(k);
+            continue;
+        }
+        EMP_TRY(e);
+        d.records = rec;
         rec += q.rounds;
+        bins += sweep_bins_max(2 * q.U, q.rounds);
+        sb.in.push_back(k);
     }
+    const size_t n_in = sb.in.size();
+    if (!n_in) return EMP_OK;
+    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + n_in), *dc = reinterpret_cast<CoopCtl *>(dj + n_in);
     SweepOut go{};
     size_t zeroed = 0;
-    EMP_TRY(ctx_ensure(ctx, sb.out, roomy(sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed)), s));
+    const emp_status bin_room = ctx_ensure(ctx, sb.out, roomy(sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed)), s);
+    if (bin_room != EMP_OK) return none(bin_room);
     sweep_out_layout(sb.out.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
     EMP_CUDA(cudaMemsetAsync(sb.out.p, 0, zeroed, s));
-    coop_ctl_init(ctx, hc, (uint32_t)nb);
+    coop_ctl_init(ctx, hc, (uint32_t)n_in);
     if (!ctx->trace_path.empty()) {
-        emp_job *j = jobs[0];
+        emp_job *j = jobs[sb.in[0]];
         EMP_TRY(ensure(j, j->coop_trace, (size_t)kSweepTraceCap * kCoopTracePhases * 8));
         EMP_CUDA(cudaMemsetAsync(j->coop_trace.p, 0, j->coop_trace.bytes, s));
         hc->trace = j->coop_trace.as<uint64_t>();
         hc->trace_cap = kSweepTraceCap;
     }
-    EMP_CUDA(cudaMemcpyAsync(dj, hj, nb * sizeof(SweepJob) + sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    EMP_CUDA(cudaMemcpyAsync(dj, hj, n_in * sizeof(SweepJob) + sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
     EMP_CUDA(cudaEventRecord(sb.ev[0], s));
     EMP_CUDA(launch_sweep(dj, dc, go, true, s));
     EMP_CUDA(cudaEventRecord(sb.ev[1], s));
@@ -1647,34 +1670,39 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     return EMP_OK;
 }
 
-// Per-job status of the launch in rc; a job whose edges did not fit, or that
-// is not one for the sweep kernel, runs again alone.
+// Per-job status of the launch in rc; a job whose edges did not fit, that is
+// not one for the sweep kernel, or that was left out, runs alone.
 emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &jobs, std::vector<emp_status> &rc,
                                cudaStream_t s) {
-    const size_t nb = jobs.size();
     const SweepJob *hj = sb.host.as<SweepJob>();
-    if (reinterpret_cast<const CoopCtl *>(hj + nb)->err & kErrSpin) return EMP_E_TIMEOUT;
-    const float ms = ms_between(sb.ev[0], sb.ev[1]);
-    if (nb && !jobs[0]->ctx->trace_path.empty()) write_sweep_trace(jobs[0], jobs[0]->ctx->trace_path.c_str(), s);
-    const RoundRecord *rec = reinterpret_cast<const RoundRecord *>(sb.host.as<uint8_t>() + sb.records);
-    for (size_t k = 0; k < nb; ++k) {
-        emp_job *j = jobs[k];
-        JobPrep &q = j->prep;
-        j->st.ms_round_kernel += ms;  // the whole batch's launch
-        if (!j->h_records.ensure((size_t)q.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
-        std::memcpy(j->h_records.p, rec, (size_t)q.rounds * sizeof(RoundRecord));
-        rec += q.rounds;
-        uint64_t needed = 0;
-        emp_status r = hj[k].crowded ? kCrowded : bucket_collect(j, 0, 2 * q.U, hj[k], &needed);
-        if (r == kNeedEdgeRoom || r == kCrowded) {
-            if (r == kCrowded) q.no_sweep = true;
-            else j->ecap_hint = q.ecap = needed + needed / 4 + 1024;
-            r = rebuild_list(j, s);
-            if (r == EMP_OK) r = job_rounds(j, s);
+    const bool timed_out = !sb.in.empty() && (reinterpret_cast<const CoopCtl *>(hj + sb.in.size())->err & kErrSpin);
+    if (!sb.in.empty() && !timed_out) {
+        const float ms = ms_between(sb.ev[0], sb.ev[1]);
+        emp_job *j0 = jobs[sb.in[0]];
+        if (!j0->ctx->trace_path.empty()) write_sweep_trace(j0, j0->ctx->trace_path.c_str(), s);
+        const RoundRecord *rec = reinterpret_cast<const RoundRecord *>(sb.host.as<uint8_t>() + sb.records);
+        for (size_t k = 0; k < sb.in.size(); ++k) {
+            emp_job *j = jobs[sb.in[k]];
+            JobPrep &q = j->prep;
+            j->st.ms_round_kernel += ms;  // the whole batch's launch
+            if (!j->h_records.ensure((size_t)q.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
+            std::memcpy(j->h_records.p, rec, (size_t)q.rounds * sizeof(RoundRecord));
+            rec += q.rounds;
+            uint64_t needed = 0;
+            emp_status r = hj[k].crowded ? kCrowded : bucket_collect(j, 0, 2 * q.U, hj[k], &needed);
+            if (r == kNeedEdgeRoom || r == kCrowded) {
+                if (r == kCrowded) q.no_sweep = true;
+                else j->ecap_hint = q.ecap = needed + needed / 4 + 1024;
+                r = rebuild_list(j, s);
+                if (r == EMP_OK) r = job_rounds(j, s);
+            }
+            rc[sb.in[k]] = r;
         }
-        rc[k] = r;
     }
-    return EMP_OK;
+    if (timed_out)
+        for (size_t k : sb.in) rc[k] = EMP_E_TIMEOUT;
+    for (size_t k : sb.out_of_it) rc[k] = job_rounds(jobs[k], s);
+    return timed_out ? EMP_E_TIMEOUT : EMP_OK;
 }
 
 // The map phase of jobs[0..n) with one stream synchronisation per stage for
@@ -1799,7 +1827,7 @@ emp_status run_batch(emp_ctx *ctx, emp_job **jobs, int n, cudaStream_t s) {
         emp_status e = sweep_batch_launch(ctx, ctx->batch_swp, js, s);
         if (e == EMP_OK) e = cuda_status(cudaStreamSynchronize(s));
         if (e == EMP_OK) e = sweep_batch_collect(ctx->batch_swp, js, src, s);
-        for (size_t k = 0; k < sweep.size(); ++k) rc[sweep[k]] = e != EMP_OK ? e : src[k];
+        for (size_t k = 0; k < sweep.size(); ++k) rc[sweep[k]] = e != EMP_OK && e != EMP_E_TIMEOUT ? e : src[k];
     }
     if (!bucket.empty()) {
         const emp_status e = batch_rounds(ctx, jobs, bucket, rc, s);
@@ -1995,11 +2023,14 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
     if (!swept.empty()) {
         swept_guard.closed = true;
         std::vector<emp_status> rc(swept.size(), EMP_OK);
+        if (sweep_rc == EMP_OK && !srv->sb.in.empty()) {
+            ss.launches += 1;
+            ss.batch_jobs += srv->sb.in.size();
+            ss.ms_kernel += ms_between(srv->sb.ev[0], srv->sb.ev[1]);
+        }
         if (sweep_rc == EMP_OK) sweep_rc = sweep_batch_collect(srv->sb, swept, rc, s);
-        if (sweep_rc != EMP_OK) rc.assign(swept.size(), sweep_rc);
-        ss.launches += 1;
-        ss.batch_jobs += swept.size();
-        ss.ms_kernel += ms_between(srv->sb.ev[0], srv->sb.ev[1]);
+        if (sweep_rc != EMP_OK && sweep_rc != EMP_E_TIMEOUT) rc.assign(swept.size(), sweep_rc);
+        ss.alone += srv->sb.out_of_it.size();
         close_jobs(swept.data(), (int)swept.size(), rc, s);
         for (emp_job *j : swept) server_complete(srv, j);
     }

@@ -1,6 +1,8 @@
 """Batches and server steps under a device-memory budget, from one that holds
 everything down to one that holds nothing: every job comes back with a status
 of its own, and what ran has the bytes it gives alone."""
+import random
+
 import pytest
 
 import cases as G
@@ -73,3 +75,31 @@ def test_every_job_comes_back(run):
         seen.add(sum(status == 0 for status, _ in got))
         budget -= budget // 30
     assert {0, len(NAMES)} <= seen
+
+
+@pytest.mark.parametrize("server", [True, False])
+def test_a_job_that_does_not_fit_fails_alone(server):
+    """Two small sets and then a large one: from the largest budget that
+    refuses the large one's rounds, the small ones run."""
+    rng = random.Random(3)
+    small, large = (G.fastq(G._reads(rng, G._genome(rng, 10 * n), n, 100)) for n in (200, 8000))
+    with emp.Engine(0) as engine:
+        want = [emp.run_bytes(d, engine=engine, min_ovlp=31)[0] for d in (small, large)]
+    budget = (8 << 20) + 16 * len(large)
+    while True:
+        with emp.Engine(0, hbm_budget_bytes=budget) as engine, engine.tuned(edge_cap=1 << 16):
+            jobs = [engine.job(min_ovlp=31) for _ in range(3)]
+            for j, d in zip(jobs, (small, small, large)):
+                j.feed(d)
+            (_serve if server else _batch)(engine, jobs)
+            status = [j.status() for j in jobs]
+            out = [j.output() if j.status() == 0 else None for j in jobs]
+            for j in jobs:
+                j.close()
+        assert status[:2] == [0, 0], budget
+        assert out[:2] == [want[0]] * 2
+        if status[2]:
+            break
+        assert out[2] == want[1]
+        budget -= budget // 200
+    assert status[2] == _native.EMP_E_NOMEM
