@@ -309,6 +309,17 @@ size_t roomy(size_t bytes) {
     while (r < bytes) r *= 2;
     return r;
 }
+// Such a buffer with at least `bytes`; exactly that many under a budget, where
+// the jobs' own buffers need what rounding up would take, and where the
+// rounded size is not to be had.
+emp_status roomy_ensure(emp_ctx *c, DevBuf &b, size_t bytes, cudaStream_t s) {
+    if (bytes <= b.bytes) return EMP_OK;
+    if (!c->budget && ctx_ensure(c, b, roomy(bytes), s) == EMP_OK) return EMP_OK;
+    return ctx_ensure(c, b, bytes, s);
+}
+bool roomy_ensure(PinnedBuf &b, size_t bytes) {
+    return bytes <= b.bytes || b.ensure(roomy(bytes)) || b.ensure(bytes);
+}
 
 // a job's buffers grow in the order of the stream its current run uses
 emp_status ensure(emp_job *j, DevBuf &b, size_t bytes) {
@@ -1147,9 +1158,9 @@ emp_status many_flush(emp_ctx *c, MapMany &m, cudaStream_t s) {
     add(m.fetch.size() * sizeof(uint64_t *));
     static_assert(kMiscSlots == 16, "a job's words as launch_gather_words takes them");
     const size_t words = m.fetch.size() * kMiscSlots * 8;
-    const size_t room = roomy(total + words + 256);
-    EMP_TRY(ctx_ensure(c, c->many, room, s));
-    if (!c->h_many.ensure(room)) return EMP_E_NOMEM;
+    const size_t room = total + words + 256;
+    EMP_TRY(roomy_ensure(c, c->many, room, s));
+    if (!roomy_ensure(c->h_many, room)) return EMP_E_NOMEM;
     uint8_t *h = c->h_many.as<uint8_t>(), *d = c->many.as<uint8_t>();
     auto put = [&](int k, const auto &v) {
         if (!v.empty()) std::memcpy(h + at[k], v.data(), v.size() * sizeof(v[0]));
@@ -1601,29 +1612,28 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
 
 // One launch of the sweep kernel over all rounds of several jobs (lists
 // ready): queued by launch, read by collect once the stream has been waited
-// for.  A job whose buffers are refused is left out of it, and all of them
-// where there is no room for what they share.
+// for.  A job whose buffers are refused is left out of it; where there is no
+// room for what the jobs share, the largest are, one by one.
 emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<emp_job *> &jobs, cudaStream_t s) {
     const size_t nb = jobs.size();
-    uint64_t side = 0, bins = 0, recs = 0;
+    uint64_t side = 0, recs = 0;
     for (emp_job *j : jobs) {
         side += j->prep.U;
         recs += (uint64_t)j->prep.rounds;
     }
     sb.in.clear();
     sb.out_of_it.clear();
-    auto none = [&](emp_status e) -> emp_status {
-        if (e != EMP_E_NOMEM) return e;
-        sb.in.clear();
-        sb.out_of_it.resize(nb);
-        for (size_t k = 0; k < nb; ++k) sb.out_of_it[k] = k;
-        return EMP_OK;
+    auto leave_out = [&](size_t k) {
+        free_buf(jobs[k], jobs[k]->swp);
+        free_buf(jobs[k], jobs[k]->dout);
+        sb.out_of_it.push_back(k);
     };
     sb.records = (nb * sizeof(SweepJob) + sizeof(CoopCtl) + 255) / 256 * 256;
     const size_t total = sb.records + recs * sizeof(RoundRecord);
-    const emp_status room = ctx_ensure(ctx, sb.jobs, roomy(total), s);
-    if (room != EMP_OK) return none(room);
-    if (!sb.host.ensure(roomy(total))) return none(EMP_E_NOMEM);
+    if (roomy_ensure(ctx, sb.jobs, total, s) != EMP_OK || !roomy_ensure(sb.host, total)) {
+        for (size_t k = 0; k < nb; ++k) leave_out(k);
+        return EMP_OK;
+    }
     if (!sb.ev[0]) {
         for (auto &e : sb.ev) EMP_CUDA(cudaEventCreate(&e));
     }
@@ -1636,22 +1646,33 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
         rounds_prelude(j);
         const emp_status e = sweep_prepare(j, s, job_env(j), 0, 0, q.U, q.U, q.ecap, side, false, &d);
         if (e == EMP_E_NOMEM) {
-            sb.out_of_it.push_back(k);
+            leave_out(k);
             continue;
         }
         EMP_TRY(e);
         d.records = rec;
         rec += q.rounds;
-        bins += sweep_bins_max(2 * q.U, q.rounds);
         sb.in.push_back(k);
     }
-    const size_t n_in = sb.in.size();
-    if (!n_in) return EMP_OK;
-    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + n_in), *dc = reinterpret_cast<CoopCtl *>(dj + n_in);
     SweepOut go{};
     size_t zeroed = 0;
-    const emp_status bin_room = ctx_ensure(ctx, sb.out, roomy(sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed)), s);
-    if (bin_room != EMP_OK) return none(bin_room);
+    uint64_t bins = 0;
+    for (;;) {
+        if (sb.in.empty()) return EMP_OK;
+        bins = 0;
+        size_t most = 0;
+        for (size_t i = 0; i < sb.in.size(); ++i) {
+            const JobPrep &q = jobs[sb.in[i]]->prep;
+            bins += sweep_bins_max(2 * q.U, q.rounds);
+            if (q.U > jobs[sb.in[most]]->prep.U) most = i;
+        }
+        if (roomy_ensure(ctx, sb.out, sweep_out_layout(nullptr, (uint32_t)bins, &go, &zeroed), s) == EMP_OK) break;
+        leave_out(sb.in[most]);
+        sb.in.erase(sb.in.begin() + (ptrdiff_t)most);
+        std::memmove(hj + most, hj + most + 1, (sb.in.size() - most) * sizeof(SweepJob));
+    }
+    const size_t n_in = sb.in.size();
+    CoopCtl *hc = reinterpret_cast<CoopCtl *>(hj + n_in), *dc = reinterpret_cast<CoopCtl *>(dj + n_in);
     sweep_out_layout(sb.out.as<uint8_t>(), (uint32_t)bins, &go, &zeroed);
     EMP_CUDA(cudaMemsetAsync(sb.out.p, 0, zeroed, s));
     coop_ctl_init(ctx, hc, (uint32_t)n_in);
@@ -1680,14 +1701,13 @@ emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &job
         const float ms = ms_between(sb.ev[0], sb.ev[1]);
         emp_job *j0 = jobs[sb.in[0]];
         if (!j0->ctx->trace_path.empty()) write_sweep_trace(j0, j0->ctx->trace_path.c_str(), s);
-        const RoundRecord *rec = reinterpret_cast<const RoundRecord *>(sb.host.as<uint8_t>() + sb.records);
         for (size_t k = 0; k < sb.in.size(); ++k) {
             emp_job *j = jobs[sb.in[k]];
             JobPrep &q = j->prep;
             j->st.ms_round_kernel += ms;  // the whole batch's launch
             if (!j->h_records.ensure((size_t)q.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
-            std::memcpy(j->h_records.p, rec, (size_t)q.rounds * sizeof(RoundRecord));
-            rec += q.rounds;
+            const size_t at = (size_t)(reinterpret_cast<uint8_t *>(hj[k].records) - sb.jobs.as<uint8_t>());
+            std::memcpy(j->h_records.p, sb.host.as<uint8_t>() + at, (size_t)q.rounds * sizeof(RoundRecord));
             uint64_t needed = 0;
             emp_status r = hj[k].crowded ? kCrowded : bucket_collect(j, 0, 2 * q.U, hj[k], &needed);
             if (r == kNeedEdgeRoom || r == kCrowded) {

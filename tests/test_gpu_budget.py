@@ -103,3 +103,37 @@ def test_a_job_that_does_not_fit_fails_alone(server):
         assert out[2] == want[1]
         budget -= budget // 200
     assert status[2] == _native.EMP_E_NOMEM
+
+
+def test_a_batch_needs_little_more_than_its_jobs():
+    """The least budget of two jobs as a batch, beside that of the two run one
+    after another: what the batch shares beyond their own buffers is a few
+    hundred bytes a job and 8 bytes a block of its launches."""
+    rng = random.Random(4)
+    sets = [G.fastq(G._reads(rng, G._genome(rng, 10 * n), n, 100)) for n in (700, 900)]
+
+    def runs(budget, batch):
+        try:
+            with emp.Engine(0, hbm_budget_bytes=budget) as engine, engine.tuned(edge_cap=1 << 13):
+                jobs = [engine.job(min_ovlp=31) for _ in sets]
+                for j, d in zip(jobs, sets):
+                    j.feed(d)
+                if batch:
+                    engine.run_batch(jobs)
+                else:
+                    for j in jobs:
+                        j.run()
+                return True
+        except emp.EmpError as e:
+            assert e.code == _native.EMP_E_NOMEM
+            return False
+
+    def least(batch):
+        lo, hi = 1 << 16, 32 << 20  # refused, enough
+        assert runs(hi, batch) and not runs(lo, batch)
+        while hi - lo > 4096:
+            mid = (lo + hi) // 2
+            lo, hi = (lo, mid) if runs(mid, batch) else (mid, hi)
+        return hi
+
+    assert least(True) <= least(False) + (256 << 10)
