@@ -1486,7 +1486,8 @@ emp_status rebuild_list(emp_job *j, cudaStream_t s) {
                      j->misc.as<uint64_t>() + kMiscU, err_word(j), s);
     q.one_half = true;
     whole_list(j, s);
-    return EMP_OK;
+    EMP_TRY(sync_and_check(j, s));  // the rounds' launches do not read the job's error word
+    return j->h_misc.as<uint64_t>()[kMiscU] == q.U ? EMP_OK : EMP_E_CUDA;
 }
 
 // All rounds of one job, restarting with a larger edge buffer when needed.

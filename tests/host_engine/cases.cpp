@@ -1,0 +1,171 @@
+// The engine's host code on the CPU: engine.cu and hostcopy.cu over the CUDA
+// runtime beside this file, with kernels that only leave the counts which the
+// host reads.  Each case makes a call fail and returns 0 when the engine says so.
+#include "../../empanada_b200/csrc/engine.cu"
+#include "../../empanada_b200/csrc/hostcopy.cu"
+
+#include <thread>
+
+namespace fake {
+constexpr uint64_t kReads = 100, kLen = 50, kUnique = 150;
+std::function<void(uint32_t *err)> on_init_list;
+std::function<void(emp::SweepJob &)> on_sweep;
+int graph_builds = 0;
+}  // namespace fake
+
+namespace emp {
+void launch_nl_count(const uint8_t *, uint64_t, uint32_t *, uint64_t *, cudaStream_t) {}
+void launch_scan_u32_u64(const uint32_t *, uint64_t *, uint64_t, uint64_t *, uint32_t *, uint64_t *total, uint32_t *,
+                         cudaStream_t) {
+    *total = 4 * fake::kReads;
+}
+void launch_scan_u32_u32(const uint32_t *, uint32_t *, uint64_t, uint64_t *, uint32_t *, uint64_t *, uint32_t *,
+                         cudaStream_t) {}
+void launch_nl_count_many(const NlArgs *, ManyBlocks, cudaStream_t) {}
+void launch_scan_many(const ScanArgs *, ManyBlocks, cudaStream_t) {}
+void launch_read_pass_many(const ReadArgs *, ManyBlocks, cudaStream_t) {}
+uint32_t read_pass_grid() { return 148; }
+void launch_dedup_many(const DedupArgs *, uint32_t, uint32_t, ManyBlocks, ManyBlocks, ManyBlocks, cudaStream_t) {}
+void launch_init_list_many(const InitArgs *, ManyBlocks, cudaStream_t) {}
+void launch_gather_words(const uint64_t *const *, uint32_t, uint64_t *, cudaStream_t) {}
+void launch_read_pass(const uint8_t *, uint64_t, const uint64_t *, const HashTables *, const ChunkWeights *, uint64_t *,
+                      uint32_t *, int, uint32_t *, uint64_t *n_kept, uint32_t *len_minmax, uint32_t *, cudaStream_t) {
+    *n_kept = fake::kReads;
+    len_minmax[0] = ~(uint32_t)fake::kLen;
+    len_minmax[1] = fake::kLen;
+}
+void launch_compact_reads(const uint32_t *, uint64_t, uint64_t, const uint64_t *, const uint32_t *, int, uint64_t *,
+                          uint32_t *, cudaStream_t) {}
+void launch_columns(const uint32_t *, uint64_t, int, int, uint32_t *, uint64_t, cudaStream_t) {}
+uint32_t dedup_buckets(uint64_t) { return 1; }
+bool dedup_args(DedupArgs *, const uint64_t *, uint64_t, uint32_t, void *, uint64_t *, uint32_t *, uint8_t *,
+                uint32_t *) { return false; }
+bool launch_dedup_hash(const uint64_t *, uint64_t, uint32_t, void *, uint64_t *, uint32_t *, uint8_t *, uint32_t *,
+                       cudaStream_t) { return true; }
+void launch_dedup_mark(const uint64_t *, const uint32_t *, uint64_t, uint8_t *, cudaStream_t) {}
+void launch_init_list(const uint64_t *, const uint8_t *, uint64_t, uint64_t *, uint32_t *, uint64_t *, uint32_t *,
+                      uint64_t *count, uint32_t *err, cudaStream_t) {
+    *count = fake::kUnique;
+    if (fake::on_init_list) fake::on_init_list(err);
+}
+void launch_dup_prefix_half(uint64_t *, uint32_t *, uint64_t, cudaStream_t) {}
+void launch_iota(uint32_t *, uint64_t, cudaStream_t) {}
+void launch_update_compact(const RoundArgs &, cudaStream_t) {}
+void launch_split_tables(const uint64_t *, const uint32_t *, uint64_t, uint64_t *, uint32_t *, uint64_t *, uint64_t *,
+                         uint32_t *, uint32_t *, cudaStream_t) {}
+void launch_search_partitions(const uint64_t *, uint64_t, const uint64_t *, uint64_t, uint64_t, const uint32_t *,
+                              const uint64_t *, uint64_t, SearchPart *, uint64_t, uint64_t *, uint64_t *, uint32_t *,
+                              cudaStream_t) {}
+void launch_write_records(const SearchPart *, uint64_t, uint64_t, int32_t, const uint32_t *, const uint32_t *, uint8_t *,
+                          cudaStream_t) {}
+void launch_join_count(const uint64_t *, const uint32_t *, uint64_t, uint32_t *, cudaStream_t) {}
+void launch_join_write(const uint64_t *, const uint32_t *, uint64_t, const uint32_t *, const uint64_t *, uint32_t *,
+                       uint32_t *, uint8_t *, uint8_t *, cudaStream_t) {}
+void launch_chunk_keys(const uint32_t *, uint64_t, const uint32_t *, uint64_t, int, uint64_t *, uint32_t *,
+                       cudaStream_t) {}
+void launch_ring_gather(const uint64_t *, const uint32_t *, const uint32_t *, uint64_t, uint64_t *, uint32_t *,
+                        cudaStream_t) {}
+void launch_ring_copy(const uint64_t *, const uint32_t *, uint64_t, uint64_t, uint64_t, uint64_t *, uint32_t *,
+                      cudaStream_t) {}
+void launch_merge(uint64_t *, uint32_t *, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t,
+                  ChunkPart *, uint64_t, uint64_t *, uint32_t *, cudaStream_t) {}
+void launch_unique_walk(const uint64_t *, uint64_t, uint64_t, uint32_t *, cudaStream_t) {}
+
+size_t sort_scratch_bytes(uint64_t) { return 4096; }
+void sort_pairs(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *, cudaStream_t,
+                cudaEvent_t *) {}
+void sort_groups(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *, cudaStream_t) {}
+void sort_radix(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *, cudaStream_t,
+                cudaEvent_t *) {}
+uint32_t *sort_flags(void *p) { return static_cast<uint32_t *>(p); }
+void sort_top_digit(const uint64_t *, const uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *,
+                    cudaStream_t) {}
+
+int bucket_grid_size() { return 148; }
+size_t bkt_scratch_bytes(uint64_t) { return 4096; }
+cudaError_t launch_bucket_rounds(BktJob *, CoopCtl *, uint32_t *, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_bucket_list(BktJob *, uint64_t *, uint32_t *, cudaStream_t) { return cudaSuccess; }
+bool bucket_prologue_apart(const BktJob &) { return false; }
+cudaError_t launch_bucket_prologue(BktJob *, cudaStream_t) { return cudaSuccess; }
+cudaError_t measure_l2_read(uint64_t, double *) { return cudaSuccess; }
+
+int sweep_grid_size() { return 148; }
+uint32_t sweep_segment_size(uint64_t) { return 32; }
+uint32_t sweep_first_rounds(uint64_t, uint64_t) { return 4; }
+uint32_t sweep_shard_log(uint64_t, uint64_t) { return 0; }
+uint32_t sweep_bins_max(uint64_t, int) { return 64; }
+size_t sweep_layout(uint8_t *, SweepJob *, size_t *zeroed) { return *zeroed = 4096; }
+size_t sweep_out_layout(uint8_t *, uint32_t, SweepOut *, size_t *zeroed) { return *zeroed = 4096; }
+cudaError_t launch_sweep(SweepJob *jobs, CoopCtl *ctl, const SweepOut &, bool, cudaStream_t) {
+    for (uint32_t k = 0; k < ctl->njobs; ++k) {
+        jobs[k].round = (uint32_t)jobs[k].r0;
+        if (fake::on_sweep) fake::on_sweep(jobs[k]);
+    }
+    return cudaSuccess;
+}
+
+void graph_paths(const uint8_t *, const uint64_t *, const uint64_t *, uint32_t, uint64_t, uint32_t, const GraphBufs &,
+                 cudaStream_t) { ++fake::graph_builds; }
+void graph_cycles(uint32_t, const GraphBufs &, cudaStream_t) {}
+void graph_place(uint32_t nodes, const GraphBufs &b, cudaStream_t) {  // every read-end a unitig of its own
+    for (uint32_t u = 0; u < nodes; ++u) {
+        b.order[u] = u;
+        b.starts[u] = u;
+    }
+    b.total[0] = b.total[1] = nodes;
+}
+}  // namespace emp
+
+// a host allocation of this thread that fails: the n-th from now
+static thread_local int alloc_countdown = 0;
+void *operator new(size_t n) {
+    if (alloc_countdown > 0 && --alloc_countdown == 0) throw std::bad_alloc();
+    if (void *p = std::malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
+
+namespace {
+
+emp_ctx *make_ctx(uint64_t budget = 0) {
+    emp_ctx *c = nullptr;
+    if (emp_ctx_create(0, budget, &c) != EMP_OK) std::abort();
+    return c;
+}
+emp_job *fed_job(emp_ctx *c) {
+    emp_params p;
+    emp_params_default(&p);
+    emp_job *j = nullptr;
+    const std::string fq(10000, 'A');
+    if (emp_job_create(c, &p, &j) != EMP_OK || emp_job_feed_fastq(j, fq.data(), fq.size(), 1) != EMP_OK) std::abort();
+    return j;
+}
+
+// The list built again for a larger edge buffer: a look-back of it that runs
+// out of its wait is the run's status.
+int rebuilt_list_times_out() {
+    emp_ctx *c = make_ctx();
+    emp_job *j = fed_job(c);
+    int sweeps = 0, lists = 0;
+    fake::on_sweep = [&](emp::SweepJob &x) {
+        x.overflow = ++sweeps == 1;
+        x.e_total = x.ecap + 1;
+    };
+    if (emp_job_run(j, nullptr) != EMP_OK || sweeps != 2) return 1;
+    sweeps = 0;
+    fake::on_init_list = [&](uint32_t *err) {
+        if (++lists == 2) *err |= emp::kErrSpin;
+    };
+    const emp_status st = emp_job_run(j, nullptr);
+    if (lists != 2) return 2;
+    return st == EMP_E_TIMEOUT ? 0 : 3;
+}
+
+}  // namespace
+
+int main(int argc, char **argv) {
+    const std::string name = argc > 1 ? argv[1] : "";
+    if (name == "rebuilt_list_times_out") return rebuilt_list_times_out();
+    return 99;
+}
