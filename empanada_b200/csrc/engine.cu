@@ -3029,7 +3029,10 @@ emp_status emp_graph_build(emp_ctx *ctx, const void *output_bin, uint64_t bytes,
     if (cudaEventCreate(&ev[0]) != cudaSuccess || cudaEventCreate(&ev[1]) != cudaSuccess) rc = EMP_E_CUDA;
     if (rc == EMP_OK) {
         cudaEventRecord(ev[0], s);
-        if (bytes) ctx->stage.to_device(ctx->device, k + o_bin, b, bytes, s);
+        // a staged copy's errors are its threads' own: its status alone tells of them
+        if (bytes && ctx->stage.to_device(ctx->device, k + o_bin, b, bytes, s) != cudaSuccess) rc = EMP_E_CUDA;
+    }
+    if (rc == EMP_OK) {
         if (nrec) cudaMemcpyAsync(d + o_roff, g->rec_off.data(), nrec * 8, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(d + o_e0, e0.data(), (nrec + 1) * 8, cudaMemcpyHostToDevice, s);
         cudaMemsetAsync(gb.status, 0, 2 * scan_t * 8, s);

@@ -162,10 +162,44 @@ int rebuilt_list_times_out() {
     return st == EMP_E_TIMEOUT ? 0 : 3;
 }
 
+// output.bin bytes of one record with n edges between the first two read-ends
+std::vector<uint8_t> one_record(uint64_t n) {
+    std::vector<uint8_t> b(12 + 8 * n, 0);
+    std::memcpy(b.data(), &n, 8);
+    return b;
+}
+
+// A piece of output.bin that does not get to the device: the graph is not
+// built over what lies there.  Copies of the caller's own thread go through
+// (after one of a helper's has failed).
+int graph_input_copy_fails() {
+    emp_ctx *c = make_ctx();
+    const std::vector<uint8_t> bin = one_record(4 << 20);
+    const auto self = std::this_thread::get_id();
+    std::atomic<int> failed{0};
+    emp_graph *g = nullptr;
+    if (emp_graph_build(c, bin.data(), bin.size(), 2, &g) != EMP_OK || fake::graph_builds != 1) return 1;
+    emp_graph_destroy(g);
+    g = nullptr;
+    fake::copy_fails = [&]() {
+        if (std::this_thread::get_id() != self) {
+            ++failed;
+            return true;
+        }
+        for (int k = 0; k < 5000 && !failed; ++k) std::this_thread::sleep_for(std::chrono::milliseconds(1));
+        return false;
+    };
+    const emp_status st = emp_graph_build(c, bin.data(), bin.size(), 2, &g);
+    fake::copy_fails = nullptr;
+    if (!failed) return std::thread::hardware_concurrency() > 1 ? 2 : 0;
+    return st == EMP_E_CUDA && !g && fake::graph_builds == 1 ? 0 : 3;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
     const std::string name = argc > 1 ? argv[1] : "";
     if (name == "rebuilt_list_times_out") return rebuilt_list_times_out();
+    if (name == "graph_input_copy_fails") return graph_input_copy_fails();
     return 99;
 }
