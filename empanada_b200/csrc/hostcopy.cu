@@ -10,7 +10,6 @@
 
 #include <atomic>
 #include <cstring>
-#include <system_error>
 #include <thread>
 
 namespace emp {
@@ -88,7 +87,7 @@ cudaError_t HostStage::run(int device, bool in, uint8_t *dev, uint8_t *host, siz
             helpers[t] = std::thread(work, t);
             ++started;
         }
-    } catch (const std::system_error &) {  // no more threads: with those there are
+    } catch (...) {  // no more threads: with those there are (they are joined below)
     }
     work(0);
     for (int t = 1; t <= started; ++t) helpers[t].join();

@@ -195,11 +195,27 @@ int graph_input_copy_fails() {
     return st == EMP_E_CUDA && !g && fake::graph_builds == 1 ? 0 : 3;
 }
 
+// A helper thread that cannot be made for want of memory: the copy goes on with those there are.
+int thread_allocation_fails() {
+    emp::HostStage stage;
+    std::vector<uint8_t> in(32 << 20), out(in.size());
+    for (size_t i = 0; i < in.size(); i += 4096) in[i] = (uint8_t)(i >> 12);
+    for (int n = 1; n <= 12; ++n) {
+        std::fill(out.begin(), out.end(), 0);
+        alloc_countdown = n;
+        const cudaError_t e = stage.to_device(0, out.data(), in.data(), in.size(), nullptr);
+        alloc_countdown = 0;
+        if (e != cudaSuccess || out != in) return n;
+    }
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
     const std::string name = argc > 1 ? argv[1] : "";
     if (name == "rebuilt_list_times_out") return rebuilt_list_times_out();
     if (name == "graph_input_copy_fails") return graph_input_copy_fails();
+    if (name == "thread_allocation_fails") return thread_allocation_fails();
     return 99;
 }
