@@ -21,6 +21,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -160,6 +161,14 @@ struct SweepBatch {
 constexpr int kMapStreams = 32;
 constexpr int kMapStreamsDefault = 8;
 
+// The graphs whose arrays lie in a context's pool.  A graph may be read and
+// destroyed by other threads than the one that uses its context: the list, and
+// where a graph's arrays are, change under the lock.
+struct GraphList {
+    std::mutex mu;
+    std::vector<emp_graph *> graphs;
+};
+
 struct emp_ctx {
     int device = 0;
     uint64_t budget = 0;
@@ -176,7 +185,7 @@ struct emp_ctx {
     uint64_t sort_calls = 0;
     HostSlab slab;
     HostStage stage;                  // pageable copies
-    std::vector<emp_graph *> graphs;  // those whose arrays lie in the pool
+    std::shared_ptr<GraphList> graphs;
     // emp_batch_run: the BktJob array and control block of one launch, their
     // host copies, and the launch's events
     DevBuf batch_jobs, batch_ctl;
@@ -2210,6 +2219,12 @@ emp_status emp_ctx_create(int device, uint64_t hbm_budget_bytes, emp_ctx **out) 
     if (cudaSetDevice(device) != cudaSuccess) return EMP_E_CUDA;
     emp_ctx *c = new (std::nothrow) emp_ctx();
     if (!c) return EMP_E_NOMEM;
+    try {
+        c->graphs = std::make_shared<GraphList>();
+    } catch (const std::bad_alloc &) {
+        delete c;
+        return EMP_E_NOMEM;
+    }
     c->device = device;
     c->budget = hbm_budget_bytes;
     if (const char *t = std::getenv("EMP_COOP_TRACE")) c->trace_path = t;
@@ -2883,7 +2898,8 @@ emp_status emp_run_file(const char *input_path, const char *output_path, const e
 // for on the host is copied from there.  When its context goes first, the
 // context copies them to the host and the graph lives on without it.
 struct emp_graph {
-    emp_ctx *ctx = nullptr;           // null: on the host
+    std::shared_ptr<GraphList> list;  // its context's, which may go first
+    emp_ctx *ctx = nullptr;           // null: on the host (under the list's lock, like the arrays' places)
     void *dev = nullptr;              // output.bin, order, starts (from the context's pool)
     const uint8_t *d_bin = nullptr;
     const uint32_t *d_order = nullptr;
@@ -2899,7 +2915,7 @@ struct emp_graph {
 
 namespace {
 
-// the graph's arrays into its host vectors
+// the graph's arrays into its host vectors, which then stay as they are
 emp_status graph_to_host(emp_graph *g) {
     if (g->order.size() == g->nodes) return EMP_OK;
     if (!g->ctx) return EMP_E_NOMEM;  // the context went while there was no room for them
@@ -2924,11 +2940,11 @@ emp_status graph_to_host(emp_graph *g) {
     return EMP_OK;
 }
 
-// the graph leaves its context
+// the graph leaves its context (under the list's lock)
 void graph_detach(emp_graph *g) {
     emp_ctx *c = g->ctx;
     if (!c) return;
-    auto &v = c->graphs;
+    auto &v = g->list->graphs;
     v.erase(std::remove(v.begin(), v.end(), g), v.end());
     if (g->dev) {
         cudaSetDevice(c->device);
@@ -2949,6 +2965,7 @@ emp_status emp_graph_build(emp_ctx *ctx, const void *output_bin, uint64_t bytes,
     const uint8_t *b = static_cast<const uint8_t *>(output_bin);
     emp_graph *g = new (std::nothrow) emp_graph();
     if (!g) return EMP_E_NOMEM;
+    g->list = ctx->graphs;
     g->ctx = ctx;
     g->nodes = 2 * n_reads;
     // the records: u64 n | i32 ovlp_len | u32 from[n] | u32 to[n]
@@ -3070,7 +3087,14 @@ emp_status emp_graph_build(emp_ctx *ctx, const void *output_bin, uint64_t bytes,
         delete g;
         return rc;
     }
-    ctx->graphs.push_back(g);
+    try {
+        std::lock_guard<std::mutex> lock(g->list->mu);
+        g->list->graphs.push_back(g);
+    } catch (const std::bad_alloc &) {
+        cudaFreeAsync(g->dev, s);
+        delete g;
+        return EMP_E_NOMEM;
+    }
     *out = g;
     return EMP_OK;
 }
@@ -3084,8 +3108,10 @@ emp_status emp_graph_get_stats(emp_graph *g, emp_graph_stats *st) {
 emp_status emp_graph_unitigs(emp_graph *g, uint32_t *order, uint64_t order_cap, uint64_t *starts, uint64_t starts_cap) {
     if (!g) return EMP_E_INVAL;
     if ((order && order_cap < g->nodes) || (starts && starts_cap < g->unitigs + 1)) return EMP_E_INVAL;
+    std::unique_lock<std::mutex> lock(g->list->mu);
     if (!g->ctx) {
         EMP_TRY(graph_to_host(g));
+        lock.unlock();
         if (order) std::memcpy(order, g->order.data(), g->nodes * 4);
         if (starts) std::memcpy(starts, g->starts.data(), (g->unitigs + 1) * 8);
         return EMP_OK;
@@ -3116,8 +3142,10 @@ char *put_u64(char *p, uint64_t v) {
 
 emp_status emp_graph_write_gfa(emp_graph *g, const char *path, int32_t read_len) {
     if (!g || !path || read_len < 0) return EMP_E_INVAL;
-    const emp_status on_host = graph_to_host(g);
-    if (on_host != EMP_OK) return on_host;
+    {
+        std::lock_guard<std::mutex> lock(g->list->mu);
+        EMP_TRY(graph_to_host(g));
+    }
     FILE *f = std::fopen(path, "wb");
     if (!f) return EMP_E_IO;
     std::vector<char> buf(1 << 22);
@@ -3206,8 +3234,9 @@ emp_status emp_graph_write_gfa(emp_graph *g, const char *path, int32_t read_len)
 
 // the graphs of a context that goes: their arrays to the host
 static void detach_graphs(emp_ctx *ctx) {
-    while (!ctx->graphs.empty()) {
-        emp_graph *g = ctx->graphs.back();
+    std::lock_guard<std::mutex> lock(ctx->graphs->mu);
+    while (!ctx->graphs->graphs.empty()) {
+        emp_graph *g = ctx->graphs->graphs.back();
         graph_to_host(g);
         graph_detach(g);
     }
@@ -3215,7 +3244,10 @@ static void detach_graphs(emp_ctx *ctx) {
 
 emp_status emp_graph_destroy(emp_graph *g) {
     if (!g) return EMP_E_INVAL;
-    graph_detach(g);
+    {
+        std::lock_guard<std::mutex> lock(g->list->mu);
+        graph_detach(g);
+    }
     delete g;
     return EMP_OK;
 }

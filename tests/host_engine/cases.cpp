@@ -210,6 +210,65 @@ int thread_allocation_fails() {
     return 0;
 }
 
+// Graphs read, written out and destroyed by other threads than the one that
+// uses their context, and beside the context's end (run under a race detector).
+int graphs_from_threads() {
+    emp_ctx *c = make_ctx();
+    const std::vector<uint8_t> bin = one_record(3);
+    auto build = [&](uint64_t reads) {
+        emp_graph *g = nullptr;
+        if (emp_graph_build(c, bin.data(), bin.size(), reads, &g) != EMP_OK) std::abort();
+        return g;
+    };
+    emp_graph *shared = build(2000);
+    std::mutex mu;
+    std::vector<emp_graph *> made;
+    std::atomic<bool> over{false};
+    std::atomic<int> wrong{0};
+    auto destroyer = [&]() {
+        for (;;) {
+            const bool last = over;
+            emp_graph *g = nullptr;
+            {
+                std::lock_guard<std::mutex> l(mu);
+                if (!made.empty()) {
+                    g = made.back();
+                    made.pop_back();
+                }
+            }
+            if (g) emp_graph_destroy(g);
+            else if (last) return;
+        }
+    };
+    auto reader = [&]() {
+        std::vector<uint32_t> order(4000);
+        std::vector<uint64_t> starts(4001);
+        for (int k = 0; k < 20; ++k) {
+            if (emp_graph_write_gfa(shared, "/dev/null", 50) != EMP_OK) ++wrong;
+            if (emp_graph_unitigs(shared, order.data(), order.size(), starts.data(), starts.size()) != EMP_OK) ++wrong;
+            for (uint32_t u = 0; u < 4000; ++u) wrong += order[u] != u || starts[u] != u;
+        }
+    };
+    std::thread a(destroyer), b(reader), d(reader);
+    for (int k = 0; k < 300; ++k) {
+        emp_graph *g = build(20);
+        std::lock_guard<std::mutex> l(mu);
+        made.push_back(g);
+    }
+    b.join();
+    d.join();
+    for (int k = 0; k < 300; ++k) {
+        emp_graph *g = build(20);
+        std::lock_guard<std::mutex> l(mu);
+        made.push_back(g);
+    }
+    emp_ctx_destroy(c);
+    over = true;
+    a.join();
+    emp_graph_destroy(shared);
+    return wrong ? 1 : fake::pool_bytes ? 2 : 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -217,5 +276,6 @@ int main(int argc, char **argv) {
     if (name == "rebuilt_list_times_out") return rebuilt_list_times_out();
     if (name == "graph_input_copy_fails") return graph_input_copy_fails();
     if (name == "thread_allocation_fails") return thread_allocation_fails();
+    if (name == "graphs_from_threads") return graphs_from_threads();
     return 99;
 }

@@ -29,3 +29,13 @@ def program(tmp_path_factory):
 def test_a_failing_call_is_a_status(program, case):
     p = subprocess.run([program, case], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0, (p.returncode, p.stderr)
+
+
+def test_graphs_from_other_threads(tmp_path):
+    """Under the thread sanitizer where the compiler has one."""
+    try:
+        exe = _build(str(tmp_path / "cases"), "-O1", "-fsanitize=thread")
+    except subprocess.CalledProcessError:
+        exe = _build(str(tmp_path / "cases"))
+    p = subprocess.run([exe, "graphs_from_threads"], capture_output=True, text=True, timeout=90)
+    assert p.returncode == 0, (p.returncode, p.stderr[-3000:])
