@@ -15,6 +15,7 @@
 // written on the device by the bucket kernel, on the host for
 // host-synchronised rounds.  Files come in through ingest.cpp.
 #include <algorithm>
+#include <atomic>
 #include <cerrno>
 #include <chrono>
 #include <cstdio>
@@ -172,7 +173,7 @@ struct GraphList {
 struct emp_ctx {
     int device = 0;
     uint64_t budget = 0;
-    uint64_t in_use = 0;
+    std::atomic<uint64_t> in_use{0};  // device bytes held (an open graph's go from any thread)
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // asynchronous FASTQ feeds
     // device memory of the jobs' work buffers: a stream-ordered pool that keeps
@@ -282,12 +283,35 @@ constexpr emp_status kCrowded = -1001;
 
 emp_status cuda_status(cudaError_t e) { return e == cudaSuccess ? EMP_OK : (e == cudaErrorMemoryAllocation ? EMP_E_NOMEM : EMP_E_CUDA); }
 
+// Arrays of open graphs to the host until `bytes` more of device memory are
+// free; returns how many became so.
+uint64_t graphs_give(emp_ctx *c, uint64_t bytes);
+
+// Whether the budget has room for `bytes` in the place of `old`, open graphs
+// moved to the host for it.
+bool budget_allows(emp_ctx *c, uint64_t old, uint64_t bytes) {
+    const uint64_t want = c->in_use - old + bytes;
+    if (!c->budget || want <= c->budget) return true;
+    graphs_give(c, want - c->budget);
+    return c->in_use - old + bytes <= c->budget;
+}
+
+cudaError_t pool_alloc(emp_ctx *c, void **p, size_t bytes, cudaStream_t s) {
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, c->pool, s);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        if (graphs_give(c, bytes)) e = cudaMallocFromPoolAsync(p, bytes, c->pool, s);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    return e;
+}
+
 // Grow b to at least `bytes` from the context's pool, in the order of stream
 // s (the old contents are not kept).
 emp_status ctx_ensure(emp_ctx *c, DevBuf &b, size_t bytes, cudaStream_t s) {
     if (bytes <= b.bytes) return EMP_OK;
     const size_t old = b.bytes;
-    if (c->budget && c->in_use - old + bytes > c->budget) return EMP_E_NOMEM;
+    if (!budget_allows(c, old, bytes)) return EMP_E_NOMEM;
     if (b.p && b.pooled) {
         cudaFreeAsync(b.p, s);
         b.p = nullptr;
@@ -297,11 +321,7 @@ emp_status ctx_ensure(emp_ctx *c, DevBuf &b, size_t bytes, cudaStream_t s) {
     b.release();
     c->in_use -= old;
     void *p = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, c->pool, s);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return EMP_E_NOMEM;
-    }
+    if (pool_alloc(c, &p, bytes ? bytes : 16, s) != cudaSuccess) return EMP_E_NOMEM;
     b.p = p;
     b.bytes = bytes;
     b.pooled = true;
@@ -2410,11 +2430,8 @@ emp_status emp_job_reserve(emp_job *job, uint64_t bytes) {
     if (job->feed_pending && cudaEventSynchronize(job->feed_ev[1]) != cudaSuccess) return EMP_E_CUDA;
     DevBuf nb;
     emp_ctx *c = job->ctx;
-    if (c->budget && c->in_use + bytes > c->budget) return EMP_E_NOMEM;
-    if (cudaMallocFromPoolAsync(&nb.p, bytes + 16, c->pool, c->stream) != cudaSuccess) {
-        cudaGetLastError();
-        return EMP_E_NOMEM;
-    }
+    if (!budget_allows(c, 0, bytes)) return EMP_E_NOMEM;
+    if (pool_alloc(c, &nb.p, bytes + 16, c->stream) != cudaSuccess) return EMP_E_NOMEM;
     nb.bytes = bytes + 16;
     nb.pooled = true;
     nb.pool_stream = c->stream;
@@ -2504,12 +2521,9 @@ emp_status emp_job_feed_fastq_async(emp_job *job, const char *bytes, uint64_t n,
     if (job->F + n > job->fq.bytes) {  // grow in the copy stream's order
         uint64_t want = job->F + n;
         if (!last) want += want / 2;
-        if (c->budget && c->in_use - job->fq.bytes + want + 16 > c->budget) return EMP_E_NOMEM;
+        if (!budget_allows(c, job->fq.bytes, want + 16)) return EMP_E_NOMEM;
         void *p = nullptr;
-        if (cudaMallocFromPoolAsync(&p, want + 16, c->pool, cs) != cudaSuccess) {
-            cudaGetLastError();
-            return EMP_E_NOMEM;
-        }
+        if (pool_alloc(c, &p, want + 16, cs) != cudaSuccess) return EMP_E_NOMEM;
         if (job->F) EMP_CUDA(cudaMemcpyAsync(p, job->fq.p, job->F, cudaMemcpyDeviceToDevice, cs));
         if (job->fq.p) {
             if (job->fq.pooled) cudaFreeAsync(job->fq.p, cs);
@@ -2904,7 +2918,7 @@ struct emp_graph {
     const uint8_t *d_bin = nullptr;
     const uint32_t *d_order = nullptr;
     const uint64_t *d_starts = nullptr;
-    uint64_t bytes = 0, unitigs = 0;
+    uint64_t dev_bytes = 0, bytes = 0, unitigs = 0;
     std::vector<uint8_t> bin;         // the output.bin bytes (the L lines come from them)
     std::vector<uint64_t> rec_off;    // byte offset of every record
     uint64_t nodes = 0, edges = 0;
@@ -2949,9 +2963,24 @@ void graph_detach(emp_graph *g) {
     if (g->dev) {
         cudaSetDevice(c->device);
         cudaFreeAsync(g->dev, c->stream);
+        c->in_use -= g->dev_bytes;
     }
     g->dev = nullptr;
     g->ctx = nullptr;
+}
+
+uint64_t graphs_give(emp_ctx *c, uint64_t bytes) {
+    std::lock_guard<std::mutex> lock(c->graphs->mu);
+    std::vector<emp_graph *> &v = c->graphs->graphs;
+    uint64_t got = 0;
+    for (size_t k = v.size(); k-- > 0 && got < bytes;) {
+        emp_graph *g = v[k];
+        if (graph_to_host(g) != EMP_OK) continue;  // no room there either: it stays
+        got += g->dev_bytes;
+        graph_detach(g);
+    }
+    if (got) cudaStreamSynchronize(c->stream);  // for an allocation in another stream's order
+    return got;
 }
 
 }  // namespace
@@ -2999,13 +3028,11 @@ emp_status emp_graph_build(emp_ctx *ctx, const void *output_bin, uint64_t bytes,
     const size_t o_tail = take(V), o_status = take(2 * scan_t * 8), o_small = take(512);
     cudaStream_t s = ctx->stream;
     void *work = nullptr;
-    if (cudaMallocFromPoolAsync(&g->dev, keep, ctx->pool, s) != cudaSuccess) {
-        cudaGetLastError();
+    if (pool_alloc(ctx, &g->dev, keep, s) != cudaSuccess) {
         delete g;
         return EMP_E_NOMEM;
     }
-    if (cudaMallocFromPoolAsync(&work, off, ctx->pool, s) != cudaSuccess) {
-        cudaGetLastError();
+    if (pool_alloc(ctx, &work, off, s) != cudaSuccess) {
         cudaFreeAsync(g->dev, s);
         delete g;
         return EMP_E_NOMEM;
@@ -3090,6 +3117,8 @@ emp_status emp_graph_build(emp_ctx *ctx, const void *output_bin, uint64_t bytes,
     try {
         std::lock_guard<std::mutex> lock(g->list->mu);
         g->list->graphs.push_back(g);
+        g->dev_bytes = keep;
+        ctx->in_use += keep;
     } catch (const std::bad_alloc &) {
         cudaFreeAsync(g->dev, s);
         delete g;

@@ -304,7 +304,8 @@ emp_status emp_graph_get_stats(emp_graph *g, emp_graph_stats *st);
  * read-end's id.  Either array may be NULL.  A graph may be read, written and
  * destroyed by any thread, beside its context's own calls (two threads that
  * destroy one graph, or use one that is being destroyed, are not); it outlives
- * its context. */
+ * its context.  While open it holds output.bin and 12 bytes a read-end of device
+ * memory, which its context counts and moves to the host when a job needs it. */
 emp_status emp_graph_unitigs(emp_graph *g, uint32_t *order, uint64_t order_cap, uint64_t *starts, uint64_t starts_cap);
 /* GFA 1.0: a header, one S line per read (length read_len), one L line per
  * edge in output.bin order (orientation + for rid 2i, - for 2i+1; overlap as

@@ -269,6 +269,48 @@ int graphs_from_threads() {
     return wrong ? 1 : fake::pool_bytes ? 2 : 0;
 }
 
+// An open graph's arrays on the device count, and make room for a job: under a
+// budget, and on a device that is full.
+int graphs_make_room() {
+    emp_ctx *c = make_ctx();
+    emp_job *j = fed_job(c);
+    if (emp_job_run(j, nullptr) != EMP_OK) return 1;
+    const long job_bytes = fake::pool_bytes;
+    emp_job_destroy(j);
+    emp_ctx_destroy(c);
+    const std::vector<uint8_t> bin = one_record(3);
+    constexpr uint64_t kNodes = 2000000;  // 24 MB on the device
+    for (const bool budget : {true, false}) {
+        const long limit = job_bytes + (20 << 20);
+        c = make_ctx(budget ? (uint64_t)limit : 0);
+        emp_graph *g = nullptr, *g2 = nullptr;
+        if (emp_graph_build(c, bin.data(), bin.size(), kNodes / 2, &g) != EMP_OK) return 2;
+        if (emp_graph_build(c, bin.data(), bin.size(), 10, &g2) != EMP_OK) return 3;
+        if (!budget) fake::pool_refuses = [&](size_t n) { return fake::pool_bytes + (long)n > limit; };
+        j = fed_job(c);
+        const emp_status st = emp_job_run(j, nullptr);
+        fake::pool_refuses = nullptr;
+        if (st != EMP_OK) return 4;
+        if (fake::pool_bytes > limit) return 5;
+        emp_job_destroy(j);
+        std::vector<uint32_t> order(kNodes);
+        std::vector<uint64_t> starts(kNodes + 1);
+        for (emp_graph *x : {g, g2}) {
+            emp_graph_stats gs;
+            emp_graph_get_stats(x, &gs);
+            if (emp_graph_unitigs(x, order.data(), kNodes, starts.data(), kNodes + 1) != EMP_OK) return 6;
+            for (uint64_t u = 0; u < gs.nodes; ++u)
+                if (order[u] != u || starts[u] != u) return 7;
+            if (starts[gs.nodes] != gs.nodes) return 8;
+            if (emp_graph_write_gfa(x, "/dev/null", 50) != EMP_OK) return 9;
+            emp_graph_destroy(x);
+        }
+        emp_ctx_destroy(c);
+        if (fake::pool_bytes) return 10;
+    }
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -277,5 +319,6 @@ int main(int argc, char **argv) {
     if (name == "graph_input_copy_fails") return graph_input_copy_fails();
     if (name == "thread_allocation_fails") return thread_allocation_fails();
     if (name == "graphs_from_threads") return graphs_from_threads();
+    if (name == "graphs_make_room") return graphs_make_room();
     return 99;
 }
