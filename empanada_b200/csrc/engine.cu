@@ -775,7 +775,7 @@ void write_coop_probe(emp_job *j, const char *path, int grid, cudaStream_t s) {
 
 // Whether rounds may run in the bucket kernel on this context (cooperative
 // launch available, not turned off by the tuning).
-bool bucket_rounds_usable(const emp_ctx *c) { return c->tune.round_driver == 0 && bucket_grid_size() > 0; }
+bool bucket_rounds_usable(const emp_ctx *c) { return c->tune.round_driver != 1 && bucket_grid_size() > 0; }
 
 // The control block of a bucket-kernel launch: the context's grid-barrier
 // limit, and the testing barrier that no arrival completes (used once).
@@ -895,12 +895,10 @@ emp_status bucket_collect(emp_job *j, int r0, uint64_t n_in, const Launched &hj,
 }
 
 // Whether rounds over a list of n entries run in the sweep kernel
-// (k_sweep.cu): not when the caller shapes the bucket kernel's buckets or
-// regions.
+// (k_sweep.cu).
 bool sweep_rounds_usable(const emp_job *j, uint64_t n) {
     const emp_tuning &t = j->ctx->tune;
-    return !j->prep.no_sweep && t.round_driver == 0 && (!t.bucket_mean || t.bucket_mean == kBktMean) &&
-           (!t.region_cap || t.region_cap == kBktRegionCap) &&
+    return !j->prep.no_sweep && t.round_driver == 0 &&
            (n <= kSweepMaxEntries ||
             (n <= kSweepMaxSparse && sweep_first_rounds(j->prep.U, 2 * j->prep.n) >= kSweepSparseR)) &&
            sweep_grid_size() > 0;
@@ -2202,7 +2200,7 @@ emp_status emp_tuning_default(emp_tuning *t) {
 
 emp_status emp_ctx_set_tuning(emp_ctx *ctx, const emp_tuning *t) {
     if (!ctx || !t) return EMP_E_INVAL;
-    if (t->round_driver < 0 || t->round_driver > 1 || t->dedup_driver < 0 || t->dedup_driver > 1) return EMP_E_INVAL;
+    if (t->round_driver < 0 || t->round_driver > 2 || t->dedup_driver < 0 || t->dedup_driver > 1) return EMP_E_INVAL;
     if (t->bucket_mean && (t->bucket_mean < kBktMeanMin || t->bucket_mean > kBktMeanMax)) return EMP_E_INVAL;
     if (t->region_cap > kBktRegionCap || t->map_streams > (uint32_t)kMapStreams) return EMP_E_INVAL;
     ctx->tune = *t;

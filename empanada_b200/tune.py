@@ -3,10 +3,11 @@
 Every choice gives the same ``output.bin`` (the tuner checks that it does on
 the workload it times); they differ in speed:
 
-``bucket_mean``  entries per key bucket of the round kernel: its tile size.
+``bucket_mean``  entries per key bucket of the bucket kernel: its tile size.
                  Smaller buckets give more of them per round (better balance
                  across the SMs, more buckets in flight), larger ones fewer
-                 per-bucket fixed costs.
+                 per-bucket fixed costs.  Offered where a list may be long
+                 enough for that kernel; a shorter one never meets it.
 ``dedup_driver`` duplicate removal by key buckets and hash sets (0) or by
                  sorting every fingerprint (1).
 
@@ -14,7 +15,8 @@ The tuner times each candidate on the caller's own workload (a fed job, or a
 list of fed jobs for a batch), keeps the fastest and records it in a JSON
 cache keyed by the workload's shape (kind, read count to a power of two,
 read length to 50 bases), so that later runs of the same shape reuse the
-choice without timing.  ``EMP_TUNE_CACHE`` names the cache file (default
+choice without timing.  An entry of another ``VERSION`` of the choices is
+timed again.  ``EMP_TUNE_CACHE`` names the cache file (default
 ``~/.cache/empanada_b200/tune.json``); ``EMP_TUNE=0`` turns the tuner off
 (the defaults stay).
 """
@@ -29,9 +31,23 @@ from typing import Callable, Iterable
 
 from . import _native
 
+# What the cached choices mean: raised with every change of the engine that can
+# turn a fast choice into a slow one.
+VERSION = 2
+
 # the defaults first: they win ties
-JOB_CANDIDATES = {"bucket_mean": [2900, 2175, 1450], "dedup_driver": [0, 1]}
-BATCH_CANDIDATES = {"bucket_mean": [2900, 2175, 1450]}
+JOB_CANDIDATES = {"dedup_driver": [0, 1]}
+BATCH_CANDIDATES: dict = {}
+BUCKET_CANDIDATES = {"bucket_mean": [2900, 2175, 1450]}
+
+# Lists of up to so many entries start in the sweep kernel, whatever their
+# density (kSweepMaxEntries of the engine).
+SWEEP_MAX_ENTRIES = 9 << 20
+
+
+def space_for(base: dict, reads: float) -> dict:
+    """The candidates of a job of `reads` reads (4 entries each at most)."""
+    return {**BUCKET_CANDIDATES, **base} if 4 * reads > SWEEP_MAX_ENTRIES else dict(base)
 
 
 def enabled() -> bool:
@@ -66,12 +82,12 @@ class Cache:
     def get(self, key: str) -> dict | None:
         """The cached choice, or None (also for an entry this version cannot read)."""
         e = self.data.get(key)
-        if not isinstance(e, dict) or not isinstance(e.get("choice"), dict):
+        if not isinstance(e, dict) or not isinstance(e.get("choice"), dict) or e.get("version") != VERSION:
             return None
         return dict(e["choice"])
 
     def put(self, key: str, choice: dict, timings: dict) -> None:
-        self.data[key] = {"choice": choice, "timings_ms": timings}
+        self.data[key] = {"choice": choice, "timings_ms": timings, "version": VERSION}
         os.makedirs(os.path.dirname(self.path) or ".", exist_ok=True)
         tmp = self.path + ".tmp"
         with open(tmp, "w") as f:
@@ -149,7 +165,8 @@ def tune_job(engine, job, reads: int, read_len: int, cache: Cache | None = None,
     if hit is not None and _apply_cached(engine, hit):
         return {"key": key, "choice": hit, "source": "cache", "timings_ms": None}
 
-    best, timings = search(space or JOB_CANDIDATES, lambda c: engine.set_tuning(**c), job.run, job.output, repeats)
+    space = space_for(JOB_CANDIDATES, reads) if space is None else space
+    best, timings = search(space, lambda c: engine.set_tuning(**c), job.run, job.output, repeats)
     engine.set_tuning(**best)
     cache.put(key, best, timings)
     return {"key": key, "choice": best, "source": "timed", "timings_ms": timings}
@@ -165,11 +182,15 @@ def tune_batch(engine, jobs: Iterable, reads: int, read_len: int, cache: Cache |
     if hit is not None and _apply_cached(engine, hit):
         return {"key": key, "choice": hit, "source": "cache", "timings_ms": None}
 
+    space = space_for(BATCH_CANDIDATES, reads / max(1, len(jobs))) if space is None else space
+    if len(candidates(space)) == 1:  # nothing to choose
+        return {"key": key, "choice": candidates(space)[0], "source": "defaults", "timings_ms": None}
+
     def outputs() -> bytes:
         crcs = [zlib.crc32(j.output()) for j in jobs]
         return json.dumps(crcs).encode()
 
-    best, timings = search(space or BATCH_CANDIDATES, lambda c: engine.set_tuning(**c),
+    best, timings = search(space, lambda c: engine.set_tuning(**c),
                            lambda: engine.run_batch(jobs), outputs, repeats)
     engine.set_tuning(**best)
     cache.put(key, best, timings)

@@ -112,9 +112,8 @@ emp_status emp_ctx_destroy(emp_ctx *ctx);
 typedef struct emp_tuning {
     int32_t round_driver;     /* 0: the sweep kernel, and the bucket kernel for long lists, for every
                                  round that cannot split into several search partitions;
-                                 1: host-synchronised rounds only */
-    uint32_t bucket_mean;     /* bucket kernel: entries per key bucket aimed at, 512..3000 (default 2900;
-                                 another value keeps every such round in the bucket kernel) */
+                                 1: host-synchronised rounds only; 2: the bucket kernel for every such round */
+    uint32_t bucket_mean;     /* bucket kernel: entries per key bucket aimed at, 512..3000 (default 2900) */
     uint32_t region_cap;      /* bucket kernel: entries per (bucket, table) region, 1..2048 (default 2048);
                                  a region's overflow goes to a spill area */
     int32_t dedup_driver;     /* 0: duplicate removal by key buckets and hash sets where 2n <= M (the

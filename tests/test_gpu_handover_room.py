@@ -50,7 +50,7 @@ def test_after_host_rounds(tmp_path, monkeypatch):
 @pytest.mark.parametrize("cap", [(1 << 40) + 1, 1 << 61, 1 << 62, (1 << 64) - 1])
 def test_edge_buffers_that_no_device_holds(engine, cap):
     fq = G.BY_NAME["tiny"].fastq()
-    for tuned in ({}, {"bucket_mean": 512}):
+    for tuned in ({}, {"round_driver": 2}):
         with engine.tuned(edge_cap=cap, **tuned), pytest.raises(emp.EmpError) as e:
             emp.run_bytes(fq, engine=engine, min_ovlp=31)
         assert e.value.code == _native.EMP_E_NOMEM
