@@ -3298,6 +3298,7 @@ emp_status emp_sort_pairs(emp_ctx *ctx, uint64_t *d_keys, uint32_t *d_vals, uint
     };
     // the working set is kept in the context for the next call
     if (n > ctx->sort_cap || ctx->sort_calls > kSortsPerClear) {
+        ctx->sort_cap = 0;  // until all of it is there again
         if (!grow(ctx->sort_k1, n * 8) || !grow(ctx->sort_v1, n * 4) || !grow(ctx->sort_scr, sort_scratch_bytes(n)))
             return EMP_E_NOMEM;
         if (cudaMemsetAsync(ctx->sort_scr.p, 0, ctx->sort_scr.bytes, s) != cudaSuccess) return EMP_E_CUDA;

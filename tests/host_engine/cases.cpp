@@ -11,6 +11,7 @@ constexpr uint64_t kReads = 100, kLen = 50, kUnique = 150;
 std::function<void(uint32_t *err)> on_init_list;
 std::function<void(emp::SweepJob &)> on_sweep;
 int graph_builds = 0;
+bool sort_buffers = false;
 }  // namespace fake
 
 namespace emp {
@@ -74,7 +75,9 @@ void launch_unique_walk(const uint64_t *, uint64_t, uint64_t, uint32_t *, cudaSt
 size_t sort_scratch_bytes(uint64_t) { return 4096; }
 void sort_pairs(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *, cudaStream_t,
                 cudaEvent_t *) {}
-void sort_groups(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *, cudaStream_t) {}
+void sort_groups(uint64_t *, uint32_t *, uint64_t *k1, uint32_t *v1, uint64_t, void *scratch, uint32_t *, cudaStream_t) {
+    fake::sort_buffers = k1 && v1 && scratch;
+}
 void sort_radix(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *, cudaStream_t,
                 cudaEvent_t *) {}
 uint32_t *sort_flags(void *p) { return static_cast<uint32_t *>(p); }
@@ -311,6 +314,24 @@ int graphs_make_room() {
     return 0;
 }
 
+// A sort whose working set could not grow leaves one that the next, smaller sort can use.
+int sort_room_refused() {
+    emp_ctx *c = make_ctx();
+    std::vector<uint64_t> k(100000);
+    std::vector<uint32_t> v(k.size());
+    for (int refused = 0; refused < 3; ++refused) {
+        if (emp_sort_pairs(c, k.data(), v.data(), 1000 << refused, nullptr) != EMP_OK || !fake::sort_buffers) return 1;
+        int asked = 0;
+        fake::malloc_refuses = [&](size_t) { return asked++ >= refused; };
+        const emp_status st = emp_sort_pairs(c, k.data(), v.data(), k.size(), nullptr);
+        fake::malloc_refuses = nullptr;
+        if (st != EMP_E_NOMEM) return refused ? 0 : 2;  // 0: the buffers had been grown before
+        if (emp_sort_pairs(c, k.data(), v.data(), 500, nullptr) != EMP_OK || !fake::sort_buffers) return 3;
+    }
+    emp_ctx_destroy(c);
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -320,5 +341,6 @@ int main(int argc, char **argv) {
     if (name == "thread_allocation_fails") return thread_allocation_fails();
     if (name == "graphs_from_threads") return graphs_from_threads();
     if (name == "graphs_make_room") return graphs_make_room();
+    if (name == "sort_room_refused") return sort_room_refused();
     return 99;
 }

@@ -38,6 +38,7 @@ namespace fake {
 inline thread_local cudaError_t last = cudaSuccess;
 inline std::function<bool()> copy_fails;  // asked by each asynchronous copy
 inline std::function<bool(size_t)> pool_refuses;  // asked by each allocation from the pool
+inline std::function<bool(size_t)> malloc_refuses;  // and by each other one
 inline std::atomic<long> pool_bytes{0};
 inline cudaError_t result(bool ok, cudaError_t e = cudaErrorUnknown) {
     if (!ok) last = e;
@@ -56,7 +57,7 @@ inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 
 template <class T>
 cudaError_t cudaMalloc(T **p, size_t n) {
-    *p = static_cast<T *>(std::calloc(1, n ? n : 1));
+    *p = fake::malloc_refuses && fake::malloc_refuses(n) ? nullptr : static_cast<T *>(std::calloc(1, n ? n : 1));
     return fake::result(*p != nullptr, cudaErrorMemoryAllocation);
 }
 inline cudaError_t cudaFree(void *p) { std::free(p); return cudaSuccess; }
