@@ -854,6 +854,9 @@ emp_status bucket_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r
 }
 
 // Queue the copy of the job's round records to the host.
+static_assert(sizeof(BktJob) <= 1024 && sizeof(SweepJob) + sizeof(CoopCtl) <= 1024 && sizeof(BktJob) % 8 == 0 &&
+                  sizeof(SweepJob) % 8 == 0 && sizeof(CoopCtl) % 8 == 0,
+              "one job's description is a copy that waits for no other; several are whole words (launch_upload)");
 emp_status bucket_fetch(emp_job *j, const RoundEnv &env, cudaStream_t s) {
     EMP_CUDA(cudaMemcpyAsync(j->h_records.p, j->records.p, (size_t)env.rounds * sizeof(RoundRecord),
                              cudaMemcpyDeviceToHost, s));
@@ -1142,8 +1145,10 @@ struct MapMany {
     uint32_t nb_max = 0;
 };
 // Queue what was collected, then the fetched jobs' words into their host
-// slots; waits for the stream.
-emp_status many_flush(emp_ctx *c, MapMany &m, cudaStream_t s) {
+// slots; waits for the stream.  started: an event to record before the kernels
+// (not as the stream's first work, where it would go where the stream's last
+// work went: after a copy in, behind all copies in flight).
+emp_status many_flush(emp_ctx *c, MapMany &m, cudaStream_t s, cudaEvent_t started) {
     if (!m.read.empty()) {  // two turns of the resident CTAs, by the jobs' tiles
         uint64_t tiles = 0;
         for (const ReadArgs &a : m.read) tiles += parse_tiles(a.F);
@@ -1206,7 +1211,8 @@ emp_status many_flush(emp_ctx *c, MapMany &m, cudaStream_t s) {
     }
     uint64_t **src = reinterpret_cast<uint64_t **>(h + at[12]);
     for (size_t k = 0; k < m.fetch.size(); ++k) src[k] = m.fetch[k]->misc.as<uint64_t>();
-    if (total) EMP_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, s));
+    launch_upload(h, d, total, s);
+    if (started) EMP_CUDA(cudaEventRecord(started, s));
     auto blocks = [&](int k) { return ManyBlocks{reinterpret_cast<const uint2 *>(d + at[5 + k]), (uint32_t)nblk[k]}; };
     launch_nl_count_many(reinterpret_cast<const NlArgs *>(d + at[0]), blocks(0), s);
     launch_scan_many(reinterpret_cast<const ScanArgs *>(d + at[1]), blocks(1), s);
@@ -1610,8 +1616,8 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
         EMP_TRY(bucket_prepare(j, s, job_env(j), 0, 0, 2 * q.U, q.ecap, 1u, &hj[k]));
     }
     coop_ctl_init(ctx, hc, (uint32_t)nb);
-    EMP_CUDA(cudaMemcpyAsync(ctx->batch_jobs.p, hj, nb * sizeof(BktJob), cudaMemcpyHostToDevice, s));
-    EMP_CUDA(cudaMemcpyAsync(ctx->batch_ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    launch_upload(hj, ctx->batch_jobs.p, nb * sizeof(BktJob), s);
+    launch_upload(hc, ctx->batch_ctl.p, sizeof(CoopCtl), s);
     EMP_CUDA(cudaEventRecord(ctx->batch_ev[0], s));
     EMP_CUDA(launch_bucket_rounds(ctx->batch_jobs.as<BktJob>(), ctx->batch_ctl.as<CoopCtl>(),
                                   err_word(jobs[idx[0]]), s));
@@ -1711,7 +1717,7 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
         hc->trace = j->coop_trace.as<uint64_t>();
         hc->trace_cap = kSweepTraceCap;
     }
-    EMP_CUDA(cudaMemcpyAsync(dj, hj, n_in * sizeof(SweepJob) + sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+    launch_upload(hj, dj, n_in * sizeof(SweepJob) + sizeof(CoopCtl), s);
     EMP_CUDA(cudaEventRecord(sb.ev[0], s));
     EMP_CUDA(launch_sweep(dj, dc, go, true, s));
     EMP_CUDA(cudaEventRecord(sb.ev[1], s));
@@ -1779,16 +1785,15 @@ emp_status map_batch_stages(emp_job **jobs, int n, std::vector<emp_status> &rc, 
     for (auto &e : ctx->many_ev)
         if (!e) EMP_CUDA(cudaEventCreate(&e));
     MapMany mm;
-    auto stage = [&](auto step) {
+    auto stage = [&](auto step, cudaEvent_t started = nullptr) {
         for (int i = 0; i < n; ++i) {
             if (!live(i)) continue;
             fail(i, step(jobs[i]));
             if (live(i)) fail(i, map_fetch(jobs[i], s, &mm));
         }
-        return many_flush(ctx, mm, s);
+        return many_flush(ctx, mm, s, started);
     };
-    EMP_CUDA(cudaEventRecord(ctx->many_ev[0], s));
-    EMP_TRY(stage([&](emp_job *j) { return map_begin(j, s, &mm); }));
+    EMP_TRY(stage([&](emp_job *j) { return map_begin(j, s, &mm); }, ctx->many_ev[0]));
     EMP_TRY(stage([&](emp_job *j) { return map_records(j, s, &mm); }));
     EMP_CUDA(cudaEventRecord(ctx->many_ev[1], s));
     EMP_TRY(stage([&](emp_job *j) { return map_keys(j, s, &mm); }));
@@ -1994,8 +1999,8 @@ emp_status server_step(emp_server *srv, cudaStream_t s) {
         }
         coop_ctl_init(ctx, hc, (uint32_t)nb);
         hc->iter_cap = any_unlimited ? 0u : share;
-        EMP_CUDA(cudaMemcpyAsync(srv->d_jobs.p, hj, nb * sizeof(BktJob), cudaMemcpyHostToDevice, s));
-        EMP_CUDA(cudaMemcpyAsync(srv->d_ctl.p, hc, sizeof(CoopCtl), cudaMemcpyHostToDevice, s));
+        launch_upload(hj, srv->d_jobs.p, nb * sizeof(BktJob), s);
+        launch_upload(hc, srv->d_ctl.p, sizeof(CoopCtl), s);
         EMP_CUDA(cudaEventRecord(srv->ev[0], s));
         EMP_CUDA(launch_bucket_rounds(srv->d_jobs.as<BktJob>(), srv->d_ctl.as<CoopCtl>(), err_word(srv->live[0]), s));
         EMP_CUDA(cudaEventRecord(srv->ev[1], s));

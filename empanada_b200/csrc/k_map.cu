@@ -585,6 +585,17 @@ void launch_read_pass_many(const ReadArgs *a, ManyBlocks b, cudaStream_t s) {
     count_launch();
     read_pass_many_kernel<<<b.n, kRT, sizeof(ReadSmem), s>>>(a, b.blk);
 }
+// volatile: the host writes `src` between launches
+__global__ void __launch_bounds__(256) upload_kernel(const volatile uint64_t *src, uint64_t *__restrict__ dst, size_t n) {
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) dst[i] = src[i];
+}
+void launch_upload(const void *host, void *dev, size_t bytes, cudaStream_t s) {
+    const size_t n = bytes / 8;
+    if (!n) return;
+    count_launch();
+    upload_kernel<<<grid_for(n, 256, 148), 256, 0, s>>>(static_cast<const uint64_t *>(host), static_cast<uint64_t *>(dev),
+                                                        n);
+}
 __global__ void __launch_bounds__(256) gather_words_kernel(const uint64_t *const *src, uint32_t jobs, uint64_t *out) {
     const uint32_t i = blockIdx.x * 256 + threadIdx.x;
     if (i < jobs * 16) out[i] = src[i >> 4][i & 15];

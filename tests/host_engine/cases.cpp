@@ -28,6 +28,7 @@ void launch_read_pass_many(const ReadArgs *, ManyBlocks, cudaStream_t) {}
 uint32_t read_pass_grid() { return 148; }
 void launch_dedup_many(const DedupArgs *, uint32_t, uint32_t, ManyBlocks, ManyBlocks, ManyBlocks, cudaStream_t) {}
 void launch_init_list_many(const InitArgs *, ManyBlocks, cudaStream_t) {}
+void launch_upload(const void *host, void *dev, size_t bytes, cudaStream_t) { std::memcpy(dev, host, bytes); }
 void launch_gather_words(const uint64_t *const *, uint32_t, uint64_t *, cudaStream_t) {}
 void launch_read_pass(const uint8_t *, uint64_t, const uint64_t *, const HashTables *, const ChunkWeights *, uint64_t *,
                       uint32_t *, int, uint32_t *, uint64_t *n_kept, uint32_t *len_minmax, uint32_t *, cudaStream_t) {
