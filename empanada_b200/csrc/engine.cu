@@ -1759,6 +1759,9 @@ emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &job
     return timed_out ? EMP_E_TIMEOUT : EMP_OK;
 }
 
+// Bytes of FASTQ that a batch's map phase is not split below (1.2 ms of copies).
+constexpr uint64_t kMapGroupLeast = 64ull << 20;
+
 // The map phase of jobs[0..n) with one stream synchronisation per stage for
 // all of them; a job that fails gets its status in rc.  Jobs left with rc
 // EMP_OK and prep.done unset have their lists ready for the rounds.
@@ -1812,7 +1815,7 @@ emp_status map_batch_stages(emp_job **jobs, int n, std::vector<emp_status> &rc, 
 // The same with a failed host allocation (the stages' lists) as a status.
 // Where there is no room for what the jobs share, they go one after another,
 // each with a status of its own.
-emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
+emp_status map_group(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) {
     auto stages = [&](emp_job **js, int k, std::vector<emp_status> &r) -> emp_status {
         try {
             return map_batch_stages(js, k, r, s);
@@ -1831,6 +1834,36 @@ emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStr
         rc[i] = e != EMP_OK ? e : one[0];
     }
     return EMP_OK;
+}
+
+// How many of jobs[0..n) go through the map phase next: all of them when their
+// FASTQ is there, else those with the first half of the bytes, so that the
+// phase of what has landed runs beside the copies of the rest and little is
+// left to do after the last one.
+int landed_first(emp_job **jobs, int n) {
+    uint64_t rest = 0, sum = 0;
+    for (int i = 0; i < n; ++i) rest += jobs[i]->F;
+    if (rest <= kMapGroupLeast) return n;
+    int last = n - 1;  // one copy stream: the last copy is the last to land
+    while (last > 0 && !jobs[last]->feed_pending) --last;
+    if (!jobs[last]->feed_pending || cudaEventQuery(jobs[last]->feed_ev[1]) == cudaSuccess) return n;
+    cudaGetLastError();
+    int k = 0;
+    while (k < n && sum < rest / 2) sum += jobs[k++]->F;
+    return k;
+}
+
+emp_status map_batch(emp_job **jobs, int n, std::vector<emp_status> &rc, cudaStream_t s) try {
+    std::vector<emp_status> part;
+    for (int i = 0, k; i < n; i += k) {
+        k = landed_first(jobs + i, n - i);
+        part.assign((size_t)k, EMP_OK);
+        EMP_TRY(map_group(jobs + i, k, part, s));
+        std::copy(part.begin(), part.end(), rc.begin() + i);
+    }
+    return EMP_OK;
+} catch (const std::bad_alloc &) {
+    return EMP_E_NOMEM;
 }
 
 // Close jobs[0..n) whose work is all queued: their last events, one
