@@ -41,8 +41,8 @@
 // an SM one cycle for a load (276 G/s on the chip), 1.5 for a reduction (188),
 // 2.3 for an exchange (121), a sixth of that rate where they leave L2; a late
 // step of 1.2M x 250 reads (16M keys) runs its reductions at 160 G/s and its
-// loads at 160.  What is left around them: a chunk's entries and bases (on
-// their way a chunk ahead), the candidates' chain of an exchange and two
+// loads at 160.  What is left around them: a chunk's entries (on their way a
+// chunk ahead; its bases too gained nothing) and bases, the candidates' chain of an exchange and two
 // stores, warps that end early (they draw their segments), and for a few
 // thousand entries the latency of 8 barriers a step, 60 us.  All rounds,
 // bucket kernel -> here: 2,000 x 100 reads 1.16 -> 0.245 ms, 100k x 150 1.90
@@ -176,14 +176,6 @@ EMP_DEV uint64_t step_bases(const SweepJob &J, uint32_t val, uint32_t r, uint32_
         x = y >> (64 - 2 * R);
     }
     return s ? x ^ 0xAAAAAAAAAAAAAAAAull : x;  // the complement's codes
-}
-
-// the line of the first of them on its way
-EMP_DEV void prefetch_bases(const SweepJob &J, uint32_t val, uint32_t r, uint32_t R) {
-    const bool inc = val >> 31 == (val & 1u);
-    const uint32_t start = inc ? r : (uint32_t)J.L - r - R;
-    const uint32_t *row = J.seq2 + (uint64_t)((val & 0x7fffffffu) >> 1) * J.wpr + (start >> 4);
-    asm volatile("prefetch.global.L2 [%0];\n" ::"l"(__cvta_generic_to_global(row)));
 }
 
 // NextSfx on the two fingerprints: t = (enc * R^(len - 1)) mod P of both
@@ -417,8 +409,6 @@ EMP_DEV void sweep_segment(SweepJob &J, const SweepLoc &l, SweepCtr &c, uint32_t
                     else flush_suffixes(J, c, w, l, tg + 1);
                 }
             }
-            if (kPass != 2 && q0 == 0 && x + 32 < cnt && t_round(nold, tg) == kNever)
-                prefetch_bases(J, nval | (half ? 0x80000000u : 0u), l.r, l.R);
         }
         if (kPass != 0 && live) kadv[en] = ((uint64_t)f1 << 32) | f2;
     }
