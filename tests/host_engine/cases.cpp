@@ -7,32 +7,46 @@
 #include <thread>
 
 namespace fake {
-constexpr uint64_t kReads = 100, kLen = 50, kUnique = 150;
+// a set has so many reads per parse tile of its FASTQ, three read-ends in four unique
+constexpr uint64_t kReads = 100, kLen = 50;
+uint64_t reads(uint64_t F) { return kReads * emp::parse_tiles(F); }
 std::function<void(uint32_t *err)> on_init_list;
 std::function<void(emp::SweepJob &)> on_sweep;
+std::function<cudaError_t()> on_bucket;
 int graph_builds = 0;
 bool sort_buffers = false;
 }  // namespace fake
 
 namespace emp {
 void launch_nl_count(const uint8_t *, uint64_t, uint32_t *, uint64_t *, cudaStream_t) {}
-void launch_scan_u32_u64(const uint32_t *, uint64_t *, uint64_t, uint64_t *, uint32_t *, uint64_t *total, uint32_t *,
+void launch_scan_u32_u64(const uint32_t *, uint64_t *, uint64_t n, uint64_t *, uint32_t *, uint64_t *total, uint32_t *,
                          cudaStream_t) {
-    *total = 4 * fake::kReads;
+    *total = 4 * fake::kReads * n;
 }
 void launch_scan_u32_u32(const uint32_t *, uint32_t *, uint64_t, uint64_t *, uint32_t *, uint64_t *, uint32_t *,
                          cudaStream_t) {}
 void launch_nl_count_many(const NlArgs *, ManyBlocks, cudaStream_t) {}
-void launch_scan_many(const ScanArgs *, ManyBlocks, cudaStream_t) {}
-void launch_read_pass_many(const ReadArgs *, ManyBlocks, cudaStream_t) {}
+void launch_scan_many(const ScanArgs *a, ManyBlocks b, cudaStream_t) {
+    for (uint32_t i = 0; i < b.n; ++i) *a[b.blk[i].x].total = 4 * fake::kReads * a[b.blk[i].x].n;
+}
+void launch_read_pass_many(const ReadArgs *a, ManyBlocks b, cudaStream_t) {
+    for (uint32_t i = 0; i < b.n; ++i) {
+        const ReadArgs &x = a[b.blk[i].x];
+        *x.n_kept = fake::reads(x.F);
+        x.len_minmax[0] = ~(uint32_t)fake::kLen;
+        x.len_minmax[1] = fake::kLen;
+    }
+}
 uint32_t read_pass_grid() { return 148; }
 void launch_dedup_many(const DedupArgs *, uint32_t, uint32_t, ManyBlocks, ManyBlocks, ManyBlocks, cudaStream_t) {}
 void launch_init_list_many(const InitArgs *, ManyBlocks, cudaStream_t) {}
 void launch_upload(const void *host, void *dev, size_t bytes, cudaStream_t) { std::memcpy(dev, host, bytes); }
-void launch_gather_words(const uint64_t *const *, uint32_t, uint64_t *, cudaStream_t) {}
-void launch_read_pass(const uint8_t *, uint64_t, const uint64_t *, const HashTables *, const ChunkWeights *, uint64_t *,
+void launch_gather_words(const uint64_t *const *src, uint32_t jobs, uint64_t *out, cudaStream_t) {
+    for (uint32_t k = 0; k < jobs; ++k) std::memcpy(out + 16 * k, src[k], 128);
+}
+void launch_read_pass(const uint8_t *, uint64_t F, const uint64_t *, const HashTables *, const ChunkWeights *, uint64_t *,
                       uint32_t *, int, uint32_t *, uint64_t *n_kept, uint32_t *len_minmax, uint32_t *, cudaStream_t) {
-    *n_kept = fake::kReads;
+    *n_kept = fake::reads(F);
     len_minmax[0] = ~(uint32_t)fake::kLen;
     len_minmax[1] = fake::kLen;
 }
@@ -45,9 +59,9 @@ bool dedup_args(DedupArgs *, const uint64_t *, uint64_t, uint32_t, void *, uint6
 bool launch_dedup_hash(const uint64_t *, uint64_t, uint32_t, void *, uint64_t *, uint32_t *, uint8_t *, uint32_t *,
                        cudaStream_t) { return true; }
 void launch_dedup_mark(const uint64_t *, const uint32_t *, uint64_t, uint8_t *, cudaStream_t) {}
-void launch_init_list(const uint64_t *, const uint8_t *, uint64_t, uint64_t *, uint32_t *, uint64_t *, uint32_t *,
+void launch_init_list(const uint64_t *, const uint8_t *, uint64_t n, uint64_t *, uint32_t *, uint64_t *, uint32_t *,
                       uint64_t *count, uint32_t *err, cudaStream_t) {
-    *count = fake::kUnique;
+    *count = 2 * n * 3 / 4;
     if (fake::on_init_list) fake::on_init_list(err);
 }
 void launch_dup_prefix_half(uint64_t *, uint32_t *, uint64_t, cudaStream_t) {}
@@ -87,7 +101,13 @@ void sort_top_digit(const uint64_t *, const uint32_t *, uint64_t *, uint32_t *, 
 
 int bucket_grid_size() { return 148; }
 size_t bkt_scratch_bytes(uint64_t) { return 4096; }
-cudaError_t launch_bucket_rounds(BktJob *, CoopCtl *, uint32_t *, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_bucket_rounds(BktJob *jobs, CoopCtl *ctl, uint32_t *, cudaStream_t) {
+    for (uint32_t k = 0; k < ctl->njobs; ++k) {
+        jobs[k].done = 1;
+        jobs[k].round = (uint32_t)jobs[k].r0;
+    }
+    return fake::on_bucket ? fake::on_bucket() : cudaSuccess;
+}
 cudaError_t launch_bucket_list(BktJob *, uint64_t *, uint32_t *, cudaStream_t) { return cudaSuccess; }
 bool bucket_prologue_apart(const BktJob &) { return false; }
 cudaError_t launch_bucket_prologue(BktJob *, cudaStream_t) { return cudaSuccess; }
@@ -137,11 +157,11 @@ emp_ctx *make_ctx(uint64_t budget = 0) {
     if (emp_ctx_create(0, budget, &c) != EMP_OK) std::abort();
     return c;
 }
-emp_job *fed_job(emp_ctx *c) {
+emp_job *fed_job(emp_ctx *c, uint64_t bytes = 10000) {
     emp_params p;
     emp_params_default(&p);
     emp_job *j = nullptr;
-    const std::string fq(10000, 'A');
+    const std::string fq(bytes, 'A');
     if (emp_job_create(c, &p, &j) != EMP_OK || emp_job_feed_fastq(j, fq.data(), fq.size(), 1) != EMP_OK) std::abort();
     return j;
 }
@@ -333,6 +353,41 @@ int sort_room_refused() {
     return 0;
 }
 
+// A server step that ends early, at its second launch: the jobs of its first
+// launch and those just admitted come back with the status, the long job that
+// was to share its rounds stays, and the next step goes on.
+int step_ends_early() {
+    emp_ctx *c = make_ctx();
+    emp_server_params p;
+    emp_server_params_default(&p);
+    p.share_min_entries = 500;
+    emp_server *srv = nullptr;
+    if (emp_server_create(c, &p, &srv) != EMP_OK) return 1;
+    emp_job *small = fed_job(c), *large = fed_job(c, 40000), *late[2] = {fed_job(c), fed_job(c)};
+    emp_job *back[8];
+    int n = 0, queued, flying, done;
+    emp_server_submit(srv, small);
+    emp_server_submit(srv, large);
+    if (emp_server_step(srv, back, 8, &n) != EMP_OK || n) return 2;
+    for (emp_job *j : late) emp_server_submit(srv, j);
+    fake::on_bucket = []() { return cudaErrorUnknown; };
+    if (emp_server_step(srv, back, 8, &n) != EMP_E_CUDA || n != 3) return 3;
+    fake::on_bucket = nullptr;
+    for (int k = 0; k < n; ++k)
+        if (back[k] == large || emp_job_status(back[k]) != EMP_E_CUDA) return 4;
+    emp_server_counts(srv, &queued, &flying, &done);
+    if (queued || flying != 1 || done) return 5;
+    if (emp_server_step(srv, back, 8, &n) != EMP_OK || n != 1 || back[0] != large) return 6;
+    if (emp_job_status(large) != EMP_OK) return 7;
+    emp_job_reset(small);  // and are free for the next set
+    if (emp_job_feed_fastq(small, "A", 1, 1) != EMP_OK || emp_job_run(small, nullptr) != EMP_OK) return 8;
+    for (emp_job *j : {small, large, late[0], late[1]})
+        if (emp_job_destroy(j) != EMP_OK) return 9;
+    emp_server_destroy(srv);
+    emp_ctx_destroy(c);
+    return fake::pool_bytes ? 10 : 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -343,5 +398,6 @@ int main(int argc, char **argv) {
     if (name == "graphs_from_threads") return graphs_from_threads();
     if (name == "graphs_make_room") return graphs_make_room();
     if (name == "sort_room_refused") return sort_room_refused();
+    if (name == "step_ends_early") return step_ends_early();
     return 99;
 }

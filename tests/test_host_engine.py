@@ -26,7 +26,8 @@ def program(tmp_path_factory):
 
 
 @pytest.mark.parametrize("case", ["rebuilt_list_times_out", "graph_input_copy_fails", "thread_allocation_fails",
-                                  "graphs_make_room", "sort_room_refused"])
+                                  "graphs_make_room", "sort_room_refused",
+                                  "step_ends_early"])
 def test_a_failing_call_is_a_status(program, case):
     p = subprocess.run([program, case], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0, (p.returncode, p.stderr)
