@@ -431,11 +431,11 @@ emp_status sync_and_check(emp_job *j, cudaStream_t s) {
 // fold the per-pass event times of the last sort into the stats (after a sync)
 void account_sort(emp_job *j) {
     if (!j->sort_timed) return;
-    for (int p = 0; p < kSortPasses; ++p) {
+    for (int p = 0; p < kSortPasses; ++p)
         j->st.ms_sort_passes += ms_between(j->sort_ev[2 * p], j->sort_ev[2 * p + 1]);
-        j->st.sort_passes += 1;
-        j->st.sort_pass_elems += j->sort_n;
-    }
+    const uint64_t moves = (uint64_t)sort_moves(j->sort_n);
+    j->st.sort_passes += moves;
+    j->st.sort_pass_elems += moves * j->sort_n;
     j->sort_timed = false;
 }
 

@@ -70,6 +70,10 @@ size_t sort_scratch_bytes(uint64_t n) {
     // group bounds: at most n / (kGroupMean / 2) groups
     return sizeof(SortScratch) + lookback_bytes(n) + (size_t)(n / (kGroupMean / 2) + 4) * sizeof(uint64_t);
 }
+int sort_moves(uint64_t n) {
+    const int bits = group_bits(n);
+    return bits == 0 ? 1 : bits <= kSortBits ? 2 : bits <= kMaxGroupBits ? 3 : kSortPasses;
+}
 uint32_t *sort_flags(void *scratch) { return &reinterpret_cast<SortScratch *>(scratch)->radix; }
 
 namespace {

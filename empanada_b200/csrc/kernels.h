@@ -211,6 +211,9 @@ void sort_groups(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_
 void sort_radix(uint64_t *k0, uint32_t *v0, uint64_t *k1, uint32_t *v1, uint64_t n, void *scratch, uint32_t *err,
                 cudaStream_t s, cudaEvent_t *events = nullptr);
 uint32_t *sort_flags(void *scratch);
+// How often a sort of n pairs moves each of them: digit passes and groups (the
+// full radix sort where there are too many pairs for groups).
+int sort_moves(uint64_t n);
 // Stable sort by the key's top digit alone (its bits kTopDigitShift ..), into
 // (k1, v1); the other bits of the sort key are zero above it.
 constexpr int kTopDigitShift = 53;

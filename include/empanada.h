@@ -74,9 +74,10 @@ typedef struct emp_stats {
     double ms_dedup;       /* fingerprint sort + duplicate removal (device time) */
     double ms_rounds;      /* overlap rounds (device time, incl. edge copies) */
     double ms_total;       /* whole run (device time) */
-    double ms_sort_passes; /* device time of all radix-sort digit passes (CUDA events per launch) */
-    uint64_t sort_passes;  /* digit-pass launches */
-    uint64_t sort_pass_elems; /* sum over those launches of the pairs each one moved */
+    double ms_sort_passes; /* device time of the run's full sorts (CUDA events) */
+    uint64_t sort_passes;  /* passes over the pairs of a sort: digit passes and the groups (a sort of
+                              uneven keys, which goes on as a radix sort, counts as the others) */
+    uint64_t sort_pass_elems; /* sum over those passes of the pairs each one moved */
     double ms_update;      /* device time of the per-round table update kernel (CUDA events per launch) */
     uint64_t update_launches; /* its launches that processed entries */
     uint64_t update_bytes;    /* their algorithmic bytes (13 B read + 1/4 B of bases per entry in, 12 B per entry out) */

@@ -95,6 +95,7 @@ void sort_groups(uint64_t *, uint32_t *, uint64_t *k1, uint32_t *v1, uint64_t, v
 }
 void sort_radix(uint64_t *, uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *, cudaStream_t,
                 cudaEvent_t *) {}
+int sort_moves(uint64_t) { return 1; }
 uint32_t *sort_flags(void *p) { return static_cast<uint32_t *>(p); }
 void sort_top_digit(const uint64_t *, const uint32_t *, uint64_t *, uint32_t *, uint64_t, void *, uint32_t *,
                     cudaStream_t) {}
