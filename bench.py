@@ -336,7 +336,7 @@ def batched_bench(args):
     outs = [j.output() for j in jobs]
     jst = [j.stats() for j in jobs]
     launches = jst[0]["gpu_launches"]  # the first job's counter spans the whole batch
-    # the batched bucket-kernel launch of the last step (every job in the batch carries its time)
+    # the batched sweep launch of the last step (every job in the batch carries its time)
     batch_kernel_ms = float(np.median([x["ms_round_kernel"] for x in jst]))
     plain_steps = max(1, min(args.steps, 3))
 
@@ -578,7 +578,7 @@ def main():
     ap.add_argument("--serve-min-jobs", type=int, default=20)
     ap.add_argument("--serve-max-jobs", type=int, default=400)
     ap.add_argument("--serve-pool", type=int, default=48)
-    ap.add_argument("--serve-rounds", type=int, default=16, help="bucket-kernel rounds per launch")
+    ap.add_argument("--serve-rounds", type=int, default=16, help="rounds per bucket launch of the long jobs")
     ap.add_argument("--serve-rounds-idle", type=int, default=64,
                     help="served: rounds per launch while no job waits to join")
     ap.add_argument("--serve-share-min", type=int, default=8_000_000,
@@ -710,8 +710,8 @@ def main():
         graph = {"ms_build": gst["ms_build"], "edges": gst["edges"], "unitigs": gst["unitigs"],
                  "long_unitigs": gst["long_unitigs"], "cycles": gst["cycles"],
                  "what": "unitigs (maximal paths of edges u->v with out-degree(u) = in-degree(v) = 1) of the "
-                         "job's output.bin on the device: edge scatter, degrees, one walk per unitig head, cycles "
-                         "cut at their smallest read-end, placement"}
+                         "job's output.bin on the device: links by compare-and-swap, heads and distances by pointer "
+                         "jumping, cycles cut at their smallest read-end, placement"}
         if rank == 0 and world == 1:
             from oracle import bind
 
@@ -783,14 +783,12 @@ def main():
     if rk_ms >= max(sort_ms, upd_ms):  # the all-rounds cooperative kernel dominates
         per_launch = rk_bytes / args.steps
         ms, nl = rk_ms, args.steps
-        if os.environ.get("EMP_NO_BUCKET"):
-            kname = "coop_rounds_kernel"
-            what = ("all rounds, Bloom-filter driver: per round 13 B + 1/4 B per entry in, 24 B per kept entry, "
-                    "72 B per candidate, 8 B per edge")
-        elif 2 * st["n_unique"] <= 9 << 20:  # lists that start in the sweep kernel whatever their density
+        if tune.starts_in_sweep(st["n_unique"], st["n_reads"]):
             kname = "sweep_kernel"
-            what = ("all rounds in one launch, many per step; counted as one pass per round over the live entries: "
-                    "16 B per entry, 16 B per entry kept for the next round, 8 B per edge")
+            what = ("all rounds in one launch, many per step; counted as one pass per round over the live entries "
+                    "(16 B per entry, 16 B per entry kept for the next round, 8 B per edge), which compares it with "
+                    "kernels that make those passes: this one reads its list once a step, its own work is random "
+                    "line accesses (see l2)")
         else:
             kname = "bucket_rounds_kernel"
             what = ("all rounds in one launch (with the prologue launch of a directly binned job and the sweep launch that "

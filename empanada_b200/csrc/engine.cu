@@ -12,8 +12,9 @@
 //                             (k_round.cu, k_sort.cu, k_chunked.cu)
 // All tables stay in HBM; the host traffic is the FASTQ in and output.bin
 // out.  output.bin records (write_edges_binary, overlap.cu:148-161) are
-// written on the device by the bucket kernel, on the host for
-// host-synchronised rounds.  Files come in through ingest.cpp.
+// written on the device: by the sweep and bucket kernels, and by
+// write_records (k_round.cu) for host-synchronised rounds (on the host where
+// the device has no room for them).  Files come in through ingest.cpp.
 #include <algorithm>
 #include <atomic>
 #include <cerrno>
@@ -1964,11 +1965,12 @@ bool shares(const emp_server *srv, const emp_job *j) {
     return !srv->p.share_min_entries || 2 * j->prep.U >= srv->p.share_min_entries;
 }
 
-// One step: the launch of at most rounds_per_launch rounds of every job in
-// the batch goes first, so that the FASTQ copies of newly admitted jobs run
-// beside it; then the admitted jobs' map phase (queued behind the launch),
-// the eligible ones joining the batch for the next step and the others run
-// alone; then the launch's results: jobs with no round left complete.
+// One step: the launches go first, so that the FASTQ copies of newly admitted
+// jobs run beside them: all rounds of the short jobs in one sweep launch, then
+// at most rounds_per_launch rounds of every long one in a bucket launch.  Then
+// the admitted jobs' map phase (queued behind the launches, as their FASTQ
+// lands), the eligible ones joining for the next step and the others run
+// alone; then the launches' results: jobs with no round left complete.
 emp_status server_step(emp_server *srv, cudaStream_t s) {
     emp_ctx *ctx = srv->ctx;
     emp_server_stats &ss = srv->st;

@@ -29,8 +29,8 @@
 // walk its whole path (thousands of reads between repeats, a memory latency
 // each).  Nothing of the node arrays crosses to the host but the result, and
 // that only when it is asked for.  Build and unitigs of 3.3M reads' overlaps
-// (6.7M read-ends, 5.6M edges, 45 MB in, 35 MB out): 48.2 -> 10.4 ms, of which
-// all but 1 ms are host copies.
+// (6.7M read-ends, 5.6M edges, 45 MB in, 35 MB out): 48.2 -> 6.9 ms (10.4
+// before the copies went through several threads), all but 1 ms host copies.
 #include "kernels.h"
 
 namespace emp {

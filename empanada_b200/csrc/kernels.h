@@ -105,7 +105,7 @@ void launch_init_list_many(const InitArgs *a, ManyBlocks b, cudaStream_t s);
 // copy of more than 1 KB that has work before it in its stream goes through the
 // copy engine, behind every FASTQ copy in flight, and all that follows it in
 // the stream with it: beside a copy of 36 ms the step of a server with 12 jobs
-// took 44.4 ms with such a copy of its 5 KB of descriptors, 9 to 13 so.
+// took 44.4 ms with such a copy of its 5 KB of descriptors, 8.5 to 13 so.
 void launch_upload(const void *host, void *dev, size_t bytes, cudaStream_t s);
 // out[16 j ..] = the 16 words at src[j]
 void launch_gather_words(const uint64_t *const *src, uint32_t jobs, uint64_t *out, cudaStream_t s);

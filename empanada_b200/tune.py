@@ -40,9 +40,21 @@ JOB_CANDIDATES = {"dedup_driver": [0, 1]}
 BATCH_CANDIDATES: dict = {}
 BUCKET_CANDIDATES = {"bucket_mean": [2900, 2175, 1450]}
 
-# Lists of up to so many entries start in the sweep kernel, whatever their
-# density (kSweepMaxEntries of the engine).
+# Lists of up to so many entries start in the sweep kernel whatever their
+# density, and sparse ones of up to so many (kSweepMaxEntries, kSweepMaxSparse
+# and kSweepSparseR of the engine).
 SWEEP_MAX_ENTRIES = 9 << 20
+SWEEP_MAX_SPARSE = 24 << 20
+SWEEP_SPARSE_R = 4
+
+
+def starts_in_sweep(unique: int, reads: int) -> bool:
+    """Whether the first round of a job of `reads` kept reads, `unique` of
+    their ends distinct, runs in the sweep kernel (the engine's rule)."""
+    n, d = 2 * unique, max(0.0, 1.0 - unique / max(1, 2 * reads))
+    lam = 2.0 * d * (1.0 + d * (2.0 / 3.0))
+    sparse = lam <= 0 or 0.8 / lam >= SWEEP_SPARSE_R
+    return n <= SWEEP_MAX_ENTRIES or (n <= SWEEP_MAX_SPARSE and sparse)
 
 
 def space_for(base: dict, reads: float) -> dict:

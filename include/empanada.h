@@ -122,8 +122,9 @@ typedef struct emp_tuning {
                                  1: always by sorting all fingerprints */
     uint64_t edge_cap;        /* first edge-buffer size in edges (default: 4 per read-end, at least 2^20);
                                  a run that needs more reruns its rounds with a larger one */
-    uint64_t wait_limit_ns;   /* time limit of every grid-barrier wait of the bucket kernel (default 20 s) */
-    int32_t block_next_wait;  /* testing: the context's next bucket-kernel launch meets a grid barrier
+    uint64_t wait_limit_ns;   /* time limit of every grid-barrier wait of the sweep and bucket kernels
+                                 (default 20 s) */
+    int32_t block_next_wait;  /* testing: the context's next launch of either kernel meets a grid barrier
                                  that no arrival completes, so its waits run out after wait_limit_ns and
                                  the run returns EMP_E_TIMEOUT; that launch clears the flag */
     uint32_t map_streams;     /* 1..32 (default 8): kept for callers that set it; a batch's map phase is
@@ -205,11 +206,11 @@ emp_status emp_job_status(emp_job *job);
  * equals its emp_job_run output.  A job held by a server (submitted, not yet
  * handed out by a step) accepts no other call. */
 typedef struct emp_server_params {
-    int32_t rounds_per_launch; /* bucket-kernel rounds per launch (default 16) */
+    int32_t rounds_per_launch; /* rounds per bucket launch of a job that shares them (default 16) */
     int32_t max_jobs;          /* jobs in the batch at most, <= 1024 (default 256) */
     uint64_t hbm_budget_bytes; /* admission budget (0: the context's, or none) */
     int32_t rounds_per_launch_idle; /* the same while no job waits to join (default 64) */
-    uint64_t batch_max_entries; /* a job whose first round list is longer runs alone (0: the bucket kernel's 16M) */
+    uint64_t batch_max_entries; /* a job whose first round list is longer runs alone (0: the bucket kernel's limit) */
     uint64_t share_min_entries; /* a job whose first round list is at least this long runs rounds_per_launch
                                    (rounds_per_launch_idle while no job waits) rounds of a launch; a shorter
                                    one runs all its rounds in the launch it joins (default 8M; 0: every job
@@ -227,9 +228,9 @@ emp_status emp_server_counts(emp_server *srv, int *queued, int *in_flight, int *
 typedef struct emp_server_stats {
     uint64_t steps;      /* emp_server_step calls */
     uint64_t admitted;   /* jobs admitted */
-    uint64_t launches;   /* bucket-kernel launches */
-    uint64_t rounds;     /* launch iterations (each runs one round of every job in the batch) */
-    uint64_t batch_jobs; /* sum over launches of the jobs in the batch */
+    uint64_t launches;   /* sweep launches and bucket-kernel launches */
+    uint64_t rounds;     /* iterations of the bucket launches (each runs one round of every job in them) */
+    uint64_t batch_jobs; /* sum over launches of the jobs in them */
     double ms_kernel;    /* device time of those launches */
     double ms_admit;     /* host wall time of admission + map phase + jobs run alone */
     double ms_map;       /* of which the map phase */

@@ -10,6 +10,7 @@ import test_gpu_handover as handover
 import test_gpu_parity as parity
 import test_gpu_sweep as sweep
 from cases import BY_NAME
+from empanada_b200 import tune
 
 pytestmark = pytest.mark.gpu
 
@@ -70,11 +71,12 @@ def test_long_lists(traced, name, mean):
         job.feed(handover._fastq(n, n, L, genome, sub))
         with engine.tuned(bucket_mean=mean, **tuned):
             job.run()
-        got, (kernel, at) = job.output(), last()
+        got, (kernel, at), job_unique = job.output(), last(), job.stats()["n_unique"]
         with engine.tuned(round_driver=2):
             job.run()
         assert job.output() == got
         assert last() == ("bucket", 0)
+    assert tune.starts_in_sweep(job_unique, n) == (kernel == "sweep" and at[0][0] == 0)
     if name == "few_rounds":
         assert (kernel, at) == ("bucket", 0)
     else:

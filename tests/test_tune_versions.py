@@ -49,10 +49,12 @@ def test_tile_sizes_are_offered_to_long_lists(tmp_path, reads, offered):
     assert (b["source"] == "timed") == offered and (b["timings_ms"] is not None) == offered
 
 
-def test_the_limit_is_the_engines():
+def test_the_limits_are_the_engines():
     import os
     import re
 
     src = open(os.path.join(os.path.dirname(tune.__file__), "csrc", "kernels.h")).read()
-    a, b = re.search(r"kSweepMaxEntries = (\d+)ull << (\d+)", src).groups()
-    assert int(a) << int(b) == tune.SWEEP_MAX_ENTRIES
+    for name, value in (("kSweepMaxEntries", tune.SWEEP_MAX_ENTRIES), ("kSweepMaxSparse", tune.SWEEP_MAX_SPARSE)):
+        a, b = re.search(name + r" = (\d+)ull << (\d+)", src).groups()
+        assert int(a) << int(b) == value
+    assert int(re.search(r"kSweepSparseR = (\d+)", src).group(1)) == tune.SWEEP_SPARSE_R
