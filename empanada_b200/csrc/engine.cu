@@ -854,10 +854,11 @@ emp_status bucket_prepare(emp_job *j, cudaStream_t s, const RoundEnv &env, int r
     return EMP_OK;
 }
 
-// Queue the copy of the job's round records to the host.
 static_assert(sizeof(BktJob) <= 1024 && sizeof(SweepJob) + sizeof(CoopCtl) <= 1024 && sizeof(BktJob) % 8 == 0 &&
                   sizeof(SweepJob) % 8 == 0 && sizeof(CoopCtl) % 8 == 0,
               "one job's description is a copy that waits for no other; several are whole words (launch_upload)");
+
+// Queue the copy of the job's round records to the host.
 emp_status bucket_fetch(emp_job *j, const RoundEnv &env, cudaStream_t s) {
     EMP_CUDA(cudaMemcpyAsync(j->h_records.p, j->records.p, (size_t)env.rounds * sizeof(RoundRecord),
                              cudaMemcpyDeviceToHost, s));
@@ -1649,7 +1650,7 @@ emp_status batch_rounds(emp_ctx *ctx, emp_job **jobs, const std::vector<int> &id
 // ready): queued by launch, read by collect once the stream has been waited
 // for.  A job whose buffers are refused is left out of it; where there is no
 // room for what the jobs share, the largest are, one by one.
-emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<emp_job *> &jobs, cudaStream_t s) {
+emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<emp_job *> &jobs, cudaStream_t s) try {
     const size_t nb = jobs.size();
     uint64_t side = 0, recs = 0;
     for (emp_job *j : jobs) {
@@ -1658,6 +1659,8 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     }
     sb.in.clear();
     sb.out_of_it.clear();
+    sb.in.reserve(nb);
+    sb.out_of_it.reserve(nb);
     auto leave_out = [&](size_t k) {
         free_buf(jobs[k], jobs[k]->swp);
         free_buf(jobs[k], jobs[k]->dout);
@@ -1724,6 +1727,8 @@ emp_status sweep_batch_launch(emp_ctx *ctx, SweepBatch &sb, const std::vector<em
     EMP_CUDA(cudaEventRecord(sb.ev[1], s));
     EMP_CUDA(cudaMemcpyAsync(hj, dj, total, cudaMemcpyDeviceToHost, s));
     return EMP_OK;
+} catch (const std::bad_alloc &) {  // the two lists of jobs: nothing is queued yet
+    return EMP_E_NOMEM;
 }
 
 // Per-job status of the launch in rc; a job whose edges did not fit, that is
@@ -1740,7 +1745,10 @@ emp_status sweep_batch_collect(SweepBatch &sb, const std::vector<emp_job *> &job
             emp_job *j = jobs[sb.in[k]];
             JobPrep &q = j->prep;
             j->st.ms_round_kernel += ms;  // the whole batch's launch
-            if (!j->h_records.ensure((size_t)q.rounds * sizeof(RoundRecord))) return EMP_E_NOMEM;
+            if (!j->h_records.ensure((size_t)q.rounds * sizeof(RoundRecord))) {
+                rc[sb.in[k]] = EMP_E_NOMEM;
+                continue;
+            }
             const size_t at = (size_t)(reinterpret_cast<uint8_t *>(hj[k].records) - sb.jobs.as<uint8_t>());
             std::memcpy(j->h_records.p, sb.host.as<uint8_t>() + at, (size_t)q.rounds * sizeof(RoundRecord));
             uint64_t needed = 0;
