@@ -2975,11 +2975,30 @@ struct emp_graph {
 
 namespace {
 
+// A graph may be used by a thread that works on another device: the device
+// that was current is so again at the end.
+struct DeviceHere {
+    int before = -1;
+    explicit DeviceHere(int device) {
+        if (cudaGetDevice(&before) != cudaSuccess) {
+            cudaGetLastError();
+            before = -1;
+        }
+        if (before != device) cudaSetDevice(device);
+        else before = -1;
+    }
+    ~DeviceHere() {
+        if (before >= 0) cudaSetDevice(before);
+    }
+    DeviceHere(const DeviceHere &) = delete;
+    DeviceHere &operator=(const DeviceHere &) = delete;
+};
+
 // the graph's arrays into its host vectors, which then stay as they are
 emp_status graph_to_host(emp_graph *g) {
     if (g->order.size() == g->nodes) return EMP_OK;
     if (!g->ctx) return EMP_E_NOMEM;  // the context went while there was no room for them
-    cudaSetDevice(g->ctx->device);
+    const DeviceHere here(g->ctx->device);
     try {
         g->bin.resize(g->bytes);
         g->starts.resize(g->unitigs + 1);
@@ -3007,7 +3026,7 @@ void graph_detach(emp_graph *g) {
     auto &v = g->list->graphs;
     v.erase(std::remove(v.begin(), v.end(), g), v.end());
     if (g->dev) {
-        cudaSetDevice(c->device);
+        const DeviceHere here(c->device);
         cudaFreeAsync(g->dev, c->stream);
         c->in_use -= g->dev_bytes;
     }
@@ -3191,7 +3210,7 @@ emp_status emp_graph_unitigs(emp_graph *g, uint32_t *order, uint64_t order_cap, 
         if (starts) std::memcpy(starts, g->starts.data(), (g->unitigs + 1) * 8);
         return EMP_OK;
     }
-    cudaSetDevice(g->ctx->device);
+    const DeviceHere here(g->ctx->device);
     emp_ctx *c = g->ctx;
     if ((order && c->stage.to_host(c->device, order, g->d_order, g->nodes * 4) != cudaSuccess) ||
         (starts && c->stage.to_host(c->device, starts, g->d_starts, (g->unitigs + 1) * 8) != cudaSuccess)) {

@@ -389,6 +389,24 @@ int step_ends_early() {
     return fake::pool_bytes ? 10 : 0;
 }
 
+// Calls on a graph leave the calling thread's device as it is.
+int graph_keeps_the_device() {
+    emp_ctx *c = make_ctx();
+    const std::vector<uint8_t> bin = one_record(3);
+    emp_graph *g[3] = {};
+    for (emp_graph *&x : g)
+        if (emp_graph_build(c, bin.data(), bin.size(), 10, &x) != EMP_OK) return 1;
+    std::vector<uint32_t> order(20);
+    std::vector<uint64_t> starts(21);
+    cudaSetDevice(1);
+    if (emp_graph_unitigs(g[0], order.data(), 20, starts.data(), 21) != EMP_OK || fake::device != 1) return 2;
+    if (emp_graph_write_gfa(g[1], "/dev/null", 50) != EMP_OK || fake::device != 1) return 3;
+    for (emp_graph *x : g)
+        if (emp_graph_destroy(x) != EMP_OK || fake::device != 1) return 4;
+    emp_ctx_destroy(c);
+    return 0;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -400,5 +418,6 @@ int main(int argc, char **argv) {
     if (name == "graphs_make_room") return graphs_make_room();
     if (name == "sort_room_refused") return sort_room_refused();
     if (name == "step_ends_early") return step_ends_early();
+    if (name == "graph_keeps_the_device") return graph_keeps_the_device();
     return 99;
 }

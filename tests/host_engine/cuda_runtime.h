@@ -51,9 +51,12 @@ inline cudaError_t cudaGetLastError() {
     fake::last = cudaSuccess;
     return e;
 }
-inline cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
-inline cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+namespace fake {
+inline thread_local int device = 0;
+}
+inline cudaError_t cudaGetDeviceCount(int *n) { *n = 2; return cudaSuccess; }
+inline cudaError_t cudaGetDevice(int *d) { *d = fake::device; return cudaSuccess; }
+inline cudaError_t cudaSetDevice(int d) { fake::device = d; return cudaSuccess; }
 
 template <class T>
 cudaError_t cudaMalloc(T **p, size_t n) {

@@ -27,7 +27,7 @@ def program(tmp_path_factory):
 
 @pytest.mark.parametrize("case", ["rebuilt_list_times_out", "graph_input_copy_fails", "thread_allocation_fails",
                                   "graphs_make_room", "sort_room_refused",
-                                  "step_ends_early"])
+                                  "step_ends_early", "graph_keeps_the_device"])
 def test_a_failing_call_is_a_status(program, case):
     p = subprocess.run([program, case], capture_output=True, text=True, timeout=120)
     assert p.returncode == 0, (p.returncode, p.stderr)
