@@ -70,7 +70,8 @@ typedef struct emp_stats {
     uint64_t output_bytes; /* output.bin size */
     uint64_t gpu_launches; /* engine kernels launched by the last run */
     double ms_h2d;         /* FASTQ host->device copy (0 for device input) */
-    double ms_map;         /* parse + fingerprint + column store (device time) */
+    double ms_map;         /* parse + fingerprint + column store (device time; in a batch or a server
+                              step that of the launches shared with other jobs, as is ms_dedup) */
     double ms_dedup;       /* fingerprint sort + duplicate removal (device time) */
     double ms_rounds;      /* overlap rounds (device time, incl. edge copies) */
     double ms_total;       /* whole run (device time) */
